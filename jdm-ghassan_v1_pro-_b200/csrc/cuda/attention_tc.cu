@@ -124,52 +124,52 @@ __global__ void __launch_bounds__(AT_THREADS) attn_tc_fwd_kernel(const __grid_co
   };
 
   if (warp == 4) {
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one();
       uint32_t kv_it = 0, q_it = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++q_it) {
+      for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++q_it) {
         int b, h, q0, k_lo, n_tiles;
         item_range(item, b, h, q0, k_lo, n_tiles);
         const int kvh = h / rep;
         const int row_base = b * p.T;
         // the tensor core has read the previous item's Q (committed after its last score tile)
-        if (!at_wait(q_empty, (q_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag)) break;
-        mbar_arrive_expect_tx(q_full, TILE);
-        load_tile<HD>(&tmQ, q_full, sQ, h * HD, row_base + q0);
+        wait_or_report(q_empty, (q_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+        mbar_arrive_expect_tx_on(on, q_full, TILE);
+        load_tile<HD>(on, &tmQ, q_full, sQ, h * HD, row_base + q0);
         for (int t = 0; t < n_tiles; ++t, ++kv_it) {
           const int s = kv_it & 1, ph = (kv_it >> 1) & 1;
-          if (!at_wait(&kv_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag)) { ok = false; break; }
-          mbar_arrive_expect_tx(&kv_full[s], 2 * TILE);
-          load_tile<HD>(&tmK, &kv_full[s], sK + s * TILE, kvh * HD, row_base + k_lo + t * AT_N);
-          load_tile<HD>(&tmV, &kv_full[s], sV + s * TILE, kvh * HD, row_base + k_lo + t * AT_N);
+          wait_or_report(&kv_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+          mbar_arrive_expect_tx_on(on, &kv_full[s], 2 * TILE);
+          load_tile<HD>(on, &tmK, &kv_full[s], sK + s * TILE, kvh * HD, row_base + k_lo + t * AT_N);
+          load_tile<HD>(on, &tmV, &kv_full[s], sV + s * TILE, kvh * HD, row_base + k_lo + t * AT_N);
         }
       }
     }
     __syncwarp();
   } else if (warp == 5) {
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one();
       constexpr int fmt = OperandFmt<T>::value;
       const uint32_t idesc_s = make_idesc_f16(fmt, 0, 0, AT_M, AT_N);
       const uint32_t idesc_o = make_idesc_f16(fmt, 0, 1, AT_M, HD);
       uint32_t kv_it = 0, q_it = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++q_it) {
+      for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++q_it) {
         int b, h, q0, k_lo, n_tiles;
         item_range(item, b, h, q0, k_lo, n_tiles);
-        if (!at_wait(q_full, q_it & 1u, p.status, ST_TIMEOUT_FULL, abort_flag)) break;
+        wait_or_report(q_full, q_it & 1u, p.status, ST_TIMEOUT_FULL, abort_flag);
         for (int t = 0; t < n_tiles; ++t, ++kv_it) {
           const int s = kv_it & 1, ph = (kv_it >> 1) & 1;
-          if (!at_wait(&kv_full[s], ph, p.status, ST_TIMEOUT_FULL, abort_flag)) { ok = false; break; }
+          wait_or_report(&kv_full[s], ph, p.status, ST_TIMEOUT_FULL, abort_flag);
           tc_fence_after();
           // S(t) may overwrite S(t-1) only after the softmax threads have read it: p_ready(t-1) was waited below
-          mma_kmajor_kmajor<HD>(tmem_S, smem_u32(sQ), smem_u32(sK + s * TILE), idesc_s, false);
-          umma_commit(s_full);
-          if (t == n_tiles - 1) umma_commit(q_empty);
-          if (!at_wait(p_ready, kv_it & 1u, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag)) { ok = false; break; }
+          mma_kmajor_kmajor<HD>(on, tmem_S, smem_u32(sQ), smem_u32(sK + s * TILE), idesc_s, false);
+          umma_commit_on(on, s_full);
+          if (t == n_tiles - 1) umma_commit_on(on, q_empty);
+          wait_or_report(p_ready, kv_it & 1u, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag);
           tc_fence_after();
-          mma_kmajor_mnmajor<AT_N>(tmem_O, smem_u32(sP), smem_u32(sV + s * TILE), idesc_o, t > 0);
-          umma_commit(o_full);
-          umma_commit(&kv_empty[s]);
+          mma_kmajor_mnmajor<AT_N>(on, tmem_O, smem_u32(sP), smem_u32(sV + s * TILE), idesc_o, t > 0);
+          umma_commit_on(on, o_full);
+          umma_commit_on(on, &kv_empty[s]);
         }
       }
     }
@@ -383,56 +383,56 @@ __global__ void __launch_bounds__(AT_BWD_THREADS) attn_tc_bwd_dq_kernel(const __
   };
 
   if (warp == AT_BWD_W_TMA) {
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one();
       uint32_t kv_it = 0, q_it = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++q_it) {
+      for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++q_it) {
         int b, h, q0, k_lo, n_tiles;
         item_range(item, b, h, q0, k_lo, n_tiles);
         const int kvh = h / rep;
         const int row_base = b * p.T;
         // Q and dO of the previous item have been read (committed after its last S / dP)
-        if (!at_wait(q_empty, (q_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag)) break;
-        mbar_arrive_expect_tx(q_full, 2 * TILE);
-        load_tile<HD>(&tmQ, q_full, sQ, h * HD, row_base + q0);
-        load_tile<HD>(&tmDO, q_full, sDO, h * HD, row_base + q0);
+        wait_or_report(q_empty, (q_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+        mbar_arrive_expect_tx_on(on, q_full, 2 * TILE);
+        load_tile<HD>(on, &tmQ, q_full, sQ, h * HD, row_base + q0);
+        load_tile<HD>(on, &tmDO, q_full, sDO, h * HD, row_base + q0);
         for (int t = 0; t < n_tiles; ++t, ++kv_it) {
           const int s = kv_it % STAGES, ph = (kv_it / STAGES) & 1;
-          if (!at_wait(&kv_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag)) { ok = false; break; }
-          mbar_arrive_expect_tx(&kv_full[s], 2 * TILE);
-          load_tile<HD>(&tmK, &kv_full[s], sK + s * TILE, kvh * HD, row_base + k_lo + t * AT_N);
-          load_tile<HD>(&tmV, &kv_full[s], sV + s * TILE, kvh * HD, row_base + k_lo + t * AT_N);
+          wait_or_report(&kv_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+          mbar_arrive_expect_tx_on(on, &kv_full[s], 2 * TILE);
+          load_tile<HD>(on, &tmK, &kv_full[s], sK + s * TILE, kvh * HD, row_base + k_lo + t * AT_N);
+          load_tile<HD>(on, &tmV, &kv_full[s], sV + s * TILE, kvh * HD, row_base + k_lo + t * AT_N);
         }
       }
     }
     __syncwarp();
   } else if (warp == AT_BWD_W_MMA) {
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one();
       constexpr int fmt = OperandFmt<T>::value;
       const uint32_t idesc_s = make_idesc_f16(fmt, 0, 0, AT_M, AT_N);
       const uint32_t idesc_dq = make_idesc_f16(fmt, 0, 1, AT_M, HD);
       uint32_t kv_it = 0, q_it = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++q_it) {
+      for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++q_it) {
         int b, h, q0, k_lo, n_tiles;
         item_range(item, b, h, q0, k_lo, n_tiles);
-        if (!at_wait(q_full, q_it & 1u, p.status, ST_TIMEOUT_FULL, abort_flag)) break;
+        wait_or_report(q_full, q_it & 1u, p.status, ST_TIMEOUT_FULL, abort_flag);
         for (int t = 0; t < n_tiles; ++t, ++kv_it) {
           const int s = kv_it % STAGES, ph = (kv_it / STAGES) & 1;
-          if (!at_wait(&kv_full[s], ph, p.status, ST_TIMEOUT_FULL, abort_flag)) { ok = false; break; }
+          wait_or_report(&kv_full[s], ph, p.status, ST_TIMEOUT_FULL, abort_flag);
           tc_fence_after();
-          mma_kmajor_kmajor<HD>(tmem_S, smem_u32(sQ), smem_u32(sK + s * TILE), idesc_s, false);
-          mma_kmajor_kmajor<HD>(tmem_dP, smem_u32(sDO), smem_u32(sV + s * TILE), idesc_s, false);
-          umma_commit(sdp_full);
-          if (t == n_tiles - 1) umma_commit(q_empty);
-          if (!at_wait(ds_ready, kv_it & 1u, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag)) { ok = false; break; }
+          mma_kmajor_kmajor<HD>(on, tmem_S, smem_u32(sQ), smem_u32(sK + s * TILE), idesc_s, false);
+          mma_kmajor_kmajor<HD>(on, tmem_dP, smem_u32(sDO), smem_u32(sV + s * TILE), idesc_s, false);
+          umma_commit_on(on, sdp_full);
+          if (t == n_tiles - 1) umma_commit_on(on, q_empty);
+          wait_or_report(ds_ready, kv_it & 1u, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag);
           tc_fence_after();
           // the first dQ of an item overwrites the accumulator: the compute warps have read the previous item's dQ
           // before they arrived on ds_ready for this tile
-          mma_kmajor_mnmajor<AT_N>(tmem_dQ, smem_u32(sDS), smem_u32(sK + s * TILE), idesc_dq, t > 0);
-          umma_commit(&kv_empty[s]);
+          mma_kmajor_mnmajor<AT_N>(on, tmem_dQ, smem_u32(sDS), smem_u32(sK + s * TILE), idesc_dq, t > 0);
+          umma_commit_on(on, &kv_empty[s]);
         }
-        if (ok) umma_commit(dq_full);
+        umma_commit_on(on, dq_full);
       }
     }
     __syncwarp();
@@ -599,53 +599,53 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dq64_kernel(co
   };
 
   if (warp == W_TMA) {
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one();
       uint32_t kv_it = 0, q_it = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++q_it) {
+      for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++q_it) {
         int b, h, q0, k_lo, n_steps;
         item_range(item, b, h, q0, k_lo, n_steps);
         const int kvh = h / rep;
         const int row_base = b * p.T;
-        if (!at_wait(q_empty, (q_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag)) break;
-        mbar_arrive_expect_tx(q_full, 2 * TILE);
-        load_tile<HD>(&tmQ, q_full, sQ, h * HD, row_base + q0);
-        load_tile<HD>(&tmDO, q_full, sDO, h * HD, row_base + q0);
+        wait_or_report(q_empty, (q_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+        mbar_arrive_expect_tx_on(on, q_full, 2 * TILE);
+        load_tile<HD>(on, &tmQ, q_full, sQ, h * HD, row_base + q0);
+        load_tile<HD>(on, &tmDO, q_full, sDO, h * HD, row_base + q0);
         for (int t = 0; t < n_steps; ++t, ++kv_it) {
           const int s = kv_it % ST, ph = (kv_it / ST) & 1;
-          if (!at_wait(&kv_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag)) { ok = false; break; }
-          mbar_arrive_expect_tx(&kv_full[s], 2 * KTILE);
-          tma_load_2d(&tmK, &kv_full[s], sK + s * KTILE, kvh * HD, row_base + k_lo + t * KN);
-          tma_load_2d(&tmV, &kv_full[s], sV + s * KTILE, kvh * HD, row_base + k_lo + t * KN);
+          wait_or_report(&kv_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+          mbar_arrive_expect_tx_on(on, &kv_full[s], 2 * KTILE);
+          tma_load_2d_on(on, &tmK, &kv_full[s], sK + s * KTILE, kvh * HD, row_base + k_lo + t * KN);
+          tma_load_2d_on(on, &tmV, &kv_full[s], sV + s * KTILE, kvh * HD, row_base + k_lo + t * KN);
         }
       }
     }
     __syncwarp();
   } else if (warp == W_MMA) {
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one();
       constexpr int fmt = OperandFmt<T>::value;
       const uint32_t idesc_s = make_idesc_f16(fmt, 0, 0, AT_M, KN);
       const uint32_t idesc_dq = make_idesc_f16(fmt, 0, 1, AT_M, HD);
       uint32_t kv_it = 0, q_it = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++q_it) {
+      for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++q_it) {
         int b, h, q0, k_lo, n_steps;
         item_range(item, b, h, q0, k_lo, n_steps);
-        if (!at_wait(q_full, q_it & 1u, p.status, ST_TIMEOUT_FULL, abort_flag)) break;
+        wait_or_report(q_full, q_it & 1u, p.status, ST_TIMEOUT_FULL, abort_flag);
         for (int t = 0; t < n_steps; ++t, ++kv_it) {
           const int s = kv_it % ST, ph = (kv_it / ST) & 1;
-          if (!at_wait(&kv_full[s], ph, p.status, ST_TIMEOUT_FULL, abort_flag)) { ok = false; break; }
+          wait_or_report(&kv_full[s], ph, p.status, ST_TIMEOUT_FULL, abort_flag);
           tc_fence_after();
-          mma_kmajor_kmajor<HD>(tmem_S, smem_u32(sQ), smem_u32(sK + s * KTILE), idesc_s, false);
-          mma_kmajor_kmajor<HD>(tmem_dP, smem_u32(sDO), smem_u32(sV + s * KTILE), idesc_s, false);
-          umma_commit(sdp_full);
-          if (t == n_steps - 1) umma_commit(q_empty);
-          if (!at_wait(ds_ready, kv_it & 1u, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag)) { ok = false; break; }
+          mma_kmajor_kmajor<HD>(on, tmem_S, smem_u32(sQ), smem_u32(sK + s * KTILE), idesc_s, false);
+          mma_kmajor_kmajor<HD>(on, tmem_dP, smem_u32(sDO), smem_u32(sV + s * KTILE), idesc_s, false);
+          umma_commit_on(on, sdp_full);
+          if (t == n_steps - 1) umma_commit_on(on, q_empty);
+          wait_or_report(ds_ready, kv_it & 1u, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag);
           tc_fence_after();
-          mma_kmajor_mnmajor<KN>(tmem_dQ, smem_u32(sDS), smem_u32(sK + s * KTILE), idesc_dq, t > 0);
-          umma_commit(&kv_empty[s]);
+          mma_kmajor_mnmajor<KN>(on, tmem_dQ, smem_u32(sDS), smem_u32(sK + s * KTILE), idesc_dq, t > 0);
+          umma_commit_on(on, &kv_empty[s]);
         }
-        if (ok) umma_commit(dq_full);
+        umma_commit_on(on, dq_full);
       }
     }
     __syncwarp();
@@ -800,60 +800,60 @@ __global__ void __launch_bounds__(AT_BWD_THREADS) attn_tc_bwd_dkv_kernel(const _
   };
 
   if (warp == AT_BWD_W_TMA) {
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one();
       uint32_t g_it = 0, item_it = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++item_it) {
+      for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++item_it) {
         int b, kvh, j0, n_qt;
         item_range(item, b, kvh, j0, n_qt);
         const int row_base = b * p.T;
         // K and V of the previous item have been read (committed after its last S^T / dP^T)
-        if (!at_wait(kv_empty, (item_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag)) break;
-        mbar_arrive_expect_tx(kv_full, 2 * TILE);
-        load_tile<HD>(&tmK, kv_full, sK, kvh * HD, row_base + j0);
-        load_tile<HD>(&tmV, kv_full, sV, kvh * HD, row_base + j0);
+        wait_or_report(kv_empty, (item_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+        mbar_arrive_expect_tx_on(on, kv_full, 2 * TILE);
+        load_tile<HD>(on, &tmK, kv_full, sK, kvh * HD, row_base + j0);
+        load_tile<HD>(on, &tmV, kv_full, sV, kvh * HD, row_base + j0);
         const int n_it = group * n_qt;
         for (int it = 0; it < n_it; ++it, ++g_it) {
           const int s = g_it % STAGES, ph = (g_it / STAGES) & 1;
           const int h = kvh * group + it / n_qt;
           const int i0 = j0 + (it % n_qt) * AT_M;
-          if (!at_wait(&q_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag)) { ok = false; break; }
-          mbar_arrive_expect_tx(&q_full[s], 2 * TILE);
-          load_tile<HD>(&tmQ, &q_full[s], sQ + s * TILE, h * HD, row_base + i0);
-          load_tile<HD>(&tmDO, &q_full[s], sDO + s * TILE, h * HD, row_base + i0);
+          wait_or_report(&q_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+          mbar_arrive_expect_tx_on(on, &q_full[s], 2 * TILE);
+          load_tile<HD>(on, &tmQ, &q_full[s], sQ + s * TILE, h * HD, row_base + i0);
+          load_tile<HD>(on, &tmDO, &q_full[s], sDO + s * TILE, h * HD, row_base + i0);
         }
       }
     }
     __syncwarp();
   } else if (warp == AT_BWD_W_MMA) {
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one();
       constexpr int fmt = OperandFmt<T>::value;
       const uint32_t idesc_s = make_idesc_f16(fmt, 0, 0, AT_M, AT_N);
       const uint32_t idesc_d = make_idesc_f16(fmt, 0, 1, AT_M, HD);
       uint32_t g_it = 0, item_it = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++item_it) {
+      for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++item_it) {
         int b, kvh, j0, n_qt;
         item_range(item, b, kvh, j0, n_qt);
-        if (!at_wait(kv_full, item_it & 1u, p.status, ST_TIMEOUT_FULL, abort_flag)) break;
+        wait_or_report(kv_full, item_it & 1u, p.status, ST_TIMEOUT_FULL, abort_flag);
         const int n_it = group * n_qt;
         for (int it = 0; it < n_it; ++it, ++g_it) {
           const int s = g_it % STAGES, ph = (g_it / STAGES) & 1;
-          if (!at_wait(&q_full[s], ph, p.status, ST_TIMEOUT_FULL, abort_flag)) { ok = false; break; }
+          wait_or_report(&q_full[s], ph, p.status, ST_TIMEOUT_FULL, abort_flag);
           tc_fence_after();
-          mma_kmajor_kmajor<HD>(tmem_ST, smem_u32(sK), smem_u32(sQ + s * TILE), idesc_s, false);
-          mma_kmajor_kmajor<HD>(tmem_dPT, smem_u32(sV), smem_u32(sDO + s * TILE), idesc_s, false);
-          umma_commit(st_full);
-          if (it == n_it - 1) umma_commit(kv_empty);
-          if (!at_wait(pt_ready, g_it & 1u, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag)) { ok = false; break; }
+          mma_kmajor_kmajor<HD>(on, tmem_ST, smem_u32(sK), smem_u32(sQ + s * TILE), idesc_s, false);
+          mma_kmajor_kmajor<HD>(on, tmem_dPT, smem_u32(sV), smem_u32(sDO + s * TILE), idesc_s, false);
+          umma_commit_on(on, st_full);
+          if (it == n_it - 1) umma_commit_on(on, kv_empty);
+          wait_or_report(pt_ready, g_it & 1u, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag);
           tc_fence_after();
           // the first dV / dK of an item overwrite the accumulators: the compute warps have read the previous item's
           // before they arrived on pt_ready for this iteration
-          mma_kmajor_mnmajor<AT_M>(tmem_dV, smem_u32(sPT), smem_u32(sDO + s * TILE), idesc_d, it > 0);
-          mma_kmajor_mnmajor<AT_M>(tmem_dK, smem_u32(sDST), smem_u32(sQ + s * TILE), idesc_d, it > 0);
-          umma_commit(&q_empty[s]);
+          mma_kmajor_mnmajor<AT_M>(on, tmem_dV, smem_u32(sPT), smem_u32(sDO + s * TILE), idesc_d, it > 0);
+          mma_kmajor_mnmajor<AT_M>(on, tmem_dK, smem_u32(sDST), smem_u32(sQ + s * TILE), idesc_d, it > 0);
+          umma_commit_on(on, &q_empty[s]);
         }
-        if (ok) umma_commit(dkv_full);
+        umma_commit_on(on, dkv_full);
       }
     }
     __syncwarp();
@@ -1065,57 +1065,57 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
   };
 
   if (warp == W_TMA) {
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one();
       uint32_t g_it = 0, item_it = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++item_it) {
+      for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++item_it) {
         int b, kvh, j0, n_qs;
         item_range(item, b, kvh, j0, n_qs);
         const int row_base = b * p.T;
-        if (!at_wait(kv_empty, (item_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag)) break;
-        mbar_arrive_expect_tx(kv_full, 2 * TILE);
-        load_tile<HD>(&tmK, kv_full, sK, kvh * HD, row_base + j0);
-        load_tile<HD>(&tmV, kv_full, sV, kvh * HD, row_base + j0);
+        wait_or_report(kv_empty, (item_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+        mbar_arrive_expect_tx_on(on, kv_full, 2 * TILE);
+        load_tile<HD>(on, &tmK, kv_full, sK, kvh * HD, row_base + j0);
+        load_tile<HD>(on, &tmV, kv_full, sV, kvh * HD, row_base + j0);
         const int n_it = group * n_qs;
         for (int it = 0; it < n_it; ++it, ++g_it) {
           const int s = g_it % ST, ph = (g_it / ST) & 1;
           const int h = kvh * group + it / n_qs;
           const int i0 = j0 + (it % n_qs) * QN;
-          if (!at_wait(&q_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag)) { ok = false; break; }
-          mbar_arrive_expect_tx(&q_full[s], 2 * QTILE);
-          tma_load_2d(&tmQ, &q_full[s], sQ + s * QTILE, h * HD, row_base + i0);
-          tma_load_2d(&tmDO, &q_full[s], sDO + s * QTILE, h * HD, row_base + i0);
+          wait_or_report(&q_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+          mbar_arrive_expect_tx_on(on, &q_full[s], 2 * QTILE);
+          tma_load_2d_on(on, &tmQ, &q_full[s], sQ + s * QTILE, h * HD, row_base + i0);
+          tma_load_2d_on(on, &tmDO, &q_full[s], sDO + s * QTILE, h * HD, row_base + i0);
         }
       }
     }
     __syncwarp();
   } else if (warp == W_MMA) {
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one();
       constexpr int fmt = OperandFmt<T>::value;
       const uint32_t idesc_s = make_idesc_f16(fmt, 0, 0, AT_N, QN);
       const uint32_t idesc_d = make_idesc_f16(fmt, 0, 1, AT_N, HD);
       uint32_t g_it = 0, item_it = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++item_it) {
+      for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++item_it) {
         int b, kvh, j0, n_qs;
         item_range(item, b, kvh, j0, n_qs);
-        if (!at_wait(kv_full, item_it & 1u, p.status, ST_TIMEOUT_FULL, abort_flag)) break;
+        wait_or_report(kv_full, item_it & 1u, p.status, ST_TIMEOUT_FULL, abort_flag);
         const int n_it = group * n_qs;
         for (int it = 0; it < n_it; ++it, ++g_it) {
           const int s = g_it % ST, ph = (g_it / ST) & 1;
-          if (!at_wait(&q_full[s], ph, p.status, ST_TIMEOUT_FULL, abort_flag)) { ok = false; break; }
+          wait_or_report(&q_full[s], ph, p.status, ST_TIMEOUT_FULL, abort_flag);
           tc_fence_after();
-          mma_kmajor_kmajor<HD>(tmem_ST, smem_u32(sK), smem_u32(sQ + s * QTILE), idesc_s, false);
-          mma_kmajor_kmajor<HD>(tmem_dPT, smem_u32(sV), smem_u32(sDO + s * QTILE), idesc_s, false);
-          umma_commit(st_full);
-          if (it == n_it - 1) umma_commit(kv_empty);
-          if (!at_wait(pt_ready, g_it & 1u, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag)) { ok = false; break; }
+          mma_kmajor_kmajor<HD>(on, tmem_ST, smem_u32(sK), smem_u32(sQ + s * QTILE), idesc_s, false);
+          mma_kmajor_kmajor<HD>(on, tmem_dPT, smem_u32(sV), smem_u32(sDO + s * QTILE), idesc_s, false);
+          umma_commit_on(on, st_full);
+          if (it == n_it - 1) umma_commit_on(on, kv_empty);
+          wait_or_report(pt_ready, g_it & 1u, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag);
           tc_fence_after();
-          mma_kmajor_mnmajor<QN>(tmem_dV, smem_u32(sPT), smem_u32(sDO + s * QTILE), idesc_d, it > 0);
-          mma_kmajor_mnmajor<QN>(tmem_dK, smem_u32(sDST), smem_u32(sQ + s * QTILE), idesc_d, it > 0);
-          umma_commit(&q_empty[s]);
+          mma_kmajor_mnmajor<QN>(on, tmem_dV, smem_u32(sPT), smem_u32(sDO + s * QTILE), idesc_d, it > 0);
+          mma_kmajor_mnmajor<QN>(on, tmem_dK, smem_u32(sDST), smem_u32(sQ + s * QTILE), idesc_d, it > 0);
+          umma_commit_on(on, &q_empty[s]);
         }
-        if (ok) umma_commit(dkv_full);
+        umma_commit_on(on, dkv_full);
       }
     }
     __syncwarp();

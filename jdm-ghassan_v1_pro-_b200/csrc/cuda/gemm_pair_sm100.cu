@@ -22,11 +22,12 @@ namespace gb {
 namespace pr {
 
 static constexpr int HM = 128;        // A rows per CTA  (pair tile: 256)
-static constexpr int HN = 128;        // B rows per CTA  (pair tile: 256 output columns)
-static constexpr int TM = 256, TN = 256;
+static constexpr int TM = 256;
+static constexpr int TN_MAX = 256;    // output columns of a pair tile (Params::tn: 128 .. 256); each CTA stages half of them
 static constexpr int BK = 64, UMMA_K = 16;
 static constexpr int THREADS = 320, W_TMA = 8, W_MMA = 9, EPI_WARPS = 8;
-static constexpr uint32_t A_BYTES = HM * BK * 2, B_BYTES = HN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+static constexpr uint32_t A_BYTES = HM * BK * 2, STAGE_BYTES = A_BYTES + TN_MAX / 2 * BK * 2;
+static constexpr int MAX_STAGES = 8;  // narrower tiles have smaller stages, and more of them
 static constexpr uint32_t SLOT_BYTES = 4096;   // 32 rows x 128 bytes
 static constexpr uint32_t TMEM_COLS = 512;
 static constexpr uint32_t BAR_BYTES = 512;
@@ -35,6 +36,7 @@ enum { EPI_STORE = 0, EPI_SWIGLU_FWD = 1, EPI_SWIGLU_BWD = 2, EPI_RELU2 = 4 };  
 
 struct Params {
   int M, N, K;
+  int tn, stages;              // output columns of a tile; pipeline depth that fits beside the epilogue's slots
   int a_mn, b_mn, fmt;
   int mode;                    // 0 dense, 1 expert-sorted rows, 2 grouped over the reduction dim
   const int* tile_expert;      // mode 1: expert of each 128-row tile (tiles 2i and 2i+1 must agree)
@@ -66,32 +68,16 @@ __device__ __forceinline__ Tile decode(const Params& p, int tile, int tiles_m, i
     const int gi = tile / per, r = tile - gi * per;
     t.g = p.groups - 1 - gi;
     t.m0 = (r % tiles_m) * TM;
-    t.n0 = (r / tiles_m) * TN;
+    t.n0 = (r / tiles_m) * p.tn;
     t.k_begin = p.seg_offsets[t.g];
     t.k_end = p.seg_offsets[t.g + 1];
   } else {
     const int tm = tile / tiles_n, tn = tile - tm * tiles_n;   // column tiles of one row block are neighbours
     t.m0 = tm * TM;
-    t.n0 = tn * TN;
+    t.n0 = tn * p.tn;
     if (p.mode == 1) t.b_row_off = p.tile_expert[2 * tm] * p.b_group_rows;
   }
   return t;
-}
-
-// Bounded wait shared by all roles of a CTA: gives up when another role has given up or after ~2 s.
-__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, int* status, int code, volatile int* abort_flag) {
-  const long long t0 = clock64();
-  for (;;) {
-#pragma unroll 1
-    for (int i = 0; i < 2048; ++i)
-      if (mbar_try_wait(bar, parity)) return true;
-    if (*abort_flag) return false;
-    if (clock64() - t0 > 4000000000LL) {
-      atomicCAS(status, 0, code);
-      *abort_flag = 1;
-      return false;
-    }
-  }
 }
 
 // 16-byte piece j of this lane's 128-byte row inside a swizzled slot (the layout TMA expects for SWIZZLE_128B)
@@ -109,8 +95,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* slots = smem + STAGES * STAGE_BYTES;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(slots + EPI_WARPS * SLOTS * SLOT_BYTES);
-  uint64_t* empty_bar = full_bar + STAGES;
-  uint64_t* tfull_bar = empty_bar + STAGES;
+  uint64_t* empty_bar = full_bar + MAX_STAGES;
+  uint64_t* tfull_bar = empty_bar + MAX_STAGES;
   uint64_t* tempty_bar = tfull_bar + 2;
   uint64_t* aux_bar = tempty_bar + 2;               // [EPI_WARPS][2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(aux_bar + 2 * EPI_WARPS);
@@ -121,7 +107,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const uint32_t rank = cluster_ctarank();          // 0 = the CTA that issues the MMAs
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int s = 0; s < MAX_STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 2 * EPI_WARPS); }
     for (int i = 0; i < 2 * EPI_WARPS; ++i) mbar_init(&aux_bar[i], 1);
     *abort_flag = 0;
@@ -140,67 +126,68 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   cluster_sync_all();        // both CTAs' barriers exist before either signals the other's
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (tmem_base != 0 && threadIdx.x == 0) { atomicCAS(p.status, 0, ST_BAD_ARGUMENT); *abort_flag = 1; }
 
   const int tiles_m = (p.mode == 1) ? (*p.num_m_tiles + 1) / 2 : (p.M + TM - 1) / TM;
-  const int tiles_n = (p.N + TN - 1) / TN;
+  const int tiles_n = (p.N + p.tn - 1) / p.tn;
+  const int hn = p.tn >> 1;                                   // B rows per CTA
+  const uint32_t stage_bytes = A_BYTES + hn * (BK * 2), nst = p.stages;
   const int total_tiles = tiles_m * tiles_n * (p.mode == 2 ? p.groups : 1);
   const int pair_id = (int)cluster_id_x(), n_pairs = (int)cluster_nctaid_x();
 
   if (warp == W_TMA) {
     // ------------------------------------------------------------- TMA producer (one per CTA, for its own halves)
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one(), on0 = on && rank == 0;
       const uint32_t full0 = mapa_shared(smem_u32(&full_bar[0]), 0);   // the full barriers that count are CTA 0's
-      uint32_t it = 0;
-      bool ok = true;
-      for (int tile = pair_id; tile < total_tiles && ok; tile += n_pairs) {
+      uint32_t s = 0, ph = 0;
+      for (int tile = pair_id; tile < total_tiles; tile += n_pairs) {
         const Tile t = decode(p, tile, tiles_m, tiles_n);
-        const int am = t.m0 + (int)rank * HM, bn = t.n0 + (int)rank * HN;
-        for (int k = t.k_begin; k < t.k_end; k += BK, ++it) {
-          const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (!wait_bar(&empty_bar[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag)) { ok = false; break; }
-          uint8_t* sa = smem + s * STAGE_BYTES;
+        const int am = t.m0 + (int)rank * HM, bn = t.n0 + (int)rank * hn;
+        for (int k = t.k_begin; k < t.k_end; k += BK) {
+          wait_or_report(&empty_bar[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+          uint8_t* sa = smem + s * stage_bytes;
           uint8_t* sb = sa + A_BYTES;
-          if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], 2 * STAGE_BYTES);   // both CTAs' bytes
+          mbar_arrive_expect_tx_on(on0, &full_bar[s], 2 * stage_bytes);   // both CTAs' bytes
           const uint32_t fb = full0 + s * 8;
           if (!p.a_mn) {
-            tma_load_2d_pair(&tmA, fb, sa, k, am);
+            tma_load_2d_pair_on(on, &tmA, fb, sa, k, am);
           } else if (p.a_mn3) {
-            tma_load_3d_pair(&tmA, fb, sa, 0, k, am >> 6);
+            tma_load_3d_pair_on(on, &tmA, fb, sa, 0, k, am >> 6);
           } else {
 #pragma unroll
-            for (int c = 0; c < HM / 64; ++c) tma_load_2d_pair(&tmA, fb, sa + c * (64 * 128), am + c * 64, k);
+            for (int c = 0; c < HM / 64; ++c) tma_load_2d_pair_on(on, &tmA, fb, sa + c * (64 * 128), am + c * 64, k);
           }
           if (!p.b_mn) {
-            tma_load_2d_pair(&tmB, fb, sb, k, t.b_row_off + bn);
+            tma_load_2d_pair_on(on, &tmB, fb, sb, k, t.b_row_off + bn);
           } else if (p.b_mn3) {
-            tma_load_3d_pair(&tmB, fb, sb, 0, t.b_row_off + k, bn >> 6);
+            tma_load_3d_pair_on(on, &tmB, fb, sb, 0, t.b_row_off + k, bn >> 6);
           } else {
-#pragma unroll
-            for (int c = 0; c < HN / 64; ++c) tma_load_2d_pair(&tmB, fb, sb + c * (64 * 128), bn + c * 64, t.b_row_off + k);
+            for (int c = 0; c < hn / 64; ++c) tma_load_2d_pair_on(on, &tmB, fb, sb + c * (64 * 128), bn + c * 64, t.b_row_off + k);
           }
+          if (++s == nst) { s = 0; ph ^= 1; }
         }
       }
     }
     __syncwarp();
   } else if (warp == W_MMA) {
     // ------------------------------------------------------------- MMA issuer (CTA 0 only)
-    if (rank == 0 && lane == 0) {
-      const uint32_t idesc = make_idesc_f16(p.fmt, p.a_mn, p.b_mn, TM, TN);
-      uint32_t it = 0, acc_it = 0;
-      bool ok = true;
-      for (int tile = pair_id; tile < total_tiles && ok; tile += n_pairs) {
+    if (rank == 0) {
+      const uint32_t on = elect_one();
+      const uint32_t idesc = make_idesc_f16(p.fmt, p.a_mn, p.b_mn, TM, p.tn);
+      uint32_t s = 0, ph = 0, acc_it = 0;
+      for (int tile = pair_id; tile < total_tiles; tile += n_pairs) {
         const Tile t = decode(p, tile, tiles_m, tiles_n);
         if (t.k_end <= t.k_begin) continue;
         const uint32_t ab = acc_it & 1, aph = (acc_it >> 1) & 1;
-        if (!wait_bar(&tempty_bar[ab], aph ^ 1, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag)) { ok = false; break; }
+        wait_or_report(&tempty_bar[ab], aph ^ 1, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag);
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + ab * TN;
+        const uint32_t d_tmem = ab * TN_MAX;      // all 512 columns are this pair's: the allocation starts at column 0 (checked above)
         bool first = true;
-        for (int k = t.k_begin; k < t.k_end; k += BK, ++it) {
-          const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (!wait_bar(&full_bar[s], ph, p.status, ST_TIMEOUT_FULL, abort_flag)) { ok = false; break; }
+        for (int k = t.k_begin; k < t.k_end; k += BK) {
+          wait_or_report(&full_bar[s], ph, p.status, ST_TIMEOUT_FULL, abort_flag);
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
+          const uint32_t sa = smem_u32(smem + s * stage_bytes);
           const uint32_t sb = sa + A_BYTES;
           // same operand layouts as the one-CTA kernel with 128-row A and B tiles; the other CTA's halves sit at
           // the same shared-memory offsets
@@ -210,12 +197,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           const uint64_t b_step = p.b_mn ? (2048 >> 4) : (32 >> 4);
 #pragma unroll
           for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-            umma_f16_pair(d_tmem, da + kk * a_step, db + kk * b_step, idesc, first ? 0u : 1u);
+            umma_f16_pair_on(on, d_tmem, da + kk * a_step, db + kk * b_step, idesc, first ? 0u : 1u);
             first = false;
           }
-          umma_commit_pair(&empty_bar[s], 3);     // frees this stage in both CTAs
+          umma_commit_pair_on(on, &empty_bar[s], 3);     // frees this stage in both CTAs
+          if (++s == nst) { s = 0; ph ^= 1; }
         }
-        if (ok) umma_commit_pair(&tfull_bar[ab], 3);
+        umma_commit_pair_on(on, &tfull_bar[ab], 3);
         ++acc_it;
       }
     }
@@ -228,7 +216,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const uint32_t tempty0 = mapa_shared(smem_u32(&tempty_bar[0]), 0);
     uint32_t acc_it = 0, n_slot = 0;
     uint32_t aux_cnt[2] = {0, 0};     // completed phases of this warp's two load barriers
-    bool ok = true;
     // next free slot; the SLOTS-1 most recent stores may still be reading theirs
     auto acquire = [&]() -> uint8_t* {
       if (lane == 0) bulk_wait_read<SLOTS - 1>();
@@ -237,11 +224,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       ++n_slot;
       return s;
     };
-    for (int tile = pair_id; tile < total_tiles && ok; tile += n_pairs) {
+    for (int tile = pair_id; tile < total_tiles; tile += n_pairs) {
       const Tile t = decode(p, tile, tiles_m, tiles_n);
       const bool empty_k = (t.k_end <= t.k_begin);
       const int row_q = t.m0 + (int)rank * HM + quarter * 32;   // first of this warp's 32 rows
-      const int colh = t.n0 + half * 128;                       // first of this warp's 128 accumulator columns
+      const int colh = t.n0 + half * 128;                       // first of this warp's 128 accumulator columns (SwiGLU: tn = 256)
       const bool rows_live = row_q < p.M;
 
       if constexpr (EPI == EPI_SWIGLU_BWD) {
@@ -266,18 +253,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (!empty_k) {
         ab = acc_it & 1;
         const uint32_t aph = (acc_it >> 1) & 1;
-        if (!wait_bar(&tfull_bar[ab], aph, p.status, ST_TIMEOUT_TMEM_FULL, abort_flag)) { ok = false; break; }
+        wait_or_report(&tfull_bar[ab], aph, p.status, ST_TIMEOUT_TMEM_FULL, abort_flag);
         tc_fence_after();
       }
-      const uint32_t taddr = tmem_base + ab * TN + half * 128 + (uint32_t(quarter * 32) << 16);
+      const uint32_t tacc = tmem_base + ab * TN_MAX + (uint32_t(quarter * 32) << 16), taddr = tacc + half * 128;
 
       if constexpr ((EPI == EPI_STORE || EPI == EPI_RELU2) && sizeof(OutT) == 2) {
 #pragma unroll 1
-        for (int c = 0; c < 2; ++c) {               // 64-column chunks
+        for (int c = half; c < p.tn >> 6; c += 2) { // 64-column chunks, in turn for the two warps of a quarter
           uint32_t r0[32], r1[32];
           if (!empty_k) {
-            tmem_ld_32x32(taddr + c * 64, r0);
-            tmem_ld_32x32(taddr + c * 64 + 32, r1);
+            tmem_ld_32x32(tacc + c * 64, r0);
+            tmem_ld_32x32(tacc + c * 64 + 32, r1);
             tmem_ld_wait();
           } else {
 #pragma unroll
@@ -309,7 +296,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           fence_proxy_async();
           __syncwarp();
           if (lane == 0) {
-            const int col = colh + c * 64;
+            const int col = t.n0 + c * 64;
             if (rows_live && col < p.N) tma_store_3d(&tmO, slot, col, row_q, t.g);
             bulk_commit();
           }
@@ -317,11 +304,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       } else if constexpr (EPI == EPI_STORE) {
         // fp32 output, 32-column chunks: plain store, store of acc + addend, or reduce-add into the matrix
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          const int col = colh + c * 32;
+        for (int c = half; c < p.tn >> 5; c += 2) {
+          const int col = t.n0 + c * 32;
           uint32_t r[32];
           if (!empty_k) {
-            tmem_ld_32x32(taddr + c * 32, r);
+            tmem_ld_32x32(tacc + c * 32, r);
             tmem_ld_wait();
           } else {
 #pragma unroll
@@ -428,7 +415,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           tmem_ld_32x32(taddr + blk * 64 + 32, r1);
           tmem_ld_wait();
           if (!live) continue;
-          if (!wait_bar(&my_aux[blk], aux_cnt[blk] & 1, p.status, ST_TIMEOUT_AUX, abort_flag)) { ok = false; break; }
+          wait_or_report(&my_aux[blk], aux_cnt[blk] & 1, p.status, ST_TIMEOUT_AUX, abort_flag);
           ++aux_cnt[blk];
           uint8_t* sg = my_slots + (2 * blk) * SLOT_BYTES;
           uint8_t* su = sg + SLOT_BYTES;
@@ -460,7 +447,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             bulk_commit();
           }
         }
-        if (!ok) break;
       }
 
       if (!empty_k) {
@@ -533,7 +519,10 @@ namespace {
 
 template <int EPI, int STAGES, int SLOTS, typename OutT>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, const CUtensorMap& tx,
-                const gb::pr::Params& p, int max_tiles, cudaStream_t st) {
+                gb::pr::Params p, int max_tiles, cudaStream_t st) {
+  const uint32_t stage = gb::pr::A_BYTES + p.tn / 2 * gb::pr::BK * 2;
+  p.stages = (int)(STAGES * gb::pr::STAGE_BYTES / stage);
+  if (p.stages > gb::pr::MAX_STAGES) p.stages = gb::pr::MAX_STAGES;
   auto kern = gb::pr::gemm_pair_kernel<EPI, STAGES, SLOTS, OutT>;
   constexpr size_t smem = gb::pr::smem_bytes<STAGES, SLOTS>();
   static_assert(smem <= 232448, "shared memory of the pair kernel exceeds 227 KB");
@@ -593,6 +582,8 @@ extern "C" int gb_gemm_pair(const gb_gemm_args* a, cudaStream_t st) {
     else { p.addend = a->addend; p.ld_add = a->ld_add; }
   }
 
+  p.tn = pr::TN_MAX;
+
   CUtensorMap ta, tb, to, tx;
   int rc;
   // An MN-major operand is fetched with one chunked 3-D load per k-block (measured 4-10 % faster on the weight
@@ -604,14 +595,14 @@ extern "C" int gb_gemm_pair(const gb_gemm_args* a, cudaStream_t st) {
     p.a_mn3 = 1;
   } else rc = gb_make_tmap_2d_16b(&ta, a->A, a->a_rows, a->a_cols, a->lda, pr::BK, 64, a->is_bf16);
   if (rc) return rc - 100;
-  if (!a->b_mn_major) rc = gb_make_tmap_2d_16b(&tb, a->B, a->b_rows, a->b_cols, a->ldb, pr::HN, pr::BK, a->is_bf16);
+  if (!a->b_mn_major) rc = gb_make_tmap_2d_16b(&tb, a->B, a->b_rows, a->b_cols, a->ldb, p.tn / 2, pr::BK, a->is_bf16);
   else if (chunked && a->b_cols % 64 == 0) {
-    rc = gb_make_tmap_mn_chunks(&tb, a->B, a->b_rows, a->b_cols, a->ldb, pr::BK, pr::HN / 64, a->is_bf16);
+    rc = gb_make_tmap_mn_chunks(&tb, a->B, a->b_rows, a->b_cols, a->ldb, pr::BK, p.tn / 128, a->is_bf16);
     p.b_mn3 = 1;
   } else rc = gb_make_tmap_2d_16b(&tb, a->B, a->b_rows, a->b_cols, a->ldb, pr::BK, 64, a->is_bf16);
   if (rc) return rc - 200;
 
-  const int tiles_m = (a->M + pr::TM - 1) / pr::TM, tiles_n = (a->N + pr::TN - 1) / pr::TN;
+  const int tiles_m = (a->M + pr::TM - 1) / pr::TM, tiles_n = (a->N + p.tn - 1) / p.tn;
   const int max_tiles = tiles_m * tiles_n * groups;
 
   switch (a->epilogue) {

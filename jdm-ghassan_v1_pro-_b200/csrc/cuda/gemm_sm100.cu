@@ -198,29 +198,29 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
   if (warp == W_TMA) {
     // ------------------------------------------------------------- TMA producer
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one();
       uint32_t it = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+      for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
         TileInfo t = decode_tile<BN>(p, tile, tiles_m, tiles_n);
         for (int k = t.k_begin; k < t.k_end; k += BK, ++it) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (!wait_or_flag(&empty_bar[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag)) { ok = false; break; }
+          wait_or_report(&empty_bar[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
           uint8_t* sa = smem + s * STAGE_BYTES;
           uint8_t* sb = sa + A_BYTES;
-          mbar_arrive_expect_tx(&full_bar[s], STAGE_BYTES);
+          mbar_arrive_expect_tx_on(on, &full_bar[s], STAGE_BYTES);
           if (!p.a_mn_major) {
-            tma_load_2d(&tmA, &full_bar[s], sa, k, t.a_row0);
+            tma_load_2d_on(on, &tmA, &full_bar[s], sa, k, t.a_row0);
           } else {
 #pragma unroll
-            for (int c = 0; c < BM / 64; ++c) tma_load_2d(&tmA, &full_bar[s], sa + c * (64 * 128), t.a_row0 + c * 64, k);
+            for (int c = 0; c < BM / 64; ++c) tma_load_2d_on(on, &tmA, &full_bar[s], sa + c * (64 * 128), t.a_row0 + c * 64, k);
           }
           if (!p.b_mn_major) {
-            tma_load_2d(&tmB, &full_bar[s], sb, k, t.b_row_off + t.n0);
+            tma_load_2d_on(on, &tmB, &full_bar[s], sb, k, t.b_row_off + t.n0);
           } else {
 #pragma unroll
             for (int c = 0; c < BN / 64; ++c)
-              tma_load_2d(&tmB, &full_bar[s], sb + c * (64 * 128), t.n0 + c * 64, t.b_row_off + k);
+              tma_load_2d_on(on, &tmB, &full_bar[s], sb + c * (64 * 128), t.n0 + c * 64, t.b_row_off + k);
           }
         }
       }
@@ -228,21 +228,21 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     __syncwarp();
   } else if (warp == W_MMA) {
     // ------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one();
       const uint32_t idesc = make_idesc_f16(p.fmt, p.a_mn_major, p.b_mn_major, BM, BN);
       uint32_t it = 0, acc_it = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+      for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
         TileInfo t = decode_tile<BN>(p, tile, tiles_m, tiles_n);
         if (t.k_end <= t.k_begin) continue;
         const uint32_t ab = acc_it & 1, aph = (acc_it >> 1) & 1;
-        if (!wait_or_flag(&tempty_bar[ab], aph ^ 1, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag)) { ok = false; break; }
+        wait_or_report(&tempty_bar[ab], aph ^ 1, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag);
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + ab * BN;
         bool first = true;
         for (int k = t.k_begin; k < t.k_end; k += BK, ++it) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          if (!wait_or_flag(&full_bar[s], ph, p.status, ST_TIMEOUT_FULL, abort_flag)) { ok = false; break; }
+          wait_or_report(&full_bar[s], ph, p.status, ST_TIMEOUT_FULL, abort_flag);
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
           const uint32_t sb = sa + A_BYTES;
@@ -254,12 +254,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           const uint64_t b_step = p.b_mn_major ? (2048 >> 4) : (32 >> 4);
 #pragma unroll
           for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-            umma_f16(d_tmem, da + kk * a_step, db + kk * b_step, idesc, first ? 0u : 1u);
+            umma_f16_on(on, d_tmem, da + kk * a_step, db + kk * b_step, idesc, first ? 0u : 1u);
             first = false;
           }
-          umma_commit(&empty_bar[s]);  // smem stage is free once these MMAs retire
+          umma_commit_on(on, &empty_bar[s]);  // smem stage is free once these MMAs retire
         }
-        if (ok) umma_commit(&tfull_bar[ab]);
+        umma_commit_on(on, &tfull_bar[ab]);
         ++acc_it;
       }
     }

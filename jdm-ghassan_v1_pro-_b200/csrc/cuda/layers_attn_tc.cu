@@ -113,48 +113,48 @@ __global__ void __launch_bounds__(LA_THREADS) ll_attn_tc_kernel(const __grid_con
   };
 
   if (warp == 4) {
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one();
       uint32_t kv_it = 0, q_it = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++q_it) {
+      for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++q_it) {
         const Item it = item_of(item);
-        if (!at_wait(q_empty, (q_it & 1u) ^ 1u, a.status, ST_TIMEOUT_EMPTY, abort_flag)) break;
-        mbar_arrive_expect_tx(q_full, TQ);
-        load_tile<DK>(&tmQ, q_full, sQ, it.h * DK, it.b * a.n + it.q0);
+        wait_or_report(q_empty, (q_it & 1u) ^ 1u, a.status, ST_TIMEOUT_EMPTY, abort_flag);
+        mbar_arrive_expect_tx_on(on, q_full, TQ);
+        load_tile<DK>(on, &tmQ, q_full, sQ, it.h * DK, it.b * a.n + it.q0);
         const int g = it.h / rep;
         for (int t = 0; t < it.n_kt + it.n_rt; ++t, ++kv_it) {
           const int s = kv_it & 1, ph = (kv_it >> 1) & 1;
-          if (!at_wait(&kv_empty[s], ph ^ 1, a.status, ST_TIMEOUT_EMPTY, abort_flag)) { ok = false; break; }
-          mbar_arrive_expect_tx(&kv_full[s], TQ + TV);
+          wait_or_report(&kv_empty[s], ph ^ 1, a.status, ST_TIMEOUT_EMPTY, abort_flag);
+          mbar_arrive_expect_tx_on(on, &kv_full[s], TQ + TV);
           const int row = tile_row(it, t);
-          load_tile<DK>(&tmK, &kv_full[s], sK + s * TQ, g * DK, row);
-          load_tile<DV>(&tmV, &kv_full[s], sV + s * TV, g * DV, row);
+          load_tile<DK>(on, &tmK, &kv_full[s], sK + s * TQ, g * DK, row);
+          load_tile<DV>(on, &tmV, &kv_full[s], sV + s * TV, g * DV, row);
         }
       }
     }
     __syncwarp();
   } else if (warp == 5) {
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one();
       const uint32_t idesc_s = make_idesc_f16(1, 0, 0, AT_M, AT_N);
       const uint32_t idesc_o = make_idesc_f16(1, 0, 1, AT_M, DV);
       uint32_t kv_it = 0, q_it = 0;
-      bool ok = true;
-      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++q_it) {
+      for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++q_it) {
         const Item it = item_of(item);
         const int n_tiles = it.n_kt + it.n_rt;
-        if (!at_wait(q_full, q_it & 1u, a.status, ST_TIMEOUT_FULL, abort_flag)) break;
+        wait_or_report(q_full, q_it & 1u, a.status, ST_TIMEOUT_FULL, abort_flag);
         for (int t = 0; t < n_tiles; ++t, ++kv_it) {
           const int s = kv_it & 1, ph = (kv_it >> 1) & 1;
-          if (!at_wait(&kv_full[s], ph, a.status, ST_TIMEOUT_FULL, abort_flag)) { ok = false; break; }
+          wait_or_report(&kv_full[s], ph, a.status, ST_TIMEOUT_FULL, abort_flag);
           tc_fence_after();
-          mma_kmajor_kmajor<DK>(tmem_S, smem_u32(sQ), smem_u32(sK + s * TQ), idesc_s, false);
-          umma_commit(s_full);
-          if (t == n_tiles - 1) umma_commit(q_empty);
-          if (!at_wait(p_ready, kv_it & 1u, a.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag)) { ok = false; break; }
+          mma_kmajor_kmajor<DK>(on, tmem_S, smem_u32(sQ), smem_u32(sK + s * TQ), idesc_s, false);
+          umma_commit_on(on, s_full);
+          if (t == n_tiles - 1) umma_commit_on(on, q_empty);
+          wait_or_report(p_ready, kv_it & 1u, a.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag);
           tc_fence_after();
-          mma_kmajor_mnmajor<AT_N>(tmem_O, smem_u32(sP), smem_u32(sV + s * TV), idesc_o, t > 0);
-          umma_commit(o_full);
-          umma_commit(&kv_empty[s]);
+          mma_kmajor_mnmajor<AT_N>(on, tmem_O, smem_u32(sP), smem_u32(sV + s * TV), idesc_o, t > 0);
+          umma_commit_on(on, o_full);
+          umma_commit_on(on, &kv_empty[s]);
         }
       }
     }

@@ -98,47 +98,49 @@ __global__ void __launch_bounds__(LT_THREADS) ll_latent_tc_kernel(const __grid_c
   const int t_lo = split * per, n_t = max(0, min(tiles, t_lo + per) - t_lo);
 
   if (warp == 4) {
-    if (lane == 0 && n_t > 0) {
-      mbar_arrive_expect_tx(q_full, panels * QP);
-      for (int p = 0; p < panels; ++p) tma_load_2d(&tmQ, q_full, sQ + p * QP, p * 64, r * a.heads_pad + h0);
+    if (n_t > 0) {
+      const uint32_t on = elect_one();
+      mbar_arrive_expect_tx_on(on, q_full, panels * QP);
+      for (int p = 0; p < panels; ++p) tma_load_2d_on(on, &tmQ, q_full, sQ + p * QP, p * 64, r * a.heads_pad + h0);
       for (int t = 0; t < n_t; ++t) {
         const int s = t % stages, ph = (t / stages) & 1;
-        if (!at_wait(&kv_empty[s], ph ^ 1, a.status, ST_TIMEOUT_EMPTY, abort_flag)) break;
-        mbar_arrive_expect_tx(&kv_full[s], panels * KP);
+        wait_or_report(&kv_empty[s], ph ^ 1, a.status, ST_TIMEOUT_EMPTY, abort_flag);
+        mbar_arrive_expect_tx_on(on, &kv_full[s], panels * KP);
         for (int p = 0; p < panels; ++p)
-          tma_load_2d(&tmC, &kv_full[s], sK + (size_t)(s * panels + p) * KP, p * 64, b * a.cap + (t_lo + t) * AT_N);
+          tma_load_2d_on(on, &tmC, &kv_full[s], sK + (size_t)(s * panels + p) * KP, p * 64, b * a.cap + (t_lo + t) * AT_N);
       }
     }
     __syncwarp();
   } else if (warp == 5) {
-    if (lane == 0 && n_t > 0) {
+    if (n_t > 0) {
+      const uint32_t on = elect_one();
       const uint32_t idesc_s = make_idesc_f16(1, 0, 0, AT_N, HP), idesc_o = make_idesc_f16(1, 1, 0, 128, HP);
       const uint64_t dq0 = make_smem_desc_sw128(smem_u32(sQ), 16, 1024), dp0 = make_smem_desc_sw128(smem_u32(sP), 16, 1024);
-      bool ok = at_wait(q_full, 0, a.status, ST_TIMEOUT_FULL, abort_flag);
-      for (int t = 0; t < n_t && ok; ++t) {
+      wait_or_report(q_full, 0, a.status, ST_TIMEOUT_FULL, abort_flag);
+      for (int t = 0; t < n_t; ++t) {
         const int s = t % stages, ph = (t / stages) & 1;
-        if (!at_wait(&kv_full[s], ph, a.status, ST_TIMEOUT_FULL, abort_flag)) break;
+        wait_or_report(&kv_full[s], ph, a.status, ST_TIMEOUT_FULL, abort_flag);
         tc_fence_after();
-        // descriptors step by whole panels (start addresses count 16 bytes): one thread issues, so few instructions per product
+        // descriptors step by whole panels (start addresses count 16 bytes): few instructions per product
         const uint32_t k0 = smem_u32(sK + (size_t)s * panels * KP);
         uint64_t dk = make_smem_desc_sw128(k0, 16, 1024), dq = dq0;
         for (int kk = 0; kk < dsteps; kk += 4, dk += KP >> 4, dq += QP >> 4) {
           const int left = dsteps - kk;
-          umma_f16(tmem_S, dk, dq, idesc_s, kk > 0);
-          if (left > 1) umma_f16(tmem_S, dk + 2, dq + 2, idesc_s, 1);
-          if (left > 2) umma_f16(tmem_S, dk + 4, dq + 4, idesc_s, 1);
-          if (left > 3) umma_f16(tmem_S, dk + 6, dq + 6, idesc_s, 1);
+          umma_f16_on(on, tmem_S, dk, dq, idesc_s, kk > 0);
+          if (left > 1) umma_f16_on(on, tmem_S, dk + 2, dq + 2, idesc_s, 1);
+          if (left > 2) umma_f16_on(on, tmem_S, dk + 4, dq + 4, idesc_s, 1);
+          if (left > 3) umma_f16_on(on, tmem_S, dk + 6, dq + 6, idesc_s, 1);
         }
-        umma_commit(s_full);
-        if (!at_wait(p_ready, t & 1, a.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag)) break;
+        umma_commit_on(on, s_full);
+        wait_or_report(p_ready, t & 1, a.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag);
         tc_fence_after();
         uint64_t dv = make_smem_desc_sw128(k0, KP, 1024);
         for (int c = 0; c < chunks; ++c, dv += 2 * (KP >> 4))
 #pragma unroll
           for (int kk = 0; kk < AT_N / 16; ++kk)      // A: latent dimensions along M (two panels), keys along K, 16 rows a step
-            umma_f16(tmem_O + c * HP, dv + kk * (2048 >> 4), dp0 + ((kk >> 2) * QP + (kk & 3) * 32) / 16, idesc_o, (t > 0 || kk > 0) ? 1u : 0u);
-        umma_commit(&kv_empty[s]);
-        umma_commit(o_full);
+            umma_f16_on(on, tmem_O + c * HP, dv + kk * (2048 >> 4), dp0 + ((kk >> 2) * QP + (kk & 3) * 32) / 16, idesc_o, (t > 0 || kk > 0) ? 1u : 0u);
+        umma_commit_on(on, &kv_empty[s]);
+        umma_commit_on(on, o_full);
       }
     }
     __syncwarp();

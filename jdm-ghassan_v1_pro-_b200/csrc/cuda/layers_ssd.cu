@@ -47,39 +47,6 @@ __device__ __forceinline__ float sd_ex2(float x) {
   return r;
 }
 
-// MMA and commit for a warp that runs converged: every lane passes the same operands, the lane with `on` != 0 issues.  The
-// operands then stay in uniform registers, which is where the instruction wants them; issued from a one-lane branch, each
-// MMA first moved its descriptors there and cost 70 to 100 cycles of issue time.
-__device__ __forceinline__ void sd_mma(uint32_t on, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      :
-      : "r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(on)
-      : "memory");
-}
-__device__ __forceinline__ void sd_mma_ts(uint32_t on, uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      :
-      : "r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(on)
-      : "memory");
-}
-__device__ __forceinline__ void sd_commit(uint32_t on, uint64_t* bar) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\t"
-      "setp.ne.b32 q, %1, 0;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-      :
-      : "r"(smem_u32(bar)), "r"(on)
-      : "memory");
-}
-
 // Out of line: the kernel has five roles with long straight-line bodies, and what bounds it once the chains overlap is the
 // instruction cache (a wait that was over cost 400 cycles with everything unrolled and inlined).
 __device__ __noinline__ bool sd_wait(uint32_t bar, uint32_t parity, int* status, int code, volatile int* abort_flag) {
@@ -200,23 +167,24 @@ __global__ void __launch_bounds__(SsdCfg<PP, SO>::THREADS, SsdCfg<PP, SO>::CTAS)
 
   if (warp == K::W_TMA) {
     // ------------------------------------------------------------------ TMA
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one();
       for (int c = 0; c < nc; ++c) {
         const int s = c % K::STAGES, ph = (c / K::STAGES) & 1;
         SD_WAIT(&empty[s], ph ^ 1, ST_TIMEOUT_EMPTY);
         uint8_t* st = smem + s * K::STAGE;
         const int row = b * p.n + (c_lo + c) * SD_Q;
-        mbar_arrive_expect_tx(&full[s], K::STAGE);
-        load_tile<SD_N>(&tmB, &full[s], st + K::OFF_B, g * SD_N, row);
-        load_tile<PP>(&tmX, &full[s], st + K::OFF_X, h * PP, row);
-        if (!so) load_tile<SD_N>(&tmC, &full[s], st, g * SD_N, row);
+        mbar_arrive_expect_tx_on(on, &full[s], K::STAGE);
+        load_tile<SD_N>(on, &tmB, &full[s], st + K::OFF_B, g * SD_N, row);
+        load_tile<PP>(on, &tmX, &full[s], st + K::OFF_X, h * PP, row);
+        if (!so) load_tile<SD_N>(on, &tmC, &full[s], st, g * SD_N, row);
       }
     }
     __syncwarp();
   } else if (warp == K::W_MMA) {
     // ------------------------------------------------------------------ MMA
     {
-      const uint32_t on = lane == 0;
+      const uint32_t on = elect_one();
       const uint32_t id_g = make_idesc_f16(1, 0, 0, SD_Q, SD_Q);
       const uint32_t id_y = make_idesc_f16(1, 0, 1, SD_Q, PP);
       const uint32_t id_y2 = make_idesc_f16(1, 0, 1, SD_Q, PP * K::NY2);
@@ -231,9 +199,9 @@ __global__ void __launch_bounds__(SsdCfg<PP, SO>::THREADS, SsdCfg<PP, SO>::CTAS)
 #pragma unroll
         for (int kk = 0; kk < SD_N / 16; ++kk) {
           const uint32_t off = (kk >> 2) * 1024 + (kk & 3) * 2;
-          sd_mma(on, to, dc + off, dc + (K::OFF_B >> 4) + off, id_g, kk ? 1u : 0u);
+          umma_f16_on(on, to, dc + off, dc + (K::OFF_B >> 4) + off, id_g, kk ? 1u : 0u);
         }
-        sd_commit(on, g_full);
+        umma_commit_on(on, g_full);
       };
       bool ok = true;
       if (!so) {
@@ -252,7 +220,7 @@ __global__ void __launch_bounds__(SsdCfg<PP, SO>::THREADS, SsdCfg<PP, SO>::CTAS)
           for (int part = 0; part < 2 / K::NY2; ++part)
 #pragma unroll
             for (int kk = 0; kk < SD_N / 16; ++kk)
-              sd_mma(on, K::COL_Y2, dc + (kk >> 2) * 1024 + (kk & 3) * 2, d_s + part * (K::TS >> 4) + kk * 128, id_y2, (part || kk) ? 1u : 0u);
+              umma_f16_on(on, K::COL_Y2, dc + (kk >> 2) * 1024 + (kk & 3) * 2, d_s + part * (K::TS >> 4) + kk * 128, id_y2, (part || kk) ? 1u : 0u);
         }
         SD_WAIT(xw_ready, c & 1, ST_TIMEOUT_EMPTY);
         tc_fence_after();
@@ -260,8 +228,8 @@ __global__ void __launch_bounds__(SsdCfg<PP, SO>::THREADS, SsdCfg<PP, SO>::CTAS)
         for (int part = 0; part < 2; ++part)
 #pragma unroll
           for (int kk = 0; kk < SD_Q / 16; ++kk)
-            sd_mma(on, tm + K::COL_S, dmn + (K::OFF_B >> 4) + kk * 128, d_xw + part * (K::TX >> 4) + kk * 128, id_s, 1u);
-        sd_commit(on, s_full);
+            umma_f16_on(on, tm + K::COL_S, dmn + (K::OFF_B >> 4) + kk * 128, d_xw + part * (K::TX >> 4) + kk * 128, id_s, 1u);
+        umma_commit_on(on, s_full);
         if (!so) {
           SD_WAIT(m_ready, c & 1, ST_TIMEOUT_TMEM_EMPTY);
           tc_fence_after();
@@ -270,11 +238,11 @@ __global__ void __launch_bounds__(SsdCfg<PP, SO>::THREADS, SsdCfg<PP, SO>::CTAS)
           for (int part = 0; part < 2; ++part)
 #pragma unroll
             for (int kk = 0; kk < SD_Q / 16; ++kk)
-              sd_mma_ts(on, K::COL_Y, m0 + (kk >> 1) * 32 + part * 16 + (kk & 1) * 8, dmn + (K::OFF_X >> 4) + kk * 128, id_y,
+              umma_f16_ts_on(on, K::COL_Y, m0 + (kk >> 1) * 32 + part * 16 + (kk & 1) * 8, dmn + (K::OFF_X >> 4) + kk * 128, id_y,
                           (part || kk) ? 1u : 0u);
-          sd_commit(on, y_full);
+          umma_commit_on(on, y_full);
         }
-        sd_commit(on, &empty[s]);
+        umma_commit_on(on, &empty[s]);
         if (!so && c + 1 < nc) {
           if (K::NG == 1) SD_WAIT(y_full, c & 1, ST_TIMEOUT_TMEM_FULL);      // the one score buffer still holds this chunk's weights
           SD_WAIT(&full[(c + 1) % K::STAGES], ((c + 1) / K::STAGES) & 1, ST_TIMEOUT_FULL);

@@ -243,31 +243,32 @@ __global__ void __launch_bounds__(RT_THREADS) moe_route_tc_kernel(const __grid_c
   const uint32_t tmem_D = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one();
       for (int kc = pre; kc < nkc; ++kc) {
         const int s = kc % RT_ST, ph = (kc / RT_ST) & 1;
-        if (!mbar_wait(&empty[s], ph ^ 1)) { atomicCAS(status, 0, ST_TIMEOUT_EMPTY); break; }
-        mbar_arrive_expect_tx(&full[s], RT_XTILE);
-        tma_load_2d(&tmX, &full[s], sX + s * RT_XTILE, kc * RT_KC, t0);
+        if (!mbar_wait(&empty[s], ph ^ 1)) atomicCAS(status, 0, ST_TIMEOUT_EMPTY);
+        mbar_arrive_expect_tx_on(on, &full[s], RT_XTILE);
+        tma_load_2d_on(on, &tmX, &full[s], sX + s * RT_XTILE, kc * RT_KC, t0);
       }
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const uint32_t on = elect_one();
       const uint32_t idesc = make_idesc_f16(kBf16 ? 1 : 0, 0, 0, RT_TOK, 16);
-      bool ok = true;
-      for (int kc = 0; kc < nkc && ok; ++kc) {
+      for (int kc = 0; kc < nkc; ++kc) {
         const int s = kc % RT_ST, ph = (kc / RT_ST) & 1;
-        if (!mbar_wait(&full[s], ph)) { atomicCAS(status, 0, ST_TIMEOUT_FULL); ok = false; break; }
+        if (!mbar_wait(&full[s], ph)) atomicCAS(status, 0, ST_TIMEOUT_FULL);
         tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < RT_KC / 16; ++kk)
-          umma_f16(tmem_D, make_smem_desc_sw128(smem_u32(sX + s * RT_XTILE) + kk * 32, 16, 1024),
+          umma_f16_on(on, tmem_D, make_smem_desc_sw128(smem_u32(sX + s * RT_XTILE) + kk * 32, 16, 1024),
                    make_smem_desc_sw128(smem_u32(sW + (size_t)kc * RT_WPANEL) + kk * 32, 16, 1024), idesc,
                    (kc > 0 || kk > 0) ? 1u : 0u);
-        umma_commit(&empty[s]);
+        umma_commit_on(on, &empty[s]);
       }
-      if (ok) umma_commit(d_full);
+      umma_commit_on(on, d_full);
     }
     __syncwarp();
   } else {

@@ -97,6 +97,31 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// Polls a few times inside one instruction sequence, so that callers' loops keep one straight path.
+__device__ __forceinline__ bool mbar_try_wait_some(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P1, P2;\n\t.reg .u32 n;\n\t"
+      "mov.u32 n, 64;\n\t"
+      "L_POLL_%=:\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+      "@P1 bra L_DONE_%=;\n\t"
+      "sub.u32 n, n, 1;\n\t"
+      "setp.ne.u32 P2, n, 0;\n\t"
+      "@P2 bra L_POLL_%=;\n\t"
+      "L_DONE_%=:\n\t"
+      "selp.b32 %0, 1, 0, P1;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// One lane of a converged warp.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t on;
+  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.b32 %0, 1, 0, P;\n\t}" : "=r"(on));
+  return on;
+}
 #ifndef GB_SPIN_LIMIT
 #define GB_SPIN_LIMIT (1u << 24)
 #endif
@@ -106,6 +131,28 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     if (mbar_try_wait(bar, parity)) return true;
   }
   return false;
+}
+
+// Bounded wait shared by all roles of a CTA: gives up when another role has given up or after ~2 s.  It reports the failure and
+// returns: the callers go on (every later wait then returns at once, on whatever the buffers hold, and the status word says
+// that the results are void).  A loop that left on a wait's result would no longer be provably uniform over the warp, and the
+// operands of the MMAs would lose their uniform registers.
+static __device__ __noinline__ void wait_or_report_slow(uint64_t* bar, uint32_t parity, int* status, int code, volatile int* abort_flag) {
+  const long long t0 = clock64();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 2048; ++i)
+      if (mbar_try_wait(bar, parity)) return;
+    if (*abort_flag) return;
+    if (clock64() - t0 > 4000000000LL) {
+      atomicCAS(status, 0, code);
+      *abort_flag = 1;
+      return;
+    }
+  }
+}
+__device__ __forceinline__ void wait_or_report(uint64_t* bar, uint32_t parity, int* status, int code, volatile int* abort_flag) {
+  if (!mbar_try_wait_some(bar, parity)) wait_or_report_slow(bar, parity, status, code, abort_flag);
 }
 
 // ----------------------------------------------------------------------------- TMA
@@ -240,23 +287,6 @@ __device__ __forceinline__ void cluster_sync_all() {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// TMA load into this CTA's shared memory whose bytes are counted on `bar_cluster_addr`, which may be the other CTA's
-__device__ __forceinline__ void tma_load_2d_pair(const CUtensorMap* map, uint32_t bar_cluster_addr, void* dst, int c0,
-                                                 int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      :
-      : "r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_3d_pair(const CUtensorMap* map, uint32_t bar_cluster_addr, void* dst, int c0,
-                                                 int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      :
-      : "r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_dst, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(ncols)
                : "memory");
@@ -267,23 +297,101 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                              uint32_t accumulate) {
+
+// ----------------------------------------------------------------------------- issue from a warp that runs converged
+// Every lane passes the same operands and the lane with `on` != 0 issues; `on` comes from elect_one().  The operands then stay
+// in uniform registers, which is where these instructions want them.  Measured in the two-CTA GEMM, cycles per 64-deep k-block
+// (four MMAs and a commit; the MMAs themselves take 512 at 256 columns and 256 at 128): 747 issued from an `if (lane == 0)`
+// branch, whatever the tile's width; 548 with the whole warp in the loop and `on = lane == 0`; 512 and 444 with elect_one().
+// The forms of one CTA are plain; *_pair_on are cta_group::2 (loads count their bytes on a barrier that may be the other CTA's;
+// the commit arrives at this shared-memory offset in every CTA of the mask, a signal, no data is copied).
+__device__ __forceinline__ void umma_f16_on(uint32_t on, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                            uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       :
-      : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(on)
       : "memory");
 }
-// When the MMAs issued so far have completed, arrive on the barrier at this shared-memory offset in every CTA of
-// `cta_mask` (an arrival signal sent to both CTAs of the pair; no data is copied).
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t cta_mask) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-                   smem_u32(bar)),
-               "h"(cta_mask)
-               : "memory");
+__device__ __forceinline__ void umma_f16_ts_on(uint32_t on, uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
+                                               uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      :
+      : "r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(on)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_on(uint32_t on, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+      :
+      : "r"(smem_u32(bar)), "r"(on)
+      : "memory");
+}
+__device__ __forceinline__ void umma_f16_pair_on(uint32_t on, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                                 uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      :
+      : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(on)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_pair_on(uint32_t on, uint64_t* bar, uint16_t cta_mask) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %2, 0;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+      :
+      : "r"(smem_u32(bar)), "h"(cta_mask), "r"(on)
+      : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_expect_tx_on(uint32_t on, uint64_t* bar, uint32_t bytes) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %2, 0;\n\t"
+      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)),
+      "r"(bytes), "r"(on)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_on(uint32_t on, const CUtensorMap* map, uint64_t* bar, void* dst, int c0, int c1) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
+      :
+      : "r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(on)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_pair_on(uint32_t on, const CUtensorMap* map, uint32_t bar_cluster_addr, void* dst,
+                                                    int c0, int c1) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
+      :
+      : "r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(on)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair_on(uint32_t on, const CUtensorMap* map, uint32_t bar_cluster_addr, void* dst,
+                                                    int c0, int c1, int c2) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "@q cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}"
+      :
+      : "r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2), "r"(on)
+      : "memory");
 }
 
 // ----------------------------------------------------------------------------- TMA stores (shared -> global)

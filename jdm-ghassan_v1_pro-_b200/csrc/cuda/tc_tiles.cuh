@@ -48,33 +48,34 @@ __device__ __forceinline__ void store_p_chunk(uint8_t* sP, int r, int c0, const 
   }
 }
 
+// Called by a whole warp: the lane with `on` issues.
 // TMA load of a [128 rows x HD] tile as HD/64 panels
 template <int HD>
-__device__ __forceinline__ void load_tile(const CUtensorMap* tm, uint64_t* bar, uint8_t* dst, int col0, int row0) {
+__device__ __forceinline__ void load_tile(uint32_t on, const CUtensorMap* tm, uint64_t* bar, uint8_t* dst, int col0, int row0) {
 #pragma unroll
-  for (int p = 0; p < HD / 64; ++p) tma_load_2d(tm, bar, dst + p * (AT_M * 128), col0 + 64 * p, row0);
+  for (int p = 0; p < HD / 64; ++p) tma_load_2d_on(on, tm, bar, dst + p * (AT_M * 128), col0 + 64 * p, row0);
 }
 
 // D[128 x N] (+)= A[128 x K] * B, all operands in the panelled SW128 layout.
 //   a_kmajor tile: K runs along the 64-column panels.   b_mn: B given as [K rows x N cols] (N contiguous).
 template <int KDIM>
-__device__ __forceinline__ void mma_kmajor_kmajor(uint32_t tmem_d, uint32_t sa, uint32_t sb, uint32_t idesc, bool accumulate) {
+__device__ __forceinline__ void mma_kmajor_kmajor(uint32_t on, uint32_t tmem_d, uint32_t sa, uint32_t sb, uint32_t idesc, bool accumulate) {
   // A: [128 x KDIM] K-major, B: [N x KDIM] K-major
 #pragma unroll
   for (int kk = 0; kk < KDIM / 16; ++kk) {
     const uint32_t off = (kk >> 2) * (AT_M * 128) + (kk & 3) * 32;
-    umma_f16(tmem_d, make_smem_desc_sw128(sa + off, 16, 1024), make_smem_desc_sw128(sb + off, 16, 1024), idesc,
+    umma_f16_on(on, tmem_d, make_smem_desc_sw128(sa + off, 16, 1024), make_smem_desc_sw128(sb + off, 16, 1024), idesc,
              (accumulate || kk > 0) ? 1u : 0u);
   }
 }
 template <int KDIM>
-__device__ __forceinline__ void mma_kmajor_mnmajor(uint32_t tmem_d, uint32_t sa, uint32_t sb, uint32_t idesc, bool accumulate) {
+__device__ __forceinline__ void mma_kmajor_mnmajor(uint32_t on, uint32_t tmem_d, uint32_t sa, uint32_t sb, uint32_t idesc, bool accumulate) {
   // A: [128 x KDIM] K-major (panels of 64 along K), B: [KDIM rows x N] with N contiguous (panels of 64 along N)
 #pragma unroll
   for (int kk = 0; kk < KDIM / 16; ++kk) {
     const uint32_t aoff = (kk >> 2) * (AT_M * 128) + (kk & 3) * 32;
     const uint32_t boff = kk * 2048;   // 16 rows of 128 bytes
-    umma_f16(tmem_d, make_smem_desc_sw128(sa + aoff, 16, 1024), make_smem_desc_sw128(sb + boff, AT_N * 128, 1024), idesc,
+    umma_f16_on(on, tmem_d, make_smem_desc_sw128(sa + aoff, 16, 1024), make_smem_desc_sw128(sb + boff, AT_N * 128, 1024), idesc,
              (accumulate || kk > 0) ? 1u : 0u);
   }
 }
