@@ -730,6 +730,22 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dq64_kernel(co
   if (warp == W_MMA) { tc_fence_after(); tmem_dealloc(tmem_base, 256); }
 }
 
+// First query position that sees none of the keys up to jl (>= jl itself): lo does not decrease along a sequence, so the queries
+// after the documents of a key tile are its tail.  Called by a whole warp; 32 probes a round, two rounds at T = 1024.
+__device__ __forceinline__ int at_query_end(const int* __restrict__ lo_seq, int T, int jl) {
+  const int lane = threadIdx.x & 31;
+  int a = jl + 1, e = T;                         // the answer lies in [a, e]
+  while (a < e) {
+    const int step = (e - a + 31) / 32, i = a + lane * step;
+    const unsigned after = __ballot_sync(0xffffffffu, i >= e || lo_seq[i] > jl);
+    const int n = after ? __ffs(after) - 1 : 32; // probes that still see key jl
+    if (n == 0) return a;
+    e = min(e, a + n * step);
+    a += (n - 1) * step + 1;
+  }
+  return e;
+}
+
 // ============================================================================================ backward: dK, dV
 // One CTA per (batch, kv head, 128 key rows).  Loops over the query heads that share the kv head and over the
 // query tiles at or after the key tile.  Per iteration: S^T = K Q^T and dP^T = V dO^T into tensor memory (rows =
@@ -789,13 +805,17 @@ __global__ void __launch_bounds__(AT_BWD_THREADS) attn_tc_bwd_dkv_kernel(const _
                  tmem_dK = tmem_base + 2 * AT_M + HD;
 
   // key tile and query tiles share the 128-row grid: the query tiles of an item start at its key tile
-  auto item_range = [&](int item, int& b, int& kvh, int& j0, int& n_qt) {
+  auto item_at = [&](int item, int& b, int& kvh, int& j0) {
     const int jt = item / BKV, bk = item - jt * BKV;
     b = bk / p.KV;
     kvh = bk - b * p.KV;
     j0 = jt * AT_N;
+  };
+  auto item_range = [&](int item, int& b, int& kvh, int& j0, int& n_qt) {
+    item_at(item, b, kvh, j0);
     int i_hi = p.T;
     if (p.window > 0) i_hi = min(p.T, j0 + AT_N - 1 + p.window);
+    if (p.lo) i_hi = min(i_hi, at_query_end(p.lo + (long long)b * p.T, p.T, min(p.T, j0 + AT_N) - 1));
     n_qt = (i_hi - j0 + AT_M - 1) / AT_M;
   };
 
@@ -869,22 +889,20 @@ __global__ void __launch_bounds__(AT_BWD_THREADS) attn_tc_bwd_dkv_kernel(const _
     // Per-query statistics of an iteration (log-sum-exp in log2 units, delta, first visible key), fetched by the four
     // cq == 0 warps (thread r = column r) one iteration ahead, the next item's first iteration included: the loads
     // of iteration n + 1 are in flight while iteration n is computed.
-    float n_lse = INFINITY, n_dl = 0.f;
-    int n_lo = 0x7fffffff;
+    // Nothing but the loads happens here: any arithmetic on them would wait for them, with every warp of the step behind
+    // that wait at the barrier below.
+    float n_lse = 0.f, n_dl = 0.f;
+    int n_lo = 0, n_i = 0;
     auto fetch_stats = [&](int b, int h, int i0) {
-      const int i = i0 + r;
-      const bool in = i < p.T;
-      const long long row = (long long)b * p.T + i;
-      n_lse = in ? p.lse[row * p.H + h] * LOG2E : INFINITY;
-      n_dl = in ? p.delta[row * p.H + h] * sc : 0.f;       // delta times the scale: dS = P (dP * scale - that)
-      int lo = 0;
-      if (in && p.lo) lo = p.lo[row];
-      if (in && p.window > 0) lo = max(lo, i - p.window + 1);
-      n_lo = in ? lo : 0x7fffffff;
+      n_i = i0 + r;
+      const long long row = (long long)b * p.T + min(n_i, p.T - 1);
+      n_lse = p.lse[row * p.H + h];
+      n_dl = p.delta[row * p.H + h];
+      if (p.lo) n_lo = p.lo[row];
     };
     if (cq == 0 && (int)blockIdx.x < n_items) {
-      int b, kvh, j0, n_qt;
-      item_range(blockIdx.x, b, kvh, j0, n_qt);
+      int b, kvh, j0;
+      item_at(blockIdx.x, b, kvh, j0);
       fetch_stats(b, kvh * group, j0);
     }
     for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++item_it) {
@@ -898,14 +916,15 @@ __global__ void __launch_bounds__(AT_BWD_THREADS) attn_tc_bwd_dkv_kernel(const _
         const int i0 = j0 + (it % n_qt) * AT_M;
         const int bufi = g_it & 1;
         if (cq == 0) {
-          sLse[bufi * AT_N + r] = n_lse;
-          sDl[bufi * AT_N + r] = n_dl;
-          sLo[bufi * AT_N + r] = n_lo;
+          const bool in = n_i < p.T;
+          sLse[bufi * AT_N + r] = in ? n_lse * LOG2E : INFINITY;
+          sDl[bufi * AT_N + r] = in ? n_dl * sc : 0.f;      // delta times the scale: dS = P (dP * scale - that)
+          sLo[bufi * AT_N + r] = !in ? 0x7fffffff : p.window > 0 ? max(n_lo, n_i - p.window + 1) : n_lo;
           if (it + 1 < n_it) {
             fetch_stats(b, kvh * group + (it + 1) / n_qt, j0 + ((it + 1) % n_qt) * AT_M);
           } else if (item + (int)gridDim.x < n_items) {
-            int b2, kvh2, j02, n_qt2;
-            item_range(item + gridDim.x, b2, kvh2, j02, n_qt2);
+            int b2, kvh2, j02;
+            item_at(item + gridDim.x, b2, kvh2, j02);
             fetch_stats(b2, kvh2 * group, j02);
           }
         }
@@ -1054,13 +1073,17 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
   const uint32_t tmem_ST = tmem_base, tmem_dPT = tmem_base + QN, tmem_dV = tmem_base + 2 * QN, tmem_dK = tmem_base + 2 * QN + HD;
 
   // the query steps of an item start at its key tile: n_qs steps of 64 queries for each head of the group
-  auto item_range = [&](int item, int& b, int& kvh, int& j0, int& n_qs) {
+  auto item_at = [&](int item, int& b, int& kvh, int& j0) {
     const int jt = item / BKV, bk = item - jt * BKV;
     b = bk / p.KV;
     kvh = bk - b * p.KV;
     j0 = jt * AT_N;
+  };
+  auto item_range = [&](int item, int& b, int& kvh, int& j0, int& n_qs) {
+    item_at(item, b, kvh, j0);
     int i_hi = p.T;
     if (p.window > 0) i_hi = min(p.T, j0 + AT_N - 1 + p.window);
+    if (p.lo) i_hi = min(i_hi, at_query_end(p.lo + (long long)b * p.T, p.T, min(p.T, j0 + AT_N) - 1));
     n_qs = (i_hi - j0 + QN - 1) / QN;
   };
 
@@ -1130,22 +1153,20 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
     bool ok = true;
     // statistics of the next step's 64 queries, fetched one step ahead by the first 64 compute threads
     const bool stat_thread = threadIdx.x < QN;
-    float n_lse = INFINITY, n_dl = 0.f;
-    int n_lo = 0x7fffffff;
+    // Nothing but the loads happens here: any arithmetic on them would wait for them, with every warp of the step behind
+    // that wait at the barrier below.
+    float n_lse = 0.f, n_dl = 0.f;
+    int n_lo = 0, n_i = 0;
     auto fetch_stats = [&](int b, int h, int i0) {
-      const int i = i0 + (int)threadIdx.x;
-      const bool in = i < p.T;
-      const long long row = (long long)b * p.T + i;
-      n_lse = in ? p.lse[row * p.H + h] * LOG2E : INFINITY;
-      n_dl = in ? p.delta[row * p.H + h] * sc : 0.f;       // delta times the scale: dS = P (dP * scale - that)
-      int lo = 0;
-      if (in && p.lo) lo = p.lo[row];
-      if (in && p.window > 0) lo = max(lo, i - p.window + 1);
-      n_lo = in ? lo : 0x7fffffff;
+      n_i = i0 + (int)threadIdx.x;
+      const long long row = (long long)b * p.T + min(n_i, p.T - 1);
+      n_lse = p.lse[row * p.H + h];
+      n_dl = p.delta[row * p.H + h];
+      if (p.lo) n_lo = p.lo[row];
     };
     if (stat_thread && (int)blockIdx.x < n_items) {
-      int b, kvh, j0, n_qs;
-      item_range(blockIdx.x, b, kvh, j0, n_qs);
+      int b, kvh, j0;
+      item_at(blockIdx.x, b, kvh, j0);
       fetch_stats(b, kvh * group, j0);
     }
     for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++item_it) {
@@ -1159,14 +1180,15 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
         const int i0 = j0 + (it % n_qs) * QN;
         const int bufi = g_it & 1;
         if (stat_thread) {
-          sLse[bufi * QN + threadIdx.x] = n_lse;
-          sDl[bufi * QN + threadIdx.x] = n_dl;
-          sLo[bufi * QN + threadIdx.x] = n_lo;
+          const bool in = n_i < p.T;
+          sLse[bufi * QN + threadIdx.x] = in ? n_lse * LOG2E : INFINITY;
+          sDl[bufi * QN + threadIdx.x] = in ? n_dl * sc : 0.f;      // delta times the scale: dS = P (dP * scale - that)
+          sLo[bufi * QN + threadIdx.x] = !in ? 0x7fffffff : p.window > 0 ? max(n_lo, n_i - p.window + 1) : n_lo;
           if (it + 1 < n_it) {
             fetch_stats(b, kvh * group + (it + 1) / n_qs, j0 + ((it + 1) % n_qs) * QN);
           } else if (item + (int)gridDim.x < n_items) {
-            int b2, kvh2, j02, n_qs2;
-            item_range(item + gridDim.x, b2, kvh2, j02, n_qs2);
+            int b2, kvh2, j02;
+            item_at(item + gridDim.x, b2, kvh2, j02);
             fetch_stats(b2, kvh2 * group, j02);
           }
         }
