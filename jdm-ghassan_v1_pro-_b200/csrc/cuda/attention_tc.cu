@@ -1016,7 +1016,15 @@ __global__ void __launch_bounds__(AT_BWD_THREADS) attn_tc_bwd_dkv_kernel(const _
 // ============================================================================================ backward: dK, dV (head_dim 64)
 // The same product in query steps of 64 instead of 128: S^T 64 + dP^T 64 + dV 64 + dK 64 = 256 tensor-memory columns
 // and under 100 KB of shared memory, so two CTAs of 8 compute warps share an SM (see the dQ kernel above for why).
-template <typename T>
+//
+// SPLIT: a cluster of H / KV CTAs per item, one query head each; their fp32 dV and dK are added through shared memory in the
+// order of the heads.  For passes whose items leave the chip idle: the item of the first key tile is a chain of H / KV times
+// all query steps (1 x 1000 tokens, 8/2 heads: 108 us whole, 29 split).
+//
+// What bounds it is the chain of a step (scores, exponentials, P^T and dS^T through shared memory, products).  The scores of the
+// next step are issued under the exponentials of this one and every warp fetches its own queries' statistics, so that no barrier
+// stands between the warps of a step: 296 -> 247 us (32 x 1024 packed tokens, 12/4 heads), 180 -> 148 us (16 x 1024).
+template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(const __grid_constant__ CUtensorMap tmQ,
                                                                            const __grid_constant__ CUtensorMap tmK,
                                                                            const __grid_constant__ CUtensorMap tmV,
@@ -1037,10 +1045,8 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
   uint8_t* sDST = sPT + TILE;
   uint8_t* sQ = sDST + TILE;                // ST
   uint8_t* sDO = sQ + ST * QTILE;           // ST
-  float* sLse = reinterpret_cast<float*>(sDO + ST * QTILE);   // [2][64]
-  float* sDl = sLse + 2 * QN;
-  int* sLo = reinterpret_cast<int*>(sDl + 2 * QN);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sLo + 2 * QN);
+  float* sStat = reinterpret_cast<float*>(sDO + ST * QTILE);  // per compute warp: log-sum-exp, delta, first visible key of its 32 queries
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + AT_DQ64_CW * 96);
   uint64_t* kv_full = bars;
   uint64_t* kv_empty = bars + 1;
   uint64_t* st_full = bars + 2;
@@ -1048,11 +1054,16 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
   uint64_t* dkv_full = bars + 4;
   uint64_t* q_full = bars + 5;              // ST
   uint64_t* q_empty = bars + 5 + ST;        // ST
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5 + 2 * ST);
+  uint64_t* st_empty = bars + 5 + 2 * ST;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6 + 2 * ST);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = p.H / p.KV;
+  const int n_heads = SPLIT ? 1 : group;                                     // heads that this CTA walks, from h0 of the group on
+  const int h0 = SPLIT ? (int)blockIdx.x % group : 0;
+  const int first = SPLIT ? (int)blockIdx.x / group : (int)blockIdx.x;       // SPLIT: one item per cluster
+  const int stride = SPLIT ? (int)gridDim.x / group : (int)gridDim.x;
   const int n_kt = (p.T + AT_N - 1) / AT_N, BKV = p.B * p.KV;
   const int n_items = n_kt * BKV;
   if (threadIdx.x == 0) {
@@ -1060,6 +1071,7 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
     mbar_init(kv_empty, 1);
     mbar_init(st_full, 1);
     mbar_init(pt_ready, AT_DQ64_CW);
+    mbar_init(st_empty, AT_DQ64_CW);
     mbar_init(dkv_full, 1);
     for (int s = 0; s < ST; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1); }
     *abort_flag = 0;
@@ -1091,7 +1103,7 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
     {
       const uint32_t on = elect_one();
       uint32_t g_it = 0, item_it = 0;
-      for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++item_it) {
+      for (int item = first; item < n_items; item += stride, ++item_it) {
         int b, kvh, j0, n_qs;
         item_range(item, b, kvh, j0, n_qs);
         const int row_base = b * p.T;
@@ -1099,15 +1111,16 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
         mbar_arrive_expect_tx_on(on, kv_full, 2 * TILE);
         load_tile<HD>(on, &tmK, kv_full, sK, kvh * HD, row_base + j0);
         load_tile<HD>(on, &tmV, kv_full, sV, kvh * HD, row_base + j0);
-        const int n_it = group * n_qs;
+        const int n_it = n_heads * n_qs;
+        int h = kvh * group + h0, qi = 0;
         for (int it = 0; it < n_it; ++it, ++g_it) {
           const int s = g_it % ST, ph = (g_it / ST) & 1;
-          const int h = kvh * group + it / n_qs;
-          const int i0 = j0 + (it % n_qs) * QN;
+          const int i0 = j0 + qi * QN;
           wait_or_report(&q_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
           mbar_arrive_expect_tx_on(on, &q_full[s], 2 * QTILE);
           tma_load_2d_on(on, &tmQ, &q_full[s], sQ + s * QTILE, h * HD, row_base + i0);
           tma_load_2d_on(on, &tmDO, &q_full[s], sDO + s * QTILE, h * HD, row_base + i0);
+          if (++qi == n_qs) { qi = 0; ++h; }
         }
       }
     }
@@ -1119,19 +1132,29 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
       const uint32_t idesc_s = make_idesc_f16(fmt, 0, 0, AT_N, QN);
       const uint32_t idesc_d = make_idesc_f16(fmt, 0, 1, AT_N, HD);
       uint32_t g_it = 0, item_it = 0;
-      for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++item_it) {
+      for (int item = first; item < n_items; item += stride, ++item_it) {
         int b, kvh, j0, n_qs;
         item_range(item, b, kvh, j0, n_qs);
         wait_or_report(kv_full, item_it & 1u, p.status, ST_TIMEOUT_FULL, abort_flag);
-        const int n_it = group * n_qs;
-        for (int it = 0; it < n_it; ++it, ++g_it) {
-          const int s = g_it % ST, ph = (g_it / ST) & 1;
-          wait_or_report(&q_full[s], ph, p.status, ST_TIMEOUT_FULL, abort_flag);
+        const int n_it = n_heads * n_qs;
+        // S^T and dP^T of step n + 1 are issued as soon as the compute warps have read those of step n, before P^T and dS^T of step n
+        // are waited for: their round trip runs under the exponentials
+        auto scores = [&](uint32_t g, bool last) {
+          const int s = g % ST;
+          wait_or_report(&q_full[s], (g / ST) & 1, p.status, ST_TIMEOUT_FULL, abort_flag);
           tc_fence_after();
           mma_kmajor_kmajor<HD>(on, tmem_ST, smem_u32(sK), smem_u32(sQ + s * QTILE), idesc_s, false);
           mma_kmajor_kmajor<HD>(on, tmem_dPT, smem_u32(sV), smem_u32(sDO + s * QTILE), idesc_s, false);
           umma_commit_on(on, st_full);
-          if (it == n_it - 1) umma_commit_on(on, kv_empty);
+          if (last) umma_commit_on(on, kv_empty);
+        };
+        scores(g_it, n_it == 1);
+        for (int it = 0; it < n_it; ++it, ++g_it) {
+          const int s = g_it % ST;
+          if (it + 1 < n_it) {
+            wait_or_report(st_empty, g_it & 1u, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag);
+            scores(g_it + 1, it + 2 == n_it);
+          }
           wait_or_report(pt_ready, g_it & 1u, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag);
           tc_fence_after();
           mma_kmajor_mnmajor<QN>(on, tmem_dV, smem_u32(sPT), smem_u32(sDO + s * QTILE), idesc_d, it > 0);
@@ -1151,103 +1174,105 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
     constexpr float LOG2E = 1.4426950408889634f;
     uint32_t g_it = 0, item_it = 0;
     bool ok = true;
-    // statistics of the next step's 64 queries, fetched one step ahead by the first 64 compute threads
-    const bool stat_thread = threadIdx.x < QN;
-    // Nothing but the loads happens here: any arithmetic on them would wait for them, with every warp of the step behind
-    // that wait at the barrier below.
+    // statistics of this warp's 32 queries of the next step, one query a lane, fetched one step ahead.  Nothing but the loads
+    // happens at the fetch: any arithmetic on them would wait for them.
+    float* lse = sStat + warp * 96;
+    float* dl = lse + 32;
+    int* lo = reinterpret_cast<int*>(dl + 32);
     float n_lse = 0.f, n_dl = 0.f;
     int n_lo = 0, n_i = 0;
     auto fetch_stats = [&](int b, int h, int i0) {
-      n_i = i0 + (int)threadIdx.x;
+      n_i = i0 + cq * 32 + lane;
       const long long row = (long long)b * p.T + min(n_i, p.T - 1);
       n_lse = p.lse[row * p.H + h];
       n_dl = p.delta[row * p.H + h];
       if (p.lo) n_lo = p.lo[row];
     };
-    if (stat_thread && (int)blockIdx.x < n_items) {
+    if (first < n_items) {
       int b, kvh, j0;
-      item_at(blockIdx.x, b, kvh, j0);
-      fetch_stats(b, kvh * group, j0);
+      item_at(first, b, kvh, j0);
+      fetch_stats(b, kvh * group + h0, j0);
     }
-    for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++item_it) {
+    for (int item = first; item < n_items && ok; item += stride, ++item_it) {
       int b, kvh, j0, n_qs;
       item_range(item, b, kvh, j0, n_qs);
       const long long row_base = (long long)b * p.T;
       const int j = j0 + r;
       const bool row_ok = j < p.T;
-      const int n_it = group * n_qs;
+      const int n_it = n_heads * n_qs;
+      int h = kvh * group + h0, qi = 0;
       for (int it = 0; it < n_it; ++it, ++g_it) {
-        const int i0 = j0 + (it % n_qs) * QN;
-        const int bufi = g_it & 1;
-        if (stat_thread) {
-          const bool in = n_i < p.T;
-          sLse[bufi * QN + threadIdx.x] = in ? n_lse * LOG2E : INFINITY;
-          sDl[bufi * QN + threadIdx.x] = in ? n_dl * sc : 0.f;      // delta times the scale: dS = P (dP * scale - that)
-          sLo[bufi * QN + threadIdx.x] = !in ? 0x7fffffff : p.window > 0 ? max(n_lo, n_i - p.window + 1) : n_lo;
-          if (it + 1 < n_it) {
-            fetch_stats(b, kvh * group + (it + 1) / n_qs, j0 + ((it + 1) % n_qs) * QN);
-          } else if (item + (int)gridDim.x < n_items) {
-            int b2, kvh2, j02;
-            item_at(item + gridDim.x, b2, kvh2, j02);
-            fetch_stats(b2, kvh2 * group, j02);
-          }
+        const int i0 = j0 + qi * QN + cq * 32;             // first of this warp's queries
+        __syncwarp();                                      // the previous step's statistics have been read
+        const bool in = n_i < p.T;
+        lse[lane] = in ? n_lse * LOG2E : INFINITY;
+        dl[lane] = in ? n_dl * sc : 0.f;                   // delta times the scale: dS = P (dP * scale - that)
+        lo[lane] = !in ? 0x7fffffff : p.window > 0 ? max(n_lo, n_i - p.window + 1) : n_lo;
+        __syncwarp();
+        if (++qi == n_qs) { qi = 0; ++h; }
+        if (it + 1 < n_it) {
+          fetch_stats(b, h, j0 + qi * QN);
+        } else if (item + stride < n_items) {
+          int b2, kvh2, j02;
+          item_at(item + stride, b2, kvh2, j02);
+          fetch_stats(b2, kvh2 * group + h0, j02);
         }
-        asm volatile("bar.sync 1, 256;" ::: "memory");   // all AT_DQ64_CW * 32 compute threads
-        // after a failed wait the loops keep running (without waiting or computing) so that every thread still
-        // reaches the named barrier above in every step
-        if (ok && !at_wait(st_full, g_it & 1u, p.status, ST_TIMEOUT_TMEM_FULL, abort_flag)) ok = false;
-        if (!ok) continue;
+        if (!at_wait(st_full, g_it & 1u, p.status, ST_TIMEOUT_TMEM_FULL, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const float* lse = sLse + bufi * QN;
-        const float* dl = sDl + bufi * QN;
-        const int* lo = sLo + bufi * QN;
-        // every (key, query) pair of the step visible: queries after the whole key tile, whole tiles, and the largest
-        // `lo` of the step (its last query) at or before the first key
-        const bool full = i0 >= j0 + AT_N && j0 + AT_N <= p.T && i0 + QN <= p.T && lo[QN - 1] <= j0;
+        // every (key, query) pair of the warp visible: queries after the whole key tile, whole tiles, and the largest
+        // `lo` of the queries (the last one's) at or before the first key
+        const bool full = i0 >= j0 + AT_N && j0 + AT_N <= p.T && i0 + 32 <= p.T && lo[31] <= j0;
         uint32_t rs[32], rp[32];
         tmem_ld_32x32(tmem_ST + lane_base + cq * 32, rs);
         tmem_ld_32x32(tmem_dPT + lane_base + cq * 32, rp);
         tmem_ld_wait();
-        float pt[32], ds[32];
-        // the statistics of this warp's 32 queries come as 16-byte loads (every lane reads the same words), four
-        // queries at a time
+        tc_fence_before();
+        if (lane == 0) mbar_arrive(st_empty);
+        // the statistics come as 16-byte loads (every lane reads the same words), four queries at a time; P and dS are
+        // packed as they come, in place of the scores
 #pragma unroll
         for (int k4 = 0; k4 < 8; ++k4) {
-          const float4 a4 = reinterpret_cast<const float4*>(lse + cq * 32)[k4];
-          const float4 d4 = reinterpret_cast<const float4*>(dl + cq * 32)[k4];
+          const float4 a4 = reinterpret_cast<const float4*>(lse)[k4];
+          const float4 d4 = reinterpret_cast<const float4*>(dl)[k4];
           const float lv[4] = {a4.x, a4.y, a4.z, a4.w};
           const float dv[4] = {d4.x, d4.y, d4.z, d4.w};
+          float pt[4], ds[4];
           if (full) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const int k = 4 * k4 + e;
-              const float pr = exp2f(fmaf(__uint_as_float(rs[k]), sc2, -lv[e]));
-              pt[k] = pr;
-              ds[k] = pr * fmaf(__uint_as_float(rp[k]), sc, -dv[e]);
+              pt[e] = exp2f(fmaf(__uint_as_float(rs[k]), sc2, -lv[e]));
+              ds[e] = pt[e] * fmaf(__uint_as_float(rp[k]), sc, -dv[e]);
             }
           } else {
-            const int4 l4 = reinterpret_cast<const int4*>(lo + cq * 32)[k4];
+            const int4 l4 = reinterpret_cast<const int4*>(lo)[k4];
             const int lov[4] = {l4.x, l4.y, l4.z, l4.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const int k = 4 * k4 + e;
-              const int i = i0 + cq * 32 + k;
-              const bool vis = row_ok && j <= i && j >= lov[e];
-              const float pr = vis ? exp2f(fmaf(__uint_as_float(rs[k]), sc2, -lv[e])) : 0.f;
-              pt[k] = pr;
-              ds[k] = pr * fmaf(__uint_as_float(rp[k]), sc, -dv[e]);
+              const bool vis = row_ok && j <= i0 + k && j >= lov[e];
+              pt[e] = vis ? exp2f(fmaf(__uint_as_float(rs[k]), sc2, -lv[e])) : 0.f;
+              ds[e] = pt[e] * fmaf(__uint_as_float(rp[k]), sc, -dv[e]);
             }
           }
+          rs[2 * k4] = Cvt<T>::pack2(pt[0], pt[1]);
+          rs[2 * k4 + 1] = Cvt<T>::pack2(pt[2], pt[3]);
+          rp[2 * k4] = Cvt<T>::pack2(ds[0], ds[1]);
+          rp[2 * k4 + 1] = Cvt<T>::pack2(ds[2], ds[3]);
         }
-        store_p_chunk<T>(sPT, r, cq * 32, pt);
-        store_p_chunk<T>(sDST, r, cq * 32, ds);
-        tc_fence_before();
+        // dV and dK of the previous step have read the buffers (they free that step's Q and dO)
+        if (g_it > 0 && !at_wait(&q_empty[(g_it - 1) % ST], ((g_it - 1) / ST) & 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag)) { ok = false; break; }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t at = sw128_off(r, cq * 32 + 8 * k);
+          *reinterpret_cast<uint4*>(sPT + at) = make_uint4(rs[4 * k], rs[4 * k + 1], rs[4 * k + 2], rs[4 * k + 3]);
+          *reinterpret_cast<uint4*>(sDST + at) = make_uint4(rp[4 * k], rp[4 * k + 1], rp[4 * k + 2], rp[4 * k + 3]);
+        }
         fence_proxy_async();
         __syncwarp();                 // every lane's writes and fences, then one arrival for the warp
         if (lane == 0) mbar_arrive(pt_ready);
       }
-      if (ok && !at_wait(dkv_full, item_it & 1u, p.status, ST_TIMEOUT_TMEM_FULL, abort_flag)) ok = false;
-      if (!ok) continue;
+      if (!ok || !at_wait(dkv_full, item_it & 1u, p.status, ST_TIMEOUT_TMEM_FULL, abort_flag)) { ok = false; break; }
       tc_fence_after();
       T* dkp = reinterpret_cast<T*>(p.dk) + (row_base + j) * p.ld_dk + (long long)kvh * HD;
       T* dvp = reinterpret_cast<T*>(p.dv) + (row_base + j) * p.ld_dv + (long long)kvh * HD;
@@ -1255,7 +1280,18 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
       tmem_ld_32x32(tmem_dV + lane_base + cq * 32, rv);
       tmem_ld_32x32(tmem_dK + lane_base + cq * 32, rk);
       tmem_ld_wait();
-      if (row_ok) {
+      if constexpr (SPLIT) {
+        // every product has been taken: the operand buffers hold the partial sums, [16 chunks of 8 columns: dV, dK][128 rows]
+        float4* part = reinterpret_cast<float4*>(sPT);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int at = ((cq * 4 + (k >> 1)) * AT_N + r) * 2 + (k & 1);
+          part[at] = make_float4(__uint_as_float(rv[4 * k]), __uint_as_float(rv[4 * k + 1]), __uint_as_float(rv[4 * k + 2]),
+                                 __uint_as_float(rv[4 * k + 3]));
+          part[at + 8 * AT_N * 2] = make_float4(__uint_as_float(rk[4 * k]), __uint_as_float(rk[4 * k + 1]),
+                                                __uint_as_float(rk[4 * k + 2]), __uint_as_float(rk[4 * k + 3]));
+        }
+      } else if (row_ok) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           uint4 qv, qk;
@@ -1278,6 +1314,35 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
   if (*abort_flag) {
     for (int k = 0; k < 64; ++k) __nanosleep(1000);
     __syncthreads();
+  }
+  if constexpr (SPLIT) {
+    cluster_sync_all();
+    int b, kvh, j0;
+    item_at(first, b, kvh, j0);
+    // (chunk, row) pairs of 8 values, every group-th chunk of 128 rows to this CTA
+    for (int u = threadIdx.x; u < 16 * AT_N; u += AT_DQ64_THREADS) {
+      const int c = u / AT_N, r = u % AT_N, j = j0 + r;
+      if (c % group != h0 || j >= p.T) continue;
+      float v[8] = {};
+      for (int g = 0; g < group; ++g) {
+        const uint32_t src = mapa_shared(smem_u32(sPT) + (uint32_t)u * 32, (uint32_t)g);
+        float4 x, y;
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(src) : "memory");
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(y.x), "=f"(y.y), "=f"(y.z), "=f"(y.w) : "r"(src + 16) : "memory");
+        v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
+        v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
+      }
+      const long long row = (long long)b * p.T + j;
+      T* dst = c < 8 ? reinterpret_cast<T*>(p.dv) + row * p.ld_dv + (long long)kvh * HD + c * 8
+                     : reinterpret_cast<T*>(p.dk) + row * p.ld_dk + (long long)kvh * HD + (c - 8) * 8;
+      uint4 q;
+      q.x = Cvt<T>::pack2(v[0], v[1]);
+      q.y = Cvt<T>::pack2(v[2], v[3]);
+      q.z = Cvt<T>::pack2(v[4], v[5]);
+      q.w = Cvt<T>::pack2(v[6], v[7]);
+      *reinterpret_cast<uint4*>(dst) = q;
+    }
+    cluster_sync_all();                          // the other CTAs have read this one's shared memory
   }
   if (warp == W_MMA) { tc_fence_after(); tmem_dealloc(tmem_base, 256); }
 }
@@ -1477,8 +1542,32 @@ int launch_tc_bwd(const gb_attn_args* a, int* lo, int* status, cudaStream_t st) 
     CUtensorMap tq64, tdo64;
     if (gb_make_tmap_2d_16b(&tq64, a->q, rows, (uint64_t)a->H * HD, a->ld_q, 64, 64, a->is_bf16)) return -20;
     if (gb_make_tmap_2d_16b(&tdo64, a->d_o, rows, (uint64_t)a->H * HD, a->ld_do, 64, 64, a->is_bf16)) return -23;
-    auto kkv64 = attn_tc_bwd_dkv64_kernel<T>;
-    constexpr size_t smem_kv64 = TILE * 4 + (size_t)64 * HD * 2 * 2 * 2 + 6 * 64 * 4 + 128;
+    constexpr size_t smem_kv64 = TILE * 4 + (size_t)64 * HD * 2 * 2 * 2 + AT_DQ64_CW * 96 * 4 + 128;
+    const int group = a->H / a->KV;
+    // An item for every SM or fewer: a cluster per item.  Between one and two items per SM, whole items are the faster (192 items of
+    // 512 tokens, 12/4 heads: 49 against 58 us; 128 items: 44 against 42 at 512 tokens, 152 against 82 at 2048).
+    if (group >= 2 && group <= 8 && items_kv <= sms) {
+      auto ks = attn_tc_bwd_dkv64_kernel<T, true>;
+      static bool attr_s = false;
+      if (!attr_s) {
+        if (cudaFuncSetAttribute(ks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv64) != cudaSuccess) return -10;
+        (void)cudaFuncSetAttribute(ks, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        attr_s = true;
+      }
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)(items_kv * group), 1, 1);
+      cfg.blockDim = dim3(AT_DQ64_THREADS, 1, 1);
+      cfg.dynamicSmemBytes = smem_kv64;
+      cfg.stream = st;
+      cudaLaunchAttribute at;
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = (unsigned)group; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      if (cudaLaunchKernelEx(&cfg, ks, tq64, tk, tv, tdo64, p) != cudaSuccess) return -10;
+      return gb_launch_rc();
+    }
+    auto kkv64 = attn_tc_bwd_dkv64_kernel<T, false>;
     static bool attr_kv64 = false;
     if (!attr_kv64) {
       if (cudaFuncSetAttribute(kkv64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv64) != cudaSuccess) return -10;

@@ -149,3 +149,21 @@ def test_tc_attention_leading_negative_segment_ids():
     ref = R.attention(q.float().view(n, H, hd), k.float().view(n, KV, hd), v.float().view(n, KV, hd), B, T, scale, 0, seg)
     ok, err, rule = near(o, ref)
     assert ok, ("o", err, rule)
+
+
+# dK/dV: a cluster per item where there are no more items (key tiles x sequences x kv heads) than SMs, whole items beyond; query steps of
+# 64 that end with the key tile's documents; one to eight query heads per kv head
+ITEM_CASES = [
+    (1, 1000, 8, 1, 64, 0, True),
+    (1, 129, 3, 1, 64, 0, False),
+    (37, 128, 12, 4, 64, 0, True),      # 148 items: the last of the clusters
+    (30, 130, 12, 4, 64, 0, True),      # 240: whole, a key tile of two rows
+    (7, 600, 12, 6, 64, 200, True),
+    (2, 700, 6, 2, 128, 0, True),
+]
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("B,T,H,KV,hd,window,use_seg", ITEM_CASES)
+def test_tc_attention_at_item_edges(dt, B, T, H, KV, hd, window, use_seg):
+    test_tc_attention_matches_oracle(dt, B, T, H, KV, hd, window, use_seg)
