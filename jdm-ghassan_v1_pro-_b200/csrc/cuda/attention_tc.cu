@@ -1,15 +1,20 @@
 // Causal flash attention on the 5th-generation tensor cores (tcgen05 + TMEM + TMA), head_dim 64 or 128.
 //
 // Forward, one CTA per (batch, head, 128 query rows):
-//   warp 4 : TMA producer  - Q tile once, then K/V tiles of 128 keys through a 2-stage ring
-//   warp 5 : MMA issuer    - S = Q K^T into tensor memory, then O_part = P V (P read from shared memory)
-//   warps 0-3 (one thread per query row): tcgen05.ld of S, scale + causal/window/segment mask, online softmax,
-//            P (16-bit) written to shared memory in the 128-byte-swizzled operand layout, O rescaled and
-//            accumulated in registers, final normalisation, O and log-sum-exp stored.
+//   warp 8 : TMA producer  - Q tile once, then K/V tiles of 128 keys through a 2-stage ring
+//   warp 9 : MMA issuer    - S = Q K^T into tensor memory, then O += P V (P read from shared memory)
+//   warps 0-7 (two threads per query row): tcgen05.ld of S, scale + causal/window/segment mask, online softmax,
+//            P (16-bit) written to shared memory in the 128-byte-swizzled operand layout, O rescaled in tensor memory where a
+//            maximum has grown, final normalisation, O and log-sum-exp stored.
 // The backward pass (further down) uses the same tile machinery: a dQ kernel per query tile and a dK/dV kernel
 // per key tile that loops over the query heads of its group, both recomputing P from the saved log-sum-exp.
 // Scores are never written to global memory (the reference materialises B*H*T^2 floats and re-runs the forward
 // in its backward, cuda/attention.cu:297-550, 805-898).
+//
+// The forward is bound by the latencies of a tile's chain (scores, maximum, exponentials, P through shared memory, P V): with one
+// thread per row that read its scores twice and let the next scores wait for P, issue slots were busy 35 % of the time.  Two
+// threads a row with the scores in registers, next scores issued at once: 93 -> 71 us (16 x 1024 tokens, 12/4 heads), 186 -> 103
+// (32 x 1024 in documents of 397: visibility is one bit per key), 37 -> 28 (16 x 512), 23 -> 18 (1 x 1000).
 //
 // Segment masks are passed as `lo[i]` = first key position visible to query i (start of its packed document,
 // or 0): visible(i, j) <=> max(lo[i], i - window + 1) <= j <= i.  Every wait is bounded (status word on expiry).
@@ -22,7 +27,8 @@
 
 namespace gb {
 
-constexpr int AT_THREADS = 192;
+constexpr int AT_FWD_CW = 8;     // soft-max warps of the forward kernel; then the TMA producer and the MMA issuer
+constexpr int AT_THREADS = (AT_FWD_CW + 2) * 32;
 // Backward kernels: sixteen compute warps.  Warp w owns the 32 tile rows of TMEM lane quarter w % 4 and the 32-column
 // chunk w / 4, so a 128 x 128 score tile is one tcgen05.ld per thread and every scheduler has four warps to switch
 // between (with four compute warps in all, the exp / multiply / pack chain of a tile ran at one warp per scheduler
@@ -47,7 +53,7 @@ struct AttnTcParams {
 
 // ============================================================================================ forward
 template <typename T, int HD>
-__global__ void __launch_bounds__(AT_THREADS) attn_tc_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
+__global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1) attn_tc_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
                                                                  const __grid_constant__ CUtensorMap tmK,
                                                                  const __grid_constant__ CUtensorMap tmV,
                                                                  const AttnTcParams p) {
@@ -55,7 +61,7 @@ __global__ void __launch_bounds__(AT_THREADS) attn_tc_fwd_kernel(const __grid_co
   constexpr uint32_t TILE = AT_M * HD * 2;
   uint8_t* smem;
   if constexpr (HD == 64) {
-    // 112 KB of tiles + barriers and not a byte more: two CTAs of this kernel share an SM (143 registers, 256 TMEM
+    // 112 KB of tiles, 640 bytes of barriers and maxima and not a byte more: two CTAs of this kernel share an SM (256 TMEM
     // columns each), which hides the latency of the short causal loops at T = 512.  That leaves no slack to align
     // the base by hand; the kernel has no static shared memory, so the dynamic window starts 1024-aligned.  Checked,
     // not assumed: a misaligned base reports and returns before any barrier or TMEM is touched.
@@ -79,8 +85,10 @@ __global__ void __launch_bounds__(AT_THREADS) attn_tc_fwd_kernel(const __grid_co
   uint64_t* p_ready = bars + 6;
   uint64_t* o_full = bars + 7;
   uint64_t* q_empty = bars + 8;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
+  uint64_t* s_empty = bars + 9;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  __nv_bfloat16* row_max = reinterpret_cast<__nv_bfloat16*>(bars + 16);     // [2 halves][128 rows]; between items 128 floats
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Work items: (query tile, batch, head), the query tile slowest and from the last one down: under a causal mask that
@@ -97,12 +105,13 @@ __global__ void __launch_bounds__(AT_THREADS) attn_tc_fwd_kernel(const __grid_co
     mbar_init(q_empty, 1);
     for (int s = 0; s < 2; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 1); }
     mbar_init(s_full, 1);
-    mbar_init(p_ready, 4);             // one arrival per soft-max warp
+    mbar_init(p_ready, AT_FWD_CW);     // one arrival per soft-max warp
+    mbar_init(s_empty, AT_FWD_CW);
     mbar_init(o_full, 1);
     *abort_flag = 0;
     fence_barrier_init();
   }
-  if (warp == 5) { tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
+  if (warp == AT_FWD_CW + 1) { tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -123,7 +132,7 @@ __global__ void __launch_bounds__(AT_THREADS) attn_tc_fwd_kernel(const __grid_co
     n_tiles = (k_hi - k_lo + AT_N - 1) / AT_N;
   };
 
-  if (warp == 4) {
+  if (warp == AT_FWD_CW) {
     {
       const uint32_t on = elect_one();
       uint32_t kv_it = 0, q_it = 0;
@@ -146,7 +155,7 @@ __global__ void __launch_bounds__(AT_THREADS) attn_tc_fwd_kernel(const __grid_co
       }
     }
     __syncwarp();
-  } else if (warp == 5) {
+  } else if (warp == AT_FWD_CW + 1) {
     {
       const uint32_t on = elect_one();
       constexpr int fmt = OperandFmt<T>::value;
@@ -157,14 +166,23 @@ __global__ void __launch_bounds__(AT_THREADS) attn_tc_fwd_kernel(const __grid_co
         int b, h, q0, k_lo, n_tiles;
         item_range(item, b, h, q0, k_lo, n_tiles);
         wait_or_report(q_full, q_it & 1u, p.status, ST_TIMEOUT_FULL, abort_flag);
-        for (int t = 0; t < n_tiles; ++t, ++kv_it) {
-          const int s = kv_it & 1, ph = (kv_it >> 1) & 1;
-          wait_or_report(&kv_full[s], ph, p.status, ST_TIMEOUT_FULL, abort_flag);
+        // the scores of tile t + 1 are issued as soon as the soft-max warps have those of tile t in registers, before the
+        // probabilities of tile t are waited for: their round trip runs under the exponentials
+        auto scores = [&](uint32_t g, bool last) {
+          const int s = g & 1;
+          wait_or_report(&kv_full[s], (g >> 1) & 1, p.status, ST_TIMEOUT_FULL, abort_flag);
           tc_fence_after();
-          // S(t) may overwrite S(t-1) only after the softmax threads have read it: p_ready(t-1) was waited below
           mma_kmajor_kmajor<HD>(on, tmem_S, smem_u32(sQ), smem_u32(sK + s * TILE), idesc_s, false);
           umma_commit_on(on, s_full);
-          if (t == n_tiles - 1) umma_commit_on(on, q_empty);
+          if (last) umma_commit_on(on, q_empty);
+        };
+        scores(kv_it, n_tiles == 1);
+        for (int t = 0; t < n_tiles; ++t, ++kv_it) {
+          const int s = kv_it & 1;
+          if (t + 1 < n_tiles) {
+            wait_or_report(s_empty, kv_it & 1u, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag);
+            scores(kv_it + 1, t + 2 == n_tiles);
+          }
           wait_or_report(p_ready, kv_it & 1u, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag);
           tc_fence_after();
           mma_kmajor_mnmajor<AT_N>(on, tmem_O, smem_u32(sP), smem_u32(sV + s * TILE), idesc_o, t > 0);
@@ -175,17 +193,18 @@ __global__ void __launch_bounds__(AT_THREADS) attn_tc_fwd_kernel(const __grid_co
     }
     __syncwarp();
   } else {
-    // Soft-max warps, one thread per query row.  The output accumulates in tensor memory over the key tiles of an item
+    // Soft-max warps: two threads per query row, each with 64 of a tile's keys in registers (warps w and w + 4 share a TMEM lane
+    // quarter) and half of the output columns.  The output accumulates in tensor memory over the key tiles of an item
     // (the P V product adds to it), so a thread touches it only at the end of the item, and in the rare tile where the
     // running maximum of a row of its warp has grown by more than 2^8: only then are the accumulator rows rescaled
     // (until then the probabilities are taken against the older, smaller maximum, at most 256 times larger than with the
     // true one; the final division by the row sum, kept against the same maximum, is exact either way).
-    const int r = threadIdx.x;                  // query row of the tile
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+    const int half = warp >> 2, r = (warp & 3) * 32 + lane;                  // key half, query row of the tile
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const float sc2 = p.scale * 1.4426950408889634f;       // scores in log2 units: exp(x * scale) = 2^(x * sc2)
+    auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"((warp & 3) + 1) : "memory"); };   // the two warps of a quarter
     uint32_t tile_it = 0;
-    bool ok = true;
-    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+    for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
       int b, h, q0, k_lo, n_tiles;
       item_range(item, b, h, q0, k_lo, n_tiles);
       const long long row_base = (long long)b * p.T;
@@ -196,115 +215,130 @@ __global__ void __launch_bounds__(AT_THREADS) attn_tc_fwd_kernel(const __grid_co
         if (p.lo) lo_i = p.lo[row_base + i];
         if (p.window > 0) lo_i = max(lo_i, i - p.window + 1);
       }
-      float m2 = -INFINITY, l = 0.f;            // maximum in use (log2 units) and the row sum against it
+      float m2 = -INFINITY, l = 0.f;            // maximum in use (log2 units) and this half's row sum against it
       for (int t = 0; t < n_tiles; ++t, ++tile_it) {
-        const int j0 = k_lo + t * AT_N;
-        if (!at_wait(s_full, tile_it & 1u, p.status, ST_TIMEOUT_TMEM_FULL, abort_flag)) { ok = false; break; }
+        const int j0 = k_lo + t * AT_N + half * 64;
+        // (a wait that fails reports and the loops go on, on whatever is there: both warps of a quarter reach their barriers)
+        wait_or_report(s_full, tile_it & 1u, p.status, ST_TIMEOUT_TMEM_FULL, abort_flag);
         tc_fence_after();
-        const bool need_mask = (j0 + AT_N - 1 > q0) || (j0 < lo_i);
-        // pass A: row maximum of the raw scores (the scale is positive: checked by the launcher)
-        float mr[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll 1
-        for (int c = 0; c < AT_N / 32; ++c) {
-          uint32_t rg[32];
-          tmem_ld_32x32(tmem_S + lane_base + c * 32, rg);
+        uint32_t r0[32], r1[32];
+        float mt;
+        {
+          tmem_ld_32x32(tmem_S + lane_base + half * 64, r0);
+          tmem_ld_32x32(tmem_S + lane_base + half * 64 + 32, r1);
           tmem_ld_wait();
-          if (!need_mask) {
-#pragma unroll
-            for (int k = 0; k < 32; ++k) mr[k & 3] = fmaxf(mr[k & 3], __uint_as_float(rg[k]));
-          } else {
+          if (!row_ok || j0 + 63 > q0 || j0 < lo_i) {
+            // the visible keys of a row are contiguous: one bit each
+            const int a0 = min(max(lo_i - j0, 0), 64), a1 = row_ok ? min(max(i - j0 + 1, 0), 64) : 0;      // [a0, a1)
+            const unsigned long long vis = a1 > a0 ? (~0ull >> (64 - (a1 - a0))) << a0 : 0ull;
+            const uint32_t v0 = (uint32_t)vis, v1 = (uint32_t)(vis >> 32);
 #pragma unroll
             for (int k = 0; k < 32; ++k) {
-              const int j = j0 + c * 32 + k;
-              if (j <= i && j >= lo_i) mr[k & 3] = fmaxf(mr[k & 3], __uint_as_float(rg[k]));
+              if (!(v0 >> k & 1u)) r0[k] = 0xff800000u;     // -inf
+              if (!(v1 >> k & 1u)) r1[k] = 0xff800000u;
             }
           }
+          // row maximum of the raw scores (the scale is positive: checked by the launcher)
+          float mr[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+          for (int k = 0; k < 32; ++k) mr[k & 3] = fmaxf(mr[k & 3], fmaxf(__uint_as_float(r0[k]), __uint_as_float(r1[k])));
+          mt = fmaxf(fmaxf(mr[0], mr[1]), fmaxf(mr[2], mr[3])) * sc2;
         }
-        float mt = fmaxf(fmaxf(mr[0], mr[1]), fmaxf(mr[2], mr[3])) * sc2;
-        if (!row_ok) mt = 0.f;
+        // The halves meet: any number that both use will do as the maximum, so it travels rounded up to 16 bits.
+        const __nv_bfloat16 m16 = __float2bfloat16_ru(mt);
+        row_max[half * AT_M + r] = m16;
+        pair_sync();
+        mt = fmaxf(__bfloat162float(m16), __bfloat162float(row_max[(half ^ 1) * AT_M + r]));
+        tc_fence_before();
+        if (lane == 0) mbar_arrive(s_empty);    // scores and the partner's maximum are in registers
         // a new maximum is taken when some row of the warp needs it (the accumulator rows are reached by warp-wide
-        // tensor-memory loads and stores, so the decision is the warp's)
+        // tensor-memory loads and stores, so the decision is the warp's; both warps of a quarter see the same maxima)
         const bool grow = mt > m2 + 8.f || (m2 == -INFINITY && mt != -INFINITY);
-        if (__any_sync(0xffffffffu, grow)) {
+        const bool rescale = __any_sync(0xffffffffu, grow);
+        float corr = 1.f;
+        if (rescale) {
           const float m_new = fmaxf(m2, mt);
-          if (t > 0) {
-            const float corr = (m2 == -INFINITY) ? 1.f : exp2f(m2 - m_new);   // nothing accumulated yet on a -inf row
-            l *= corr;
-            // the previous tile's P V has to be in the accumulator before it is rescaled
-            if (!at_wait(o_full, (tile_it - 1u) & 1u, p.status, ST_TIMEOUT_TMEM_FULL, abort_flag)) { ok = false; break; }
+          if (m2 != -INFINITY) corr = exp2f(m2 - m_new);                    // else nothing accumulated yet
+          l *= corr;
+          m2 = m_new;
+        }
+        const float mu = m2 == -INFINITY ? 0.f : m2;       // a row that sees no key so far: every score is -inf
+        float ls[2] = {0.f, 0.f};
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          const float e0 = exp2f(fmaf(__uint_as_float(r0[2 * k]), sc2, -mu)), e1 = exp2f(fmaf(__uint_as_float(r0[2 * k + 1]), sc2, -mu));
+          ls[0] += e0;
+          ls[1] += e1;
+          r0[k] = Cvt<T>::pack2(e0, e1);
+        }
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          const float e0 = exp2f(fmaf(__uint_as_float(r1[2 * k]), sc2, -mu)), e1 = exp2f(fmaf(__uint_as_float(r1[2 * k + 1]), sc2, -mu));
+          ls[0] += e0;
+          ls[1] += e1;
+          r1[k] = Cvt<T>::pack2(e0, e1);
+        }
+        l += ls[0] + ls[1];
+        if (t > 0) {
+          // the previous tile's P V has read the buffer, and is in the accumulator before that is rescaled
+          wait_or_report(o_full, (tile_it - 1u) & 1u, p.status, ST_TIMEOUT_TMEM_FULL, abort_flag);
+          if (rescale) {
             tc_fence_after();
 #pragma unroll
-            for (int c = 0; c < HD / 16; ++c) {
-              uint32_t rg[16];
-              tmem_ld_32x16(tmem_O + lane_base + c * 16, rg);
+            for (int c = 0; c < HD / 32; ++c) {
+              uint32_t ro[16];
+              tmem_ld_32x16(tmem_O + lane_base + half * (HD / 2) + c * 16, ro);
               tmem_ld_wait();
 #pragma unroll
-              for (int k = 0; k < 16; ++k) rg[k] = __float_as_uint(__uint_as_float(rg[k]) * corr);
-              tmem_st_32x16(tmem_O + lane_base + c * 16, rg);
+              for (int k = 0; k < 16; ++k) ro[k] = __float_as_uint(__uint_as_float(ro[k]) * corr);
+              tmem_st_32x16(tmem_O + lane_base + half * (HD / 2) + c * 16, ro);
             }
             tmem_st_wait();
           }
-          m2 = m_new;
         }
-        float ls[2] = {0.f, 0.f};
-        const bool dead = m2 == -INFINITY;       // no visible key so far in this row
-        // pass B: probabilities -> shared memory (operand layout)
-#pragma unroll 1
-        for (int c = 0; c < AT_N / 32; ++c) {
-          uint32_t rg[32];
-          tmem_ld_32x32(tmem_S + lane_base + c * 32, rg);
-          tmem_ld_wait();
-          float pv[32];
-          if (!need_mask) {
 #pragma unroll
-            for (int k = 0; k < 32; ++k) {
-              const float e = exp2f(fmaf(__uint_as_float(rg[k]), sc2, -m2));
-              pv[k] = e;
-              ls[k & 1] += e;
-            }
-          } else {
-#pragma unroll
-            for (int k = 0; k < 32; ++k) {
-              const int j = j0 + c * 32 + k;
-              const bool vis = row_ok && !dead && j <= i && j >= lo_i;
-              const float e = vis ? exp2f(fmaf(__uint_as_float(rg[k]), sc2, -m2)) : 0.f;
-              pv[k] = e;
-              ls[k & 1] += e;
-            }
-          }
-          store_p_chunk<T>(sP, r, c * 32, pv);
+        for (int k = 0; k < 4; ++k) {           // this half's 64 keys are one panel of the operand layout
+          uint8_t* panel = sP + half * (AT_M * 128);
+          *reinterpret_cast<uint4*>(panel + sw128_off(r, 8 * k)) = make_uint4(r0[4 * k], r0[4 * k + 1], r0[4 * k + 2], r0[4 * k + 3]);
+          *reinterpret_cast<uint4*>(panel + sw128_off(r, 8 * k + 32)) = make_uint4(r1[4 * k], r1[4 * k + 1], r1[4 * k + 2], r1[4 * k + 3]);
         }
-        l += ls[0] + ls[1];
         tc_fence_before();
         fence_proxy_async();          // generic-proxy writes of P must be visible to the tensor core
         __syncwarp();                 // every lane's writes and fences, then one arrival for the warp
         if (lane == 0) mbar_arrive(p_ready);
       }
-      if (!ok) break;
-      // the item's last P V
-      if (!at_wait(o_full, (tile_it - 1u) & 1u, p.status, ST_TIMEOUT_TMEM_FULL, abort_flag)) { ok = false; break; }
+      // the item's last P V (every warp is past its last exchange of maxima then)
+      wait_or_report(o_full, (tile_it - 1u) & 1u, p.status, ST_TIMEOUT_TMEM_FULL, abort_flag);
+      float* row_sum = reinterpret_cast<float*>(row_max);
+      pair_sync();
+      if (half == 1) row_sum[r] = l;
+      pair_sync();
+      if (half == 0) { l += row_sum[r]; row_sum[r] = l; }
+      pair_sync();
+      if (half == 1) l = row_sum[r];
+      pair_sync();                    // read before the next item's maxima take the place
       tc_fence_after();
       const float inv_l = l > 0.f ? 1.f / l : 0.f;
-      T* op = reinterpret_cast<T*>(p.o) + (row_base + i) * p.ld_o + (long long)h * HD;
+      T* op = reinterpret_cast<T*>(p.o) + (row_base + i) * p.ld_o + (long long)h * HD + half * (HD / 2);
 #pragma unroll
-      for (int c = 0; c < HD / 32; ++c) {
-        uint32_t rg[32];
-        tmem_ld_32x32(tmem_O + lane_base + c * 32, rg);
+      for (int c = 0; c < HD / 64; ++c) {
+        uint32_t ro[32];
+        tmem_ld_32x32(tmem_O + lane_base + half * (HD / 2) + c * 32, ro);
         tmem_ld_wait();
         if (row_ok) {
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             uint4 q;
-            q.x = Cvt<T>::pack2(__uint_as_float(rg[8 * k + 0]) * inv_l, __uint_as_float(rg[8 * k + 1]) * inv_l);
-            q.y = Cvt<T>::pack2(__uint_as_float(rg[8 * k + 2]) * inv_l, __uint_as_float(rg[8 * k + 3]) * inv_l);
-            q.z = Cvt<T>::pack2(__uint_as_float(rg[8 * k + 4]) * inv_l, __uint_as_float(rg[8 * k + 5]) * inv_l);
-            q.w = Cvt<T>::pack2(__uint_as_float(rg[8 * k + 6]) * inv_l, __uint_as_float(rg[8 * k + 7]) * inv_l);
+            q.x = Cvt<T>::pack2(__uint_as_float(ro[8 * k + 0]) * inv_l, __uint_as_float(ro[8 * k + 1]) * inv_l);
+            q.y = Cvt<T>::pack2(__uint_as_float(ro[8 * k + 2]) * inv_l, __uint_as_float(ro[8 * k + 3]) * inv_l);
+            q.z = Cvt<T>::pack2(__uint_as_float(ro[8 * k + 4]) * inv_l, __uint_as_float(ro[8 * k + 5]) * inv_l);
+            q.w = Cvt<T>::pack2(__uint_as_float(ro[8 * k + 6]) * inv_l, __uint_as_float(ro[8 * k + 7]) * inv_l);
             reinterpret_cast<uint4*>(op)[c * 4 + k] = q;
           }
         }
       }
       tc_fence_before();              // the next item's first P V overwrites the accumulator
-      if (row_ok && p.lse) p.lse[(row_base + i) * p.H + h] = l > 0.f ? (m2 + log2f(l)) * 0.6931471805599453f : INFINITY;
+      if (half == 0 && row_ok && p.lse) p.lse[(row_base + i) * p.H + h] = l > 0.f ? (m2 + log2f(l)) * 0.6931471805599453f : INFINITY;
     }
   }
   __syncthreads();
@@ -312,7 +346,7 @@ __global__ void __launch_bounds__(AT_THREADS) attn_tc_fwd_kernel(const __grid_co
     for (int k = 0; k < 64; ++k) __nanosleep(1000);
     __syncthreads();
   }
-  if (warp == 5) { tc_fence_after(); tmem_dealloc(tmem_base, 256); }
+  if (warp == AT_FWD_CW + 1) { tc_fence_after(); tmem_dealloc(tmem_base, 256); }
 }
 
 // ============================================================================================ backward: dQ
@@ -1425,7 +1459,7 @@ int launch_tc_fwd(const gb_attn_args* a, int* lo, int* status, cudaStream_t st) 
   AttnTcParams p{};
   p.B = a->B; p.T = a->T; p.H = a->H; p.KV = a->KV; p.window = a->window; p.scale = a->scale;
   p.lo = lo; p.o = a->o; p.ld_o = a->ld_o; p.lse = a->lse; p.status = status;
-  constexpr size_t smem = (size_t)AT_M * HD * 2 * 5 + AT_M * AT_N * 2 + 128 + (HD == 64 ? 0 : 1024);
+  constexpr size_t smem = (size_t)AT_M * HD * 2 * 5 + AT_M * AT_N * 2 + 128 + 512 + (HD == 64 ? 0 : 1024);
   auto kern = attn_tc_fwd_kernel<T, HD>;
   static bool attr = false;
   if (!attr) {
