@@ -41,6 +41,9 @@ typedef struct gb_gemm_args {
   int pair;                   // 1: two-CTA 256 x 256 tiles (gemm_pair_sm100.cu).  Needs a 16-byte aligned output whose
                               // row pitch is a multiple of 16 bytes, no tile_out, an addend only with fp32 output, and
                               // in mode 1 expert segments padded to GB_MOE_PAD rows; block_n is ignored
+  float* part; int part_slots, part_cut;  // pair, mode 2, fp32 out accumulated in place, contiguous: scratch of part_slots [M, N] matrices for the
+                              // partial sums of reductions that are cut into pieces (at most 64 groups; seg_offsets may be
+                              // null for one group over K; part_cut > 0: k-blocks of its pieces).  null: reductions stay whole
 } gb_gemm_args;
 int gb_gemm(const gb_gemm_args* args, cudaStream_t stream);
 int gb_gemm_pair(const gb_gemm_args* args, cudaStream_t stream);   // what gb_gemm calls when args->pair != 0

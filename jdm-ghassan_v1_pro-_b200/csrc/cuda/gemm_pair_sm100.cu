@@ -31,6 +31,8 @@ static constexpr int MAX_STAGES = 8;  // narrower tiles have smaller stages, and
 static constexpr uint32_t SLOT_BYTES = 4096;   // 32 rows x 128 bytes
 static constexpr uint32_t TMEM_COLS = 512;
 static constexpr uint32_t BAR_BYTES = 512;
+static constexpr int MAX_PIECE_GROUPS = 64;    // groups that a plan of pieces covers
+static constexpr uint32_t PLAN_BYTES = 1024;
 
 enum { EPI_STORE = 0, EPI_SWIGLU_FWD = 1, EPI_SWIGLU_BWD = 2, EPI_RELU2 = 4 };   // numbered as in gemm_sm100.cu
 
@@ -49,20 +51,123 @@ struct Params {
   int reduce;                  // fp32 out only: out += acc through TMA reduce-add
   int has_aux_out;             // SwiGLU forward: also store the interleaved gate/up pre-activations
   int a_mn3, b_mn3;            // the MN-major operand's map is the chunked 3-D view: one load per k-block
+  int part_slots;              // mode 2, reduce: slots of [M, N] partial sums for the pieces of cut reductions (0: whole reductions)
+  int part_cut;                // k-blocks of a piece where the caller knows them (one group), else 0
   int* status;
 };
 
 struct Tile {
   int m0, n0, b_row_off, k_begin, k_end, g;
+  int slot;                    // of the partial sums, or -1: into the matrix
 };
 
-__device__ __forceinline__ Tile decode(const Params& p, int tile, int tiles_m, int tiles_n) {
+// How the reductions of a weight gradient are cut into pieces.  Whole reductions are the items of a persistent kernel only when
+// there are many of them and none is long: the always-on expert sees every token (512 k-blocks where the others have 128, at
+// 32768 tokens and top 2 of 8), and pairs without one of its tiles are done long before.  Every group's reduction is cut evenly
+// into pieces of at most C k-blocks; the items are (group, piece, tile), tiles fastest, so pairs that run at the same time
+// read the same rows.  The first piece adds into the matrix, the others store partial sums, which piece_add_kernel adds in order.
+// C is the candidate with the least estimate (k-blocks of the pair that starts with the longest group, and what the slots cost to
+// write and add), found by one warp from the lengths at hand; it depends on nothing else, so results repeat.
+// Whole against cut, with the addition (us; 9 groups, the last 4 times as long; 98304 rows): 1536 x 768 330 -> 190, 768 x 768
+// 270 -> 115 (floor at 1668 TFLOP/s: 139 and 70); 49152 rows: 1024 x 512 113 -> 62, 512 x 512 113 -> 38.  One group: 1280 x 768 over
+// 32768 rows 67 -> 59, 4096 x 768 over 16384 (one-CTA tiles before) 141 -> 64.
+struct PiecePlan {
+  int base[MAX_PIECE_GROUPS + 1];      // first item of the i-th group from the last
+  short len[MAX_PIECE_GROUPS];         // k-blocks of a piece (at most 32767)
+  short slot[MAX_PIECE_GROUPS];        // first slot
+};
+static_assert(sizeof(PiecePlan) <= PLAN_BYTES, "plan");
+
+__device__ __forceinline__ int piece_kblocks(const int* seg, int K, int g) {
+  return seg ? (seg[g + 1] - seg[g] + BK - 1) / BK : (K + BK - 1) / BK;
+}
+__device__ __forceinline__ int warp_prefix(int v, int& total) {        // sum over the lanes below
+  const int lane = threadIdx.x & 31;
+  int s = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, s, o);
+    if (lane >= o) s += x;
+  }
+  total = __shfl_sync(0xffffffffu, s, 31);
+  return s - v;
+}
+// Called by one whole warp; `per` tiles per group.  Lane l holds groups l and l + 32 from the last, and estimates candidate l.
+__device__ __forceinline__ void plan_pieces(PiecePlan* pl, const int* seg, int K, int groups, int per, long long mn, int n_pairs, int slots,
+                                            int fixed) {
+  const int lane = threadIdx.x & 31;
+  int kb[2], cb = fixed;
+  float units = 0.f;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int i = lane + 32 * h;
+    kb[h] = i < groups ? max(0, piece_kblocks(seg, K, groups - 1 - i)) : 0;
+    units += (float)kb[h];
+  }
+  if (fixed <= 0) {
+    for (int o = 16; o; o >>= 1) units += __shfl_xor_sync(0xffffffffu, units, o);
+    // candidates: 1/16 to 31/16 of a pair's even share, at least 16 k-blocks (an epilogue's time); the last one cuts only at 32767
+    const float share = units * (float)per / (float)n_pairs;
+    const float c = lane == 31 ? 32767.f : fminf(32767.f, fmaxf(16.f, ceilf(share * (float)(lane + 1) / 16.f)));
+    // a slot is written and read, the matrix of a group that is cut is read and written: 8 bytes a value each, at about 5 TB/s, in
+    // k-blocks of 0.4 us
+    const float slot_cost = (float)mn * 4e-6f;
+    const float inv_c = 1.f / c, inv_pairs = 1.f / (float)n_pairs;
+    float load = 0.f, items = 0.f, turn = 0.f, extra = 0.f, cut = 0.f;      // turn: items of the first pair so far
+#pragma unroll 4
+    for (int i = 0; i < groups; ++i) {
+      const float k = (float)__shfl_sync(0xffffffffu, i < 32 ? kb[0] : kb[1], i & 31), n = ceilf(k * inv_c);
+      items = fmaf(n, (float)per, items);
+      const float t = ceilf(items * inv_pairs);
+      load = fmaf(t - turn, __fdividef(k, fmaxf(n, 1.f)), load);
+      turn = t;
+      extra += fmaxf(n - 1.f, 0.f);
+      cut += n > 1.f ? 1.f : 0.f;
+    }
+    const float score = extra + cut > (float)slots ? 3e38f : load + (extra + cut) * slot_cost;   // the real plan has no more pieces than this
+    float best = score;
+    for (int o = 16; o; o >>= 1) best = fminf(best, __shfl_xor_sync(0xffffffffu, best, o));
+    const unsigned who = __ballot_sync(0xffffffffu, score == best);
+    cb = (int)__shfl_sync(0xffffffffu, c, 31 - __clz(who));                 // the fewest pieces among equals
+  }
+  int item0 = 0, slot = 0;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    if (32 * h >= groups) break;
+    const int i = lane + 32 * h, n0 = (kb[h] + cb - 1) / cb, len = n0 ? (kb[h] + n0 - 1) / n0 : 0, n = len ? (kb[h] + len - 1) / len : 0;
+    int all, used;
+    const int at = item0 + warp_prefix(n * per, all), sl = slot + warp_prefix(n > 0 ? n - 1 : 0, used);
+    if (i < groups) {
+      pl->base[i] = at;
+      pl->len[i] = (short)len;
+      pl->slot[i] = (short)sl;
+    }
+    item0 += all;
+    slot += used;
+  }
+  if (lane == 0) pl->base[groups] = item0;
+}
+
+__device__ __forceinline__ Tile decode(const Params& p, const PiecePlan* pl, int tile, int tiles_m, int tiles_n) {
   Tile t;
   t.b_row_off = 0;
+  t.slot = -1;
   t.k_begin = 0;
   t.k_end = p.K;
   t.g = 0;
-  if (p.mode == 2) {
+  if (p.part_slots) {
+    int i = 0;
+    while (tile >= pl->base[i + 1]) ++i;                // groups without rows have no items
+    const int per = tiles_m * tiles_n, at = tile - pl->base[i], piece = at / per, r = at - piece * per;
+    const int len = pl->len[i] * BK;
+    t.g = p.groups - 1 - i;
+    t.m0 = (r % tiles_m) * TM;
+    t.n0 = (r / tiles_m) * p.tn;
+    const int k0 = p.seg_offsets ? p.seg_offsets[t.g] : 0, k1 = p.seg_offsets ? p.seg_offsets[t.g + 1] : p.K;
+    t.k_begin = k0 + piece * len;
+    t.k_end = min(k1, t.k_begin + len);
+    if (piece > 0) t.slot = pl->slot[i] + piece - 1;
+  } else if (p.mode == 2) {
     // groups from the last to the first: the always-on expert is the last group and the longest reduction
     const int per = tiles_m * tiles_n;
     const int gi = tile / per, r = tile - gi * per;
@@ -101,6 +206,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint64_t* aux_bar = tempty_bar + 2;               // [EPI_WARPS][2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(aux_bar + 2 * EPI_WARPS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  PiecePlan* plan = reinterpret_cast<PiecePlan*>(reinterpret_cast<uint8_t*>(full_bar) + BAR_BYTES);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -121,6 +227,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB); tma_prefetch_desc(&tmO);
     if (EPI != EPI_STORE && EPI != EPI_RELU2) tma_prefetch_desc(&tmX);
   }
+  if (EPI == EPI_STORE && sizeof(OutT) == 4 && p.part_slots && warp == 0)
+    plan_pieces(plan, p.seg_offsets, p.K, p.groups, ((p.M + TM - 1) / TM) * ((p.N + p.tn - 1) / p.tn), (long long)p.M * p.N,
+                (int)cluster_nctaid_x(), p.part_slots, p.part_cut);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();        // both CTAs' barriers exist before either signals the other's
@@ -132,7 +241,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int tiles_n = (p.N + p.tn - 1) / p.tn;
   const int hn = p.tn >> 1;                                   // B rows per CTA
   const uint32_t stage_bytes = A_BYTES + hn * (BK * 2), nst = p.stages;
-  const int total_tiles = tiles_m * tiles_n * (p.mode == 2 ? p.groups : 1);
+  const int total_tiles = p.part_slots ? plan->base[p.groups] : tiles_m * tiles_n * (p.mode == 2 ? p.groups : 1);
   const int pair_id = (int)cluster_id_x(), n_pairs = (int)cluster_nctaid_x();
 
   if (warp == W_TMA) {
@@ -142,7 +251,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const uint32_t full0 = mapa_shared(smem_u32(&full_bar[0]), 0);   // the full barriers that count are CTA 0's
       uint32_t s = 0, ph = 0;
       for (int tile = pair_id; tile < total_tiles; tile += n_pairs) {
-        const Tile t = decode(p, tile, tiles_m, tiles_n);
+        const Tile t = decode(p, plan, tile, tiles_m, tiles_n);
         const int am = t.m0 + (int)rank * HM, bn = t.n0 + (int)rank * hn;
         for (int k = t.k_begin; k < t.k_end; k += BK) {
           wait_or_report(&empty_bar[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
@@ -177,7 +286,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const uint32_t idesc = make_idesc_f16(p.fmt, p.a_mn, p.b_mn, TM, p.tn);
       uint32_t s = 0, ph = 0, acc_it = 0;
       for (int tile = pair_id; tile < total_tiles; tile += n_pairs) {
-        const Tile t = decode(p, tile, tiles_m, tiles_n);
+        const Tile t = decode(p, plan, tile, tiles_m, tiles_n);
         if (t.k_end <= t.k_begin) continue;
         const uint32_t ab = acc_it & 1, aph = (acc_it >> 1) & 1;
         wait_or_report(&tempty_bar[ab], aph ^ 1, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag);
@@ -225,7 +334,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       return s;
     };
     for (int tile = pair_id; tile < total_tiles; tile += n_pairs) {
-      const Tile t = decode(p, tile, tiles_m, tiles_n);
+      const Tile t = decode(p, plan, tile, tiles_m, tiles_n);
       const bool empty_k = (t.k_end <= t.k_begin);
       const int row_q = t.m0 + (int)rank * HM + quarter * 32;   // first of this warp's 32 rows
       const int colh = t.n0 + half * 128;                       // first of this warp's 128 accumulator columns (SwiGLU: tn = 256)
@@ -346,7 +455,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           __syncwarp();
           if (lane == 0) {
             if (rows_live && col < p.N) {
-              if (p.reduce) tma_reduce_add_3d(&tmO, slot, col, row_q, t.g);
+              if (t.slot >= 0) tma_store_3d(&tmX, slot, col, row_q, t.slot);
+              else if (p.reduce) tma_reduce_add_3d(&tmO, slot, col, row_q, t.g);
               else tma_store_3d(&tmO, slot, col, row_q, t.g);
             }
             bulk_commit();
@@ -474,7 +584,34 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
 template <int STAGES, int SLOTS>
 constexpr size_t smem_bytes() {
-  return size_t(STAGES) * STAGE_BYTES + size_t(EPI_WARPS) * SLOTS * SLOT_BYTES + BAR_BYTES + 1024;
+  return size_t(STAGES) * STAGE_BYTES + size_t(EPI_WARPS) * SLOTS * SLOT_BYTES + BAR_BYTES + PLAN_BYTES + 1024;
+}
+
+// out[g] += the group's partial sums, in the order of its pieces.  Bound by their bytes, which the product has just written: 16
+// bytes a thread, every block a stride of each group that was cut.
+__global__ void __launch_bounds__(256) piece_add_kernel(const float* __restrict__ part, float* __restrict__ out, const int* seg, int K,
+                                                        int groups, int per, long long mn, int n_pairs, int slots, int fixed) {
+  __shared__ PiecePlan pl;
+  // the offsets come from kernels before the product, which is not itself launched ahead of them
+  if (threadIdx.x < 32) plan_pieces(&pl, seg, K, groups, per, mn, n_pairs, slots, fixed);
+  __syncthreads();
+  pdl_wait();
+  const long long n4 = mn / 4;
+  for (int i = 0; i < groups; ++i) {
+    const int n = (pl.base[i + 1] - pl.base[i]) / per - 1;
+    if (n <= 0) continue;
+    const float4* src = reinterpret_cast<const float4*>(part) + pl.slot[i] * n4;
+    float4* dst = reinterpret_cast<float4*>(out) + (groups - 1 - i) * n4;
+    for (long long e = (long long)blockIdx.x * 256 + threadIdx.x; e < n4; e += (long long)gridDim.x * 256) {
+      float4 v = dst[e];
+#pragma unroll 4
+      for (int j = 0; j < n; ++j) {
+        const float4 x = __ldcs(src + j * n4 + e);
+        v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+      }
+      dst[e] = v;
+    }
+  }
 }
 
 }  // namespace pr
@@ -519,7 +656,7 @@ namespace {
 
 template <int EPI, int STAGES, int SLOTS, typename OutT>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, const CUtensorMap& tx,
-                gb::pr::Params p, int max_tiles, cudaStream_t st) {
+                gb::pr::Params p, int max_tiles, cudaStream_t st, int* used_pairs = nullptr) {
   const uint32_t stage = gb::pr::A_BYTES + p.tn / 2 * gb::pr::BK * 2;
   p.stages = (int)(STAGES * gb::pr::STAGE_BYTES / stage);
   if (p.stages > gb::pr::MAX_STAGES) p.stages = gb::pr::MAX_STAGES;
@@ -550,6 +687,8 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   }
   int pairs = max_tiles < max_pairs ? max_tiles : max_pairs;
   if (pairs < 1) pairs = 1;
+  if (p.part_slots) pairs = max_pairs;
+  if (used_pairs) *used_pairs = pairs;
   kern<<<2 * pairs, gb::pr::THREADS, smem, st>>>(ta, tb, to, tx, p);
   return gb_launch_rc();
 }
@@ -574,7 +713,7 @@ extern "C" int gb_gemm_pair(const gb_gemm_args* a, cudaStream_t st) {
   p.b_group_rows = a->b_group_rows;
   p.status = a->status;
   if (a->mode == 1 && (!a->tile_expert || !a->num_m_tiles)) return -1;
-  if (a->mode == 2 && !a->seg_offsets) return -1;
+  if (a->mode == 2 && !a->seg_offsets && !a->part) return -1;
   const int groups = a->mode == 2 ? p.groups : 1;
   if (a->addend) {
     if (a->addend == a->out && a->ld_add == a->ldo) p.reduce = 1;
@@ -583,6 +722,16 @@ extern "C" int gb_gemm_pair(const gb_gemm_args* a, cudaStream_t st) {
   }
 
   p.tn = pr::TN_MAX;
+  if (a->part) {
+    // pieces of reductions: fp32 sums into [groups, M, N] without gaps
+    if (a->mode != 2 || !p.reduce || ot != 2 || a->part_slots < 1 || p.groups > pr::MAX_PIECE_GROUPS || a->epilogue != pr::EPI_STORE ||
+        a->ldo != a->N || a->N % 4 || (groups > 1 && (!a->seg_offsets || a->out_group_stride != (long long)a->M * a->N)) ||
+        (reinterpret_cast<uintptr_t>(a->part) & 15)) return -26;
+    p.part_slots = a->part_slots;
+    p.part_cut = a->part_cut;
+    // a cut given by the caller is for one group, whose pieces have to fit
+    if (p.part_cut > 0 && (p.groups > 1 || a->seg_offsets || p.part_cut > 32767 || ((a->K + pr::BK - 1) / pr::BK - 1) / p.part_cut > p.part_slots)) return -27;
+  }
 
   CUtensorMap ta, tb, to, tx;
   int rc;
@@ -610,6 +759,18 @@ extern "C" int gb_gemm_pair(const gb_gemm_args* a, cudaStream_t st) {
       rc = gb_make_tmap_3d_box128(&to, a->out, ot, a->N, a->M, groups, a->ldo, a->out_group_stride, 32);
       if (rc) return rc - 300;
       tx = to;
+      if (p.part_slots) {
+        const long long mn = (long long)a->M * a->N;
+        rc = gb_make_tmap_3d_box128(&tx, a->part, 2, a->N, a->M, p.part_slots, a->N, mn, 32);
+        if (rc) return rc - 400;
+        int pairs = 0;
+        rc = launch_pair<pr::EPI_STORE, 5, 2, float>(ta, tb, to, tx, p, max_tiles, st, &pairs);
+        if (rc) return rc;
+        const long long blocks = (mn / 4 + 255) / 256;
+        GB_PDL_LAUNCH(pr::piece_add_kernel, dim3((unsigned)(blocks < 4 * pairs ? blocks : 4 * pairs)), dim3(256), st, a->part,
+                      reinterpret_cast<float*>(a->out), a->seg_offsets, a->K, p.groups, tiles_m * tiles_n, mn, pairs, p.part_slots, p.part_cut);
+        return gb_launch_rc();
+      }
       if (ot == 2) return launch_pair<pr::EPI_STORE, 5, 2, float>(ta, tb, to, tx, p, max_tiles, st);
       if (ot == 1) return launch_pair<pr::EPI_STORE, 5, 2, __nv_bfloat16>(ta, tb, to, tx, p, max_tiles, st);
       return launch_pair<pr::EPI_STORE, 5, 2, __half>(ta, tb, to, tx, p, max_tiles, st);

@@ -483,13 +483,14 @@ class CudaModel:
             self.ep.backward(l, b)
         elif cfg.use_moe:
             ws = b.ws
+            every = self.N if cfg.moe_shared else 0       # the shared expert's rows
             K.moe_combine_bwd(ws, t.dx, b.yperm, t.dy_perm, t.gdot)
             G.gemm_swiglu_bwd(t.dy_perm, self.w16(p + "w_down"), b.gu, dgu_out=t.dgu, tile_expert=ws.tile_expert,
                               num_m_tiles=ws.num_tiles, group_rows=d, n=E)
-            G.gemm_grouped_reduce(t.dy_perm, b.act, ws.seg_offsets, ne1, self.g(p + "w_down").view(ne1, d, E))
+            G.gemm_grouped_reduce(t.dy_perm, b.act, ws.seg_offsets, ne1, self.g(p + "w_down").view(ne1, d, E), longest=every)
             G.gemm_grouped_rows(t.dgu, self.w16(p + "w_gu"), ws.tile_expert, ws.num_tiles, n=d, b_mn=True,
                                 group_rows=2 * E, out=t.dxperm)
-            G.gemm_grouped_reduce(t.dgu, b.xperm, ws.seg_offsets, ne1, self.g(p + "w_gu").view(ne1, 2 * E, d))
+            G.gemm_grouped_reduce(t.dgu, b.xperm, ws.seg_offsets, ne1, self.g(p + "w_gu").view(ne1, 2 * E, d), longest=every)
             want_aux = cfg.moe_aux_scale > 0
             K.moe_router_bwd(ws, b.xb2, self.w(p + "router"), t.gdot, t.dxperm, t.dxb, self.g(p + "router"), t.part,
                              jitter=cfg.moe_jitter, seed_dev=self.seed_dev if cfg.moe_jitter > 0 else None,
@@ -497,10 +498,10 @@ class CudaModel:
         else:
             G.gemm_swiglu_bwd(t.dx16, self.w16(p + "w_down"), b.gu, dgu_out=t.dgu, n=E)
             gd = self.g(p + "w_down")
-            G.gemm(t.dx16, b.act, a_mn=True, b_mn=True, out=gd, addend=gd)
+            G.gemm_wgrad(t.dx16, b.act, gd.view(d, E))
             G.gemm(t.dgu, self.w16(p + "w_gu"), b_mn=True, out=t.dxb)
             gg = self.g(p + "w_gu")
-            G.gemm(t.dgu, b.xb2, a_mn=True, b_mn=True, out=gg, addend=gg)
+            G.gemm_wgrad(t.dgu, b.xb2, gg.view(2 * E, d))
         K.rmsnorm_bwd(t.dxb, b.x_mid, self.w(p + "ffn_norm"), b.rrms2, t.dx, t.dx, t.dx16, t.norm_part,
                       self.g(p + "ffn_norm"))
         # attention branch

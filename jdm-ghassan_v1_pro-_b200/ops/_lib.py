@@ -39,6 +39,7 @@ class GemmArgs(ctypes.Structure):
         ("status", c_vp),
         ("tile_out", c_vp),
         ("pair", c_int),
+        ("part", c_vp), ("part_slots", c_int), ("part_cut", c_int),
     ]
 
 

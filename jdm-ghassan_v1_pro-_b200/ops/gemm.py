@@ -198,22 +198,26 @@ def gemm_grouped_rows(a, b, tile_expert, num_m_tiles, *, n, b_mn=False, group_ro
     return out
 
 
-def gemm_grouped_reduce(a, b, seg_offsets, groups, out, *, accumulate=True, block_n=0, pair=None):
+def gemm_grouped_reduce(a, b, seg_offsets, groups, out, *, accumulate=True, block_n=0, pair=None, longest=0):
     """Per-expert weight gradient: ``out[g] (+)= a[rows_g]^T @ b[rows_g]`` with ``rows_g`` given by the padded
     offsets ``seg_offsets[g] .. seg_offsets[g+1]`` (device int32, multiples of 128; pad rows must be zero).
-    ``a`` is ``[rows, M]``, ``b`` is ``[rows, N]``, ``out`` is fp32 ``[groups, M, N]``.
+    ``a`` is ``[rows, M]``, ``b`` is ``[rows, N]``, ``out`` is fp32 ``[groups, M, N]``.  ``longest``: rows of the last group where that is
+    known to be the longest (an expert that every token visits), for the choice of the schedule only.
     """
     M, N = a.shape[1], b.shape[1]
     if out.dtype != torch.float32 or out.shape != (groups, M, N) or not out.is_contiguous():
         raise ValueError("out must be contiguous fp32 [groups, M, N]")
     if not block_n:    # 256-wide tiles measured 1.47x faster once the groups supply tiles for every SM
         block_n = 256 if (N % 256 == 0 and groups * ((M + 127) // 128) * (N // 256) >= 222) else 128
+    part = _piece_scratch(M, N, a.shape[0] // 64, groups, out, longest // 64) if accumulate and pair is not False else None
     if pair is None:
         pair = pair_ok(M, N, out, groups=groups)
     g = _base_args(a, b, M, N, 0, True, True, out, block_n)
     g.epilogue = EPI_STORE
     g.mode = 2
     g.pair = int(bool(pair))
+    if part is not None:
+        _use_pieces(g, (part[0], 0))         # how many rows the groups really have is known on the device
     g.seg_offsets = seg_offsets.data_ptr()
     g.groups = groups
     g.out_group_stride = M * N
@@ -222,6 +226,55 @@ def gemm_grouped_reduce(a, b, seg_offsets, groups, out, *, accumulate=True, bloc
         g.addend, g.ld_add = out.data_ptr(), N
     _launch(g)
     return out
+
+
+# Weight gradients whose reductions are cut into pieces (csrc/cuda/gemm_pair_sm100.cu): partial sums take at most this much scratch,
+# and the product has at least this many k-blocks of 64 for each of the 74 pairs, half as many where it is one group (below, an
+# epilogue costs as much as a piece).
+PIECE_BYTES = 96 << 20
+PIECE_MIN_KBLOCKS = 16
+
+
+def _best_cut(tiles, lens, mn):
+    """The estimate of the plan on the device for reductions of these lengths (k-blocks, the longest first): k-blocks of the best
+    pieces, or 0 where they do not gain a tenth."""
+    def cost(c):
+        load, items, turn, extra = 0.0, 0, 0, 0
+        for k in lens:
+            n = -(-k // c)
+            items += n * tiles
+            load, turn = load + (-(-items // 74) - turn) * (k / n), -(-items // 74)
+            extra += n if n > 1 else 0
+        return load + extra * mn * 4e-6
+    share = tiles * sum(lens) / 74.0
+    c = min((max(PIECE_MIN_KBLOCKS, int(share * i / 16)) for i in range(1, 32)), key=cost)
+    return c if cost(c) < 0.9 * cost(1 << 30) else 0
+
+
+def _piece_scratch(M, N, kblocks, groups, out, longest=0):
+    """(fp32 ``[slots, M, N]``, k-blocks of a piece where that is settled) for the pieces of ``groups`` reductions that have ``kblocks``
+    blocks of 64 rows in all, or None where they stay whole.  ``longest``: k-blocks of a group known to be longer than the others.  Taken from the allocator for this call, so
+    calls on other streams have their own."""
+    tiles = pair_tiles(M, N)
+    if not PAIR_ENABLED or N % 4 or groups > 64 or tiles * kblocks * (2 if groups == 1 else 1) < 74 * PIECE_MIN_KBLOCKS or not pair_ok(M, N, out, groups=60):
+        return None
+    if tiles * groups >= 3 * 74:             # three rounds of whole reductions and more: little idles at the end
+        return None
+    cut = 0
+    if groups == 1 or longest:
+        rest = max(1, (kblocks - longest) // (groups - 1)) if groups > 1 else 0
+        cut = _best_cut(tiles, [longest or kblocks] + [rest] * (groups - 1), M * N)
+        if not cut:
+            return None
+    slots = min(64, PIECE_BYTES // (4 * M * N), kblocks // PIECE_MIN_KBLOCKS)      # a piece has at least that many k-blocks
+    if groups == 1:
+        slots = -(-kblocks // cut) - 1 if slots >= -(-kblocks // cut) - 1 else 0
+    return (torch.empty(slots, M, N, dtype=torch.float32, device=out.device), cut if groups == 1 else 0) if slots >= 1 else None
+
+
+def _use_pieces(g, pieces, K=0):
+    g.pair, g.mode, g.K = 1, 2, K
+    g.part, g.part_slots, g.part_cut = pieces[0].data_ptr(), pieces[0].shape[0], pieces[1]
 
 
 class SplitK:
@@ -263,30 +316,27 @@ _WGRAD_PLANS = {}
 
 def gemm_wgrad(a, b, grad):
     """``grad += a^T @ b`` for a weight gradient: ``a`` is ``[tokens, M]``, ``b`` is ``[tokens, N]``, ``grad`` is
-    contiguous fp32 ``[M, N]``.  A product with few output tiles and a long token dimension (the attention
-    projections: 36-60 tiles for 148 SMs) is split over the tokens: ``splits`` CTAs per tile write fp32 partials and
+    contiguous fp32 ``[M, N]``.  A long token dimension is cut into pieces that fill the CTA pairs (:func:`_piece_scratch`).  A shorter
+    one with few output tiles is split over the tokens on the one-CTA kernel: ``splits`` CTAs per tile write fp32 partials and
     a second kernel adds them to ``grad`` in a fixed order (measured 60 us -> 23-36 us on the pro_1b shapes).
     Everything else takes the plain accumulate path."""
     Kt, M = a.shape
     N = b.shape[1]
     splittable = not (Kt % 64 or not grad.is_contiguous() or grad.shape != (M, N) or (M * N) % 4)
-    use_pair = False
-    if PAIR_ENABLED and splittable and pair_tiles(M, N) < PAIR_MIN_TILES:
-        # two-CTA tiles: the split count that best fills the 74 CTA pairs (at most 8 partials, 1024 tokens or more each)
-        t, best = pair_tiles(M, N), (0.0, 1)
-        for sp in range(1, 9):
-            if sp > 1 and Kt // sp < 1024:
-                break
-            eff = t * sp / (-(-t * sp // 74) * 74.0)
-            if eff > best[0] + 0.04:
-                best = (eff, sp)
-        if best[1] >= 2 and t * best[1] >= 30:
-            use_pair, splits = True, best[1]
-    if not use_pair:
-        tiles = ((M + 127) // 128) * ((N + 127) // 128)
-        splits = min(8, 148 // max(1, tiles), Kt // 1024)
-        if splits < 2 or not splittable:
-            return gemm(a, b, a_mn=True, b_mn=True, out=grad, addend=grad)
+    part = _piece_scratch(M, N, Kt // 64, 1, grad) if splittable else None
+    if part is not None:
+        g = _base_args(a, b, M, N, Kt, True, True, grad, 256)
+        g.epilogue = EPI_STORE
+        g.groups = 1
+        g.addend, g.ld_add = grad.data_ptr(), N
+        g.out_group_stride = M * N
+        _use_pieces(g, part, Kt)
+        _launch(g)
+        return grad
+    tiles = ((M + 127) // 128) * ((N + 127) // 128)
+    splits = min(8, 148 // max(1, tiles), Kt // 1024)
+    if splits < 2 or not splittable:
+        return gemm(a, b, a_mn=True, b_mn=True, out=grad, addend=grad)
     key = (M, N, Kt, splits, a.device.index)
     plan = _WGRAD_PLANS.get(key)
     if plan is None:
@@ -299,7 +349,6 @@ def gemm_wgrad(a, b, grad):
     g = _base_args(a, b, M, N, 0, True, True, part, 128)
     g.epilogue = EPI_STORE
     g.mode = 2
-    g.pair = int(use_pair)
     g.seg_offsets = offsets.data_ptr()
     g.groups = splits
     g.out_group_stride = M * N

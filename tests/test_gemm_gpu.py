@@ -328,3 +328,39 @@ def test_pair_grouped_rows_and_grouped_reduce():
     G.gemm_grouped_reduce(y16, x, seg, ne, dw2, accumulate=False, pair=True)     # an empty group must store zeros
     L.check_status(what="pair grouped reduce store")
     assert torch.allclose(dw2, dw - 1.0, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("M,N,lens", [
+    (768, 768, [1024, 0, 2048, 128, 16384]),        # a long last group is cut, an empty one has no items
+    (200, 328, [65536]),                            # edges of the 256 x 256 tile
+    (512, 256, [128] * 63 + [32768]),               # as many groups as a plan holds
+    (2560, 512, [512] * 8 + [4096]),
+])
+def test_weight_gradients_in_pieces(M, N, lens):
+    G, L = _ops()
+    offs = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    a, b = _rand(offs[-1], M, seed=80) * 0.2, _rand(offs[-1], N, seed=81) * 0.2
+    assert G._piece_scratch(M, N, offs[-1] // 64, len(lens), torch.empty(len(lens), M, N, device="cuda")) is not None
+    seg = torch.tensor(offs, dtype=torch.int32, device="cuda")
+    out = torch.full((len(lens), M, N), 0.5, dtype=torch.float32, device="cuda")
+    G.gemm_grouped_reduce(a, b, seg, len(lens), out)
+    L.check_status(what="pieces")
+    again = torch.full_like(out, 0.5)
+    G.gemm_grouped_reduce(a, b, seg, len(lens), again)
+    assert torch.equal(out, again)                  # pieces are added in order
+    for g, n in enumerate(lens):
+        ref = 0.5 + a[offs[g]:offs[g + 1]].float().t() @ b[offs[g]:offs[g + 1]].float()
+        rel, ok = _close(out[g], ref)
+        assert ok, (g, n, rel)
+
+
+@pytest.mark.parametrize("M,N,K", [(4096, 768, 16384), (768, 2048, 16384), (264, 776, 16448)])
+def test_weight_gradient_of_one_group_in_pieces(M, N, K):
+    G, L = _ops()
+    a, b = _rand(K, M, seed=82) * 0.2, _rand(K, N, seed=83) * 0.2
+    grad = torch.full((M, N), 0.5, dtype=torch.float32, device="cuda")
+    assert G._piece_scratch(M, N, K // 64, 1, grad) is not None
+    G.gemm_wgrad(a, b, grad)
+    L.check_status(what="pieces")
+    rel, ok = _close(grad, 0.5 + a.float().t() @ b.float())
+    assert ok, rel
