@@ -541,3 +541,34 @@ def test_tensor_core_token_step_matches_gemv_chain(moe, fmt, B):
     gemm.decode_steps(12, sp)                             # through the captured graph
     out = np.asarray(gemm.transcript(13))
     assert out.shape == (B, 13) and int(gemm.state[0, 0]) == 9 + 12
+
+
+@pytest.mark.parametrize("V,top_k", [(300, 300), (1000, 40), (5000, 512), (5000, 513), (32001, 40), (32001, 1024)])
+def test_device_sampler_candidate_edges(V, top_k):
+    """Fewer logits than threads, both ways to the k-th largest value, ties across it (values on a grid of 1/16)."""
+    from ghassan_b200 import _gb200_host as H
+    from ghassan_b200.inference.engine import SamplingParams
+    D = _D()
+    B = 4
+    n = SamplingParams(temperature=1.5, top_k=top_k, top_p=0.99, min_p=0.0, repetition_penalty=1.0, seed=5).to_native()
+    lg = (_rand(B, V, seed=900 + top_k, scale=2.0) * 16).round() / 16
+    lg[3] = lg[3].clamp(max=0.5)                                # many ties at the top
+    rng, host = [H.Rng(70 + b) for b in range(B)], []
+    for b in range(B):
+        c = SamplingParams(temperature=1.5, top_k=top_k, top_p=0.99, min_p=0.0, repetition_penalty=1.0, seed=5).to_native()
+        c.seed = 70 + b
+        host.append(H.Sampler(c))
+    out = torch.zeros(B, dtype=torch.int32, device="cuda")
+    for _ in range(6):
+        logits = lg.cuda()
+        uniforms = torch.tensor([r.uniform() for r in rng], device="cuda")
+        a = D.SampleArgs()
+        a.logits, a.ld, a.B, a.V = logits.data_ptr(), V, B, V
+        a.temperature, a.top_k, a.top_p, a.min_p = n.temperature, n.top_k, n.top_p, n.min_p
+        a.rep_penalty, a.uniforms, a.out_tok = 1.0, uniforms.data_ptr(), out.data_ptr()
+        D.sample(a)
+        rows = range(B) if V <= 5000 else range(3)              # the tied row has more ties than the device keeps
+        assert [out.tolist()[b] for b in rows] == [host[b].sample(lg[b].numpy(), []) for b in rows]
+        if V > 5000:
+            host[3].sample(lg[3].numpy(), [])
+            assert 0 <= out.tolist()[3] < V
