@@ -227,8 +227,13 @@ __global__ void decode_advance_kernel(gb_seq_state* __restrict__ st, int* __rest
 
 // ---------------------------------------------------------------------------------------------- decode attention
 // grid (B*KV, splits), 4 warps.  A block serves the G = H/KV query heads that share one K/V head, so each cached
-// row is read once per group.  Each warp walks its share of the slots with an online softmax per query head; the
-// four warps and then the splits are merged with the usual (max, sum, weighted output) rule.
+// row is read once per group.  HD / 8 lanes share a slot with one 16-byte load of its key and one of its value, so a warp works on
+// 256 / HD slots side by side and a dot product is reduced over HD / 8 lanes; the loads of four slots per lane come before the
+// first use.  Every group of lanes keeps an online softmax per query head; groups, warps and then the splits are merged
+// with the usual (max, sum, weighted output) rule.
+// Bound by the latency of a trip (load, reduce, exponentials, accumulate).  One slot a trip over all 32 lanes took sixteen trips where
+// this takes one (32 sequences, 500 slots, 8 splits): 18.6 -> 11.4 us a launch,
+// and its merge, which overlaps it, 17.9 -> 6.2.
 template <typename T, int HD, int G>
 __global__ void __launch_bounds__(128) decode_attn_kernel(const T* __restrict__ q, long long ld_q, const T* __restrict__ cK,
                                                          const T* __restrict__ cV, const int* __restrict__ slot_pos,
@@ -236,54 +241,130 @@ __global__ void __launch_bounds__(128) decode_attn_kernel(const T* __restrict__ 
                                                          int splits, int H, int KV, int cap, int window, float scale,
                                                          int* __restrict__ ticket, T* __restrict__ out, long long ld_o) {
   pdl_wait();
-  constexpr int EPL = HD / 32;   // elements per lane
+  constexpr int LPS = HD / 8, SPW = 32 / LPS, U = G <= 4 ? 4 : 2;      // lanes per slot, slots side by side, slots in flight per lane
   const int b = blockIdx.x / KV, kvh = blockIdx.x % KV, split = blockIdx.y;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane / LPS, sub = lane % LPS;
   const gb_seq_state s = st[b];
   // the step's own token was appended before this kernel and is not counted in cache_len yet
   const int n_slots = min(cap, s.cache_len + 1);
-  const int own_slot = s.cache_len < cap ? s.cache_len : -1;   // when the ring is full the new token replaced a slot
-  (void)own_slot;
-  float qv[G][EPL], m[G], l[G], o[G][EPL];
+  const bool wide = ((reinterpret_cast<uintptr_t>(cK) | reinterpret_cast<uintptr_t>(cV)) & 15) == 0;    // rows are whole 64 bytes
+  auto load8 = [&](const T* p) {
+    uint4 r;
+    if (wide) r = *reinterpret_cast<const uint4*>(p);
+    else {
+      uint32_t w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) w[i] = Cvt<T>::pack2(Cvt<T>::to_f(p[2 * i]), Cvt<T>::to_f(p[2 * i + 1]));
+      r = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    return r;
+  };
+  auto unpack8 = [](const uint4& r, float (&f)[8]) {
+    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { const float2 x = Cvt<T>::unpack2(w[i]); f[2 * i] = x.x; f[2 * i + 1] = x.y; }
+  };
+  float qv[G][8], m[G], l[G], o[G][8];
 #pragma unroll
   for (int g = 0; g < G; ++g) {
-    const T* qp = q + b * ld_q + (long long)(kvh * G + g) * HD + lane * EPL;
+    const T* qp = q + b * ld_q + (long long)(kvh * G + g) * HD + sub * 8;
 #pragma unroll
-    for (int e = 0; e < EPL; ++e) { qv[g][e] = Cvt<T>::to_f(qp[e]) * scale; o[g][e] = 0.f; }
+    for (int e = 0; e < 8; ++e) { qv[g][e] = Cvt<T>::to_f(qp[e]) * scale; o[g][e] = 0.f; }
     m[g] = -INFINITY;
     l[g] = 0.f;
   }
   const int per = (n_slots + splits - 1) / splits;
   const int lo = split * per, hi = min(n_slots, lo + per);
   const long long kvd = (long long)KV * HD;
-  for (int j = lo + warp; j < hi; j += 4) {
-    if (window > 0 && s.abs_pos - slot_pos[(long long)b * cap + j] >= window) continue;
-    const T* kp = cK + ((long long)b * cap + j) * kvd + kvh * HD + lane * EPL;
-    const T* vp = cV + ((long long)b * cap + j) * kvd + kvh * HD + lane * EPL;
-    float kf[EPL], vf[EPL];
+  const T* kb = cK + (long long)b * cap * kvd + kvh * HD + sub * 8;
+  const T* vb = cV + (long long)b * cap * kvd + kvh * HD + sub * 8;
+  for (int j0 = lo + warp * SPW; j0 < hi; j0 += U * 4 * SPW) {         // the warp's first slot of the trip
+    uint4 kr[U], vr[U];
+    bool ok[U];
 #pragma unroll
-    for (int e = 0; e < EPL; ++e) { kf[e] = Cvt<T>::to_f(kp[e]); vf[e] = Cvt<T>::to_f(vp[e]); }
+    for (int u = 0; u < U; ++u) {
+      const int j = j0 + u * 4 * SPW + grp;
+      ok[u] = j < hi && !(window > 0 && s.abs_pos - slot_pos[(long long)b * cap + j] >= window);
+      kr[u] = vr[u] = make_uint4(0u, 0u, 0u, 0u);
+      if (ok[u]) {
+        kr[u] = load8(kb + (long long)j * kvd);
+        vr[u] = load8(vb + (long long)j * kvd);
+      }
+    }
+    float d[U][G];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float kf[8];
+      unpack8(kr[u], kf);
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        float x = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x += qv[g][e] * kf[e];
+        d[u][g] = x;
+      }
+    }
+#pragma unroll
+    for (int off = LPS / 2; off > 0; off >>= 1)
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int g = 0; g < G; ++g) d[u][g] += __shfl_xor_sync(0xffffffffu, d[u][g], off);
+    float p[U][G];
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-      float d = 0.f;
+      float mn = m[g];
 #pragma unroll
-      for (int e = 0; e < EPL; ++e) d += qv[g][e] * kf[e];
-      d = warp_sum(d);
-      const float mn = fmaxf(m[g], d);
-      const float c = __expf(m[g] - mn), p = __expf(d - mn);
-      l[g] = l[g] * c + p;
+      for (int u = 0; u < U; ++u) if (ok[u]) mn = fmaxf(mn, d[u][g]);
+      const float mu = mn == -INFINITY ? 0.f : mn;                     // nothing seen so far in this group of lanes
+      const float c = __expf(m[g] - mu);
+      l[g] *= c;
 #pragma unroll
-      for (int e = 0; e < EPL; ++e) o[g][e] = o[g][e] * c + p * vf[e];
+      for (int e = 0; e < 8; ++e) o[g][e] *= c;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        p[u][g] = ok[u] ? __expf(d[u][g] - mu) : 0.f;
+        l[g] += p[u][g];
+      }
       m[g] = mn;
     }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float vf[8];
+      unpack8(vr[u], vf);
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[g][e] += p[u][g] * vf[e];
+    }
   }
+  // the groups of a warp
+#pragma unroll
+  for (int off = LPS; off < 32; off <<= 1)
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const float mo = __shfl_xor_sync(0xffffffffu, m[g], off), mm = fmaxf(m[g], mo);
+      const float f = m[g] == -INFINITY ? 0.f : __expf(m[g] - mm);
+      l[g] *= f;
+      l[g] += __shfl_xor_sync(0xffffffffu, l[g], off);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        o[g][e] *= f;
+        o[g][e] += __shfl_xor_sync(0xffffffffu, o[g][e], off);
+      }
+      m[g] = mm;
+    }
   // merge the four warps through shared memory
-  __shared__ float sm_m[4][G], sm_l[4][G], sm_o[4][G][HD];
+  __shared__ float sm_m[4][G], sm_l[4][G];
+  __shared__ __align__(16) float sm_o[4][G][HD];
 #pragma unroll
   for (int g = 0; g < G; ++g) {
     if (lane == 0) { sm_m[warp][g] = m[g]; sm_l[warp][g] = l[g]; }
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) sm_o[warp][g][lane * EPL + e] = o[g][e];
+    if (grp == 0) {
+      float4* dst = reinterpret_cast<float4*>(&sm_o[warp][g][sub * 8]);
+      dst[0] = make_float4(o[g][0], o[g][1], o[g][2], o[g][3]);
+      dst[1] = make_float4(o[g][4], o[g][5], o[g][6], o[g][7]);
+    }
   }
   __syncthreads();
   for (int t = threadIdx.x; t < G * HD; t += 128) {

@@ -572,3 +572,34 @@ def test_device_sampler_candidate_edges(V, top_k):
         if V > 5000:
             host[3].sample(lg[3].numpy(), [])
             assert 0 <= out.tolist()[3] < V
+
+
+@pytest.mark.parametrize("hd,H,KV", [(64, 3, 1), (64, 8, 1), (32, 6, 1), (128, 2, 2), (128, 4, 2)])
+@pytest.mark.parametrize("n,splits,window", [(1, 1, 0), (15, 1, 0), (16, 1, 0), (17, 1, 7), (64, 2, 0), (129, 1, 0), (200, 8, 33)])
+@pytest.mark.parametrize("off", [0, 1])
+def test_decode_attention_at_slot_edges(hd, H, KV, n, splits, window, off):
+    """Whole and partial trips over the slots, windows that hide whole lanes, caches that are not 16-byte aligned."""
+    D = _D()
+    B, cap, kvd = 3, 208, KV * hd
+    def cache(seed):
+        flat = torch.zeros(B * cap * kvd + 8, device="cuda", dtype=torch.float16)
+        c = flat[off * 2:off * 2 + B * cap * kvd].view(B, cap, kvd)
+        c[:, :n] = _rand(B, n, kvd, seed=seed).cuda().half()
+        c[:, n:] = 60000.0                                      # never read
+        return c
+    cK, cV = cache(1), cache(2)
+    slot_pos = torch.arange(cap, dtype=torch.int32, device="cuda").repeat(B, 1)
+    state = torch.zeros(B, D.STATE_INTS, dtype=torch.int32, device="cuda")
+    state[:, 0] = n - 1                                         # position of the newest token, which is not counted yet
+    state[:, 1] = n - 1
+    q = _rand(B, H * hd, seed=3).cuda().half()
+    out = torch.zeros(B, H * hd, device="cuda", dtype=torch.float16)
+    scratch = torch.zeros(B * H * splits * (hd + 2), device="cuda")
+    D.decode_attn(q, cK, cV, slot_pos, state, out, scratch, splits, H, KV, hd, cap, window, hd ** -0.5)
+    lo = max(0, n - window) if window else 0
+    g = H // KV
+    for h in range(H):
+        s = torch.einsum("bd,bld->bl", q.float()[:, h * hd:(h + 1) * hd], cK[:, lo:n, (h // g) * hd:(h // g + 1) * hd].float()) * hd ** -0.5
+        ref = torch.einsum("bl,bld->bd", torch.softmax(s, -1), cV[:, lo:n, (h // g) * hd:(h // g + 1) * hd].float())
+        # fp32 throughout, rounded once: half a unit of fp16 at these values (below 4)
+        assert (out.float()[:, h * hd:(h + 1) * hd] - ref).abs().max() < 2e-3, (h, lo)
