@@ -70,7 +70,7 @@ struct Tile {
 // write and add), found by one warp from the lengths at hand; it depends on nothing else, so results repeat.
 // Whole against cut, with the addition (us; 9 groups, the last 4 times as long; 98304 rows): 1536 x 768 330 -> 190, 768 x 768
 // 270 -> 115 (floor at 1668 TFLOP/s: 139 and 70); 49152 rows: 1024 x 512 113 -> 62, 512 x 512 113 -> 38.  One group: 1280 x 768 over
-// 32768 rows 67 -> 59, 4096 x 768 over 16384 (one-CTA tiles before) 141 -> 64.
+// 32768 rows 67 -> 59; 4096 x 768 and 768 x 2048 over 16384 (one-CTA tiles before) 142 -> 91 and 113 -> 47.
 struct PiecePlan {
   int base[MAX_PIECE_GROUPS + 1];      // first item of the i-th group from the last
   short len[MAX_PIECE_GROUPS];         // k-blocks of a piece (at most 32767)
