@@ -196,6 +196,22 @@ __global__ void __launch_bounds__(256) decode_route_kernel(const XT* __restrict_
 }
 
 // ---------------------------------------------------------------------------------------------- KV cache
+// Keys, values and positions of the first *n of T prompt rows per sequence into the cache: one warp per row.
+template <typename T>
+__global__ void __launch_bounds__(256) kv_rows_kernel(const T* __restrict__ k, long long ld_k, const T* __restrict__ v, long long ld_v,
+                                                      T* __restrict__ cK, T* __restrict__ cV, int* __restrict__ slot_pos,
+                                                      const int* __restrict__ n, int rows, int Tlen, int cap, int kv_dim) {
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int b = row / Tlen, t = row - b * Tlen;
+  if (row >= rows || t >= min(*n, cap)) return;
+  const long long dst = ((long long)b * cap + t) * kv_dim;
+  for (int i = lane * 8; i < kv_dim; i += 256) {
+    *reinterpret_cast<uint4*>(cK + dst + i) = *reinterpret_cast<const uint4*>(k + row * ld_k + i);
+    *reinterpret_cast<uint4*>(cV + dst + i) = *reinterpret_cast<const uint4*>(v + row * ld_v + i);
+  }
+  if (lane == 0) slot_pos[(long long)b * cap + t] = t;
+}
+
 template <typename T>
 __global__ void kv_append_kernel(const T* __restrict__ k, long long ld_k, const T* __restrict__ v, long long ld_v,
                                  T* __restrict__ cK, T* __restrict__ cV, int* __restrict__ slot_pos,
@@ -778,6 +794,17 @@ extern "C" int gb_kv_append(const void* k16, long long ld_k, const void* v16, lo
   // 16-bit elements of either type are copied as raw bits
   GB_PDL_LAUNCH(kv_append_kernel<__half>, dim3(B), dim3(128), st, (const __half*)k16, ld_k, (const __half*)v16, ld_v, (__half*)cacheK,
                                               (__half*)cacheV, slot_pos, state, cap, pinned, kv_dim);
+  return gb_launch_rc();
+}
+
+extern "C" int gb_kv_rows(const void* k, long long ld_k, const void* v, long long ld_v, void* cK, void* cV, int* slot_pos, const int* n,
+                          int B, int T, int cap, int kv_dim, cudaStream_t st) {
+  if (!k || !v || !cK || !cV || !slot_pos || !n || B <= 0 || T <= 0 || cap < T || kv_dim <= 0 || kv_dim % 8 || ld_k % 8 || ld_v % 8 ||
+      ((reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(cK) | reinterpret_cast<uintptr_t>(cV)) & 15))
+    return -1;
+  const int rows = B * T;                       // copied as they are: one instantiation serves both 16-bit types
+  kv_rows_kernel<__half><<<(rows + 7) / 8, 256, 0, st>>>((const __half*)k, ld_k, (const __half*)v, ld_v, (__half*)cK, (__half*)cV, slot_pos, n,
+                                                         rows, T, cap, kv_dim);
   return gb_launch_rc();
 }
 

@@ -59,6 +59,10 @@ int gb_kv_append(const void* k16, long long ld_k, const void* v16, long long ld_
 int gb_decode_attn(const void* q16, long long ld_q, const void* cacheK, const void* cacheV, const int* slot_pos,
                    const gb_seq_state* state, void* out16, long long ld_o, float* scratch, int splits, int B, int H,
                    int KV, int hd, int cap, int window, float scale, int is_bf16, cudaStream_t st);
+// The first *n (device) of T prompt rows per sequence into slots 0 .. *n - 1 of the caches [B, cap, kv_dim], 16-bit values, and their
+// positions; pointers 16-byte aligned, kv_dim and row pitches multiples of 8, cap >= T.
+int gb_kv_rows(const void* k, long long ld_k, const void* v, long long ld_v, void* cK, void* cV, int* slot_pos, const int* n, int B, int T,
+               int cap, int kv_dim, cudaStream_t st);
 // After the step: abs_pos++, cache_len / ring_start move on; pos_out[b] = new abs_pos (feeds RoPE of the next step).
 int gb_decode_advance(gb_seq_state* state, int* pos_out, int B, int cap, int pinned, cudaStream_t st);
 

@@ -362,10 +362,10 @@ class CudaModel:
         d, qd, kvd, H, KV, hd = cfg.hidden_size, cfg.q_dim, cfg.kv_dim, cfg.num_heads, cfg.num_kv_heads, cfg.head_dim
         E = self.layout.Eff
         K.rmsnorm_fwd(x_in, self.w(p + "attn_norm"), b.xb, b.rrms1, cfg.rms_eps)
+        dec = getattr(self, "decode_engine", None)
         G.gemm(b.xb, self.w16(p + "wqkv"), out=b.qkv)
         qw = self.w(p + "qk_qnorm") if cfg.use_qk_norm else None
         kw = self.w(p + "qk_knorm") if cfg.use_qk_norm else None
-        dec = getattr(self, "decode_engine", None)
         if dec is not None:    # token step of the inference engine (T == 1): this token's k/v go into the cache, the
             #                    query attends over the cache; everything else in this layer is the batched pass
             from ..ops import decode as D
@@ -386,9 +386,8 @@ class CudaModel:
         K.qk_norm_rope_fwd(b.qkv, b.qk, qw, kw, self.cos_sin, self.pos, H, KV, hd, cfg.rms_eps, cfg.rope_type)
         sink = getattr(self, "kv_sink", None)
         if sink is not None:   # prompt pass of the inference engine: keep this layer's keys (after RoPE) and values
-            eng, n = sink
-            eng.layers[l].cK[:, :n].copy_(b.qk.view(self.B, self.T, -1)[:, :n, qd:])
-            eng.layers[l].cV[:, :n].copy_(b.qkv.view(self.B, self.T, -1)[:, :n, qd + kvd:])
+            from ..ops import decode as D
+            D.kv_rows(b.qk[:, qd:], b.qkv[:, qd + kvd:], sink.layers[l].cK, sink.layers[l].cV, sink.slot_pos, sink.prompt_len, self.T)
         if self.attn_tc:   # tcgen05 path (packed-document segment ids are contiguous runs, as the loader emits them)
             K.attn_tc_fwd(b.qk[:, :qd], b.qk[:, qd:], b.qkv[:, qd + kvd:], b.att, b.lse, None, self.seg_lo,
                           self.B, self.T, H, KV, hd, cfg.sliding_window, cfg.attn_scale(), lo_ready=self.use_segments)
@@ -416,6 +415,17 @@ class CudaModel:
         else:
             G.gemm_swiglu(b.xb2, self.w16(p + "w_gu"), act_out=b.act, gu_out=b.gu if train else None)
             G.gemm(b.act, self.w16(p + "w_down"), out=x_out, addend=b.x_mid)
+
+    def prompt_forward(self, eng):
+        """The rows in ``ids`` through all layers, for the keys and values that they leave in the cache of ``eng`` (the logits of a
+        prompt come from the token step of its last token)."""
+        self.kv_sink = eng
+        try:
+            K.embed_fwd(self.ids, self.w("tok_embeddings"), self.x[0])
+            for l in range(self.cfg.num_layers):
+                self._layer_forward(l, self.x[l % 2], self.x[(l + 1) % 2], self.layers[0], False, False)
+        finally:
+            self.kv_sink = None
 
     def decode_forward(self, eng):
         """One token per sequence for the inference engine ``eng`` (this model has T == 1 and B == eng.B): embedding of

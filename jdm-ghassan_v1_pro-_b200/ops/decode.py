@@ -203,6 +203,15 @@ def decode_attn_fused(q16, cacheK, cacheV, slot_pos, state, out16, scratch, tick
     _lib.check_rc(rc, "gb_decode_attn_fused")
 
 
+def kv_rows(k, v, cacheK, cacheV, slot_pos, n_dev, T):
+    """The first ``n_dev`` (device int32) of ``T`` prompt rows of every sequence into the cache, with their positions."""
+    B, cap, kvd = cacheK.shape
+    rc = _lib.lib().gb_kv_rows(c_vp(k.data_ptr()), c_ll(k.stride(0)), c_vp(v.data_ptr()), c_ll(v.stride(0)), c_vp(cacheK.data_ptr()),
+                               c_vp(cacheV.data_ptr()), c_vp(slot_pos.data_ptr()), c_vp(n_dev.data_ptr()), c_int(B), c_int(T), c_int(cap),
+                               c_int(kvd), _lib.stream_ptr())
+    _lib.check_rc(rc, "gb_kv_rows")
+
+
 def decode_advance(state, pos_out, cap, pinned):
     rc = _lib.lib().gb_decode_advance(c_vp(state.data_ptr()), c_vp(pos_out.data_ptr()), c_int(state.shape[0]), c_int(cap),
                                       c_int(pinned), _lib.stream_ptr())

@@ -603,3 +603,29 @@ def test_decode_attention_at_slot_edges(hd, H, KV, n, splits, window, off):
         ref = torch.einsum("bl,bld->bd", torch.softmax(s, -1), cV[:, lo:n, (h // g) * hd:(h // g + 1) * hd].float())
         # fp32 throughout, rounded once: half a unit of fp16 at these values (below 4)
         assert (out.float()[:, h * hd:(h + 1) * hd] - ref).abs().max() < 2e-3, (h, lo)
+
+
+def test_prompt_pass_replays_for_other_prompts():
+    """The second prompt of an engine replays the first one's captured pass: other lengths and tokens, two sequences; cache rows
+    behind the prompt stay as they were."""
+    from ghassan_b200.inference.engine import InferenceEngine
+    from ghassan_b200.models.config import init_parameters
+    cfg = _tiny_cfg(num_heads=4, num_kv_heads=2, hidden_size=256)
+    named = init_parameters(cfg, 5)
+    g = torch.Generator().manual_seed(6)
+    a = InferenceEngine(cfg, named, fmt="f16", batch=2, max_len=160, prefill_chunk=128)
+    for n in (100, 129, 66, 140):                           # 66: a shorter prompt, 140: longer than the chunk
+        prompt = torch.randint(16, 512, (2, n), generator=g, dtype=torch.int32)
+        a.reset(1)
+        for L in a.layers:
+            L.cK.fill_(7.0)
+            L.cV.fill_(7.0)
+        a.prefill(prompt)
+        b = InferenceEngine(cfg, named, fmt="f16", batch=2, max_len=160, prefill_chunk=128)
+        b.reset(1)
+        b.prefill(prompt)                                   # this engine's first: eager
+        assert torch.equal(a.logits, b.logits), n
+        assert a.state.cpu().tolist() == b.state.cpu().tolist() and torch.equal(a.slot_pos[:, :n], b.slot_pos[:, :n])
+        for La, Lb in zip(a.layers, b.layers):
+            assert torch.equal(La.cK[:, :n], Lb.cK[:, :n]) and torch.equal(La.cV[:, :n], Lb.cV[:, :n])
+            assert (La.cK[:, n:] == 7).all() and (La.cV[:, n:] == 7).all()
