@@ -148,6 +148,7 @@ typedef struct gb_moe_args {
   int seg_tokens;
   const float* seg_weight;
   int* status;                       // device status word for kernels with bounded waits (tensor-core router), or NULL
+  int forward_only;                  // gb_moe_group: the pad rows of x_perm keep what they hold (only sums over its rows need zeros)
 } gb_moe_args;
 int gb_moe_seg_ok(int n_tok, int seg_tokens);   // 1 when seg_tokens is usable for a pass of n_tok tokens
 #define GB_ROUTER_WGRAD_CHUNKS 256

@@ -406,7 +406,8 @@ class CudaModel:
             jit = cfg.moe_jitter if train else 0.0
             K.moe_route_group(b.ws, b.xb2, self.w(p + "router"), bias, b.xperm, counts, jitter=jit,
                               seed_dev=self.seed_dev if jit > 0 else None, want_aux=want_aux,
-                              aux_acc=self.aux_acc if want_aux else None, seg_weight=self.dyn_segw if want_aux else None)
+                              aux_acc=self.aux_acc if want_aux else None, seg_weight=self.dyn_segw if want_aux else None,
+                              forward_only=not train)
             G.gemm_swiglu(b.xperm, self.w16(p + "w_gu"), act_out=b.act, gu_out=b.gu if train else None,
                           tile_expert=b.ws.tile_expert, num_m_tiles=b.ws.num_tiles, group_rows=2 * E)
             G.gemm_grouped_rows(b.act, self.w16(p + "w_down"), b.ws.tile_expert, b.ws.num_tiles, n=d, group_rows=d,

@@ -48,7 +48,7 @@ class MoeArgs(ctypes.Structure):
                 ("aux_coef", c_float), ("f_frac", c_void_p), ("d_router_w", c_void_p), ("dx16", c_void_p),
                 ("aux_m", c_void_p), ("part", c_void_p), ("aux_acc", c_void_p), ("dyn_seed", c_void_p),
                 ("dyn_aux_coef", c_void_p), ("part2", c_void_p), ("seg_tokens", c_int), ("seg_weight", c_void_p),
-                ("status", c_void_p)]
+                ("status", c_void_p), ("forward_only", c_int)]
 
 ROUTER_WGRAD_CHUNKS = 256
 
@@ -268,8 +268,9 @@ class MoeWorkspace:
 
 
 def moe_route_group(ws: MoeWorkspace, x16, router_w, bias, x_perm, counts=None, jitter=0.0, jitter_seed=None,
-                    want_aux=False, aux_acc=None, seed_dev=None, seg_weight=None):
-    """``jitter_seed`` (host int) or ``seed_dev`` (uint64 device tensor, read at run time) enables the jitter.
+                    want_aux=False, aux_acc=None, seed_dev=None, seg_weight=None, forward_only=False):
+    """``forward_only``: no weight gradient will sum over the rows of ``x_perm``, so the pad rows between the experts keep what they hold.
+    ``jitter_seed`` (host int) or ``seed_dev`` (uint64 device tensor, read at run time) enables the jitter.
     ``seg_weight`` (fp32 device [ws.n_seg]): weight of each micro-batch's balance loss in ``aux_acc`` (default 1)."""
     a = ws.args()
     a.x16, a.router_w, a.bias = _p(x16), _p(router_w), _p(bias)
@@ -280,6 +281,7 @@ def moe_route_group(ws: MoeWorkspace, x16, router_w, bias, x_perm, counts=None, 
     a.x_perm, a.counts = _p(x_perm), _p(counts)
     a.aux_acc = _p(aux_acc)
     a.seg_weight = _p(seg_weight)
+    a.forward_only = int(forward_only)
     if not want_aux:
         a.aux_m = None
         a.f_frac = None
