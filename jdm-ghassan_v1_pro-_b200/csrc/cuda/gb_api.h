@@ -44,9 +44,13 @@ typedef struct gb_gemm_args {
   float* part; int part_slots, part_cut;  // pair, mode 2, fp32 out accumulated in place, contiguous: scratch of part_slots [M, N] matrices for the
                               // partial sums of reductions that are cut into pieces (at most 64 groups; seg_offsets may be
                               // null for one group over K; part_cut > 0: k-blocks of its pieces).  null: reductions stay whole
+  int skinny;                 // 1: few rows (gemm_skinny_sm100.cu): M <= 128, mode 0, both operands with K contiguous, N a multiple of 8,
+                              // rows of out and addend 16-byte aligned; epilogue 0 or 4.  block_n is ignored
+  int b_static;               // skinny: B is no output of the launch before this one (weights): it may be read ahead of that launch's end
 } gb_gemm_args;
 int gb_gemm(const gb_gemm_args* args, cudaStream_t stream);
 int gb_gemm_pair(const gb_gemm_args* args, cudaStream_t stream);   // what gb_gemm calls when args->pair != 0
+int gb_gemm_skinny(const gb_gemm_args* args, cudaStream_t stream); // what gb_gemm calls when args->skinny != 0
 // Expert segments of the sorted MoE buffers start at multiples of this many rows (two 128-row tiles: one pair tile).
 #define GB_MOE_PAD 256
 

@@ -511,6 +511,7 @@ int dispatch_bn(int bn, const CUtensorMap& ta, const CUtensorMap& tb, const gb::
 extern "C" int gb_gemm(const gb_gemm_args* a, cudaStream_t st) {
   if (!a || a->M <= 0 || a->N <= 0 || a->K < 0) return -1;
   if (a->pair) return gb_gemm_pair(a, st);
+  if (a->skinny) return gb_gemm_skinny(a, st);
   const int bn = a->block_n ? a->block_n : 128;
   if (bn != 64 && bn != 128 && bn != 256) return -1;
   gb::GemmParams p{};

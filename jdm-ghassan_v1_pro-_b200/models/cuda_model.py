@@ -363,7 +363,7 @@ class CudaModel:
         E = self.layout.Eff
         K.rmsnorm_fwd(x_in, self.w(p + "attn_norm"), b.xb, b.rrms1, cfg.rms_eps)
         dec = getattr(self, "decode_engine", None)
-        G.gemm(b.xb, self.w16(p + "wqkv"), out=b.qkv)
+        G.gemm(b.xb, self.w16(p + "wqkv"), out=b.qkv, b_static=dec is not None)
         qw = self.w(p + "qk_qnorm") if cfg.use_qk_norm else None
         kw = self.w(p + "qk_knorm") if cfg.use_qk_norm else None
         if dec is not None:    # token step of the inference engine (T == 1): this token's k/v go into the cache, the
@@ -376,7 +376,7 @@ class CudaModel:
                           dec.cap, cfg.sliding_window, cfg.attn_scale())
         else:
             self._attention_forward(l, b, qw, kw)
-        G.gemm(b.att, self.w16(p + "wo"), out=b.x_mid, addend=x_in)
+        G.gemm(b.att, self.w16(p + "wo"), out=b.x_mid, addend=x_in, b_static=dec is not None)
         K.rmsnorm_fwd(b.x_mid, self.w(p + "ffn_norm"), b.xb2, b.rrms2, cfg.rms_eps)
         self._ffn_forward(l, p, b, x_out, train, want_aux)
 

@@ -196,7 +196,7 @@ class LayerModel:
         if self.dtype == torch.float32:
             K.gemm_f32(a, w, out, rows)
         else:
-            G.gemm(a[:rows], w, out=out[:rows, :w.shape[0]])
+            G.gemm(a[:rows], w, out=out[:rows, :w.shape[0]], b_static=True)
         return out
 
     def _mlp_act(self, w: LayerWeights, rows):
@@ -441,7 +441,7 @@ class LayerModel:
             K.relu2_f32(act, rows, w.w_up.shape[0])
             self.launches += 2
         else:
-            G.gemm(self.x16[:rows], w.w_up, out=act[:rows, :w.w_up.shape[0]], relu2=True)
+            G.gemm(self.x16[:rows], w.w_up, out=act[:rows, :w.w_up.shape[0]], relu2=True, b_static=True)
             self.launches += 1
 
     def _rows_parallel(self, ids, mem, st, slot, B, n, pos0, on_layer):

@@ -40,6 +40,7 @@ class GemmArgs(ctypes.Structure):
         ("tile_out", c_vp),
         ("pair", c_int),
         ("part", c_vp), ("part_slots", c_int), ("part_cut", c_int),
+        ("skinny", c_int), ("b_static", c_int),
     ]
 
 

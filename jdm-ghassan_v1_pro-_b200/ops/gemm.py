@@ -85,18 +85,28 @@ def pick_block_n(M, N, mn_major=False):
     return 128
 
 
-def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_dtype=None, addend=None, block_n=0, pair=None, relu2=False):
+def skinny_ok(M, N, out, addend=None):
+    """True for a product of at most 128 rows (both operands with K contiguous) whose 64-column tiles do not fill the SMs: a cluster
+    of CTAs shares each of them over K (csrc/cuda/gemm_skinny_sm100.cu)."""
+    if M > 128 or N % 8 or (N + 63) // 64 > 148:
+        return False
+    return not any(t.data_ptr() % 16 or (t.stride(-2) * t.element_size()) % 16 for t in (out, addend) if t is not None)
+
+
+def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_dtype=None, addend=None, block_n=0, pair=None, relu2=False, b_static=False):
     """``out = A @ B^T (+ addend)``; ``addend`` is fp32 and may alias an fp32 ``out`` (accumulate).
     ``relu2``: store ``max(A @ B^T, 0) ** 2`` (bf16, no addend).
-    ``pair``: force (True) or forbid (False) the two-CTA kernel; None picks by size."""
+    ``pair``: force (True) or forbid (False) the two-CTA kernel; None picks by size.
+    ``b_static``: ``b`` is not written by the launch before this one (weights), so reading it may begin before that ends."""
     M, K = (a.shape[1], a.shape[0]) if a_mn else (a.shape[0], a.shape[1])
     N, Kb = (b.shape[1], b.shape[0]) if b_mn else (b.shape[0], b.shape[1])
     if K != Kb:
         raise ValueError(f"reduction dims differ: {K} vs {Kb}")
     if out is None:
         out = torch.empty(M, N, dtype=out_dtype or a.dtype, device=a.device)
+    skinny = pair is None and not (block_n or a_mn or b_mn) and skinny_ok(M, N, out, addend)
     if pair is None:
-        pair = (block_n in (0, 256) and (addend is None or out.dtype == torch.float32) and pair_ok(M, N, out))
+        pair = (not skinny and block_n in (0, 256) and (addend is None or out.dtype == torch.float32) and pair_ok(M, N, out))
     if not block_n:
         block_n = pick_block_n(M, N, mn_major=a_mn and b_mn)
     g = _base_args(a, b, M, N, K, a_mn, b_mn, out, block_n)
@@ -104,6 +114,7 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_dtype=None, addend=None,
         raise ValueError("relu2 needs a bf16 output and no addend")
     g.epilogue = EPI_RELU2 if relu2 else EPI_STORE
     g.pair = int(bool(pair))
+    g.skinny, g.b_static = int(skinny), int(b_static)
     if addend is not None:
         if addend.dtype != torch.float32:
             raise ValueError("addend must be fp32")

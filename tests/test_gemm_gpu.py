@@ -364,3 +364,27 @@ def test_weight_gradient_of_one_group_in_pieces(M, N, K):
     L.check_status(what="pieces")
     rel, ok = _close(grad, 0.5 + a.float().t() @ b.float())
     assert ok, rel
+
+
+@pytest.mark.parametrize("M", [1, 7, 8, 31, 33, 64, 100, 128])
+@pytest.mark.parametrize("N,K", [(64, 64), (8, 200), (1000, 72), (1024, 3840), (9472, 128), (2824, 1032)])
+def test_few_rows(M, N, K):
+    """Products of at most 128 rows: edges of the row tile, of 64 columns and of 64-deep k-blocks, one to eight CTAs per tile."""
+    G, L = _ops()
+    for dt in (torch.float16, torch.bfloat16):
+        a, b = _rand(M, K, seed=90).to(dt), (_rand(N, K, seed=91) * 0.3).to(dt)
+        ref = a.float() @ b.float().t()
+        add = torch.randn(M, N + 8, device="cuda")[:, :N]
+        assert G.skinny_ok(M, N, torch.empty(M, N, device="cuda"), add)
+        out = G.gemm(a, b, out_dtype=torch.float32, addend=add)
+        rel, ok = _close(out, ref + add)
+        assert ok, (dt, rel)
+        wide = torch.full((M, N + 16), 7.0, dtype=dt, device="cuda")
+        G.gemm(a, b, out=wide[:, 8:N + 8], b_static=True)
+        rel, ok = _close(wide[:, 8:N + 8], ref)
+        assert ok, (dt, rel)
+        assert (wide[:, :8] == 7).all() and (wide[:, N + 8:] == 7).all()
+    sq = G.gemm(a, b, relu2=True)
+    rel, ok = _close(sq, torch.relu(ref) ** 2)
+    assert ok, rel
+    L.check_status(what="few rows")
