@@ -49,11 +49,18 @@ struct LlGemv {
   void* out; long long ldo; int out_f32; float softcap;
   const float* x0; float alpha; const float* b1; int norm_mode;
   int n1; void* out2; long long ldo2;
+  int staged;                    // the norm weights have room in shared memory
 };
 
-// Input vector of sequence b into xs[0, K).
+// Vectors of norm weights that a prologue applies.  They are constants that a token step reads once, so they come from DRAM: the block
+// has them in shared memory before it waits for the kernel ahead (read where they are applied, behind the sum over the row, they
+// put another DRAM round trip into every product's chain; with the state of the recurrence asked for early, too, a request of 64 tokens
+// went from 26.6 to 25.6 ms: 12 layers, width 1024).
+__host__ __device__ constexpr int ll_norm_vectors(int pro) { return pro == 1 || pro == 5 ? 2 : pro == 3 || pro == 4 ? 1 : 0; }
+
+// Input vector of sequence b into xs[0, K).  w1, w2: the norm weights in shared memory (w2: the last norm's, or the norm's bias).
 template <int PRO, typename XT>
-__device__ __forceinline__ void ll_prologue(const LlGemv& a, int b, XT* __restrict__ xs, float* red, float* part_inv) {
+__device__ __forceinline__ void ll_prologue(const LlGemv& a, int b, XT* __restrict__ xs, float* red, float* part_inv, const float* w1, const float* w2) {
   const int tid = threadIdx.x, d = a.d;
   if constexpr (PRO == 1) {
     const float* xr = a.x + (long long)b * d;
@@ -76,10 +83,10 @@ __device__ __forceinline__ void ll_prologue(const LlGemv& a, int b, XT* __restri
 #pragma unroll
       for (int k = 0; k < KEEP; ++k) {
         const int i = tid + k * LV_THREADS;
-        if (i < d) v[k] = xv[k] + v[k] * inv * a.w1[i];
+        if (i < d) v[k] = xv[k] + v[k] * inv * w1[i];
       }
       for (int i = tid + KEEP * LV_THREADS; i < d; i += LV_THREADS) {
-        const float o = xr[i] + yr[i] * inv * a.w1[i];
+        const float o = xr[i] + yr[i] * inv * w1[i];
         if (writes) a.x_out[(long long)b * d + i] = o;
         xs[i] = Cvt<XT>::from_f(o);
       }
@@ -109,7 +116,7 @@ __device__ __forceinline__ void ll_prologue(const LlGemv& a, int b, XT* __restri
 #pragma unroll
       for (int k = 0; k < KEEP; ++k) {
         const int i = tid + k * LV_THREADS;
-        if (i < d) v[k] = v[k] * inv * a.w2[i];
+        if (i < d) v[k] = v[k] * inv * w2[i];
       }
     }
 #pragma unroll
@@ -122,7 +129,7 @@ __device__ __forceinline__ void ll_prologue(const LlGemv& a, int b, XT* __restri
     float ss = 0.f;
     for (int i = tid; i < d; i += LV_THREADS) { const float v = Cvt<XT>::to_f(xr[i]); ss += v * v; }
     const float inv = ll_inv_rms(ll_block_sum(ss, red), d, a.eps);
-    for (int i = tid; i < d; i += LV_THREADS) xs[i] = Cvt<XT>::from_f(Cvt<XT>::to_f(xr[i]) * inv * a.w1[i]);
+    for (int i = tid; i < d; i += LV_THREADS) xs[i] = Cvt<XT>::from_f(Cvt<XT>::to_f(xr[i]) * inv * w1[i]);
   } else if constexpr (PRO == 5) {                 // residual add, then the norm ahead of the sublayers
     const float* xr = a.x + (long long)b * d;
     const float* yr = a.y ? a.y + b * a.ldy : nullptr;
@@ -154,7 +161,7 @@ __device__ __forceinline__ void ll_prologue(const LlGemv& a, int b, XT* __restri
     const float inv = ll_inv_rms(ll_block_sum(dev, red), d, a.eps);
     auto put = [&](int i, float u) {
       if (xo) xo[i] = u;
-      xs[i] = Cvt<XT>::from_f((u - mean) * inv * a.w1[i] + (a.b1 ? a.b1[i] : 0.f));
+      xs[i] = Cvt<XT>::from_f((u - mean) * inv * w1[i] + (a.b1 ? w2[i] : 0.f));
     };
 #pragma unroll
     for (int k = 0; k < KEEP; ++k) {
@@ -174,7 +181,7 @@ __device__ __forceinline__ void ll_prologue(const LlGemv& a, int b, XT* __restri
     }
     __syncthreads();
 #pragma unroll 4
-    for (int i = tid; i < d; i += LV_THREADS) xs[i] = Cvt<XT>::from_f(vr[i] * part_inv[i / per] * a.w1[i]);
+    for (int i = tid; i < d; i += LV_THREADS) xs[i] = Cvt<XT>::from_f(vr[i] * part_inv[i / per] * w1[i]);
     __syncthreads();                               // part_inv is the next sequence's, too
   } else {                                         // PRO == 2: gated norm in equal parts, one warp per part
     const XT* yr = reinterpret_cast<const XT*>(a.y16) + b * a.ldy16;
@@ -280,11 +287,21 @@ __global__ void __launch_bounds__(LV_THREADS) ll_gemv_kernel(const __grid_consta
       }
   };
   fetch(blockIdx.x * RPB + ric);
+  constexpr int NV = ll_norm_vectors(PRO);
+  float* norm_w = reinterpret_cast<float*>(lv_dyn + (((size_t)a.B * a.K * sizeof(XT) + 15) & ~(size_t)15));
+  const float* second = PRO == 1 ? a.w2 : a.b1;
+  if (NV > 0 && a.staged) {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < a.d; i += LV_THREADS) {
+      if (PRO != 1 || a.y) norm_w[i] = a.w1[i];
+      if (NV > 1 && second) norm_w[a.d + i] = second[i];
+    }
+  }
   pdl_wait();
   const XT* xin = reinterpret_cast<const XT*>(a.x16);
   long long ldx = a.ldx;
   if constexpr (PRO != 0) {
-    for (int b = 0; b < a.B; ++b) ll_prologue<PRO, XT>(a, b, xs + (long long)b * a.K, red, part_inv);
+    for (int b = 0; b < a.B; ++b) ll_prologue<PRO, XT>(a, b, xs + (long long)b * a.K, red, part_inv, a.staged ? norm_w : a.w1, a.staged ? norm_w + a.d : second);
     __syncthreads();
     xin = xs;
     ldx = a.K;
@@ -357,9 +374,11 @@ __global__ void __launch_bounds__(LV_THREADS) ll_gemv_kernel(const __grid_consta
 }
 
 template <int FMT, typename XT, int PRO, int SWI>
-static int ll_gemv_go(const LlGemv& a, cudaStream_t st) {
-  const size_t smem = PRO ? (size_t)a.B * a.K * sizeof(XT) : 0;
-  if (smem > 200 * 1024) return -3;
+static int ll_gemv_go(LlGemv a, cudaStream_t st) {
+  const size_t rows = PRO ? ((size_t)a.B * a.K * sizeof(XT) + 15) & ~(size_t)15 : 0, norms = (size_t)ll_norm_vectors(PRO) * a.d * sizeof(float);
+  if (PRO && (size_t)a.B * a.K * sizeof(XT) > 200 * 1024) return -3;
+  a.staged = rows + norms <= 200 * 1024;
+  const size_t smem = rows + (a.staged ? norms : 0);
   const int n_out = SWI ? a.N / 2 : a.N;
   // warps per row: enough of them to keep loads in flight on every SM, more for long rows
   const int units = a.K >> 3;

@@ -397,3 +397,24 @@ def test_embedding_gather_scatter():
     for t in torch.nonzero(ids == first).flatten().tolist():
         seq = seq + dx[t]
     assert torch.equal(runs[0][first], 0.25 + seq) or near(runs[0][first], 0.25 + seq)[0]
+
+
+@pytest.mark.parametrize("n,d", [(1, 768), (7, 256), (8, 1024), (9, 512), (32, 768)])
+def test_moe_few_tokens_and_forward_only(n, d):
+    """A token per warp up to eight a block; a pass without weight gradients leaves the pad rows as they are."""
+    k, r = K(), R()
+    from ghassan_b200.models.config import ModelConfig
+    ne, Kk = 8, 2
+    x16, rw = _moe_setup(n, d, ne, Kk, True)
+    probs, idx, w = r.route(x16.float(), rw, None, ModelConfig(num_experts=ne, moe_top_k=Kk, moe_allow_dense=True), None)
+    ws = [k.MoeWorkspace(n, d, ne, Kk, True, torch.float16, "cuda") for _ in range(2)]
+    xp = [torch.full((ws[0].cap, d), 7.0, dtype=torch.float16, device="cuda") for _ in range(2)]
+    for i in range(2):
+        k.moe_route_group(ws[i], x16, rw, None, xp[i], forward_only=bool(i))
+    assert near(ws[0].probs, probs)[0] and torch.equal(ws[0].idx.long(), idx)
+    assert torch.equal(ws[0].slot_pos, ws[1].slot_pos) and torch.equal(ws[0].seg_offsets, ws[1].seg_offsets)
+    real = torch.zeros(ws[0].cap, dtype=torch.bool, device="cuda")
+    real[ws[0].slot_pos.reshape(-1).long()] = True
+    used = int(ws[0].seg_offsets[ne + 1])
+    assert torch.equal(xp[0][real], xp[1][real])
+    assert (xp[0][:used][~real[:used]] == 0).all() and (xp[1][~real] == 7).all()
