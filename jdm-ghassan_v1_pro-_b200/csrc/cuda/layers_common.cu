@@ -271,9 +271,12 @@ extern "C" int gb_ll_norm_rows(const float* x, const int* row_idx, const float* 
 }
 
 // a warp per row while the row fits its registers, else a block per row
+// A warp per row of up to 1024 values, once there are more rows than the SMs hold blocks: fewer rows get a block each, whose threads
+// have one load to wait for instead of eight (add and layer norm of 32 x 1024: 5.0 -> 2.6 us, 300 x 1024: 5.2 -> 3.0).
+constexpr int LL_BLOCK_ROWS = 4 * 148;
 #define LL_ROWS(KERN, T, ...)                                                                                                 \
   do {                                                                                                                       \
-    if (d <= 1024) {                                                                                                         \
+    if (d <= 1024 && rows > LL_BLOCK_ROWS) {                                                                                 \
       if (vec) GB_PDL_LAUNCH((KERN<T, 32, 4>), dim3((rows + 7) / 8), dim3(256), st, __VA_ARGS__);                               \
       else GB_PDL_LAUNCH((KERN<T, 32, 1>), dim3((rows + 7) / 8), dim3(256), st, __VA_ARGS__);                                   \
     } else if (vec) GB_PDL_LAUNCH((KERN<T, 256, 4>), dim3(rows), dim3(256), st, __VA_ARGS__);                                   \
