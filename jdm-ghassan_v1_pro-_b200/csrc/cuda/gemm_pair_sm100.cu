@@ -726,7 +726,7 @@ extern "C" int gb_gemm_pair(const gb_gemm_args* a, cudaStream_t st) {
     // pieces of reductions: fp32 sums into [groups, M, N] without gaps
     if (a->mode != 2 || !p.reduce || ot != 2 || a->part_slots < 1 || p.groups > pr::MAX_PIECE_GROUPS || a->epilogue != pr::EPI_STORE ||
         a->ldo != a->N || a->N % 4 || (groups > 1 && (!a->seg_offsets || a->out_group_stride != (long long)a->M * a->N)) ||
-        (reinterpret_cast<uintptr_t>(a->part) & 15)) return -26;
+        (reinterpret_cast<uintptr_t>(a->part) & 15) || a->a_rows > 32767ll * pr::BK) return -26;      // a whole reduction is a plan, too
     p.part_slots = a->part_slots;
     p.part_cut = a->part_cut;
     // a cut given by the caller is for one group, whose pieces have to fit

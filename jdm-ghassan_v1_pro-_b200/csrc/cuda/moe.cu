@@ -132,8 +132,8 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const gb_moe_args a) {
 #pragma unroll
           for (int u = 0; u < 2; ++u)
             if (u == 0 || two)
-            s[u] += xf[u][k][0] * w0.x + xf[u][k][1] * w0.y + xf[u][k][2] * w0.z + xf[u][k][3] * w0.w +
-                    xf[u][k][4] * w1.x + xf[u][k][5] * w1.y + xf[u][k][6] * w1.z + xf[u][k][7] * w1.w;
+              s[u] += xf[u][k][0] * w0.x + xf[u][k][1] * w0.y + xf[u][k][2] * w0.z + xf[u][k][3] * w0.w +
+                      xf[u][k][4] * w1.x + xf[u][k][5] * w1.y + xf[u][k][6] * w1.z + xf[u][k][7] * w1.w;
         }
 #pragma unroll
         for (int u = 0; u < 2; ++u) {

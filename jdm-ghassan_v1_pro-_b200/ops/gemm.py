@@ -267,7 +267,7 @@ def _piece_scratch(M, N, kblocks, groups, out, longest=0):
     blocks of 64 rows in all, or None where they stay whole.  ``longest``: k-blocks of a group known to be longer than the others.  Taken from the allocator for this call, so
     calls on other streams have their own."""
     tiles = pair_tiles(M, N)
-    if not PAIR_ENABLED or N % 4 or groups > 64 or tiles * kblocks * (2 if groups == 1 else 1) < 74 * PIECE_MIN_KBLOCKS or not pair_ok(M, N, out, groups=60):
+    if not PAIR_ENABLED or N % 4 or groups > 64 or kblocks > 32000 or tiles * kblocks * (2 if groups == 1 else 1) < 74 * PIECE_MIN_KBLOCKS or not pair_ok(M, N, out, groups=60):
         return None
     if tiles * groups >= 3 * 74:             # three rounds of whole reductions and more: little idles at the end
         return None
