@@ -88,7 +88,9 @@ __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1) attn_tc_fwd_kern
   uint64_t* s_empty = bars + 9;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  __nv_bfloat16* row_max = reinterpret_cast<__nv_bfloat16*>(bars + 16);     // [2 halves][128 rows]; between items 128 floats
+  // 128 bytes for each lane quarter: its rows' maxima ([2 halves][32], 16 bits), between items its rows' sums ([32], fp32).  The two warps
+  // of a quarter are all that its named barrier joins, and another quarter may be an item ahead, so no byte is shared by quarters.
+  uint8_t* exchange = reinterpret_cast<uint8_t*>(bars + 16);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Work items: (query tile, batch, head), the query tile slowest and from the last one down: under a causal mask that
@@ -202,6 +204,8 @@ __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1) attn_tc_fwd_kern
     const int half = warp >> 2, r = (warp & 3) * 32 + lane;                  // key half, query row of the tile
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const float sc2 = p.scale * 1.4426950408889634f;       // scores in log2 units: exp(x * scale) = 2^(x * sc2)
+    __nv_bfloat16* row_max = reinterpret_cast<__nv_bfloat16*>(exchange + (warp & 3) * 128);
+    float* row_sum = reinterpret_cast<float*>(row_max);
     auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"((warp & 3) + 1) : "memory"); };   // the two warps of a quarter
     uint32_t tile_it = 0;
     for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
@@ -246,9 +250,9 @@ __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1) attn_tc_fwd_kern
         }
         // The halves meet: any number that both use will do as the maximum, so it travels rounded up to 16 bits.
         const __nv_bfloat16 m16 = __float2bfloat16_ru(mt);
-        row_max[half * AT_M + r] = m16;
+        row_max[half * 32 + lane] = m16;
         pair_sync();
-        mt = fmaxf(__bfloat162float(m16), __bfloat162float(row_max[(half ^ 1) * AT_M + r]));
+        mt = fmaxf(__bfloat162float(m16), __bfloat162float(row_max[(half ^ 1) * 32 + lane]));
         tc_fence_before();
         if (lane == 0) mbar_arrive(s_empty);    // scores and the partner's maximum are in registers
         // a new maximum is taken when some row of the warp needs it (the accumulator rows are reached by warp-wide
@@ -307,16 +311,15 @@ __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1) attn_tc_fwd_kern
         __syncwarp();                 // every lane's writes and fences, then one arrival for the warp
         if (lane == 0) mbar_arrive(p_ready);
       }
-      // the item's last P V (every warp is past its last exchange of maxima then)
+      // the item's last P V
       wait_or_report(o_full, (tile_it - 1u) & 1u, p.status, ST_TIMEOUT_TMEM_FULL, abort_flag);
-      float* row_sum = reinterpret_cast<float*>(row_max);
       pair_sync();
-      if (half == 1) row_sum[r] = l;
+      if (half == 1) row_sum[lane] = l;
       pair_sync();
-      if (half == 0) { l += row_sum[r]; row_sum[r] = l; }
+      if (half == 0) { l += row_sum[lane]; row_sum[lane] = l; }
       pair_sync();
-      if (half == 1) l = row_sum[r];
-      pair_sync();                    // read before the next item's maxima take the place
+      if (half == 1) l = row_sum[lane];
+      pair_sync();                    // read before the quarter's next maxima take the place
       tc_fence_after();
       const float inv_l = l > 0.f ? 1.f / l : 0.f;
       T* op = reinterpret_cast<T*>(p.o) + (row_base + i) * p.ld_o + (long long)h * HD + half * (HD / 2);

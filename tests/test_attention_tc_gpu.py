@@ -167,3 +167,42 @@ ITEM_CASES = [
 @pytest.mark.parametrize("B,T,H,KV,hd,window,use_seg", ITEM_CASES)
 def test_tc_attention_at_item_edges(dt, B, T, H, KV, hd, window, use_seg):
     test_tc_attention_matches_oracle(dt, B, T, H, KV, hd, window, use_seg)
+
+
+def _lse(q, k, B, T, H, KV, scale, vis):
+    """Log-sum-exp [B * T, H] of the visible scores, in fp64, a sequence at a time; ``vis`` is [B, T, T]."""
+    hd = q.shape[1] // H
+    out = []
+    for b in range(B):
+        s = torch.einsum("ihd,jhd->hij", q.view(B, T, H, hd)[b].double(), k.view(B, T, KV, hd)[b].double().repeat_interleave(H // KV, dim=1)) * scale
+        out.append(torch.logsumexp(s.masked_fill(~vis[b], float("-inf")), dim=-1).t())
+    return torch.cat(out).contiguous()
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("B,T,H,KV,hd", [(24, 700, 12, 4, 64), (8, 520, 16, 4, 128)])
+def test_tc_attention_forward_many_uneven_items_per_block(dt, B, T, H, KV, hd):
+    """Every CTA walks many work items whose numbers of key tiles differ (documents of uneven lengths), so its warps are an item apart
+    now and then: outputs and log-sum-exp equal the oracle's and, bit for bit, those of every other run."""
+    from ghassan_b200.models import reference as R
+    from ghassan_b200.ops import _lib, kernels as K
+    n, scale = B * T, hd ** -0.5
+    q, k, v = rnd(n, H * hd, seed=31, dtype=dt), rnd(n, KV * hd, seed=32, dtype=dt), rnd(n, KV * hd, seed=33, dtype=dt)
+    g = torch.Generator().manual_seed(34)
+    seg = (torch.rand(B, T, generator=g) < torch.tensor([0.0, 0.003, 0.01, 0.1])[torch.arange(B) % 4, None]).cumsum(1).to(torch.int32).cuda()
+    lo = torch.empty(n, dtype=torch.int32, device="cuda")
+    first = None
+    for _ in range(20):
+        o, lse = torch.empty(n, H * hd, dtype=dt, device="cuda"), torch.empty(n, H, device="cuda")
+        K.attn_tc_fwd(q, k, v, o, lse, seg.view(-1), lo, B, T, H, KV, hd, 0, scale)
+        _lib.check_status(what="attn_tc_fwd")
+        if first is None:
+            first = (o, lse)
+            ref = R.attention(q.float().view(n, H, hd), k.float().view(n, KV, hd), v.float().view(n, KV, hd), B, T, scale, 0, seg.view(-1))
+            ok, err, rule = near(o, ref)
+            assert ok, ("o", err, rule)
+            ar = torch.arange(T, device="cuda")
+            vis = (ar[None, :] <= ar[:, None])[None] & (seg[:, None, :] == seg[:, :, None])
+            ok, err, rule = near(lse, _lse(q, k, B, T, H, KV, scale, vis).float(), chain=False)
+            assert ok, ("lse", err, rule)
+        assert torch.equal(o, first[0]) and torch.equal(lse, first[1])
