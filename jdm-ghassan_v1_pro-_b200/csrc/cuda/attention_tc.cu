@@ -51,6 +51,10 @@ struct AttnTcParams {
   int* status;
 };
 
+// Integers in the order of the floats (and back).
+__device__ __forceinline__ int at_order(float f) { const int i = __float_as_int(f); return i ^ ((i >> 31) & 0x7fffffff); }
+__device__ __forceinline__ float at_order_back(int i) { return __int_as_float(i ^ ((i >> 31) & 0x7fffffff)); }
+
 // ============================================================================================ forward
 template <typename T, int HD>
 __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1) attn_tc_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
@@ -61,7 +65,7 @@ __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1) attn_tc_fwd_kern
   constexpr uint32_t TILE = AT_M * HD * 2;
   uint8_t* smem;
   if constexpr (HD == 64) {
-    // 112 KB of tiles, 640 bytes of barriers and maxima and not a byte more: two CTAs of this kernel share an SM (256 TMEM
+    // 112 KB of tiles, 640 bytes of barriers and row words and not a byte more: two CTAs of this kernel share an SM (256 TMEM
     // columns each), which hides the latency of the short causal loops at T = 512.  That leaves no slack to align
     // the base by hand; the kernel has no static shared memory, so the dynamic window starts 1024-aligned.  Checked,
     // not assumed: a misaligned base reports and returns before any barrier or TMEM is touched.
@@ -88,9 +92,10 @@ __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1) attn_tc_fwd_kern
   uint64_t* s_empty = bars + 9;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  // 128 bytes for each lane quarter: its rows' maxima ([2 halves][32], 16 bits), between items its rows' sums ([32], fp32).  The two warps
-  // of a quarter are all that its named barrier joins, and another quarter may be an item ahead, so no byte is shared by quarters.
-  uint8_t* exchange = reinterpret_cast<uint8_t*>(bars + 16);
+  // One word a row, where the two threads of a row meet: during an item its maximum so far, at the end its sum.  Both layouts are by
+  // row, so a lane quarter keeps to its own 128 bytes: its two warps are all that its named barrier joins, and another quarter may be
+  // an item ahead.
+  int* row_word = reinterpret_cast<int*>(bars + 16);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Work items: (query tile, batch, head), the query tile slowest and from the last one down: under a causal mask that
@@ -113,6 +118,7 @@ __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1) attn_tc_fwd_kern
     *abort_flag = 0;
     fence_barrier_init();
   }
+  if (threadIdx.x < AT_M) row_word[threadIdx.x] = at_order(-INFINITY);
   if (warp == AT_FWD_CW + 1) { tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
@@ -204,8 +210,6 @@ __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1) attn_tc_fwd_kern
     const int half = warp >> 2, r = (warp & 3) * 32 + lane;                  // key half, query row of the tile
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const float sc2 = p.scale * 1.4426950408889634f;       // scores in log2 units: exp(x * scale) = 2^(x * sc2)
-    __nv_bfloat16* row_max = reinterpret_cast<__nv_bfloat16*>(exchange + (warp & 3) * 128);
-    float* row_sum = reinterpret_cast<float*>(row_max);
     auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"((warp & 3) + 1) : "memory"); };   // the two warps of a quarter
     uint32_t tile_it = 0;
     for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
@@ -248,12 +252,13 @@ __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1) attn_tc_fwd_kern
           for (int k = 0; k < 32; ++k) mr[k & 3] = fmaxf(mr[k & 3], fmaxf(__uint_as_float(r0[k]), __uint_as_float(r1[k])));
           mt = fmaxf(fmaxf(mr[0], mr[1]), fmaxf(mr[2], mr[3])) * sc2;
         }
-        // The halves meet: any number that both use will do as the maximum, so it travels rounded up to 16 bits.
-        const __nv_bfloat16 m16 = __float2bfloat16_ru(mt);
-        row_max[half * 32 + lane] = m16;
+        // The halves meet: the row's maximum over this tile and the ones before it, exact (rounded to 16 bits it would leave
+        // scores of thousands with probabilities that fp16 cannot hold).
+        atomicMax(&row_word[r], at_order(mt));
         pair_sync();
-        mt = fmaxf(__bfloat162float(m16), __bfloat162float(row_max[(half ^ 1) * 32 + lane]));
+        mt = at_order_back(row_word[r]);
         tc_fence_before();
+        __syncwarp();                           // every lane has read its word: it is written again once s_empty is complete
         if (lane == 0) mbar_arrive(s_empty);    // scores and the partner's maximum are in registers
         // a new maximum is taken when some row of the warp needs it (the accumulator rows are reached by warp-wide
         // tensor-memory loads and stores, so the decision is the warp's; both warps of a quarter see the same maxima)
@@ -261,10 +266,9 @@ __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1) attn_tc_fwd_kern
         const bool rescale = __any_sync(0xffffffffu, grow);
         float corr = 1.f;
         if (rescale) {
-          const float m_new = fmaxf(m2, mt);
-          if (m2 != -INFINITY) corr = exp2f(m2 - m_new);                    // else nothing accumulated yet
+          if (m2 != -INFINITY) corr = exp2f(m2 - mt);                       // else nothing accumulated yet
           l *= corr;
-          m2 = m_new;
+          m2 = mt;
         }
         const float mu = m2 == -INFINITY ? 0.f : m2;       // a row that sees no key so far: every score is -inf
         float ls[2] = {0.f, 0.f};
@@ -314,12 +318,12 @@ __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1) attn_tc_fwd_kern
       // the item's last P V
       wait_or_report(o_full, (tile_it - 1u) & 1u, p.status, ST_TIMEOUT_TMEM_FULL, abort_flag);
       pair_sync();
-      if (half == 1) row_sum[lane] = l;
+      if (half == 1) row_word[r] = __float_as_int(l);
       pair_sync();
-      if (half == 0) { l += row_sum[lane]; row_sum[lane] = l; }
+      if (half == 0) { l += __int_as_float(row_word[r]); row_word[r] = __float_as_int(l); }
       pair_sync();
-      if (half == 1) l = row_sum[lane];
-      pair_sync();                    // read before the quarter's next maxima take the place
+      if (half == 1) { l = __int_as_float(row_word[r]); row_word[r] = at_order(-INFINITY); }
+      pair_sync();                    // the word is free for the next item's maxima
       tc_fence_after();
       const float inv_l = l > 0.f ? 1.f / l : 0.f;
       T* op = reinterpret_cast<T*>(p.o) + (row_base + i) * p.ld_o + (long long)h * HD + half * (HD / 2);

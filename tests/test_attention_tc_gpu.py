@@ -206,3 +206,50 @@ def test_tc_attention_forward_many_uneven_items_per_block(dt, B, T, H, KV, hd):
             ok, err, rule = near(lse, _lse(q, k, B, T, H, KV, scale, vis).float(), chain=False)
             assert ok, ("lse", err, rule)
         assert torch.equal(o, first[0]) and torch.equal(lse, first[1])
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T,H,KV,hd,use_seg", [(100, 2, 2, 64, False), (700, 4, 2, 64, True), (96, 2, 1, 128, False), (520, 4, 2, 128, True)])
+def test_tc_attention_scores_of_thousands(dt, T, H, KV, hd, use_seg):
+    """Row maxima of about 3,000 to 9,000 in log2 units (nothing bounds scores without a norm on queries and keys): the largest
+    probability of a row still has to be stored as about 1.  Allowances are sums of absolute values times eps: 16-bit probabilities, score gradients
+    and outputs (2^-10, bf16 2^-7), and the exponent's fp32 roundings (scores, log-sum-exp, their difference: 8 x 2^-23 of the score's terms)."""
+    from ghassan_b200.ops import _lib, kernels as K
+    B, scale, rep = 2, hd ** -0.5, H // KV
+    n = B * T
+    for top in (3000.0, 9000.0):
+        amp = (top / 1.4427 / 3.0) ** 0.5                   # scores are N(0, amp^4): a row's largest is about three deviations
+        q, k = ((rnd(n, m * hd, seed=40 + m, dtype=torch.float32) * amp).to(dt) for m in (H, KV))
+        v, g = rnd(n, KV * hd, seed=51, dtype=dt), rnd(n, H * hd, seed=52, dtype=dt)
+        seg = (torch.arange(T, device="cuda") // 150).repeat(B).to(torch.int32) if use_seg else None
+        lo = torch.empty(n, dtype=torch.int32, device="cuda")
+        o, lse, delta = torch.empty_like(q), torch.empty(n, H, device="cuda"), torch.empty(n, H, device="cuda")
+        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+        K.attn_tc_fwd(q, k, v, o, lse, seg, lo, B, T, H, KV, hd, 0, scale)
+        K.attn_tc_bwd(q, k, v, o, lse, seg, lo, g, delta, dq, dk, dv, B, T, H, KV, hd, 0, scale)
+        _lib.check_status(what="attention")
+        ar = torch.arange(T, device="cuda")
+        vis = ar[None, :] <= ar[:, None]
+        if use_seg:
+            vis = vis & (ar[None, :] // 150 == ar[:, None] // 150)
+        heads = lambda t, m: t.double().view(B, T, m, hd).transpose(1, 2)
+        Q, G, Ov = heads(q, H), heads(g, H), heads(o, H)
+        Kh, V = (heads(t, KV).repeat_interleave(rep, dim=1) for t in (k, v))
+        S = (Q @ Kh.transpose(2, 3) * scale).masked_fill(~vis, float("-inf"))
+        P = torch.softmax(S, dim=-1)
+        terms = float((Q.abs() @ Kh.abs().transpose(2, 3) * scale * vis).max())
+        eps = (2.0 ** -10 if dt == torch.float16 else 2.0 ** -7) + 8 * 2.0 ** -23 * terms
+        want = P @ V
+        dP = G @ V.transpose(2, 3)
+        dS = P * (dP - (P * dP).sum(-1, keepdim=True))
+        aS = P * (G.abs() @ V.abs().transpose(2, 3) + (G.abs() * want.abs()).sum(-1, keepdim=True))
+        fold = lambda t: t.view(B, KV, rep, T, hd).sum(2)
+        tiny = 2.0 ** -24 * T                               # probabilities and score gradients below fp16's smallest step
+        for name, got, ref, room in (("o", Ov, want, P @ V.abs()), ("dq", heads(dq, H), dS @ Kh * scale, aS @ Kh.abs() * scale),
+                                     ("dk", heads(dk, KV), fold(dS.transpose(2, 3) @ Q) * scale, fold(aS.transpose(2, 3) @ Q.abs()) * scale),
+                                     ("dv", heads(dv, KV), fold(P.transpose(2, 3) @ G), fold(P.transpose(2, 3) @ G.abs()))):
+            mag = {"o": V, "dq": Kh, "dk": Q, "dv": G}[name].abs().max()
+            worst = float(((got - ref).abs() / (eps * room + tiny * mag)).max())
+            assert worst <= 1.0, (name, top, worst)
+        err = float((heads(lse.repeat_interleave(hd, dim=1), H)[..., 0] - torch.logsumexp(S, dim=-1)).abs().max())
+        assert err <= 8 * 2.0 ** -23 * terms, ("lse", top, err)
