@@ -736,6 +736,7 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dq64_kernel(co
         tmem_ld_32x32(tmem_dP + lane_base + cq * 32, rp);
         tmem_ld_wait();
         tc_fence_before();
+        __syncwarp();                 // every lane's reads and fences, then one arrival for the warp
         if (lane == 0) mbar_arrive(sdp_empty);
         float ds[32];
         if (!need_mask) {
@@ -1285,6 +1286,7 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
         tmem_ld_32x32(tmem_dPT + lane_base + cq * 32, rp);
         tmem_ld_wait();
         tc_fence_before();
+        __syncwarp();                 // every lane's reads and fences, then one arrival for the warp
         if (lane == 0) mbar_arrive(st_empty);
         // the statistics come as 16-byte loads (every lane reads the same words), four queries at a time; P and dS are
         // packed as they come, in place of the scores
