@@ -150,12 +150,12 @@ __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1) attn_tc_fwd_kern
         const int kvh = h / rep;
         const int row_base = b * p.T;
         // the tensor core has read the previous item's Q (committed after its last score tile)
-        wait_or_report(q_empty, (q_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+        wait_or_leave(q_empty, (q_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag);
         mbar_arrive_expect_tx_on(on, q_full, TILE);
         load_tile<HD>(on, &tmQ, q_full, sQ, h * HD, row_base + q0);
         for (int t = 0; t < n_tiles; ++t, ++kv_it) {
           const int s = kv_it & 1, ph = (kv_it >> 1) & 1;
-          wait_or_report(&kv_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+          wait_or_leave(&kv_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
           mbar_arrive_expect_tx_on(on, &kv_full[s], 2 * TILE);
           load_tile<HD>(on, &tmK, &kv_full[s], sK + s * TILE, kvh * HD, row_base + k_lo + t * AT_N);
           load_tile<HD>(on, &tmV, &kv_full[s], sV + s * TILE, kvh * HD, row_base + k_lo + t * AT_N);
@@ -433,13 +433,13 @@ __global__ void __launch_bounds__(AT_BWD_THREADS) attn_tc_bwd_dq_kernel(const __
         const int kvh = h / rep;
         const int row_base = b * p.T;
         // Q and dO of the previous item have been read (committed after its last S / dP)
-        wait_or_report(q_empty, (q_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+        wait_or_leave(q_empty, (q_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag);
         mbar_arrive_expect_tx_on(on, q_full, 2 * TILE);
         load_tile<HD>(on, &tmQ, q_full, sQ, h * HD, row_base + q0);
         load_tile<HD>(on, &tmDO, q_full, sDO, h * HD, row_base + q0);
         for (int t = 0; t < n_tiles; ++t, ++kv_it) {
           const int s = kv_it % STAGES, ph = (kv_it / STAGES) & 1;
-          wait_or_report(&kv_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+          wait_or_leave(&kv_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
           mbar_arrive_expect_tx_on(on, &kv_full[s], 2 * TILE);
           load_tile<HD>(on, &tmK, &kv_full[s], sK + s * TILE, kvh * HD, row_base + k_lo + t * AT_N);
           load_tile<HD>(on, &tmV, &kv_full[s], sV + s * TILE, kvh * HD, row_base + k_lo + t * AT_N);
@@ -652,13 +652,13 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dq64_kernel(co
         item_range(item, b, h, q0, k_lo, n_steps);
         const int kvh = h / rep;
         const int row_base = b * p.T;
-        wait_or_report(q_empty, (q_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+        wait_or_leave(q_empty, (q_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag);
         mbar_arrive_expect_tx_on(on, q_full, 2 * TILE);
         load_tile<HD>(on, &tmQ, q_full, sQ, h * HD, row_base + q0);
         load_tile<HD>(on, &tmDO, q_full, sDO, h * HD, row_base + q0);
         for (int t = 0; t < n_steps; ++t, ++kv_it) {
           const int s = kv_it % ST, ph = (kv_it / ST) & 1;
-          wait_or_report(&kv_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+          wait_or_leave(&kv_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
           mbar_arrive_expect_tx_on(on, &kv_full[s], 2 * KTILE);
           tma_load_2d_on(on, &tmK, &kv_full[s], sK + s * KTILE, kvh * HD, row_base + k_lo + t * KN);
           tma_load_2d_on(on, &tmV, &kv_full[s], sV + s * KTILE, kvh * HD, row_base + k_lo + t * KN);
@@ -887,7 +887,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS) attn_tc_bwd_dkv_kernel(const _
         item_range(item, b, kvh, j0, n_qt);
         const int row_base = b * p.T;
         // K and V of the previous item have been read (committed after its last S^T / dP^T)
-        wait_or_report(kv_empty, (item_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+        wait_or_leave(kv_empty, (item_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag);
         mbar_arrive_expect_tx_on(on, kv_full, 2 * TILE);
         load_tile<HD>(on, &tmK, kv_full, sK, kvh * HD, row_base + j0);
         load_tile<HD>(on, &tmV, kv_full, sV, kvh * HD, row_base + j0);
@@ -896,7 +896,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS) attn_tc_bwd_dkv_kernel(const _
           const int s = g_it % STAGES, ph = (g_it / STAGES) & 1;
           const int h = kvh * group + it / n_qt;
           const int i0 = j0 + (it % n_qt) * AT_M;
-          wait_or_report(&q_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+          wait_or_leave(&q_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
           mbar_arrive_expect_tx_on(on, &q_full[s], 2 * TILE);
           load_tile<HD>(on, &tmQ, &q_full[s], sQ + s * TILE, h * HD, row_base + i0);
           load_tile<HD>(on, &tmDO, &q_full[s], sDO + s * TILE, h * HD, row_base + i0);
@@ -1166,7 +1166,7 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
         int b, kvh, j0, n_qs;
         item_range(item, b, kvh, j0, n_qs);
         const int row_base = b * p.T;
-        wait_or_report(kv_empty, (item_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+        wait_or_leave(kv_empty, (item_it & 1u) ^ 1u, p.status, ST_TIMEOUT_EMPTY, abort_flag);
         mbar_arrive_expect_tx_on(on, kv_full, 2 * TILE);
         load_tile<HD>(on, &tmK, kv_full, sK, kvh * HD, row_base + j0);
         load_tile<HD>(on, &tmV, kv_full, sV, kvh * HD, row_base + j0);
@@ -1175,7 +1175,7 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
         for (int it = 0; it < n_it; ++it, ++g_it) {
           const int s = g_it % ST, ph = (g_it / ST) & 1;
           const int i0 = j0 + qi * QN;
-          wait_or_report(&q_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+          wait_or_leave(&q_empty[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
           mbar_arrive_expect_tx_on(on, &q_full[s], 2 * QTILE);
           tma_load_2d_on(on, &tmQ, &q_full[s], sQ + s * QTILE, h * HD, row_base + i0);
           tma_load_2d_on(on, &tmDO, &q_full[s], sDO + s * QTILE, h * HD, row_base + i0);

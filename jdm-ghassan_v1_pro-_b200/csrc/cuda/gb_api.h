@@ -51,6 +51,10 @@ typedef struct gb_gemm_args {
 int gb_gemm(const gb_gemm_args* args, cudaStream_t stream);
 int gb_gemm_pair(const gb_gemm_args* args, cudaStream_t stream);   // what gb_gemm calls when args->pair != 0
 int gb_gemm_skinny(const gb_gemm_args* args, cudaStream_t stream); // what gb_gemm calls when args->skinny != 0
+// One CTA whose producer and consumer warps each wait `waits` times for barriers that nothing completes, with the bounded waits of the
+// kernels above and `limit` cycles as their bound.  out[0]: cycles until both were through; out[1]: times the producer would have
+// issued.  Loads nothing; the status word gets the code of the wait that ran out.
+int gb_wait_check(int waits, long long limit, long long* out, int* status, cudaStream_t stream);
 // Expert segments of the sorted MoE buffers start at multiples of this many rows (two 128-row tiles: one pair tile).
 #define GB_MOE_PAD 256
 

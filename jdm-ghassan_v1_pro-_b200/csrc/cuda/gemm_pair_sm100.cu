@@ -254,7 +254,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const Tile t = decode(p, plan, tile, tiles_m, tiles_n);
         const int am = t.m0 + (int)rank * HM, bn = t.n0 + (int)rank * hn;
         for (int k = t.k_begin; k < t.k_end; k += BK) {
-          wait_or_report(&empty_bar[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+          wait_or_leave(&empty_bar[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
           uint8_t* sa = smem + s * stage_bytes;
           uint8_t* sb = sa + A_BYTES;
           mbar_arrive_expect_tx_on(on0, &full_bar[s], 2 * stage_bytes);   // both CTAs' bytes

@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(THREADS) gemm_skinny_kernel(const __grid_const
     for (int i = 0; i < early; ++i) load_w(i);
     pdl_wait();
     for (int i = 0; i < nkb; ++i) {
-      if (i >= STAGES) wait_or_report(&empty_bar[i % STAGES], ((i / STAGES) & 1) ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+      if (i >= STAGES) wait_or_leave(&empty_bar[i % STAGES], ((i / STAGES) & 1) ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
       if (i >= early) load_w(i);
       tma_load_2d_on(on, &tmA, &full_bar[i % STAGES], stage(i), (kb0 + i) * BK, 0);
     }

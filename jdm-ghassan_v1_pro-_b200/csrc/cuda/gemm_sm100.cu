@@ -205,7 +205,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         TileInfo t = decode_tile<BN>(p, tile, tiles_m, tiles_n);
         for (int k = t.k_begin; k < t.k_end; k += BK, ++it) {
           const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
-          wait_or_report(&empty_bar[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+          wait_or_leave(&empty_bar[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
           uint8_t* sa = smem + s * STAGE_BYTES;
           uint8_t* sb = sa + A_BYTES;
           mbar_arrive_expect_tx_on(on, &full_bar[s], STAGE_BYTES);

@@ -118,13 +118,13 @@ __global__ void __launch_bounds__(LA_THREADS) ll_attn_tc_kernel(const __grid_con
       uint32_t kv_it = 0, q_it = 0;
       for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++q_it) {
         const Item it = item_of(item);
-        wait_or_report(q_empty, (q_it & 1u) ^ 1u, a.status, ST_TIMEOUT_EMPTY, abort_flag);
+        wait_or_leave(q_empty, (q_it & 1u) ^ 1u, a.status, ST_TIMEOUT_EMPTY, abort_flag);
         mbar_arrive_expect_tx_on(on, q_full, TQ);
         load_tile<DK>(on, &tmQ, q_full, sQ, it.h * DK, it.b * a.n + it.q0);
         const int g = it.h / rep;
         for (int t = 0; t < it.n_kt + it.n_rt; ++t, ++kv_it) {
           const int s = kv_it & 1, ph = (kv_it >> 1) & 1;
-          wait_or_report(&kv_empty[s], ph ^ 1, a.status, ST_TIMEOUT_EMPTY, abort_flag);
+          wait_or_leave(&kv_empty[s], ph ^ 1, a.status, ST_TIMEOUT_EMPTY, abort_flag);
           mbar_arrive_expect_tx_on(on, &kv_full[s], TQ + TV);
           const int row = tile_row(it, t);
           load_tile<DK>(on, &tmK, &kv_full[s], sK + s * TQ, g * DK, row);

@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(LT_THREADS) ll_latent_tc_kernel(const __grid_c
       for (int p = 0; p < panels; ++p) tma_load_2d_on(on, &tmQ, q_full, sQ + p * QP, p * 64, r * a.heads_pad + h0);
       for (int t = 0; t < n_t; ++t) {
         const int s = t % stages, ph = (t / stages) & 1;
-        wait_or_report(&kv_empty[s], ph ^ 1, a.status, ST_TIMEOUT_EMPTY, abort_flag);
+        wait_or_leave(&kv_empty[s], ph ^ 1, a.status, ST_TIMEOUT_EMPTY, abort_flag);
         mbar_arrive_expect_tx_on(on, &kv_full[s], panels * KP);
         for (int p = 0; p < panels; ++p)
           tma_load_2d_on(on, &tmC, &kv_full[s], sK + (size_t)(s * panels + p) * KP, p * 64, b * a.cap + (t_lo + t) * AT_N);

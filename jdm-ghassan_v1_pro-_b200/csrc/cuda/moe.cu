@@ -204,6 +204,7 @@ __global__ void __launch_bounds__(RT_THREADS) moe_route_tc_kernel(const __grid_c
   uint64_t* empty = bars + RT_ST;          // RT_ST
   uint64_t* d_full = bars + 2 * RT_ST;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * RT_ST + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* s_hist = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(bars) + 128);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int bt = blk_tok(a.n_tok);                       // routing block (<= RT_TOK: checked by the launcher)
@@ -215,6 +216,7 @@ __global__ void __launch_bounds__(RT_THREADS) moe_route_tc_kernel(const __grid_c
   if (threadIdx.x == 0) {
     for (int s = 0; s < RT_ST; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(d_full, 1);
+    *abort_flag = 0;
     fence_barrier_init();
   }
   if (warp == 1) { tmem_alloc(tmem_slot, 32); tmem_relinquish(); }
@@ -250,7 +252,7 @@ __global__ void __launch_bounds__(RT_THREADS) moe_route_tc_kernel(const __grid_c
       const uint32_t on = elect_one();
       for (int kc = pre; kc < nkc; ++kc) {
         const int s = kc % RT_ST, ph = (kc / RT_ST) & 1;
-        if (!mbar_wait(&empty[s], ph ^ 1)) atomicCAS(status, 0, ST_TIMEOUT_EMPTY);
+        wait_or_leave(&empty[s], ph ^ 1, status, ST_TIMEOUT_EMPTY, abort_flag);
         mbar_arrive_expect_tx_on(on, &full[s], RT_XTILE);
         tma_load_2d_on(on, &tmX, &full[s], sX + s * RT_XTILE, kc * RT_KC, t0);
       }
@@ -262,7 +264,7 @@ __global__ void __launch_bounds__(RT_THREADS) moe_route_tc_kernel(const __grid_c
       const uint32_t idesc = make_idesc_f16(kBf16 ? 1 : 0, 0, 0, RT_TOK, 16);
       for (int kc = 0; kc < nkc; ++kc) {
         const int s = kc % RT_ST, ph = (kc / RT_ST) & 1;
-        if (!mbar_wait(&full[s], ph)) atomicCAS(status, 0, ST_TIMEOUT_FULL);
+        wait_or_report(&full[s], ph, status, ST_TIMEOUT_FULL, abort_flag);
         tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < RT_KC / 16; ++kk)
@@ -279,9 +281,8 @@ __global__ void __launch_bounds__(RT_THREADS) moe_route_tc_kernel(const __grid_c
     const int q = warp & 3;
     const int r = q * 32 + lane;
     const int t = t0 + r;
-    const bool got = mbar_wait(d_full, 0);
-    if (!got && lane == 0) atomicCAS(status, 0, ST_TIMEOUT_TMEM_FULL);
-    if (got) {
+    wait_or_report(d_full, 0, status, ST_TIMEOUT_TMEM_FULL, abort_flag);
+    if (__all_sync(0xffffffffu, *abort_flag == 0)) {
       tc_fence_after();
       uint32_t v[16];
       tmem_ld_32x16(tmem_D + ((uint32_t)(q * 32) << 16), v);
@@ -342,6 +343,10 @@ __global__ void __launch_bounds__(RT_THREADS) moe_route_tc_kernel(const __grid_c
     }
   }
   __syncthreads();
+  if (*abort_flag) {
+    for (int k = 0; k < 64; ++k) __nanosleep(1000);      // copies still in flight get time to land
+    __syncthreads();
+  }
   const int nb = (a.n_tok + bt - 1) / bt;
   for (int i = threadIdx.x; i < nsub * (ne + 1); i += RT_THREADS) {
     const int b = blockIdx.x * nsub + i / (ne + 1);

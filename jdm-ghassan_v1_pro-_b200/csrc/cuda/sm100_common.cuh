@@ -1,7 +1,7 @@
 // Thin inline-PTX layer for Blackwell (sm_100a): mbarrier, TMA (cp.async.bulk.tensor),
 // tcgen05 (alloc / mma / commit / ld / fences) and shared-memory matrix descriptors.
-// Every wait in this file is bounded: after SPIN_LIMIT unsuccessful polls the caller gets
-// `false` back and is expected to record an error code and drain, never to spin forever.
+// Every wait in this file is bounded, by polls (mbar_wait: the caller gets `false` and is expected to
+// record an error code and drain) or by cycles (wait_or_report, wait_or_leave: they record it themselves).
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -133,26 +133,43 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
-// Bounded wait shared by all roles of a CTA: gives up when another role has given up or after ~2 s.  It reports the failure and
-// returns: the callers go on (every later wait then returns at once, on whatever the buffers hold, and the status word says
-// that the results are void).  A loop that left on a wait's result would no longer be provably uniform over the warp, and the
-// operands of the MMAs would lose their uniform registers.
-static __device__ __noinline__ void wait_or_report_slow(uint64_t* bar, uint32_t parity, int* status, int code, volatile int* abort_flag) {
+// Bounded wait shared by all roles of a CTA: gives up once another role has given up (looked at before anything else), or after
+// ~2 s, and reports that in the status word, which says that the results are void.
+static constexpr long long WAIT_CYCLES = 4000000000LL;      // ~2 s
+__device__ __forceinline__ bool wait_poll(uint64_t* bar, uint32_t parity, int* status, int code, volatile int* abort_flag, long long limit) {
   const long long t0 = clock64();
-  for (;;) {
+  while (!*abort_flag) {
 #pragma unroll 1
-    for (int i = 0; i < 2048; ++i)
-      if (mbar_try_wait(bar, parity)) return;
-    if (*abort_flag) return;
-    if (clock64() - t0 > 4000000000LL) {
+    for (int i = 0; i < 256; ++i)
+      if (mbar_try_wait(bar, parity)) return true;
+    if (clock64() - t0 > limit) {
       atomicCAS(status, 0, code);
       *abort_flag = 1;
-      return;
     }
   }
+  return false;
 }
-__device__ __forceinline__ void wait_or_report(uint64_t* bar, uint32_t parity, int* status, int code, volatile int* abort_flag) {
-  if (!mbar_try_wait_some(bar, parity)) wait_or_report_slow(bar, parity, status, code, abort_flag);
+static __device__ __noinline__ void wait_or_report_slow(uint64_t* bar, uint32_t parity, int* status, int code, volatile int* abort_flag,
+                                                        long long limit) {
+  (void)wait_poll(bar, parity, status, code, abort_flag, limit);
+}
+static __device__ __noinline__ void wait_or_leave_slow(uint64_t* bar, uint32_t parity, int* status, int code, volatile int* abort_flag,
+                                                       long long limit) {
+  if (!wait_poll(bar, parity, status, code, abort_flag, limit)) asm volatile("exit;");
+}
+// For MMA issuers and epilogues: after a failure the loops go on, on whatever the buffers hold, and no later wait of the CTA takes longer
+// than its first polls.  A loop that left on a wait's result would no longer be provably uniform over the warp, and the operands
+// of the MMAs would lose their uniform registers.  What still runs stays in the CTA's own buffers and barriers.
+__device__ __forceinline__ void wait_or_report(uint64_t* bar, uint32_t parity, int* status, int code, volatile int* abort_flag,
+                                               long long limit = WAIT_CYCLES) {
+  if (!mbar_try_wait_some(bar, parity)) wait_or_report_slow(bar, parity, status, code, abort_flag, limit);
+}
+// For the warps that load: after a failure the thread ends, so that nothing more is expected of a barrier or loaded into a stage that may
+// be in use; the barriers of the block and the cluster wait for the threads that are left.  Not for a warp that holds anything
+// (tensor memory).  Clearing `on` instead, which makes it an ordinary predicate, cost the two-CTA GEMM 2 to 6 %.
+__device__ __forceinline__ void wait_or_leave(uint64_t* bar, uint32_t parity, int* status, int code, volatile int* abort_flag,
+                                              long long limit = WAIT_CYCLES) {
+  if (!mbar_try_wait_some(bar, parity)) wait_or_leave_slow(bar, parity, status, code, abort_flag, limit);
 }
 
 // ----------------------------------------------------------------------------- TMA

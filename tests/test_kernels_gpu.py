@@ -418,3 +418,20 @@ def test_moe_few_tokens_and_forward_only(n, d):
     used = int(ws[0].seg_offsets[ne + 1])
     assert torch.equal(xp[0][real], xp[1][real])
     assert (xp[0][:used][~real[:used]] == 0).all() and (xp[1][~real] == 7).all()
+
+
+def test_bounded_waits_give_up_together():
+    """A producer and a consumer that wait 200 times each for barriers that nothing completes: one wait runs out and is reported, all others
+    (of either role) see that it has, and the producer issues nothing more.  The time is that of one limit, not of one per wait."""
+    from ghassan_b200.ops import _lib
+    import ctypes
+    out = torch.zeros(2, dtype=torch.int64, device="cuda")
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    waits, limit = 200, 400_000_000                     # about a fifth of a second
+    rc = _lib.lib().gb_wait_check(waits, ctypes.c_longlong(limit), ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(status.data_ptr()),
+                                  _lib.stream_ptr())
+    _lib.check_rc(rc, "gb_wait_check")
+    cycles, issued = out.tolist()
+    assert int(status[0]) in (101, 102)
+    assert issued == 0
+    assert limit <= cycles < 1.5 * limit, cycles
