@@ -161,6 +161,7 @@ class InferenceEngine(TokenLoop):
             self._build_mega()
         self.prefill_chunk = min(prefill_chunk, max_len)
         self._prefill_model: Optional[CudaModel] = None
+        self._prompt_seen = False
         self._prompt_graph: Optional[torch.cuda.CUDAGraph] = None
         self.prompt_len = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self._named = named
@@ -325,18 +326,19 @@ class InferenceEngine(TokenLoop):
     def _prompt_pass(self, m: CudaModel):
         """The prompt pass over ``m.ids``.  Its launches are the same for every prompt (the shape is the chunk's, the prompt's length
         is on the device), and issuing 370 of them from Python took longer than running them: 7.2 ms for 3.6 ms of kernels
-        (26 layers, 1501 tokens).  So the first pass, which also does the first-use set-up, is followed by a capture, and later
-        ones are replays."""
-        if self._prompt_graph is not None and not torch.cuda.is_current_stream_capturing():
-            self._prompt_graph.replay()
+        (26 layers, 1501 tokens).  The first prompt runs as it comes, which does the first-use set-up, and may be the only one; the
+        second is captured and replayed, and so are all others."""
+        if torch.cuda.is_current_stream_capturing() or not self._prompt_seen:
+            m.prompt_forward(self)
+            self._prompt_seen = True
             return
-        m.prompt_forward(self)
-        if not torch.cuda.is_current_stream_capturing():
+        if self._prompt_graph is None:
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g, capture_error_mode="thread_local"):
+            with torch.cuda.graph(g, capture_error_mode="thread_local"):   # records the launches, runs nothing
                 m.prompt_forward(self)
             self._prompt_graph = g
+        self._prompt_graph.replay()
 
     def prefill(self, prompts: torch.Tensor):
         """``prompts``: int32 [B, n] (same length for every sequence).  The first ``prefill_chunk`` tokens go through

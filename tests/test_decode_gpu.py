@@ -606,21 +606,22 @@ def test_decode_attention_at_slot_edges(hd, H, KV, n, splits, window, off):
 
 
 def test_prompt_pass_replays_for_other_prompts():
-    """The second prompt of an engine replays the first one's captured pass: other lengths and tokens, two sequences; cache rows
-    behind the prompt stay as they were."""
+    """An engine's first prompt runs as it comes (it may be the only one), the second is captured and replayed, as are all others: other
+    lengths and tokens, two sequences; cache rows behind the prompt stay as they were."""
     from ghassan_b200.inference.engine import InferenceEngine
     from ghassan_b200.models.config import init_parameters
     cfg = _tiny_cfg(num_heads=4, num_kv_heads=2, hidden_size=256)
     named = init_parameters(cfg, 5)
     g = torch.Generator().manual_seed(6)
     a = InferenceEngine(cfg, named, fmt="f16", batch=2, max_len=160, prefill_chunk=128)
-    for n in (100, 129, 66, 140):                           # 66: a shorter prompt, 140: longer than the chunk
+    for at, n in enumerate((100, 129, 66, 140)):            # 66: a shorter prompt, 140: longer than the chunk
         prompt = torch.randint(16, 512, (2, n), generator=g, dtype=torch.int32)
         a.reset(1)
         for L in a.layers:
             L.cK.fill_(7.0)
             L.cV.fill_(7.0)
         a.prefill(prompt)
+        assert (a._prompt_graph is not None) == (at > 0)
         b = InferenceEngine(cfg, named, fmt="f16", batch=2, max_len=160, prefill_chunk=128)
         b.reset(1)
         b.prefill(prompt)                                   # this engine's first: eager
