@@ -239,16 +239,17 @@ def gemm_grouped_reduce(a, b, seg_offsets, groups, out, *, accumulate=True, bloc
     return out
 
 
-# Weight gradients whose reductions are cut into pieces (csrc/cuda/gemm_pair_sm100.cu): partial sums take at most this much scratch,
-# and the product has at least this many k-blocks of 64 for each of the 74 pairs, half as many where it is one group (below, an
-# epilogue costs as much as a piece).
+# Weight gradients whose reductions are cut into pieces (csrc/cuda/gemm_pair_sm100.cu): partial sums take at most this much scratch
+# (inside the slack of the trainer's memory guard), and the product has at least this many k-blocks of 64 for each of the 74 pairs,
+# half as many where it is one group (below, an epilogue costs as much as a piece).
 PIECE_BYTES = 96 << 20
 PIECE_MIN_KBLOCKS = 16
 
 
 def _best_cut(tiles, lens, mn):
-    """The estimate of the plan on the device for reductions of these lengths (k-blocks, the longest first): k-blocks of the best
-    pieces, or 0 where they do not gain a tenth."""
+    """k-blocks of the best pieces for reductions of these lengths (k-blocks, the longest first), or 0 where cutting does not gain a
+    tenth.  Costs as the plan on the device estimates them (``plan_pieces``), with the 74 pairs of a whole B200; for one group the
+    result is the cut that the device uses, for several it only decides whether the device plans at all, so the two need not agree."""
     def cost(c):
         load, items, turn, extra = 0.0, 0, 0, 0
         for k in lens:
@@ -264,8 +265,8 @@ def _best_cut(tiles, lens, mn):
 
 def _piece_scratch(M, N, kblocks, groups, out, longest=0):
     """(fp32 ``[slots, M, N]``, k-blocks of a piece where that is settled) for the pieces of ``groups`` reductions that have ``kblocks``
-    blocks of 64 rows in all, or None where they stay whole.  ``longest``: k-blocks of a group known to be longer than the others.  Taken from the allocator for this call, so
-    calls on other streams have their own."""
+    blocks of 64 rows in all, or None where they stay whole.  ``longest``: k-blocks of a group known to be longer than the others.
+    Taken from the allocator for this call, so calls on other streams have their own."""
     tiles = pair_tiles(M, N)
     if not PAIR_ENABLED or N % 4 or groups > 64 or kblocks > 32000 or tiles * kblocks * (2 if groups == 1 else 1) < 74 * PIECE_MIN_KBLOCKS or not pair_ok(M, N, out, groups=60):
         return None
@@ -280,7 +281,13 @@ def _piece_scratch(M, N, kblocks, groups, out, longest=0):
     slots = min(64, PIECE_BYTES // (4 * M * N), kblocks // PIECE_MIN_KBLOCKS)      # a piece has at least that many k-blocks
     if groups == 1:
         slots = -(-kblocks // cut) - 1 if slots >= -(-kblocks // cut) - 1 else 0
-    return (torch.empty(slots, M, N, dtype=torch.float32, device=out.device), cut if groups == 1 else 0) if slots >= 1 else None
+    if slots < 1:
+        return None
+    try:
+        part = torch.empty(slots, M, N, dtype=torch.float32, device=out.device)
+    except torch.OutOfMemoryError:           # whole reductions need no scratch
+        return None
+    return part, cut if groups == 1 else 0
 
 
 def _use_pieces(g, pieces, K=0):

@@ -1,7 +1,8 @@
 """Closed-form device memory of the CUDA engine for a recipe: what ``--dry-run`` prints, what the trainer's memory
 guard compares with the device, and what picks the number of micro-batches per pass.  Nothing is allocated.
 Plays the role of the reference's ``Model::plan_memory`` / ``workspace_plan`` (model/model.cpp:919-1238) for this
-engine's buffers (``models/cuda_model.py``), which are not the reference's arenas."""
+engine's buffers (``models/cuda_model.py``), which are not the reference's arenas.  Scratch of single launches (partial sums of weight
+gradients: ``ops.gemm.PIECE_BYTES`` at most) is left to the guard's slack of 1 GiB."""
 from __future__ import annotations
 
 from ..models.config import ModelConfig

@@ -118,3 +118,17 @@ def test_trainer_refuses_before_training(tmp_path, monkeypatch):
     tr = Trainer(ModelConfig.from_config(c), TrainerConfig.from_config(c), device="cpu")
     tr.prefetch.stop()
     assert np.isfinite(tr.scaler.for_step())
+
+
+def test_cut_weight_gradients_do_without_their_scratch(monkeypatch):
+    """Where the partial sums of cut reductions find no memory, the reductions stay whole instead of failing."""
+    import torch
+    from ghassan_b200.ops import gemm
+    out = torch.zeros(768, 1280)
+    part, cut = gemm._piece_scratch(768, 1280, 512, 1, out)
+    assert part.shape == (-(-512 // cut) - 1, 768, 1280)
+
+    def full(*a, **k):
+        raise torch.OutOfMemoryError("no room")
+    monkeypatch.setattr(torch, "empty", full)
+    assert gemm._piece_scratch(768, 1280, 512, 1, out) is None
