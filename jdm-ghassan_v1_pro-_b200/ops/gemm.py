@@ -329,7 +329,7 @@ class SplitK:
         return out16
 
 
-_WGRAD_PLANS = {}
+_WGRAD_SPLITS = {}        # token offsets of a split: only read once made
 
 
 def gemm_wgrad(a, b, grad):
@@ -355,15 +355,13 @@ def gemm_wgrad(a, b, grad):
     splits = min(8, 148 // max(1, tiles), Kt // 1024)
     if splits < 2 or not splittable:
         return gemm(a, b, a_mn=True, b_mn=True, out=grad, addend=grad)
-    key = (M, N, Kt, splits, a.device.index)
-    plan = _WGRAD_PLANS.get(key)
-    if plan is None:
+    key = (Kt, splits, a.device.index)
+    offsets = _WGRAD_SPLITS.get(key)
+    if offsets is None:
         kc = (Kt // splits + 63) // 64 * 64
         offs = [min(Kt, i * kc) for i in range(splits)] + [Kt]
-        plan = (torch.tensor(offs, dtype=torch.int32, device=a.device),
-                torch.empty(splits, M, N, dtype=torch.float32, device=a.device))
-        _WGRAD_PLANS[key] = plan
-    offsets, part = plan
+        offsets = _WGRAD_SPLITS[key] = torch.tensor(offs, dtype=torch.int32, device=a.device)
+    part = torch.empty(splits, M, N, dtype=torch.float32, device=a.device)      # of this call: other streams have their own
     g = _base_args(a, b, M, N, 0, True, True, part, 128)
     g.epilogue = EPI_STORE
     g.mode = 2

@@ -197,7 +197,7 @@ def test_weight_gradient_split_over_tokens(M, N, K):
     b = _rand(K, N, seed=71) * 0.2
     grad = torch.full((M, N), 0.5, dtype=torch.float32, device="cuda")
     G.gemm_wgrad(a, b, grad)
-    G.gemm_wgrad(a, b, grad)                  # accumulates, and the cached plan is reused
+    G.gemm_wgrad(a, b, grad)                  # accumulates, and the cached offsets are reused
     L.check_status(what="wgrad")
     ref = 0.5 + 2.0 * (a.float().t() @ b.float())
     rel, ok = _close(grad, ref)
@@ -388,3 +388,24 @@ def test_few_rows(M, N, K):
     rel, ok = _close(sq, torch.relu(ref) ** 2)
     assert ok, rel
     L.check_status(what="few rows")
+
+
+def test_wgrad_split_on_two_streams_at_once():
+    """Calls of one shape on two streams keep their partial sums apart (256 x 256 over 4096 tokens: four splits on the one-CTA kernel)."""
+    G, L = _ops()
+    T, M, N = 4096, 256, 256
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    g = torch.Generator(device="cuda").manual_seed(9)
+    ops = [[torch.randint(-3, 4, (T, m), device="cuda", generator=g).half() for m in (M, N)] for _ in streams]
+    grads = [torch.zeros(M, N, device="cuda") for _ in streams]
+    warm = torch.zeros(M, N, device="cuda")
+    G.gemm_wgrad(*ops[0], warm)
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for s, (a, b), gr in zip(streams, ops, grads):
+            with torch.cuda.stream(s):
+                G.gemm_wgrad(a, b, gr)
+    torch.cuda.synchronize()
+    L.check_status(what="wgrad")
+    for (a, b), gr in zip(ops, grads):
+        assert torch.equal(gr, 20 * (a.double().t() @ b.double()).float())       # whole numbers below 2^24: exact in any order
