@@ -22,12 +22,11 @@ namespace gb {
 namespace pr {
 
 static constexpr int HM = 128;        // A rows per CTA  (pair tile: 256)
-static constexpr int TM = 256;
-static constexpr int TN_MAX = 256;    // output columns of a pair tile (Params::tn: 128 .. 256); each CTA stages half of them
+static constexpr int HN = 128;        // B rows per CTA  (pair tile: 256 output columns)
+static constexpr int TM = 256, TN = 256;
 static constexpr int BK = 64, UMMA_K = 16;
 static constexpr int THREADS = 320, W_TMA = 8, W_MMA = 9, EPI_WARPS = 8;
-static constexpr uint32_t A_BYTES = HM * BK * 2, STAGE_BYTES = A_BYTES + TN_MAX / 2 * BK * 2;
-static constexpr int MAX_STAGES = 8;  // narrower tiles have smaller stages, and more of them
+static constexpr uint32_t A_BYTES = HM * BK * 2, B_BYTES = HN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
 static constexpr uint32_t SLOT_BYTES = 4096;   // 32 rows x 128 bytes
 static constexpr uint32_t TMEM_COLS = 512;
 static constexpr uint32_t BAR_BYTES = 512;
@@ -38,7 +37,6 @@ enum { EPI_STORE = 0, EPI_SWIGLU_FWD = 1, EPI_SWIGLU_BWD = 2, EPI_RELU2 = 4 };  
 
 struct Params {
   int M, N, K;
-  int tn, stages;              // output columns of a tile; pipeline depth that fits beside the epilogue's slots
   int a_mn, b_mn, fmt;
   int mode;                    // 0 dense, 1 expert-sorted rows, 2 grouped over the reduction dim
   const int* tile_expert;      // mode 1: expert of each 128-row tile (tiles 2i and 2i+1 must agree)
@@ -92,6 +90,7 @@ __device__ __forceinline__ int warp_prefix(int v, int& total) {        // sum ov
   total = __shfl_sync(0xffffffffu, s, 31);
   return s - v;
 }
+// The product and the addition behind it each make the plan: whatever could be rounded in two ways is written as fmaf, so both get the same.
 // Called by one whole warp; `per` tiles per group.  Lane l holds groups l and l + 32 from the last, and estimates candidate l.
 __device__ __forceinline__ void plan_pieces(PiecePlan* pl, const int* seg, int K, int groups, int per, long long mn, int n_pairs, int slots,
                                             int fixed) {
@@ -124,7 +123,7 @@ __device__ __forceinline__ void plan_pieces(PiecePlan* pl, const int* seg, int K
       extra += fmaxf(n - 1.f, 0.f);
       cut += n > 1.f ? 1.f : 0.f;
     }
-    const float score = extra + cut > (float)slots ? 3e38f : load + (extra + cut) * slot_cost;   // the real plan has no more pieces than this
+    const float score = extra + cut > (float)slots ? 3e38f : fmaf(extra + cut, slot_cost, load);   // the real plan has no more pieces than this
     float best = score;
     for (int o = 16; o; o >>= 1) best = fminf(best, __shfl_xor_sync(0xffffffffu, best, o));
     const unsigned who = __ballot_sync(0xffffffffu, score == best);
@@ -162,7 +161,7 @@ __device__ __forceinline__ Tile decode(const Params& p, const PiecePlan* pl, int
     const int len = pl->len[i] * BK;
     t.g = p.groups - 1 - i;
     t.m0 = (r % tiles_m) * TM;
-    t.n0 = (r / tiles_m) * p.tn;
+    t.n0 = (r / tiles_m) * TN;
     const int k0 = p.seg_offsets ? p.seg_offsets[t.g] : 0, k1 = p.seg_offsets ? p.seg_offsets[t.g + 1] : p.K;
     t.k_begin = k0 + piece * len;
     t.k_end = min(k1, t.k_begin + len);
@@ -173,13 +172,13 @@ __device__ __forceinline__ Tile decode(const Params& p, const PiecePlan* pl, int
     const int gi = tile / per, r = tile - gi * per;
     t.g = p.groups - 1 - gi;
     t.m0 = (r % tiles_m) * TM;
-    t.n0 = (r / tiles_m) * p.tn;
+    t.n0 = (r / tiles_m) * TN;
     t.k_begin = p.seg_offsets[t.g];
     t.k_end = p.seg_offsets[t.g + 1];
   } else {
     const int tm = tile / tiles_n, tn = tile - tm * tiles_n;   // column tiles of one row block are neighbours
     t.m0 = tm * TM;
-    t.n0 = tn * p.tn;
+    t.n0 = tn * TN;
     if (p.mode == 1) t.b_row_off = p.tile_expert[2 * tm] * p.b_group_rows;
   }
   return t;
@@ -200,8 +199,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* slots = smem + STAGES * STAGE_BYTES;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(slots + EPI_WARPS * SLOTS * SLOT_BYTES);
-  uint64_t* empty_bar = full_bar + MAX_STAGES;
-  uint64_t* tfull_bar = empty_bar + MAX_STAGES;
+  uint64_t* empty_bar = full_bar + STAGES;
+  uint64_t* tfull_bar = empty_bar + STAGES;
   uint64_t* tempty_bar = tfull_bar + 2;
   uint64_t* aux_bar = tempty_bar + 2;               // [EPI_WARPS][2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(aux_bar + 2 * EPI_WARPS);
@@ -213,7 +212,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const uint32_t rank = cluster_ctarank();          // 0 = the CTA that issues the MMAs
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < MAX_STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 2 * EPI_WARPS); }
     for (int i = 0; i < 2 * EPI_WARPS; ++i) mbar_init(&aux_bar[i], 1);
     *abort_flag = 0;
@@ -228,7 +227,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (EPI != EPI_STORE && EPI != EPI_RELU2) tma_prefetch_desc(&tmX);
   }
   if (EPI == EPI_STORE && sizeof(OutT) == 4 && p.part_slots && warp == 0)
-    plan_pieces(plan, p.seg_offsets, p.K, p.groups, ((p.M + TM - 1) / TM) * ((p.N + p.tn - 1) / p.tn), (long long)p.M * p.N,
+    plan_pieces(plan, p.seg_offsets, p.K, p.groups, ((p.M + TM - 1) / TM) * ((p.N + TN - 1) / TN), (long long)p.M * p.N,
                 (int)cluster_nctaid_x(), p.part_slots, p.part_cut);
   tc_fence_before();
   __syncthreads();
@@ -238,9 +237,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (tmem_base != 0 && threadIdx.x == 0) { atomicCAS(p.status, 0, ST_BAD_ARGUMENT); *abort_flag = 1; }
 
   const int tiles_m = (p.mode == 1) ? (*p.num_m_tiles + 1) / 2 : (p.M + TM - 1) / TM;
-  const int tiles_n = (p.N + p.tn - 1) / p.tn;
-  const int hn = p.tn >> 1;                                   // B rows per CTA
-  const uint32_t stage_bytes = A_BYTES + hn * (BK * 2), nst = p.stages;
+  const int tiles_n = (p.N + TN - 1) / TN;
   const int total_tiles = p.part_slots ? plan->base[p.groups] : tiles_m * tiles_n * (p.mode == 2 ? p.groups : 1);
   const int pair_id = (int)cluster_id_x(), n_pairs = (int)cluster_nctaid_x();
 
@@ -252,12 +249,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       uint32_t s = 0, ph = 0;
       for (int tile = pair_id; tile < total_tiles; tile += n_pairs) {
         const Tile t = decode(p, plan, tile, tiles_m, tiles_n);
-        const int am = t.m0 + (int)rank * HM, bn = t.n0 + (int)rank * hn;
+        const int am = t.m0 + (int)rank * HM, bn = t.n0 + (int)rank * HN;
         for (int k = t.k_begin; k < t.k_end; k += BK) {
           wait_or_leave(&empty_bar[s], ph ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
-          uint8_t* sa = smem + s * stage_bytes;
+          uint8_t* sa = smem + s * STAGE_BYTES;
           uint8_t* sb = sa + A_BYTES;
-          mbar_arrive_expect_tx_on(on0, &full_bar[s], 2 * stage_bytes);   // both CTAs' bytes
+          mbar_arrive_expect_tx_on(on0, &full_bar[s], 2 * STAGE_BYTES);   // both CTAs' bytes
           const uint32_t fb = full0 + s * 8;
           if (!p.a_mn) {
             tma_load_2d_pair_on(on, &tmA, fb, sa, k, am);
@@ -272,9 +269,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           } else if (p.b_mn3) {
             tma_load_3d_pair_on(on, &tmB, fb, sb, 0, t.b_row_off + k, bn >> 6);
           } else {
-            for (int c = 0; c < hn / 64; ++c) tma_load_2d_pair_on(on, &tmB, fb, sb + c * (64 * 128), bn + c * 64, t.b_row_off + k);
+#pragma unroll
+            for (int c = 0; c < HN / 64; ++c) tma_load_2d_pair_on(on, &tmB, fb, sb + c * (64 * 128), bn + c * 64, t.b_row_off + k);
           }
-          if (++s == nst) { s = 0; ph ^= 1; }
+          if (++s == STAGES) { s = 0; ph ^= 1; }
         }
       }
     }
@@ -283,7 +281,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // ------------------------------------------------------------- MMA issuer (CTA 0 only)
     if (rank == 0) {
       const uint32_t on = elect_one();
-      const uint32_t idesc = make_idesc_f16(p.fmt, p.a_mn, p.b_mn, TM, p.tn);
+      const uint32_t idesc = make_idesc_f16(p.fmt, p.a_mn, p.b_mn, TM, TN);
       uint32_t s = 0, ph = 0, acc_it = 0;
       for (int tile = pair_id; tile < total_tiles; tile += n_pairs) {
         const Tile t = decode(p, plan, tile, tiles_m, tiles_n);
@@ -291,12 +289,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const uint32_t ab = acc_it & 1, aph = (acc_it >> 1) & 1;
         wait_or_report(&tempty_bar[ab], aph ^ 1, p.status, ST_TIMEOUT_TMEM_EMPTY, abort_flag);
         tc_fence_after();
-        const uint32_t d_tmem = ab * TN_MAX;      // all 512 columns are this pair's: the allocation starts at column 0 (checked above)
+        const uint32_t d_tmem = ab * TN;      // all 512 columns are this pair's: the allocation starts at column 0 (checked above)
         bool first = true;
         for (int k = t.k_begin; k < t.k_end; k += BK) {
           wait_or_report(&full_bar[s], ph, p.status, ST_TIMEOUT_FULL, abort_flag);
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + s * stage_bytes);
+          const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
           const uint32_t sb = sa + A_BYTES;
           // same operand layouts as the one-CTA kernel with 128-row A and B tiles; the other CTA's halves sit at
           // the same shared-memory offsets
@@ -310,7 +308,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             first = false;
           }
           umma_commit_pair_on(on, &empty_bar[s], 3);     // frees this stage in both CTAs
-          if (++s == nst) { s = 0; ph ^= 1; }
+          if (++s == STAGES) { s = 0; ph ^= 1; }
         }
         umma_commit_pair_on(on, &tfull_bar[ab], 3);
         ++acc_it;
@@ -337,7 +335,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const Tile t = decode(p, plan, tile, tiles_m, tiles_n);
       const bool empty_k = (t.k_end <= t.k_begin);
       const int row_q = t.m0 + (int)rank * HM + quarter * 32;   // first of this warp's 32 rows
-      const int colh = t.n0 + half * 128;                       // first of this warp's 128 accumulator columns (SwiGLU: tn = 256)
+      const int colh = t.n0 + half * 128;                       // first of this warp's 128 accumulator columns (SwiGLU)
       const bool rows_live = row_q < p.M;
 
       if constexpr (EPI == EPI_SWIGLU_BWD) {
@@ -365,11 +363,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         wait_or_report(&tfull_bar[ab], aph, p.status, ST_TIMEOUT_TMEM_FULL, abort_flag);
         tc_fence_after();
       }
-      const uint32_t tacc = tmem_base + ab * TN_MAX + (uint32_t(quarter * 32) << 16), taddr = tacc + half * 128;
+      const uint32_t tacc = tmem_base + ab * TN + (uint32_t(quarter * 32) << 16), taddr = tacc + half * 128;
 
       if constexpr ((EPI == EPI_STORE || EPI == EPI_RELU2) && sizeof(OutT) == 2) {
 #pragma unroll 1
-        for (int c = half; c < p.tn >> 6; c += 2) { // 64-column chunks, in turn for the two warps of a quarter
+        for (int c = half; c < TN / 64; c += 2) { // 64-column chunks, in turn for the two warps of a quarter
           uint32_t r0[32], r1[32];
           if (!empty_k) {
             tmem_ld_32x32(tacc + c * 64, r0);
@@ -413,7 +411,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       } else if constexpr (EPI == EPI_STORE) {
         // fp32 output, 32-column chunks: plain store, store of acc + addend, or reduce-add into the matrix
 #pragma unroll 1
-        for (int c = half; c < p.tn >> 5; c += 2) {
+        for (int c = half; c < TN / 32; c += 2) {
           const int col = t.n0 + c * 32;
           uint32_t r[32];
           if (!empty_k) {
@@ -656,10 +654,7 @@ namespace {
 
 template <int EPI, int STAGES, int SLOTS, typename OutT>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, const CUtensorMap& tx,
-                gb::pr::Params p, int max_tiles, cudaStream_t st, int* used_pairs = nullptr) {
-  const uint32_t stage = gb::pr::A_BYTES + p.tn / 2 * gb::pr::BK * 2;
-  p.stages = (int)(STAGES * gb::pr::STAGE_BYTES / stage);
-  if (p.stages > gb::pr::MAX_STAGES) p.stages = gb::pr::MAX_STAGES;
+                const gb::pr::Params& p, int max_tiles, cudaStream_t st, int* used_pairs = nullptr) {
   auto kern = gb::pr::gemm_pair_kernel<EPI, STAGES, SLOTS, OutT>;
   constexpr size_t smem = gb::pr::smem_bytes<STAGES, SLOTS>();
   static_assert(smem <= 232448, "shared memory of the pair kernel exceeds 227 KB");
@@ -721,7 +716,6 @@ extern "C" int gb_gemm_pair(const gb_gemm_args* a, cudaStream_t st) {
     else { p.addend = a->addend; p.ld_add = a->ld_add; }
   }
 
-  p.tn = pr::TN_MAX;
   if (a->part) {
     // pieces of reductions: fp32 sums into [groups, M, N] without gaps
     if (a->mode != 2 || !p.reduce || ot != 2 || a->part_slots < 1 || p.groups > pr::MAX_PIECE_GROUPS || a->epilogue != pr::EPI_STORE ||
@@ -744,14 +738,14 @@ extern "C" int gb_gemm_pair(const gb_gemm_args* a, cudaStream_t st) {
     p.a_mn3 = 1;
   } else rc = gb_make_tmap_2d_16b(&ta, a->A, a->a_rows, a->a_cols, a->lda, pr::BK, 64, a->is_bf16);
   if (rc) return rc - 100;
-  if (!a->b_mn_major) rc = gb_make_tmap_2d_16b(&tb, a->B, a->b_rows, a->b_cols, a->ldb, p.tn / 2, pr::BK, a->is_bf16);
+  if (!a->b_mn_major) rc = gb_make_tmap_2d_16b(&tb, a->B, a->b_rows, a->b_cols, a->ldb, pr::HN, pr::BK, a->is_bf16);
   else if (chunked && a->b_cols % 64 == 0) {
-    rc = gb_make_tmap_mn_chunks(&tb, a->B, a->b_rows, a->b_cols, a->ldb, pr::BK, p.tn / 128, a->is_bf16);
+    rc = gb_make_tmap_mn_chunks(&tb, a->B, a->b_rows, a->b_cols, a->ldb, pr::BK, pr::HN / 64, a->is_bf16);
     p.b_mn3 = 1;
   } else rc = gb_make_tmap_2d_16b(&tb, a->B, a->b_rows, a->b_cols, a->ldb, pr::BK, 64, a->is_bf16);
   if (rc) return rc - 200;
 
-  const int tiles_m = (a->M + pr::TM - 1) / pr::TM, tiles_n = (a->N + p.tn - 1) / p.tn;
+  const int tiles_m = (a->M + pr::TM - 1) / pr::TM, tiles_n = (a->N + pr::TN - 1) / pr::TN;
   const int max_tiles = tiles_m * tiles_n * groups;
 
   switch (a->epilogue) {
