@@ -899,8 +899,10 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
   XT* act = reinterpret_cast<XT*>(a.act);
 
   // number of cache splits: 64 slots per CTA (four per warp, side by side), up to 128 (two trips' loads at once) rather than more
-  // than 24 splits, since every CTA reads all partial results in the next phase; at most what the grid and the scratch hold
-  // (4-bit weights, 26 layers: 3001 slots 1146 us a token with 37 splits, 1062 with 24, 1142 with 9; 1024 slots 1004 with 17, 1012 with 9)
+  // than 24 splits, since every CTA reads all partial results in the next phase; at most what the grid and the scratch hold.
+  // us a step without the sampler, at most 16 / 24 / 32 / 64 splits before the 128: 36 layers, 12/4 heads, fp16: 1024 slots 1678 / 1651 / 1650 / 1650,
+  // 2000 1705 / 1722 / 1796 / 1798, 3001 1740 / 1740 / 1844 / 1864; 26 layers, 12/4, 4 bits: 975 / 962 / 962 / 962, 996 / 998 / 1060 / 1060,
+  // 1011 / 1012 / 1087 / 1097; 12 layers, 8/2, 8 bits: 417 / 411 / 410 / 411, 428 / 435 / 455 / 456, 441 / 440 / 468 / 470
   const gb_seq_state s0 = a.state[0];
   const int pos_now = a.pos[0];
   const int n_slots = min(a.cap, s0.cache_len + 1);

@@ -61,6 +61,7 @@ int gb_ll_advance(gb_seq_state* state, int* pos_out, int B, int n, cudaStream_t 
 // n1 > 0: rows from n1 on go to out2 (compute type, pitch ldo2) as max(v, 0)^2.
 // swiglu != 0: W holds gate/up rows interleaved in blocks of 64 (N = 2 E rows) and out[b, j] = silu(gate_j) * up_j.
 // softcap > 0: out = cap * tanh(out / cap).
+// W, w1, w2 and b1 are constants: they are read before the wait for the launch ahead, which must not write them.
 typedef struct gb_ll_gemv_args {
   const void* W; int fmt, N, K;          // K: stored row length (values beyond `d` are zero)
   int B, dtype, prologue, swiglu;
@@ -134,7 +135,7 @@ typedef struct gb_ll_latent_args {
   void* cache; int ldc; int cap;         // [B, cap, ldc]
   const void* qc; long long ld_qc;       // [rows, H, dn + dr] queries as projected
   void* q;                               // [rows, H, dkp] rotated queries
-  const void* W_kv; long long ld_w;      // rows h*dkp + d: key map of head h, rows H*dkp + h*dvp + e: its value map; columns: rank ..
+  const void* W_kv; long long ld_w;      // rows h*dkp + d: key map of head h, rows H*dkp + h*dvp + e: its value map; columns: rank .. (not written by the launch ahead)
   float* qa;                             // [rows, H, ldc] queries against cache rows, or
   void* qa16; int heads_pad, ld_qa16;    // [rows, heads_pad, ld_qa16] the same in bf16 for the tensor cores (padding is zero)
   const void* gate; long long ld_gate;   // [rows, H*dv] or NULL

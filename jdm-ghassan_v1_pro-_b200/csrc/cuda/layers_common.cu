@@ -270,9 +270,9 @@ extern "C" int gb_ll_norm_rows(const float* x, const int* row_idx, const float* 
   return gb_launch_rc();
 }
 
-// a warp per row while the row fits its registers, else a block per row
-// A warp per row of up to 1024 values, once there are more rows than the SMs hold blocks: fewer rows get a block each, whose threads
-// have one load to wait for instead of eight (add and layer norm of 32 x 1024: 5.0 -> 2.6 us, 300 x 1024: 5.2 -> 3.0).
+// A warp per row while the row fits its registers (1024 values) and there are more rows than the SMs hold blocks, else a block per row:
+// its threads have one load to wait for instead of eight (add and layer norm of 32 x 1024: 5.0 -> 2.6 us, 300 x 1024: 5.2 -> 3.0).
+// The two sum a row in different orders, so its last bits depend on which is taken.
 constexpr int LL_BLOCK_ROWS = 4 * 148;
 #define LL_ROWS(KERN, T, ...)                                                                                                 \
   do {                                                                                                                       \

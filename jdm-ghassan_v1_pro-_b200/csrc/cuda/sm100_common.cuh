@@ -33,8 +33,10 @@ static inline int gb_launch_rc() {
 }
 
 // Programmatic dependent launch for chains of short kernels (the decode step): the next kernel's blocks are set up
-// while this one drains.  A kernel launched through GB_PDL_LAUNCH must call gb::pdl_wait() before it touches global
-// memory; until then nothing its predecessors wrote is guaranteed visible.  GB200_NO_PDL=1 turns the attribute off.
+// while this one drains.  A kernel launched through GB_PDL_LAUNCH must call gb::pdl_wait() before it writes global memory and
+// before it reads anything that the launch ahead of it may write; until then nothing that launch wrote is guaranteed
+// visible.  What only earlier launches write may be read before: a launch starts once every block of the one ahead is past its own
+// wait.  GB200_NO_PDL=1 turns the attribute off.
 #include <cstdlib>
 static inline cudaLaunchConfig_t gb_pdl_config(dim3 grid, dim3 block, size_t smem, cudaStream_t st, cudaLaunchAttribute* attr) {
   static const int enabled = []() { const char* e = std::getenv("GB200_NO_PDL"); return (e && e[0] == '1') ? 0 : 1; }();
@@ -58,8 +60,10 @@ static inline cudaLaunchConfig_t gb_pdl_config(dim3 grid, dim3 block, size_t sme
 
 namespace gb {
 
-// First statement of every kernel that GB_PDL_LAUNCH starts: wait until the kernels before it have finished and
-// their writes are visible, then let the kernel after it begin its own set-up.
+// Wait until the kernels before this one have finished and their writes are visible, then let the kernel after it begin its own
+// set-up.  The first statement of every kernel that GB_PDL_LAUNCH starts, but for those that first ask for constants (weights in
+// gemm_skinny_sm100.cu, layers_gemv.cu and layers_latent.cu, prefetches in layers_mamba.cu, the offsets in piece_add_kernel): their launchers say
+// which arguments the launch ahead must not write.
 __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
