@@ -14,7 +14,7 @@
 // The forward is bound by the latencies of a tile's chain (scores, maximum, exponentials, P through shared memory, P V): with one
 // thread per row that read its scores twice and let the next scores wait for P, issue slots were busy 35 % of the time.  Two
 // threads a row with the scores in registers, next scores issued at once: 93 -> 71 us (16 x 1024 tokens, 12/4 heads), 186 -> 103
-// (32 x 1024 in documents of 397: visibility is one bit per key), 37 -> 28 (16 x 512), 23 -> 18 (1 x 1000).
+// (32 x 1024 in documents of 397: visibility is one bit per key; 105 with exact maxima), 37 -> 28 (16 x 512), 23 -> 18 (1 x 1000).
 //
 // Segment masks are passed as `lo[i]` = first key position visible to query i (start of its packed document,
 // or 0): visible(i, j) <=> max(lo[i], i - window + 1) <= j <= i.  Every wait is bounded (status word on expiry).
