@@ -333,10 +333,15 @@ class InferenceEngine(TokenLoop):
             self._prompt_seen = True
             return
         if self._prompt_graph is None:
-            torch.cuda.synchronize()
+            # recorded on a stream of its own, nothing runs; torch.cuda.graph() would also empty the allocator's cache, which costs
+            # this prompt up to 20 ms
             g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g, capture_error_mode="thread_local"):   # records the launches, runs nothing
-                m.prompt_forward(self)
+            with torch.cuda.stream(torch.cuda.Stream(self.dev)):
+                g.capture_begin(capture_error_mode="thread_local")         # other threads may call CUDA
+                try:
+                    m.prompt_forward(self)
+                finally:
+                    g.capture_end()
             self._prompt_graph = g
         self._prompt_graph.replay()
 
