@@ -8,6 +8,7 @@ bf16, accumulation is fp32, the output dtype is chosen by the caller.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 
 import torch
@@ -246,10 +247,12 @@ PIECE_BYTES = 96 << 20
 PIECE_MIN_KBLOCKS = 16
 
 
+@functools.lru_cache(maxsize=256)
 def _best_cut(tiles, lens, mn):
     """k-blocks of the best pieces for reductions of these lengths (k-blocks, the longest first), or 0 where cutting does not gain a
     tenth.  Costs as the plan on the device estimates them (``plan_pieces``), with the 74 pairs of a whole B200; for one group the
-    result is the cut that the device uses, for several it only decides whether the device plans at all, so the two need not agree."""
+    result is the cut that the device uses, for several it only decides whether the device plans at all, so the two need not agree.
+    A function of sizes alone, so remembered (20 to 65 us a call)."""
     def cost(c):
         load, items, turn, extra = 0.0, 0, 0, 0
         for k in lens:
@@ -275,7 +278,7 @@ def _piece_scratch(M, N, kblocks, groups, out, longest=0):
     cut = 0
     if groups == 1 or longest:
         rest = max(1, (kblocks - longest) // (groups - 1)) if groups > 1 else 0
-        cut = _best_cut(tiles, [longest or kblocks] + [rest] * (groups - 1), M * N)
+        cut = _best_cut(tiles, (longest or kblocks,) + (rest,) * (groups - 1), M * N)
         if not cut:
             return None
     slots = min(64, PIECE_BYTES // (4 * M * N), kblocks // PIECE_MIN_KBLOCKS)      # a piece has at least that many k-blocks
