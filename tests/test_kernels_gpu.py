@@ -435,3 +435,19 @@ def test_bounded_waits_give_up_together():
     assert int(status[0]) in (101, 102)
     assert issued == 0
     assert limit <= cycles < 1.5 * limit, cycles
+
+
+def test_router_rows_at_any_address():
+    """Router rows that do not start on 16 bytes (the tensor-core kernel reads them in fours of four bytes then)."""
+    from ghassan_b200.ops import kernels as K
+    N, d, ne, top = 512, 256, 8, 2
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(N, d, device="cuda", generator=g).half()
+    rows = torch.randn(ne * d + 1, device="cuda", generator=g) * d ** -0.5
+    outs = []
+    for w in (rows[1:].view(ne, d), rows[1:].clone().view(ne, d)):
+        ws = K.MoeWorkspace(N, d, ne, top, True, torch.float16, "cuda")
+        K.moe_route_group(ws, x, w, None, torch.zeros(ws.cap, d, device="cuda", dtype=torch.float16), None, forward_only=True)
+        outs.append((ws.probs.clone(), ws.w.clone()))
+    assert rows[1:].data_ptr() % 16 == 4
+    assert float((outs[0][0] - outs[1][0]).abs().max()) <= 1e-5
