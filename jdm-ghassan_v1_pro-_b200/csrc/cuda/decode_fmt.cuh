@@ -1,6 +1,6 @@
 // Stored weight rows of the decode kernels: how eight consecutive values of a row are expanded into floats, per
-// storage format (formats and block layouts in gb_decode.h).  Shared by the per-kernel token step (decode.cu) and
-// the single-kernel token step (decode_mega.cu).
+// storage format (formats and block layouts in gb_decode.h), and the router's choice by one warp.  Shared by the per-kernel token step
+// (decode.cu) and the single-kernel token step (decode_mega.cu).
 #pragma once
 #include "sm100_common.cuh"
 #include "gb_decode.h"
@@ -58,6 +58,73 @@ __device__ __forceinline__ void load8(const uint8_t* __restrict__ row, int u, fl
 #pragma unroll
     for (int i = 0; i < 8; ++i) w[i] = d * (float)((v >> (4 * i)) & 0xF) + m;
   }
+}
+
+// Soft-max over ne <= 64 logits, lane e holding experts e (l0) and e + 32 (l1; -inf where there is none), and the top_k picks by
+// probability + bias (ties: the lower index), their probabilities renormalised.  Lane k < top_k gets pick k: expert my_e, weight my_w.
+__device__ __forceinline__ void warp_route(float l0, float l1, const float* __restrict__ bias, int ne, int top_k, int& my_e, float& my_w) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  if (ne <= 8) {                        // eight lanes do: three steps instead of five, nothing in a second register
+    float mx = lane < ne ? l0 : -INFINITY;
+#pragma unroll
+    for (int o = 4; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(full, mx, o));
+    const float p0 = lane < ne ? __expf(l0 - mx) : 0.f;
+    float sum = p0;
+#pragma unroll
+    for (int o = 4; o; o >>= 1) sum += __shfl_xor_sync(full, sum, o);
+    const float p = p0 * (1.f / sum), score = lane < ne ? p + (bias ? bias[lane] : 0.f) : -INFINITY;
+    int place = 0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float v = __shfl_sync(full, score, e);
+      place += e < ne && (v > score || (v == score && e < lane)) ? 1 : 0;
+    }
+    float psum = 0.f;
+    my_w = 0.f;
+    my_e = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const unsigned who = __ballot_sync(full, lane < ne && place == k);
+      const int e = who ? __ffs(who) - 1 : 0;
+      const float w = __shfl_sync(full, p, e);
+      if (k < top_k) {
+        if (lane == k) { my_e = e; my_w = w; }
+        psum += w;
+      }
+    }
+    my_w *= psum > 1e-8f ? 1.f / psum : 0.f;
+    return;
+  }
+  const bool h0 = lane < ne, h1 = lane + 32 < ne;
+  const float mx = warp_max(fmaxf(l0, l1));
+  float p0 = h0 ? __expf(l0 - mx) : 0.f, p1 = h1 ? __expf(l1 - mx) : 0.f;
+  const float inv = 1.f / warp_sum(p0 + p1);
+  p0 *= inv;
+  p1 *= inv;
+  float s0 = h0 ? p0 + (bias ? bias[lane] : 0.f) : -INFINITY;
+  float s1 = h1 ? p1 + (bias ? bias[lane + 32] : 0.f) : -INFINITY;
+  // An expert's place is the number of experts ahead of it: independent shuffles, where picking the best top_k times was a chain of ten
+  // shuffles a pick.
+  int r0 = 0, r1 = 0;
+#pragma unroll 8
+  for (int e = 0; e < ne; ++e) {
+    const float v = __shfl_sync(full, e < 32 ? s0 : s1, e & 31);
+    r0 += v > s0 || (v == s0 && e < lane) ? 1 : 0;
+    r1 += v > s1 || (v == s1 && e < lane + 32) ? 1 : 0;
+  }
+  float psum = 0.f;
+  my_w = 0.f;
+  my_e = 0;
+#pragma unroll 4
+  for (int k = 0; k < top_k; ++k) {
+    const unsigned b0 = __ballot_sync(full, h0 && r0 == k), b1 = __ballot_sync(full, h1 && r1 == k);
+    const int e = b0 ? __ffs(b0) - 1 : b1 ? __ffs(b1) + 31 : 0;
+    const float w = __shfl_sync(full, b0 ? p0 : p1, e & 31);
+    if (lane == k) { my_e = e; my_w = w; }
+    psum += w;
+  }
+  my_w *= psum > 1e-8f ? 1.f / psum : 0.f;
 }
 
 }  // namespace gb

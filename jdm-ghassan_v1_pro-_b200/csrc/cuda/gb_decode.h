@@ -124,19 +124,16 @@ typedef struct gb_mega_args {
   const float* cos_sin; int* pos;                // RoPE table [positions, hd]; pos[0] = position of the token
   gb_seq_state* state; int* slot_pos;            // advanced by the kernel at the end of the step
   int cap, pinned, window;
-  float* xbuf;                                   // 2 * d floats
-  void* qkv;                                     // (H + 2 KV) * hd 16-bit
-  float* att_scratch; int max_splits;            // H * max_splits * (hd + 2) floats
-  void* act;                                     // slots * E 16-bit
+  unsigned long long* words; int max_splits;     // exchange words (gb_decode_mega_words), zero before the first launch, the kernel's afterwards
   int* r_idx; float* r_w;                        // router choice of the last layer (may be NULL)
   unsigned* sync;                                // 4 words, zero before the first launch, owned by the kernel afterwards
-  int* status;                                   // set to 401 when a grid-wide wait ran out
-  unsigned long long* prof;                      // NULL, or 16 * n_layers + 2 words: CTA 0's global-timer marks in
-                                                 // nanoseconds (start; per layer both sides of each of the five
-                                                 // barriers and six points inside the phases; end)
-  int stage_bytes;                               // filled in by the launcher: shared-memory bytes per warp for staged rows
+  int* status;                                   // set to 401 when a wait for other CTAs ran out, 402 for a copy
+  unsigned long long* prof;                      // NULL, or 13 * n_layers + 2 words: CTA 0's global-timer marks in
+                                                 // nanoseconds (start; thirteen points of every layer; end)
+  int stage_bytes, at_stage, at_merge, at_rows;   // filled in by the launcher: shared-memory bytes per warp for staged rows, and offsets
 } gb_mega_args;
 int gb_decode_mega_ok(const gb_mega_args* a);    // 0 when the shapes are covered, else a negative code
+long long gb_decode_mega_words(const gb_mega_args* a);   // 64-bit words of `words`, from the sizes and max_splits
 int gb_decode_mega_grid(void);                   // CTAs of the launch (one per SM)
 int gb_decode_mega(const gb_mega_args* a, cudaStream_t st);
 

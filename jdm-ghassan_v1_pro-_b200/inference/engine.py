@@ -198,11 +198,9 @@ class InferenceEngine(TokenLoop):
         a.cos_sin, a.pos = self.cos_sin.data_ptr(), self.pos.data_ptr()
         a.state, a.slot_pos = self.state.data_ptr(), self.slot_pos.data_ptr()
         a.cap, a.pinned, a.window = self.cap, PINNED_TOKENS, cfg.sliding_window
-        self._mega_x = torch.zeros(2 * cfg.hidden_size, dtype=torch.float32, device=self.dev)
-        a.xbuf, a.qkv = self._mega_x.data_ptr(), self.qkv.data_ptr()
         a.max_splits = max(1, min(64, grid // max(1, cfg.num_kv_heads)))
-        self._mega_scratch = torch.zeros(cfg.num_heads * a.max_splits * (cfg.head_dim + 2), dtype=torch.float32, device=self.dev)
-        a.att_scratch, a.act = self._mega_scratch.data_ptr(), self.act.data_ptr()
+        self._mega_words = CA.zeros(D.mega_words(a), dtype=torch.int64, device=self.dev)
+        a.words = self._mega_words.data_ptr()
         a.r_idx, a.r_w = self.r_idx.data_ptr(), self.r_w.data_ptr()
         self._mega_sync = torch.zeros(4, dtype=torch.int32, device=self.dev)
         a.sync, a.status = self._mega_sync.data_ptr(), _lib_status(self.dev).data_ptr()
@@ -210,13 +208,13 @@ class InferenceEngine(TokenLoop):
             self.mega = a
 
     def trace_phases(self, n_tokens: int = 16) -> Dict[str, float]:
-        """Mean microseconds that CTA 0 of the one-kernel step spends in each phase of a layer and at the barrier
-        behind it, over ``n_tokens`` eager steps from the current state (the marks come from the device's global
-        timer).  Keys: A (norm + QKV), B (attention: ``B_rope``, ``B_walk``, ``B_merge``), C (``C_factors``, ``C_sum``,
-        ``C_proj``), D (``D_norm``, ``D_route``, ``D_experts``), E (down projection), ``wait_X`` for the barrier after
-        phase X, ``head`` and ``step``."""
+        """Mean microseconds that CTA 0 of the one-kernel step spends in each part of a layer, over ``n_tokens`` eager steps from the
+        current state (the marks come from the device's global timer).  Keys ending in ``_in`` are the wait for the vector that
+        a phase reads, up to its being in shared memory: A (norm; QKV projection), B (attention: ``B_in`` queries rotated, ``B_walk``,
+        ``B_join`` of the warps, ``B_merge`` of the splits), C (output projection), D (norm; ``D_route``, ``D_experts``), E (down
+        projection); ``layer``, ``head`` and ``step``."""
         assert self.mega is not None, "the one-kernel token step is not in use"
-        nl, M = self.cfg.num_layers, 16
+        nl, M = self.cfg.num_layers, 13
         buf = torch.zeros(M * nl + 2, dtype=torch.int64, device=self.dev)
         self.mega.prof = buf.data_ptr()
         acc = np.zeros(M * nl + 1)
@@ -229,11 +227,8 @@ class InferenceEngine(TokenLoop):
             self.mega.prof = None
         acc /= n_tokens * 1e3
         per = acc[:M * nl].reshape(nl, M)
-        names = ["A", "wait_A", "B_rope", "B_walk", "B_merge", "wait_B", "C_factors", "C_sum", "C_proj", "wait_C", "D_norm",
-                 "D_route", "D_experts", "wait_D", "E", "wait_E"]
+        names = ["A_in", "A", "B_in", "B_walk", "B_join", "B_merge", "C_in", "C", "D_in", "D_route", "D_experts", "E_in", "E"]
         out = {k: float(per[:, i].mean()) for i, k in enumerate(names)}
-        for ph in "BCD":
-            out[ph] = sum(v for k, v in out.items() if k.startswith(ph + "_"))
         out["layer"] = float(per.sum(1).mean())
         out["head"] = float(acc[M * nl])
         out["step"] = float(acc.sum())

@@ -241,11 +241,9 @@ class MegaArgs(ctypes.Structure):
         ("cos_sin", c_vp), ("pos", c_vp),
         ("state", c_vp), ("slot_pos", c_vp),
         ("cap", c_int), ("pinned", c_int), ("window", c_int),
-        ("xbuf", c_vp), ("qkv", c_vp),
-        ("att_scratch", c_vp), ("max_splits", c_int),
-        ("act", c_vp),
+        ("words", c_vp), ("max_splits", c_int),
         ("r_idx", c_vp), ("r_w", c_vp),
-        ("sync", c_vp), ("status", c_vp), ("prof", c_vp), ("stage_bytes", c_int),
+        ("sync", c_vp), ("status", c_vp), ("prof", c_vp), ("stage_bytes", c_int), ("at_stage", c_int), ("at_merge", c_int), ("at_rows", c_int),
     ]
 
 
@@ -258,6 +256,13 @@ def mega_layer_table(layers, device) -> torch.Tensor:
 
 def mega_grid() -> int:
     return int(_lib.lib().gb_decode_mega_grid())
+
+
+def mega_words(a: MegaArgs) -> int:
+    """64-bit words of the exchange buffer for these sizes and ``max_splits``."""
+    f = _lib.lib().gb_decode_mega_words
+    f.restype = ctypes.c_longlong
+    return int(f(ctypes.byref(a)))
 
 
 def mega_ok(a: MegaArgs) -> int:

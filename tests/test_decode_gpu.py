@@ -471,6 +471,50 @@ def test_single_kernel_step_matches_kernel_chain(case):
     assert outs[0][0, 0] == outs[1][0, 0] and same >= 1, (outs[0], outs[1])
 
 
+# Query heads per key head (one to four are passes of their own, eight go four at a time), head sizes, and how many slots the cache holds: up to 64 a
+# CTA is one trip, more is several; 1537 and up make a CTA walk more than 64; a full ring wraps.
+@pytest.mark.parametrize("n", [1, 64, 65, 700, 1537, 2500])
+@pytest.mark.parametrize("hidden,H,KV", [(256, 4, 4), (512, 8, 4), (768, 12, 4), (512, 8, 2), (512, 8, 1), (256, 2, 1), (256, 8, 4)])
+def test_single_kernel_step_over_long_caches(hidden, H, KV, n):
+    """One step of the cooperative kernel against the kernel chain, from the same cache of ``n`` - 1 drawn keys and values."""
+    from ghassan_b200.inference.engine import InferenceEngine
+    from ghassan_b200.models.config import init_parameters
+    from ghassan_b200.ops import _lib
+    cap = 2400
+    cfg = _tiny_cfg(hidden_size=hidden, num_heads=H, num_kv_heads=KV, moe_expert_dim=256, max_seq_len=4096)
+    named = init_parameters(cfg, 7)
+    one = InferenceEngine(cfg, named, fmt="f16", batch=1, max_len=cap, prefill_chunk=32, single_kernel=True)
+    chain = InferenceEngine(cfg, named, fmt="f16", batch=1, max_len=cap, prefill_chunk=32, single_kernel=False)
+    assert one.mega is not None and chain.mega is None
+    g = torch.Generator(device="cuda").manual_seed(n)
+    seen, held = n - 1, min(n - 1, cap)
+    ring = max(0, seen - cap) % (cap - 8)
+    for e in (one, chain):
+        e.reset(1)
+    for La, Lb in zip(one.layers, chain.layers):
+        La.cK.copy_(torch.randn(La.cK.shape, device="cuda", generator=g))
+        La.cV.copy_(torch.randn(La.cV.shape, device="cuda", generator=g))
+        Lb.cK.copy_(La.cK)
+        Lb.cV.copy_(La.cV)
+    one.slot_pos.copy_(torch.randint(0, max(1, seen), one.slot_pos.shape, device="cuda", generator=g, dtype=torch.int32))
+    chain.slot_pos.copy_(one.slot_pos)
+    one.state.copy_(torch.tensor([[held, seen, ring, 0][:one.state.shape[1]]], dtype=torch.int32))
+    chain.state.copy_(one.state)
+    for e in (one, chain):
+        e.pos.fill_(seen)
+    for step in range(3):
+        for e in (one, chain):
+            e.cur_tok.fill_(100 + step)
+            e._forward_token()
+        err, scale = float((one.logits - chain.logits).abs().max()), float(chain.logits.abs().max())
+        assert err <= 4e-3 * max(1.0, scale), (step, err, scale)        # as in the test above: the order of fp32 sums, between 16-bit stores
+        assert one.state.cpu().tolist() == chain.state.cpu().tolist()
+    _lib.check_status(what="single-kernel step over a long cache")
+    assert torch.equal(one.slot_pos, chain.slot_pos)
+    for La, Lb in zip(one.layers, chain.layers):
+        assert torch.allclose(La.cK.float(), Lb.cK.float(), atol=3.2e-2) and torch.allclose(La.cV.float(), Lb.cV.float(), atol=3.2e-2)
+
+
 def test_single_kernel_step_is_refused_for_uncovered_shapes():
     from ghassan_b200.inference.engine import InferenceEngine
     from ghassan_b200.models.config import init_parameters
