@@ -601,6 +601,80 @@ __global__ void __launch_bounds__(GV_THREADS) route_norm_kernel(const float* __r
   }
 }
 
+// RMSNorm and router of a batch's tokens, one block per token: the 16-bit normed row, and the token's weight for every expert (zero where it
+// is not chosen; 1 for the shared expert, the last).  The norm's and the router's weights are asked for before the wait for
+// the kernel ahead.  Up to 1024 columns and 8 experts everything stays in registers; more of either takes the loops behind.
+// Bound by its chain of round trips: 32 tokens of width 768, 8 experts 3.2 us (norm, router, scan and sorted copy were 21).
+template <typename XT>
+__global__ void __launch_bounds__(GV_THREADS) norm_route_few_kernel(const float* __restrict__ x32, const float* __restrict__ norm_w, float eps,
+                                                                    const float* __restrict__ rw, const float* __restrict__ bias, int d, int ne,
+                                                                    int top_k, int shared, XT* __restrict__ x16, float* __restrict__ weights) {
+  extern __shared__ __align__(16) uint8_t gv_dyn[];
+  XT* xs = reinterpret_cast<XT*>(gv_dyn);                 // [d]
+  __shared__ float lg[64], red[GV_WARPS];
+  const int b = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, n4 = d / 4;
+  constexpr int NR = 8;                                   // 16-byte loads of a router row per lane that are kept
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 r[NR], g = tid < n4 ? reinterpret_cast<const float4*>(norm_w)[tid] : zero;
+#pragma unroll
+  for (int k = 0; k < NR; ++k)
+    r[k] = warp < ne && lane + 32 * k < n4 ? reinterpret_cast<const float4*>(rw + (size_t)warp * d)[lane + 32 * k] : zero;
+  pdl_wait();
+  const float4* xr = reinterpret_cast<const float4*>(x32 + (long long)b * d);
+  const float4 x = tid < n4 ? xr[tid] : zero;
+  float ss = x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
+  for (int i = tid + GV_THREADS; i < n4; i += GV_THREADS) { const float4 v = xr[i]; ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w; }
+  ss = warp_sum(ss);
+  if (lane == 0) red[warp] = ss;
+  __syncthreads();
+  float tot = 0.f;
+#pragma unroll
+  for (int i = 0; i < GV_WARPS; ++i) tot += red[i];
+  float inv = rsqrtf(tot / (float)d + eps);
+  if (!isfinite(inv)) inv = 0.f;
+  uint2* out = reinterpret_cast<uint2*>(x16 + (long long)b * d);
+  auto put = [&](int i, const float4& v, const float4& w) {
+    const uint2 q = make_uint2(Cvt<XT>::pack2(v.x * inv * w.x, v.y * inv * w.y), Cvt<XT>::pack2(v.z * inv * w.z, v.w * inv * w.w));
+    reinterpret_cast<uint2*>(xs)[i] = q;
+    out[i] = q;
+  };
+  if (tid < n4) put(tid, x, g);
+  for (int i = tid + GV_THREADS; i < n4; i += GV_THREADS) put(i, xr[i], reinterpret_cast<const float4*>(norm_w)[i]);
+  __syncthreads();
+  for (int e = warp; e < ne; e += GV_WARPS) {
+    const float4* wr = reinterpret_cast<const float4*>(rw + (size_t)e * d);
+    float s = 0.f;
+    auto dot = [&](int i, const float4& w) {
+      const uint2 q = reinterpret_cast<const uint2*>(xs)[i];
+      const float2 u = Cvt<XT>::unpack2(q.x), v = Cvt<XT>::unpack2(q.y);
+      s += u.x * w.x + u.y * w.y + v.x * w.z + v.y * w.w;
+    };
+#pragma unroll
+    for (int k = 0; k < NR; ++k)
+      if (lane + 32 * k < n4) dot(lane + 32 * k, e == warp ? r[k] : wr[lane + 32 * k]);
+    for (int i = lane + 32 * NR; i < n4; i += 32) dot(i, wr[i]);
+    s = warp_sum(s);
+    if (lane == 0) lg[e] = s;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    int my_e;
+    float my_w;
+    warp_route(lane < ne ? lg[lane] : -INFINITY, lane + 32 < ne ? lg[lane + 32] : -INFINITY, bias, ne, top_k, my_e, my_w);
+    float w0 = 0.f, w1 = 0.f;
+    for (int k = 0; k < top_k; ++k) {
+      const int e = __shfl_sync(0xffffffffu, my_e, k);
+      const float w = __shfl_sync(0xffffffffu, my_w, k);
+      if (e == lane) w0 = w;
+      if (e == lane + 32) w1 = w;
+    }
+    float* dst = weights + (long long)b * (ne + (shared ? 1 : 0));
+    if (lane < ne) dst[lane] = w0;
+    if (lane + 32 < ne) dst[lane + 32] = w1;
+    if (shared && lane == 0) dst[ne] = 1.f;
+  }
+}
+
 // grid (ceil(E / rows per block), B * slots).  idx == nullptr: dense feed-forward (one "expert" 0).
 template <int FMT, int KS, typename XT>
 __global__ void __launch_bounds__(GV_THREADS) swiglu_norm_kernel(
@@ -912,6 +986,23 @@ extern "C" int gb_route_norm(const float* x32, const float* norm_w, float eps, c
   cudaLaunchConfig_t cfg = gb_pdl_config(dim3(B), dim3(GV_THREADS), smem, st, &attr);
   if (is_bf16) (void)cudaLaunchKernelEx(&cfg, route_norm_kernel<__nv_bfloat16>, x32, norm_w, eps, router_w, bias, d, ne, top_k, idx_out, w_out);
   else (void)cudaLaunchKernelEx(&cfg, route_norm_kernel<__half>, x32, norm_w, eps, router_w, bias, d, ne, top_k, idx_out, w_out);
+  return gb_launch_rc();
+}
+
+// RMSNorm of x32 [B, d] into x16 [B, d], and the weight of every token for every expert: weights [B, ne (+ 1 shared)] fp32.  norm_w, router_w
+// and bias are not what the launch ahead writes.
+extern "C" int gb_norm_route_few(const float* x32, const float* norm_w, float eps, const float* router_w, const float* bias, int B, int d,
+                                 int ne, int top_k, int shared, void* x16, float* weights, int is_bf16, cudaStream_t st) {
+  if (!x32 || !norm_w || !router_w || !x16 || !weights || B <= 0 || ne <= 0 || ne > 64 || top_k <= 0 || top_k > 8 || top_k > ne || d <= 0 || d % 8)
+    return -1;
+  if ((reinterpret_cast<uintptr_t>(x32) | reinterpret_cast<uintptr_t>(norm_w) | reinterpret_cast<uintptr_t>(router_w) | reinterpret_cast<uintptr_t>(x16)) & 15)
+    return -1;
+  const size_t smem = (size_t)d * 2;
+  if (smem > 40 * 1024) return -2;
+  cudaLaunchAttribute attr;
+  cudaLaunchConfig_t cfg = gb_pdl_config(dim3(B), dim3(GV_THREADS), smem, st, &attr);
+  if (is_bf16) (void)cudaLaunchKernelEx(&cfg, norm_route_few_kernel<__nv_bfloat16>, x32, norm_w, eps, router_w, bias, d, ne, top_k, shared, (__nv_bfloat16*)x16, weights);
+  else (void)cudaLaunchKernelEx(&cfg, norm_route_few_kernel<__half>, x32, norm_w, eps, router_w, bias, d, ne, top_k, shared, (__half*)x16, weights);
   return gb_launch_rc();
 }
 

@@ -45,8 +45,12 @@ typedef struct gb_gemm_args {
                               // partial sums of reductions that are cut into pieces (at most 64 groups; seg_offsets may be
                               // null for one group over K; part_cut > 0: k-blocks of its pieces).  null: reductions stay whole
   int skinny;                 // 1: few rows (gemm_skinny_sm100.cu): M <= 128, mode 0, both operands with K contiguous, N a multiple of 8,
-                              // rows of out and addend 16-byte aligned; epilogue 0 or 4.  block_n is ignored
+                              // rows of out and addend 16-byte aligned; epilogue 0, 1 (N counts output columns; no addend, 16-bit out,
+                              // nothing saved) or 4.  block_n is ignored
   int b_static;               // skinny: B is no output of the launch before this one (weights): it may be read ahead of that launch's end
+  int k_group;                // skinny, epilogue 0: > 0 (a multiple of 64 that divides K): values g * k_group .. of K meet rows g * b_group_rows ..
+                              // of B (b_cols == k_group), as the down projections of several experts do
+  const float* scale; int ld_scale, scale_cols;  // skinny, epilogue 1: out(m, j) *= scale[m * ld_scale + j / scale_cols]; where that is 0 out is 0
 } gb_gemm_args;
 int gb_gemm(const gb_gemm_args* args, cudaStream_t stream);
 int gb_gemm_pair(const gb_gemm_args* args, cudaStream_t stream);   // what gb_gemm calls when args->pair != 0

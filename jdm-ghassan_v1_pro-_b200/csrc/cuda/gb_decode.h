@@ -90,6 +90,10 @@ int gb_gemv_norm(const void* W, int fmt, int N, int K, const float* x32, int ldx
 // Router of rmsnorm(x32) [B, d]: picks to idx_out / w_out [B, top_k].
 int gb_route_norm(const float* x32, const float* norm_w, float eps, const float* router_w, const float* bias, int B, int d,
                   int ne, int top_k, int* idx_out, float* w_out, int is_bf16, cudaStream_t st);
+// The same for a batch whose tokens go through all experts: the normed rows x16 [B, d] and weights [B, ne (+ 1 shared)], zero where an expert
+// is not chosen.
+int gb_norm_route_few(const float* x32, const float* norm_w, float eps, const float* router_w, const float* bias, int B, int d,
+                      int ne, int top_k, int shared, void* x16, float* weights, int is_bf16, cudaStream_t st);
 // act = SwiGLU(gate, up) of the experts named by idx [B, top_k] (+ the shared one) applied to rmsnorm(x32).
 // idx == NULL: dense feed-forward block.
 int gb_swiglu_norm(const void* Wg, const void* Wu, int fmt, int ne, int E, int d, const float* x32, const float* norm_w, float eps,

@@ -250,6 +250,10 @@ class CudaModel:
         f32 = dict(dtype=torch.float32, device=dev)
         c16 = dict(dtype=dt, device=dev)
         nl = cfg.num_layers if train else 1     # evaluation reuses one layer's buffers
+        # Few tokens visit nearly all experts: 1 - (1 - top_k / ne)^N of them, two thirds from here on.  All rows then go through all experts, with no
+        # sorting and no rows padded to 256 (32 tokens, 2 of 8 experts and a shared one of 768, width 768: 47 us a layer's feed-forward -> 20).
+        self.experts_few = (not train and cfg.use_moe and N <= 128 and N * cfg.moe_top_k >= cfg.num_experts and cfg.num_experts <= 64
+                            and cfg.moe_top_k <= 8 and E % 64 == 0 and d <= 20480)
         self.x = [CA.empty(N, d, **f32) for _ in range((cfg.num_layers + 1) if train else 2)]
         self.layers: List[_LayerBuf] = []
         for _ in range(nl):
@@ -266,6 +270,8 @@ class CudaModel:
                 b.xperm, b.yperm = CA.zeros(rows, d, **c16), CA.zeros(rows, d, **c16)
             else:
                 rows = N
+            if self.experts_few:
+                b.few_w, b.few_act = CA.zeros(N, self.layout.ne1, **f32), CA.zeros(N, self.layout.ne1 * E, **c16)
             b.gu, b.act = CA.zeros(rows, 2 * E, **c16), CA.zeros(rows, E, **c16)
             self.layers.append(b)
         rows = self.layers[0].ws.cap if cfg.use_moe else N
@@ -377,6 +383,12 @@ class CudaModel:
         else:
             self._attention_forward(l, b, qw, kw)
         G.gemm(b.att, self.w16(p + "wo"), out=b.x_mid, addend=x_in, b_static=dec is not None)
+        if self.experts_few and not train and self.ep is None:
+            from ..ops import decode as D
+            D.norm_route_few(b.x_mid, self.w(p + "ffn_norm"), cfg.rms_eps, self.w(p + "router"), self.moe_bias[l] if self.moe_bias is not None else None,
+                             cfg.moe_top_k, cfg.moe_shared, b.xb2, b.few_w)
+            G.experts_few(b.xb2, self.w16(p + "w_gu"), self.w16(p + "w_down"), b.few_w, b.few_act, x_out, b.x_mid)
+            return
         K.rmsnorm_fwd(b.x_mid, self.w(p + "ffn_norm"), b.xb2, b.rrms2, cfg.rms_eps)
         self._ffn_forward(l, p, b, x_out, train, want_aux)
 

@@ -174,6 +174,16 @@ def route_norm(x32, norm_w, eps, router_w, bias, top_k, idx, w, is_bf16=False):
     _lib.check_rc(rc, "gb_route_norm")
 
 
+def norm_route_few(x32, norm_w, eps, router_w, bias, top_k, shared, x16, weights):
+    """RMSNorm of every row into ``x16`` and its weights for all experts (fp32 ``[B, ne (+ 1 shared)]``, zero where not chosen)."""
+    B, d = x32.shape
+    rc = _lib.lib().gb_norm_route_few(c_vp(x32.data_ptr()), c_vp(norm_w.data_ptr()), c_float(eps), c_vp(router_w.data_ptr()),
+                                      c_vp(bias.data_ptr()) if bias is not None else None, c_int(B), c_int(d), c_int(router_w.shape[0]),
+                                      c_int(top_k), c_int(int(shared)), c_vp(x16.data_ptr()), c_vp(weights.data_ptr()), c_int(_bf(x16)),
+                                      _lib.stream_ptr())
+    _lib.check_rc(rc, "gb_norm_route_few")
+
+
 def swiglu_norm(wg: QWeight, wu: QWeight, ne, E, d, x32, norm_w, eps, idx, top_k, shared, act):
     """RMSNorm + gate/up of the experts in ``idx`` (``None``: dense block) in one launch."""
     rc = _lib.lib().gb_swiglu_norm(c_vp(wg.data.data_ptr()), c_vp(wu.data.data_ptr()), c_int(wg.fmt), c_int(ne), c_int(E),

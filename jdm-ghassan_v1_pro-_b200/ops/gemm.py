@@ -124,6 +124,27 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_dtype=None, addend=None,
     return out
 
 
+def experts_few(a, w_gu, w_down, weights, act, out, addend):
+    """All rows of ``a`` through all experts, for batches so small that their tokens visit nearly every expert: ``out = addend +
+    sum_e weights[:, e] * expert_e(a)``.  ``w_gu`` ``[ne * 2E, d]`` interleaved, ``w_down`` ``[ne * d, E]``, ``weights`` fp32 ``[M, ne]``,
+    ``act`` 16-bit ``[M, ne * E]`` scratch, ``out`` and ``addend`` fp32 ``[M, d]``.  Weights may be read ahead of the launch before."""
+    (M, d), ne, E = a.shape, weights.shape[1], w_down.shape[1]
+    if M > 128 or act.shape != (M, ne * E) or w_gu.shape != (ne * 2 * E, d) or w_down.shape != (ne * d, E) or E % 64:
+        raise ValueError("experts_few: shapes")
+    g = _base_args(a, w_gu, M, ne * E, d, False, False, act, 0)
+    g.epilogue = EPI_SWIGLU_FWD
+    g.skinny = g.b_static = 1
+    g.scale, g.ld_scale, g.scale_cols = weights.data_ptr(), weights.stride(0), E
+    _launch(g)
+    g = _base_args(act, w_down, M, d, ne * E, False, False, out, 0)
+    g.epilogue = EPI_STORE
+    g.skinny = g.b_static = 1
+    g.k_group, g.b_group_rows = E, d
+    g.addend, g.ld_add = addend.data_ptr(), addend.stride(0)
+    _launch(g)
+    return out
+
+
 def gemm_swiglu(a, w_gu, *, act_out=None, gu_out=None, tile_expert=None, num_m_tiles=None, group_rows=0, pair=None):
     """Fused ``[gate|up]`` projection + SwiGLU.
 

@@ -1,0 +1,61 @@
+"""All tokens of a small batch through all experts (``gemm_skinny_sm100.cu``) and the norm + router kernel ahead of it, against fp32."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+CASES = [  # tokens, width, experts, picks, shared, expert width: tile edges of 8, 32 and 128 rows, 32 / 64 columns, clusters over K, more experts than warps
+    (1, 64, 2, 2, False, 64), (7, 256, 4, 2, True, 64), (8, 512, 8, 2, True, 512), (31, 768, 8, 4, True, 192), (33, 776, 3, 1, False, 128),
+    (64, 256, 12, 3, True, 64), (100, 1032, 40, 8, False, 64), (128, 768, 8, 2, True, 768)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "-".join(str(int(x)) for x in c))
+def test_experts_few(case, dtype):
+    from ghassan_b200.ops import _lib, decode as D, gemm as G
+    B, d, ne, top, shared, E = case
+    g = torch.Generator(device="cuda").manual_seed(B * d)
+    n = lambda *s: torch.randn(s, device="cuda", generator=g)
+    x, norm_w, router, bias = n(B, d), 1.0 + 0.1 * n(d), n(ne, d) * d ** -0.5, 0.01 * n(ne)
+    ne1 = ne + int(shared)
+    gate, up, down = (n(ne1, E, d) * d ** -0.5).to(dtype), (n(ne1, E, d) * d ** -0.5).to(dtype), (n(ne1, d, E) * E ** -0.5).to(dtype)
+    x16, weights = torch.empty(B, d, device="cuda", dtype=dtype), torch.full((B, ne1), 7.0, device="cuda")
+    D.norm_route_few(x, norm_w, 1e-5, router, bias, top, shared, x16, weights)
+    want16 = x * torch.rsqrt(x.pow(2).mean(1, keepdim=True) + 1e-5) * norm_w
+    eps = torch.finfo(dtype).eps
+    assert float((x16.float() - want16).abs().max()) <= eps * float(want16.abs().max())          # half a unit in the last place, and the fp32 norm
+    p = torch.softmax(x16.float() @ router.t(), 1)
+    pick = (p + bias).topk(top, 1).indices
+    want_w = torch.zeros(B, ne, device="cuda").scatter_(1, pick, p.gather(1, pick))
+    want_w /= want_w.sum(1, keepdim=True)
+    near = (p + bias).sort(1, descending=True).values
+    clear = torch.ones(B, dtype=torch.bool, device="cuda") if top == ne else near[:, top - 1] - near[:, top] > 1e-4        # no tie in the last bits
+    assert int(clear.sum()) >= B // 2
+    assert float((weights[:, :ne] - want_w)[clear].abs().max()) <= 1e-5
+    assert not shared or bool((weights[:, ne] == 1.0).all())
+    act, out, resid = torch.full((B, ne1 * E), 3.0, device="cuda", dtype=dtype), torch.empty(B, d, device="cuda"), n(B, d)
+    w_gu = G.interleave_gate_up(gate, up).reshape(ne1 * 2 * E, d)
+    G.experts_few(x16, w_gu, down.reshape(ne1 * d, E), weights, act, out, resid)
+    _lib.check_status(what="experts_few")
+    h = x16.float()
+    want_act = torch.stack([torch.nn.functional.silu(h @ gate[e].float().t()) * (h @ up[e].float().t()) * weights[:, e:e + 1] for e in range(ne1)], 1)
+    assert float((act.float().view(B, ne1, E) - want_act).abs().max()) <= eps * float(want_act.abs().max())
+    assert bool((act.view(B, ne1, E)[weights == 0] == 0).all())
+    want = resid + torch.einsum("bek,edk->bd", act.float().view(B, ne1, E), down.float())
+    assert float((out - want).abs().max()) <= 2e-5 * float(want.abs().max()) + 1e-6 * (ne1 * E) ** 0.5       # fp32 sums in another order
+
+
+def test_unchosen_expert_does_not_matter():
+    """An expert that no token has chosen may hold infinities."""
+    from ghassan_b200.ops import gemm as G
+    B, d, ne, E = 16, 256, 4, 64
+    g = torch.Generator(device="cuda").manual_seed(5)
+    h = torch.randn(B, d, device="cuda", generator=g).half()
+    w_gu = (torch.randn(ne * 2 * E, d, device="cuda", generator=g) * 0.05).half()
+    down = (torch.randn(ne * d, E, device="cuda", generator=g) * 0.1).half()
+    w_gu[2 * E:4 * E] = float("inf")
+    weights = torch.rand(B, ne, device="cuda", generator=g)
+    weights[:, 1] = 0.0
+    act, out = torch.empty(B, ne * E, device="cuda", dtype=torch.float16), torch.empty(B, d, device="cuda")
+    G.experts_few(h, w_gu, down, weights, act, out, torch.zeros(B, d, device="cuda"))
+    assert bool(torch.isfinite(out).all()) and bool((act[:, E:2 * E] == 0).all())
