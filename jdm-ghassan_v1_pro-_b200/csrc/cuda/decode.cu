@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(GV_THREADS) route_norm_kernel(const float* __r
 }
 
 // RMSNorm and router of a batch's tokens, one block per token: the 16-bit normed row, and the token's weight for every expert (zero where it
-// is not chosen; 1 for the shared expert, the last).  The norm's and the router's weights are asked for before the wait for
+// is not chosen; 1 for the shared expert, the last).  ne == 0: the norm alone.  The norm's and the router's weights are asked for before the wait for
 // the kernel ahead.  Up to 1024 columns and 8 experts everything stays in registers; more of either takes the loops behind.
 // Bound by its chain of round trips: 32 tokens of width 768, 8 experts 3.2 us (norm, router, scan and sorted copy were 21).
 template <typename XT>
@@ -640,6 +640,7 @@ __global__ void __launch_bounds__(GV_THREADS) norm_route_few_kernel(const float*
   };
   if (tid < n4) put(tid, x, g);
   for (int i = tid + GV_THREADS; i < n4; i += GV_THREADS) put(i, xr[i], reinterpret_cast<const float4*>(norm_w)[i]);
+  if (ne == 0) return;
   __syncthreads();
   for (int e = warp; e < ne; e += GV_WARPS) {
     const float4* wr = reinterpret_cast<const float4*>(rw + (size_t)e * d);
@@ -989,12 +990,12 @@ extern "C" int gb_route_norm(const float* x32, const float* norm_w, float eps, c
   return gb_launch_rc();
 }
 
-// RMSNorm of x32 [B, d] into x16 [B, d], and the weight of every token for every expert: weights [B, ne (+ 1 shared)] fp32.  norm_w, router_w
+// RMSNorm of x32 [B, d] into x16 [B, d], and the weight of every token for every expert: weights [B, ne (+ 1 shared)] fp32 (ne == 0: the norm alone).  norm_w, router_w
 // and bias are not what the launch ahead writes.
 extern "C" int gb_norm_route_few(const float* x32, const float* norm_w, float eps, const float* router_w, const float* bias, int B, int d,
                                  int ne, int top_k, int shared, void* x16, float* weights, int is_bf16, cudaStream_t st) {
-  if (!x32 || !norm_w || !router_w || !x16 || !weights || B <= 0 || ne <= 0 || ne > 64 || top_k <= 0 || top_k > 8 || top_k > ne || d <= 0 || d % 8)
-    return -1;
+  if (!x32 || !norm_w || !x16 || B <= 0 || d <= 0 || d % 8) return -1;
+  if (ne != 0 && (!router_w || !weights || ne < 0 || ne > 64 || top_k <= 0 || top_k > 8 || top_k > ne)) return -1;
   if ((reinterpret_cast<uintptr_t>(x32) | reinterpret_cast<uintptr_t>(norm_w) | reinterpret_cast<uintptr_t>(router_w) | reinterpret_cast<uintptr_t>(x16)) & 15)
     return -1;
   const size_t smem = (size_t)d * 2;

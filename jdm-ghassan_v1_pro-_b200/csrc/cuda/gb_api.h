@@ -50,6 +50,7 @@ typedef struct gb_gemm_args {
   int b_static;               // skinny: B is no output of the launch before this one (weights): it may be read ahead of that launch's end
   int k_group;                // skinny, epilogue 0: > 0 (a multiple of 64 that divides K): values g * k_group .. of K meet rows g * b_group_rows ..
                               // of B (b_cols == k_group), as the down projections of several experts do
+  int n1;                     // skinny, epilogue 4: > 0 (a multiple of 8): columns below n1 are stored as they are, the others in aux_out
   const float* scale; int ld_scale, scale_cols;  // skinny, epilogue 1: out(m, j) *= scale[m * ld_scale + j / scale_cols]; where that is 0 out is 0
 } gb_gemm_args;
 int gb_gemm(const gb_gemm_args* args, cudaStream_t stream);

@@ -1,11 +1,13 @@
 // GEMM of few rows for sm_100a: C[M, N] = A[M, K] * W[N, K]^T with M <= 128 (a batch of token steps, a short prompt).  Such a
 // product is a stream of weights with one tile of rows, and in the persistent kernel (gemm_sm100.cu) a chain: 32 x 3840 by
 // 1024 x 3840 has sixteen 64-column tiles, so sixteen SMs walk sixty k-blocks each while the others idle.  Here a cluster of S
-// CTAs shares a 128 x 64 tile: each takes K / S of the reduction, keeps its part of the sum in its tensor memory, writes it to
-// its shared memory, and every CTA adds and stores 1 / S of the tile, the parts in the order of K.
-// us, the persistent kernel -> this one with early weights (floor by bytes at 6.5 TB/s): 32 x 3840 x 1024 16.7 -> 7.7 (1.2), 32 x 1024 x
-// 2816 7.5 -> 6.0 (0.9), 32 x 768 x 1280 6.6 -> 4.5 (0.3), 8 x 6912 x 2560 26.9 -> 11.2 (5.5), 128 x 6912 x 2560 28.9 -> 14.3; 100 x 2816
-// x 1024 14.2 -> 7.0 (15.0 with clusters of eight).  What is left is launch, the round trips of the first loads and the exchange.
+// CTAs shares a 128 x 64 tile: each takes K / S of the reduction, keeps its part of the sum in its tensor memory and writes 1 / S of it
+// into the shared memory of each of the others with a bulk copy; every CTA then adds and stores its share of the tile, the parts in the order of K.
+// Row by row, in pieces of four columns, the same writes took 1 us; fetched from the others when all were there, another round trip and a second wait
+// for the cluster so that nobody leaves early, 1 to 1.8 us more than now (from the last product to the last store 1.3 us).
+// us, the persistent kernel -> this one with early weights (floor by bytes at 6.5 TB/s), before the exchange by bulk copies: 32 x 3840 x 1024
+// 16.7 -> 7.7 (1.2), 32 x 1024 x 2816 7.5 -> 6.0 (0.9), 32 x 768 x 1280 6.6 -> 4.5 (0.3), 8 x 6912 x 2560 26.9 -> 11.2 (5.5), 128 x 6912 x 2560
+// 28.9 -> 14.3, 100 x 2816 x 1024 14.2 -> 7.0.  What is left is launch, the round trips of the first loads and the exchange.
 //
 // The kernel is launched with programmatic dependency: barriers, tensor memory and, where the caller says that W is not what
 // the kernel before writes (weights), the first eight k-blocks of W are under way before griddepcontrol.wait.
@@ -19,6 +21,8 @@
 // one product whose K runs over all experts, each with a row block of its own in W.
 // 32 tokens, 9 experts of 768, width 768 (32 MB of weights, 4.9 us at the copy rate): gate and up 7.3 us, down 8.7; sorted by expert 12.6, 9.1, and 14 for
 // sorting and adding up.
+#include <atomic>
+
 #include "sm100_common.cuh"
 #include "gb_api.h"
 
@@ -28,10 +32,10 @@ namespace sk {
 static constexpr int BN = 64, BK = 64, STAGES = 8, THREADS = 192;   // warps 0-3 accumulators, 4 TMA, 5 MMA
 static constexpr int W_TMA = 4, W_MMA = 5;
 static constexpr uint32_t W_BYTES = BN * BK * 2;
-static constexpr int PITCH = BN + 4;                                // floats of a row of the partial sums: lanes hit all banks
 
 struct Params {
-  int M, N, K, fmt, split;      // split: CTAs of a cluster
+  int M, N, K, fmt, split, lg;  // split: CTAs of a cluster, 2 to the power lg
+  int stages;                   // at most STAGES
   int a_rows;                   // rows of A per stage
   int w_early, relu2;
   void* out; int ldo;
@@ -39,13 +43,14 @@ struct Params {
   int* status;
   int k_group, w_group;         // K is cut into groups of k_group k-blocks (0: one), each with its own w_group rows of W
   const float* scale; int ld_scale, scale_cols;    // SwiGLU: factor of (row, column / scale_cols)
+  int n1; void* out2; int ldo2;                    // relu2: columns below n1 as they are into out, the others into out2
 };
 
 template <typename OutT, bool SWIGLU>
 __global__ void __launch_bounds__(THREADS) gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW,
                                                               const Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], done_bar;
+  __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], done_bar, parts_bar;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_word;
   volatile int* abort_flag = &abort_word;
@@ -56,62 +61,95 @@ __global__ void __launch_bounds__(THREADS) gemm_skinny_kernel(const __grid_const
   const uint32_t a_bytes = (uint32_t)p.a_rows * (BK * 2), stage_bytes = a_bytes + W_BYTES;
   const int blocks = (p.K + BK - 1) / BK;
   const int kb0 = rank * blocks / p.split, nkb = (rank + 1) * blocks / p.split - kb0;      // at least one: split <= blocks
+  // Parts of this CTA's share of the tile: [source][row][BN / split columns and four more, so that lanes hit all banks].  They lie behind the stages, where
+  // the MMAs read rows that nothing uses.
+  const int width = BN >> p.lg, pitch = width + 4, share = p.M * pitch;
+  float* parts = reinterpret_cast<float*>(smem + (uint32_t)p.stages * stage_bytes);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     mbar_init(&done_bar, 1);
+    mbar_init(&parts_bar, 1);
     abort_word = 0;
     fence_barrier_init();
+    if (p.split > 1) mbar_arrive_expect_tx(&parts_bar, (uint32_t)(p.split * share) * 4);
   }
   if (warp == W_MMA) { tmem_alloc(&tmem_slot, BN); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");       // waited for before the first write to another CTA
+  // units of four columns; what a thread's first two are added to or scaled by is asked for before the sums are there
+  constexpr int LG_ROW = SWIGLU ? 3 : 4;
+  const int per_row = 1 << (LG_ROW - p.lg), units = p.M * per_row;
+  auto column = [&](int u) { return n0 + rank * (COLS >> p.lg) + (u & (per_row - 1)) * 4; };
+  auto addend_of = [&](int u) {
+    const int row = u >> (LG_ROW - p.lg), col = column(u);
+    return p.addend && u < units && col < p.N ? *reinterpret_cast<const float4*>(p.addend + (long long)row * p.ld_add + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  float4 add0 = make_float4(0.f, 0.f, 0.f, 0.f), add1 = add0;
+  float scale0 = 1.f, scale1 = 1.f;
+  auto scale_of = [&](int u) {
+    const int col = column(u);
+    return SWIGLU && p.scale && u < units && col < p.N ? p.scale[(long long)(u >> (LG_ROW - p.lg)) * p.ld_scale + col / p.scale_cols] : 1.f;
+  };
+  auto ahead = [&]() {
+    add0 = addend_of(threadIdx.x);
+    add1 = addend_of(threadIdx.x + THREADS);
+    scale0 = scale_of(threadIdx.x);
+    scale1 = scale_of(threadIdx.x + THREADS);
+  };
 
   if (warp == W_TMA) {
     const uint32_t on = elect_one();
-    auto stage = [&](int i) { return smem + (uint32_t)(i % STAGES) * stage_bytes; };
-    auto load_w = [&](int i) {
-      mbar_arrive_expect_tx_on(on, &full_bar[i % STAGES], stage_bytes);        // both operands' bytes
+    if (on) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmA)) : "memory");
+    auto load_w = [&](int i, int slot) {
+      uint8_t* dst = smem + (uint32_t)slot * stage_bytes + a_bytes;
+      mbar_arrive_expect_tx_on(on, &full_bar[slot], stage_bytes);              // both operands' bytes
       if constexpr (SWIGLU) {        // stored in blocks of 64 gate rows and 64 up rows
         const int row = (n0 >> 6) * 128 + (n0 & 63);
-        tma_load_2d_on(on, &tmW, &full_bar[i % STAGES], stage(i) + a_bytes, (kb0 + i) * BK, row);
-        tma_load_2d_on(on, &tmW, &full_bar[i % STAGES], stage(i) + a_bytes + W_BYTES / 2, (kb0 + i) * BK, row + 64);
+        tma_load_2d_on(on, &tmW, &full_bar[slot], dst, (kb0 + i) * BK, row);
+        tma_load_2d_on(on, &tmW, &full_bar[slot], dst + W_BYTES / 2, (kb0 + i) * BK, row + 64);
       } else {
         const int kb = kb0 + i, g = p.k_group ? kb / p.k_group : 0;
-        tma_load_2d_on(on, &tmW, &full_bar[i % STAGES], stage(i) + a_bytes, (kb - g * p.k_group) * BK, g * p.w_group + n0);
+        tma_load_2d_on(on, &tmW, &full_bar[slot], dst, (kb - g * p.k_group) * BK, g * p.w_group + n0);
       }
     };
-    const int early = p.w_early ? min(nkb, STAGES) : 0;
-    for (int i = 0; i < early; ++i) load_w(i);
+    const int early = p.w_early ? min(nkb, p.stages) : 0;
+    for (int i = 0; i < early; ++i) load_w(i, i);
     pdl_wait();
-    for (int i = 0; i < nkb; ++i) {
-      if (i >= STAGES) wait_or_leave(&empty_bar[i % STAGES], ((i / STAGES) & 1) ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
-      if (i >= early) load_w(i);
-      tma_load_2d_on(on, &tmA, &full_bar[i % STAGES], stage(i), (kb0 + i) * BK, 0);
+    for (int i = 0, slot = 0, round = 0; i < nkb; ++i) {
+      if (round > 0) wait_or_leave(&empty_bar[slot], (round & 1) ^ 1, p.status, ST_TIMEOUT_EMPTY, abort_flag);
+      if (i >= early) load_w(i, slot);
+      tma_load_2d_on(on, &tmA, &full_bar[slot], smem + (uint32_t)slot * stage_bytes, (kb0 + i) * BK, 0);
+      if (++slot == p.stages) { slot = 0; ++round; }
     }
     __syncwarp();
+    ahead();
   } else if (warp == W_MMA) {
     const uint32_t on = elect_one();
     const uint32_t idesc = make_idesc_f16(p.fmt, 0, 0, 128, BN);
-    for (int i = 0; i < nkb; ++i) {
-      wait_or_report(&full_bar[i % STAGES], (i / STAGES) & 1, p.status, ST_TIMEOUT_FULL, abort_flag);
+    for (int i = 0, slot = 0, round = 0; i < nkb; ++i) {
+      wait_or_report(&full_bar[slot], round & 1, p.status, ST_TIMEOUT_FULL, abort_flag);
       tc_fence_after();
-      const uint32_t sa = smem_u32(smem) + (uint32_t)(i % STAGES) * stage_bytes;
+      const uint32_t sa = smem_u32(smem) + (uint32_t)slot * stage_bytes;
       const uint64_t da = make_smem_desc_sw128(sa, 16, 1024), dw = make_smem_desc_sw128(sa + a_bytes, 16, 1024);
 #pragma unroll
       for (int kk = 0; kk < BK / 16; ++kk) umma_f16_on(on, tmem, da + kk * 2, dw + kk * 2, idesc, i > 0 || kk > 0 ? 1u : 0u);
-      umma_commit_on(on, &empty_bar[i % STAGES]);
+      umma_commit_on(on, &empty_bar[slot]);
+      if (++slot == p.stages) { slot = 0; ++round; }
     }
     umma_commit_on(on, &done_bar);
     __syncwarp();
     pdl_wait();
+    ahead();
   } else {
     pdl_wait();
+    ahead();
     wait_or_report(&done_bar, 0, p.status, ST_TIMEOUT_TMEM_FULL, abort_flag);
     tc_fence_after();
-    // every product is taken: the stages hold the partial sums now
+    // every product is taken: the stages hold this CTA's part of the tile now, a share behind the other (SwiGLU: gate and up columns in one)
     const int row = warp * 32 + lane;
     if (warp * 32 < p.M) {
 #pragma unroll
@@ -120,78 +158,79 @@ __global__ void __launch_bounds__(THREADS) gemm_skinny_kernel(const __grid_const
         tmem_ld_32x32(tmem + ((uint32_t)(warp * 32) << 16) + c * 32, r);
         tmem_ld_wait();
         if (row < p.M) {
-          float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(smem) + row * PITCH + c * 32);
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            dst[k] = make_float4(__uint_as_float(r[4 * k]), __uint_as_float(r[4 * k + 1]), __uint_as_float(r[4 * k + 2]), __uint_as_float(r[4 * k + 3]));
+          for (int k = 0; k < 4; ++k) {
+            const int cg = c * 4 + k, own = SWIGLU ? k << p.lg >> 2 : cg << p.lg >> 3;
+            const int at = SWIGLU ? c * (width >> 1) + ((k * 8) & ((width >> 1) - 1)) : (cg * 8) & (width - 1);
+            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<float*>(smem) + own * share + row * pitch + at);
+            dst[0] = make_uint4(r[8 * k], r[8 * k + 1], r[8 * k + 2], r[8 * k + 3]);
+            dst[1] = make_uint4(r[8 * k + 4], r[8 * k + 5], r[8 * k + 6], r[8 * k + 7]);
+          }
         }
       }
     }
     tc_fence_before();
+    fence_proxy_async();                               // read by the copies below
   }
   __syncthreads();
   if (*abort_flag) {
     for (int i = 0; i < 64; ++i) __nanosleep(1000);    // copies still in flight get time to land
     __syncthreads();
   }
-  cluster_sync_all();
-  const int units = p.M * (COLS / 8), u0 = rank * units / p.split, u1 = (rank + 1) * units / p.split;
-  for (int u = u0 + (int)threadIdx.x; u < u1; u += THREADS) {
-    const int row = u / (COLS / 8), c = (u - row * (COLS / 8)) * 8, col = n0 + c;
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");          // the others have begun, their barriers are set up
+  if (p.split > 1) {
+    if (threadIdx.x == 0)
+      for (int r = 0; r < p.split; ++r) {
+        const uint32_t own = (uint32_t)((rank + r) & (p.split - 1));
+        asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         mapa_shared(smem_u32(parts) + (uint32_t)(rank * share) * 4, own)),
+                     "r"(smem_u32(smem) + own * (uint32_t)share * 4), "r"((uint32_t)share * 4), "r"(mapa_shared(smem_u32(&parts_bar), own))
+                     : "memory");
+      }
+    wait_or_report(&parts_bar, 0, p.status, ST_TIMEOUT_AUX, abort_flag);
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // all copies into this CTA have landed
+  } else {
+    parts = reinterpret_cast<float*>(smem);
+  }
+  for (int u = (int)threadIdx.x; u < units; u += THREADS) {
+    const int row = u >> (LG_ROW - p.lg), col = column(u);
     if (col >= p.N) continue;                          // N is a multiple of 8
-    const uint32_t at = smem_u32(smem) + (uint32_t)(row * PITCH + c) * 4;
-    float4 add[2];
-    float scale = 1.f;
-    if (p.addend) {
-      const float4* src = reinterpret_cast<const float4*>(p.addend + (long long)row * p.ld_add + col);
-      add[0] = src[0];
-      add[1] = src[1];
-    }
-    if (SWIGLU && p.scale) scale = p.scale[(long long)row * p.ld_scale + col / p.scale_cols];
-    auto total = [&](uint32_t from, float (&v)[8]) {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) v[k] = 0.f;
+    const int turn = u / THREADS;
+    const float4 add = turn == 0 ? add0 : turn == 1 ? add1 : addend_of(u);
+    const float scale = turn == 0 ? scale0 : turn == 1 ? scale1 : scale_of(u);
+    const float* src = parts + row * pitch + (u & (per_row - 1)) * 4;
+    auto total = [&](const float* from) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
       for (int g = 0; g < p.split; ++g) {
-        const uint32_t src = mapa_shared(from, (uint32_t)g);
-        float4 x, y;
-        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(src) : "memory");
-        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(y.x), "=f"(y.y), "=f"(y.z), "=f"(y.w) : "r"(src + 16) : "memory");
-        v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
-        v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
+        const float4 x = *reinterpret_cast<const float4*>(from + g * share);
+        v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
       }
+      return v;
     };
-    float v[8];
-    total(at, v);
+    const float4 t = total(src);
+    float v[4] = {t.x, t.y, t.z, t.w};
     if constexpr (SWIGLU) {
-      float up[8];
-      total(at + (BN / 2) * 4, up);
+      const float4 t2 = total(src + (width >> 1));
+      const float up[4] = {t2.x, t2.y, t2.z, t2.w};
 #pragma unroll
-      for (int k = 0; k < 8; ++k) v[k] = scale == 0.f ? 0.f : v[k] / (1.f + __expf(-v[k])) * up[k] * scale;   // not chosen: zero, whatever the product is
+      for (int k = 0; k < 4; ++k) v[k] = scale == 0.f ? 0.f : v[k] / (1.f + __expf(-v[k])) * up[k] * scale;   // not chosen: zero, whatever the product is
     }
-    if (p.addend) {
-      v[0] += add[0].x; v[1] += add[0].y; v[2] += add[0].z; v[3] += add[0].w;
-      v[4] += add[1].x; v[5] += add[1].y; v[6] += add[1].z; v[7] += add[1].w;
-    }
-    if (p.relu2) {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) { v[k] = fmaxf(v[k], 0.f); v[k] *= v[k]; }
-    }
+    v[0] += add.x; v[1] += add.y; v[2] += add.z; v[3] += add.w;
     OutT* dst = reinterpret_cast<OutT*>(p.out) + (long long)row * p.ldo + col;
-    if constexpr (sizeof(OutT) == 4) {
-      reinterpret_cast<float4*>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
-      reinterpret_cast<float4*>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
-    } else {
-      uint4 q;
-      q.x = Cvt<OutT>::pack2(v[0], v[1]);
-      q.y = Cvt<OutT>::pack2(v[2], v[3]);
-      q.z = Cvt<OutT>::pack2(v[4], v[5]);
-      q.w = Cvt<OutT>::pack2(v[6], v[7]);
-      *reinterpret_cast<uint4*>(dst) = q;
+    if (p.relu2 && col >= p.n1) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) { v[k] = fmaxf(v[k], 0.f); v[k] *= v[k]; }
+      if (p.out2) dst = reinterpret_cast<OutT*>(p.out2) + (long long)row * p.ldo2 + col - p.n1;
     }
+    if constexpr (sizeof(OutT) == 4) *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+    else *reinterpret_cast<uint2*>(dst) = make_uint2(Cvt<OutT>::pack2(v[0], v[1]), Cvt<OutT>::pack2(v[2], v[3]));
   }
-  cluster_sync_all();                                  // the other CTAs have read this one's shared memory
   if (warp == W_MMA) { tc_fence_after(); tmem_dealloc(tmem, BN); }
+  __syncwarp();
+  if (p.split > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");       // and all copies out of it
+  if (*abort_flag)
+    for (int i = 0; i < 64; ++i) __nanosleep(1000);    // copies of a CTA whose waits ran out may still be on their way
 }
 
 }  // namespace sk
@@ -199,25 +238,62 @@ __global__ void __launch_bounds__(THREADS) gemm_skinny_kernel(const __grid_const
 
 namespace {
 
-template <typename OutT, bool SWIGLU = false>
-int launch_skinny(const CUtensorMap& ta, const CUtensorMap& tw, const gb::sk::Params& p, cudaStream_t st) {
+constexpr size_t MOST_SMEM = 226 * 1024;
+
+// Shared memory of a launch: stages, and behind them the larger of the parts and of the rows that the MMAs read past the last stage.
+size_t skinny_smem(const gb::sk::Params& p) {
   namespace sk = gb::sk;
-  auto kern = sk::gemm_skinny_kernel<OutT, SWIGLU>;
-  // behind the last stage the MMA still reads up to 128 rows; the partial sums are smaller than eight stages
-  const size_t smem = (size_t)sk::STAGES * (p.a_rows * 128 + sk::W_BYTES) + (128 - p.a_rows) * 128 + 1024;
-  static_assert((size_t)sk::STAGES * (8 * 128 + sk::W_BYTES) >= 128 * sk::PITCH * 4, "partial sums fit the stages");
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sk::STAGES * (128 * 128 + (int)sk::W_BYTES) + 1024) != cudaSuccess) return -10;
-    attr = true;
-  }
+  const size_t parts = (size_t)p.M * (sk::BN + 4 * p.split) * 4, tail = (size_t)(128 - p.a_rows) * 128;
+  return (size_t)p.stages * (p.a_rows * 128 + sk::W_BYTES) + (parts > tail ? parts : tail) + 1024;
+}
+
+template <typename OutT, bool SWIGLU>
+cudaLaunchConfig_t skinny_config(const gb::sk::Params& p, cudaStream_t st, cudaLaunchAttribute* at) {
+  namespace sk = gb::sk;
   constexpr int COLS = SWIGLU ? sk::BN / 2 : sk::BN;
-  cudaLaunchAttribute at[2];
-  cudaLaunchConfig_t cfg = gb_pdl_config(dim3((unsigned)((p.N + COLS - 1) / COLS * p.split)), dim3(sk::THREADS), smem, st, &at[1]);
+  cudaLaunchConfig_t cfg = gb_pdl_config(dim3((unsigned)((p.N + COLS - 1) / COLS * p.split)), dim3(sk::THREADS), skinny_smem(p), st, &at[1]);
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = (unsigned)p.split; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs += 1;
+  return cfg;
+}
+
+template <typename OutT, bool SWIGLU = false>
+int launch_skinny(const CUtensorMap& ta, const CUtensorMap& tw, gb::sk::Params p, cudaStream_t st) {
+  namespace sk = gb::sk;
+  auto kern = sk::gemm_skinny_kernel<OutT, SWIGLU>;
+  static bool attr = false;
+  if (!attr) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST_SMEM) != cudaSuccess) { (void)cudaGetLastError(); return -10; }
+    attr = true;
+  }
+  // CTAs of a tile: as many as leave all tiles resident at once, which the driver is asked for (296 CTAs of half an SM each do not all fit where they come
+  // in fours: 32 x 4352 x 1024 with four CTAs a tile had a few late clusters, 10.2 us, with two it has none, 6.0).  Fewer than two k-blocks per
+  // CTA do not pay for the exchange.
+  constexpr int COLS = SWIGLU ? sk::BN / 2 : sk::BN, MOST = SWIGLU ? 4 : 8;
+  const int tiles = (p.N + COLS - 1) / COLS, blocks = (p.K + sk::BK - 1) / sk::BK;
+  static std::atomic<int> fits[4][17];                // clusters of 2, 4, 8 CTAs that fit, plus one, by rows of A in eights
+  cudaLaunchAttribute at[2];
+  p.split = 1;
+  for (int lg = 1; (1 << lg) <= MOST && blocks >= (1 << lg) * 2; ++lg) {
+    sk::Params q = p;
+    q.split = 1 << lg;
+    q.lg = lg;
+    q.M = q.a_rows;
+    for (q.stages = sk::STAGES; skinny_smem(q) > MOST_SMEM;) --q.stages;
+    int n = fits[lg][p.a_rows / 8].load(std::memory_order_relaxed);
+    if (!n) {
+      const cudaLaunchConfig_t cfg = skinny_config<OutT, SWIGLU>(q, st, at);
+      if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = 0; }
+      fits[lg][p.a_rows / 8].store(++n, std::memory_order_relaxed);
+    }
+    if (tiles > n - 1) break;
+    p.split = q.split;
+    p.lg = lg;
+  }
+  for (p.stages = sk::STAGES; skinny_smem(p) > MOST_SMEM;) --p.stages;
+  const cudaLaunchConfig_t cfg = skinny_config<OutT, SWIGLU>(p, st, at);
   if (cudaLaunchKernelEx(&cfg, kern, ta, tw, p) != cudaSuccess) return -10;
   return gb_launch_rc();
 }
@@ -226,6 +302,7 @@ int launch_skinny(const CUtensorMap& ta, const CUtensorMap& tw, const gb::sk::Pa
 
 // gb_gemm with args->skinny: M <= 128, mode 0, K contiguous in both operands, N a multiple of 8, 16-byte aligned rows of out and addend.
 // k_group > 0: K runs over groups of k_group values, group g against rows g * b_group_rows + (0 .. N - 1) of B.
+// epilogue 4 with n1: columns below n1 into out as they are, the others, squared where positive, into aux_out from its column 0.
 // epilogue 1: SwiGLU over 2 N interleaved rows of B, column j times scale[row, j / scale_cols] where scale is given; 16-bit out.
 extern "C" int gb_gemm_skinny(const gb_gemm_args* a, cudaStream_t st) {
   namespace sk = gb::sk;
@@ -244,14 +321,11 @@ extern "C" int gb_gemm_skinny(const gb_gemm_args* a, cudaStream_t st) {
   p.out = a->out; p.ldo = a->ldo; p.addend = a->addend; p.ld_add = a->ld_add; p.status = a->status;
   p.k_group = a->k_group / sk::BK; p.w_group = a->b_group_rows;
   p.scale = a->scale; p.ld_scale = a->ld_scale; p.scale_cols = a->scale_cols;
-  // As many CTAs as the SMs hold at once: two per SM while their stages are small.  Fewer than two k-blocks per CTA do not
-  // pay for the exchange.
-  const int cols = swiglu ? sk::BN / 2 : sk::BN;
-  const int tiles = (a->N + cols - 1) / cols, blocks = (a->K + sk::BK - 1) / sk::BK;
-  const bool two = p.a_rows <= 32;
-  const int room = 148 * (two ? 2 : 1), most = two ? 8 : 4;      // eight CTAs that need an SM each do not fit a GPC twice
-  p.split = 1;
-  while (p.split < most && tiles * p.split * 2 <= room && blocks >= p.split * 4) p.split *= 2;
+  if (a->n1) {
+    if (a->epilogue != 4 || a->n1 < 0 || a->n1 % 8 || a->n1 > a->N || !a->aux_out || (reinterpret_cast<uintptr_t>(a->aux_out) & 15) || ((long long)a->ld_aux * es) % 16)
+      return -1;
+    p.n1 = a->n1; p.out2 = a->aux_out; p.ldo2 = a->ld_aux;
+  }
   CUtensorMap ta, tw;
   int rc = gb_make_tmap_2d_16b(&ta, a->A, a->a_rows, a->a_cols, a->lda, p.a_rows, sk::BK, a->is_bf16);
   if (rc) return rc - 100;

@@ -367,8 +367,12 @@ class CudaModel:
         p = f"L{l}."
         d, qd, kvd, H, KV, hd = cfg.hidden_size, cfg.q_dim, cfg.kv_dim, cfg.num_heads, cfg.num_kv_heads, cfg.head_dim
         E = self.layout.Eff
-        K.rmsnorm_fwd(x_in, self.w(p + "attn_norm"), b.xb, b.rrms1, cfg.rms_eps)
         dec = getattr(self, "decode_engine", None)
+        if dec is not None and d <= 20480:
+            from ..ops import decode as D
+            D.norm_few(x_in, self.w(p + "attn_norm"), cfg.rms_eps, b.xb)
+        else:
+            K.rmsnorm_fwd(x_in, self.w(p + "attn_norm"), b.xb, b.rrms1, cfg.rms_eps)
         G.gemm(b.xb, self.w16(p + "wqkv"), out=b.qkv, b_static=dec is not None)
         qw = self.w(p + "qk_qnorm") if cfg.use_qk_norm else None
         kw = self.w(p + "qk_knorm") if cfg.use_qk_norm else None

@@ -41,7 +41,7 @@ class GemmArgs(ctypes.Structure):
         ("pair", c_int),
         ("part", c_vp), ("part_slots", c_int), ("part_cut", c_int),
         ("skinny", c_int), ("b_static", c_int),
-        ("k_group", c_int), ("scale", c_vp), ("ld_scale", c_int), ("scale_cols", c_int),
+        ("k_group", c_int), ("n1", c_int), ("scale", c_vp), ("ld_scale", c_int), ("scale_cols", c_int),
     ]
 
 

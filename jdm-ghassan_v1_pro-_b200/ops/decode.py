@@ -174,6 +174,14 @@ def route_norm(x32, norm_w, eps, router_w, bias, top_k, idx, w, is_bf16=False):
     _lib.check_rc(rc, "gb_route_norm")
 
 
+def norm_few(x32, norm_w, eps, x16):
+    """RMSNorm of a few fp32 rows into ``x16``, as a link of the token step's chain of launches."""
+    B, d = x32.shape
+    rc = _lib.lib().gb_norm_route_few(c_vp(x32.data_ptr()), c_vp(norm_w.data_ptr()), c_float(eps), None, None, c_int(B), c_int(d), c_int(0), c_int(0),
+                                      c_int(0), c_vp(x16.data_ptr()), None, c_int(_bf(x16)), _lib.stream_ptr())
+    _lib.check_rc(rc, "gb_norm_route_few")
+
+
 def norm_route_few(x32, norm_w, eps, router_w, bias, top_k, shared, x16, weights):
     """RMSNorm of every row into ``x16`` and its weights for all experts (fp32 ``[B, ne (+ 1 shared)]``, zero where not chosen)."""
     B, d = x32.shape

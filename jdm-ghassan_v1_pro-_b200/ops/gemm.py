@@ -124,6 +124,20 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_dtype=None, addend=None,
     return out
 
 
+def gemm_two(a, w, n1, out1, out2):
+    """``out1 = a @ w[:n1]^T`` and ``out2 = max(a @ w[n1:]^T, 0) ** 2`` (bf16) of at most 128 rows in one launch, or False where
+    :func:`gemm` would not take the few-rows kernel for it.  ``w`` may be read ahead of the launch before."""
+    (M, K), N = a.shape, w.shape[0]
+    if not skinny_ok(M, N, out1) or n1 % 8 or not skinny_ok(M, N, out2) or out1.dtype != torch.bfloat16 or out2.dtype != torch.bfloat16:
+        return False
+    g = _base_args(a, w, M, N, K, False, False, out1, 0)
+    g.epilogue = EPI_RELU2
+    g.skinny = g.b_static = 1
+    g.n1, g.aux_out, g.ld_aux = n1, out2.data_ptr(), out2.stride(0)
+    _launch(g)
+    return True
+
+
 def experts_few(a, w_gu, w_down, weights, act, out, addend):
     """All rows of ``a`` through all experts, for batches so small that their tokens visit nearly every expert: ``out = addend +
     sum_e weights[:, e] * expert_e(a)``.  ``w_gu`` ``[ne * 2E, d]`` interleaved, ``w_down`` ``[ne * d, E]``, ``weights`` fp32 ``[M, ne]``,
@@ -145,7 +159,13 @@ def experts_few(a, w_gu, w_down, weights, act, out, addend):
     return out
 
 
-def gemm_swiglu(a, w_gu, *, act_out=None, gu_out=None, tile_expert=None, num_m_tiles=None, group_rows=0, pair=None):
+def swiglu_skinny_ok(M, N, act_out):
+    """True where a product of at most 128 rows with SwiGLU takes the few-rows kernel: 32 output columns a tile, as many tiles as the SMs
+    hold at once (two an SM up to 32 rows). """
+    return M <= 128 and N // 64 <= (296 if M <= 32 else 148) and act_out.data_ptr() % 16 == 0 and act_out.stride(-2) % 8 == 0
+
+
+def gemm_swiglu(a, w_gu, *, act_out=None, gu_out=None, tile_expert=None, num_m_tiles=None, group_rows=0, pair=None, b_static=False):
     """Fused ``[gate|up]`` projection + SwiGLU.
 
     ``w_gu`` stores gate and up rows interleaved in blocks of 64 (``g0..g63,u0..u63,g64..``) so that one
@@ -161,6 +181,10 @@ def gemm_swiglu(a, w_gu, *, act_out=None, gu_out=None, tile_expert=None, num_m_t
         act_out = torch.empty(M, N // 2, dtype=a.dtype, device=a.device)
     g = _base_args(a, w_gu, M, N, K, False, False, act_out, 256 if (N % 256 == 0 and M >= 4096) else 128)
     g.epilogue = EPI_SWIGLU_FWD
+    if pair is None and tile_expert is None and gu_out is None and swiglu_skinny_ok(M, N, act_out):
+        g.N, g.skinny, g.b_static = N // 2, 1, int(b_static)
+        _launch(g)
+        return act_out
     g.pair = int(pair_ok(M, N, act_out, extra=(gu_out,)) if pair is None else bool(pair))
     if gu_out is not None:
         g.aux_out, g.ld_aux = gu_out.data_ptr(), gu_out.stride(0)

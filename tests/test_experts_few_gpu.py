@@ -19,10 +19,13 @@ def test_experts_few(case, dtype):
     x, norm_w, router, bias = n(B, d), 1.0 + 0.1 * n(d), n(ne, d) * d ** -0.5, 0.01 * n(ne)
     ne1 = ne + int(shared)
     gate, up, down = (n(ne1, E, d) * d ** -0.5).to(dtype), (n(ne1, E, d) * d ** -0.5).to(dtype), (n(ne1, d, E) * E ** -0.5).to(dtype)
+    eps = torch.finfo(dtype).eps
     x16, weights = torch.empty(B, d, device="cuda", dtype=dtype), torch.full((B, ne1), 7.0, device="cuda")
     D.norm_route_few(x, norm_w, 1e-5, router, bias, top, shared, x16, weights)
     want16 = x * torch.rsqrt(x.pow(2).mean(1, keepdim=True) + 1e-5) * norm_w
-    eps = torch.finfo(dtype).eps
+    alone = torch.empty_like(x16)
+    D.norm_few(x, norm_w, 1e-5, alone)
+    assert torch.equal(alone, x16)
     assert float((x16.float() - want16).abs().max()) <= eps * float(want16.abs().max())          # half a unit in the last place, and the fp32 norm
     p = torch.softmax(x16.float() @ router.t(), 1)
     pick = (p + bias).topk(top, 1).indices
@@ -59,3 +62,47 @@ def test_unchosen_expert_does_not_matter():
     act, out = torch.empty(B, ne * E, device="cuda", dtype=torch.float16), torch.empty(B, d, device="cuda")
     G.experts_few(h, w_gu, down, weights, act, out, torch.zeros(B, d, device="cuda"))
     assert bool(torch.isfinite(out).all()) and bool((act[:, E:2 * E] == 0).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 64, 64), (9, 256, 1024), (32, 2816, 1024), (33, 192, 200), (100, 2816, 1024), (128, 4736, 320)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_swiglu_of_few_rows(M, N, K, dtype):
+    from ghassan_b200.ops import gemm as G
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a, gate, up = (torch.randn(*s, device="cuda", generator=g).mul(k).to(dtype) for s, k in (((M, K), 1.0), ((N, K), K ** -0.5), ((N, K), K ** -0.5)))
+    out = torch.full((M, N), 3.0, device="cuda", dtype=dtype)
+    assert G.swiglu_skinny_ok(M, 2 * N, out)
+    G.gemm_swiglu(a, G.interleave_gate_up(gate, up), act_out=out)
+    want = torch.nn.functional.silu(a.float() @ gate.float().t()) * (a.float() @ up.float().t())
+    assert float((out.float() - want).abs().max()) <= torch.finfo(dtype).eps * float(want.abs().max())
+
+
+@pytest.mark.parametrize("M,n1,n2,K", [(1, 8, 8, 64), (31, 136, 248, 512), (32, 1536, 2816, 1024), (64, 1824, 512, 328), (128, 64, 64, 1024)])
+def test_two_outputs_of_few_rows(M, n1, n2, K):
+    from ghassan_b200.ops import gemm as G
+    g = torch.Generator(device="cuda").manual_seed(M + n1)
+    a, w = torch.randn(M, K, device="cuda", generator=g).bfloat16(), (torch.randn(n1 + n2, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    out1, both = torch.full((M, n1), 3.0, device="cuda", dtype=torch.bfloat16), torch.full((M, 8 + n2), 3.0, device="cuda", dtype=torch.bfloat16)
+    assert G.gemm_two(a, w, n1, out1, both[:, 8:])
+    want = a.float() @ w.float().t()
+    up = want[:, n1:].clamp(min=0) ** 2
+    eps = torch.finfo(torch.bfloat16).eps
+    assert float((out1.float() - want[:, :n1]).abs().max()) <= eps * float(want.abs().max())
+    assert float((both[:, 8:].float() - up).abs().max()) <= eps * float(up.abs().max()) and bool((both[:, :8] == 3).all())
+
+
+@pytest.mark.parametrize("splits", [1, 4, 8])
+def test_decode_attention_of_a_full_ring(splits):
+    """A cluster's splits over a cache whose next slot lies inside the ring."""
+    from ghassan_b200.ops import decode as D
+    B, H, KV, hd, cap = 2, 6, 2, 64, 300
+    g = torch.Generator(device="cuda").manual_seed(splits)
+    cK, cV = (torch.randn(B, cap, KV * hd, device="cuda", generator=g).half() for _ in range(2))
+    q, out = torch.randn(B, H * hd, device="cuda", generator=g).half(), torch.zeros(B, H * hd, device="cuda", dtype=torch.float16)
+    state = torch.zeros(B, D.STATE_INTS, dtype=torch.int32, device="cuda")
+    state[:, 0], state[:, 1], state[:, 2] = 1000, cap, 17
+    D.decode_attn(q, cK, cV, torch.zeros(B, cap, dtype=torch.int32, device="cuda"), state, out, torch.zeros(B * H * splits * (hd + 2), device="cuda"), splits,
+                  H, KV, hd, cap, 0, hd ** -0.5)
+    k, v = (c.float().view(B, cap, KV, hd).repeat_interleave(H // KV, 2) for c in (cK, cV))
+    want = torch.einsum("bhl,blhd->bhd", torch.softmax(torch.einsum("bhd,blhd->bhl", q.float().view(B, H, hd), k) * hd ** -0.5, -1), v)
+    assert float((out.float().view(B, H, hd) - want).abs().max()) < 2e-3          # fp32 throughout, rounded once, values below 4
