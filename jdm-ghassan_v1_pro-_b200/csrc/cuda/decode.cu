@@ -429,6 +429,227 @@ __global__ void __launch_bounds__(128) decode_attn_kernel(const T* __restrict__ 
   }
 }
 
+// The same for up to eight splits (1, 2, 4 or 8): the splits of a (sequence, kv head) are a cluster, whose CTAs exchange their results through
+// distributed shared memory and write the output, so there is no merge kernel behind it.  Keys and values are loaded two slots a lane ahead of
+// the ones being worked on, the first ones before the wait for the kernel ahead, which writes the step's own row and the queries and nothing
+// else that is read here (a full ring's next slot is not known here, so it loads behind the wait).
+// Bound by the latency of the chain and the instructions of the scores at short caches, by memory at long ones: 32 sequences, 500 slots, 3 query
+// heads a key head, 4 splits (16 MB, 2.5 us at the copy rate): 8.3 us of the step, before 9.9 with 8 splits and 2.4 for the merge.
+template <typename T, int HD, int G>
+__global__ void __launch_bounds__(128, G <= 4 ? 4 : 2) decode_attn_cluster_kernel(const T* __restrict__ q, long long ld_q, const T* __restrict__ cK,
+                                                                     const T* __restrict__ cV, const int* __restrict__ slot_pos,
+                                                                     const gb_seq_state* __restrict__ st, int splits, int H, int KV, int cap, int window,
+                                                                     float scale, T* __restrict__ out, long long ld_o) {
+  constexpr int LPS = HD / 8, SPW = 32 / LPS, TRIP = 2 * 4 * SPW;       // lanes per slot, slots side by side, slots of a trip of the CTA
+  __shared__ __align__(16) float sm_q[G][HD];
+  constexpr int PARTS = 4 * SPW;                                        // groups of lanes that share a slot, in the CTA
+  __shared__ float sm_m[PARTS + 1][G], sm_l[PARTS + 1][G], sm_f[PARTS][G];      // theirs, and the CTA's
+  __shared__ __align__(16) float sm_o[PARTS + 1][G][HD];
+  const int split = (int)cluster_ctarank(), item = (int)cluster_id_x(), b = item / KV, kvh = item - b * KV;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane / LPS, sub = lane % LPS;
+  const gb_seq_state s = st[b];
+  // the step's own token was appended before this kernel and is not counted in cache_len yet
+  const int n_slots = min(cap, s.cache_len + 1);
+  const bool full = s.cache_len >= cap;
+  const bool wide = ((reinterpret_cast<uintptr_t>(cK) | reinterpret_cast<uintptr_t>(cV)) & 15) == 0;    // rows are whole 64 bytes
+  const int per = (n_slots + splits - 1) / splits, lo = split * per, hi = min(n_slots, lo + per);
+  const long long kvd = (long long)KV * HD;
+  const T* kb = cK + (long long)b * cap * kvd + kvh * HD + sub * 8;
+  const T* vb = cV + (long long)b * cap * kvd + kvh * HD + sub * 8;
+  auto load8 = [&](const T* p) {
+    uint4 r;
+    if (wide) r = __ldcg(reinterpret_cast<const uint4*>(p));
+    else {
+      uint32_t w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) w[i] = Cvt<T>::pack2(Cvt<T>::to_f(__ldcg(p + 2 * i)), Cvt<T>::to_f(__ldcg(p + 2 * i + 1)));
+      r = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    return r;
+  };
+  struct Pair { uint4 k[2], v[2]; bool ok[2]; };
+  const int first = lo + warp * SPW + grp;                              // the lane's slot u of trip t: first + (2 t + u) * 4 SPW
+  auto fetch = [&](Pair& x, int t, bool own, bool rest) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int j = first + (2 * t + u) * 4 * SPW;
+      const bool mine = j == n_slots - 1;                               // the step's own slot, unless the ring is full
+      if (rest) {
+        x.ok[u] = j < hi;
+        x.k[u] = x.v[u] = make_uint4(0u, 0u, 0u, 0u);
+      }
+      if (j < hi && (mine ? own : rest)) {
+        x.k[u] = load8(kb + (long long)j * kvd);
+        x.v[u] = load8(vb + (long long)j * kvd);
+        if (window > 0) x.ok[u] = s.abs_pos - __ldcg(slot_pos + (long long)b * cap + j) < window;
+      }
+    }
+  };
+  Pair A, B2;
+  const int trips = hi > lo ? (hi - lo + TRIP - 1) / TRIP : 0;
+  if (!full) { fetch(A, 0, false, true); fetch(B2, 1, false, true); }
+  pdl_wait();
+  fetch(A, 0, true, full);
+  fetch(B2, 1, true, full);
+  for (int i = threadIdx.x; i < G * HD; i += 128) sm_q[i / HD][i % HD] = Cvt<T>::to_f(q[b * ld_q + (long long)kvh * G * HD + i]) * scale;
+  __syncthreads();
+  auto unpack8 = [](const uint4& r, float (&f)[8]) {
+    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { const float2 x = Cvt<T>::unpack2(w[i]); f[2 * i] = x.x; f[2 * i + 1] = x.y; }
+  };
+  // The scores of a trip are one to a lane: the sums over the lanes of a slot are exchanged so that lane `sub` ends up with sum number sub & (NS - 1)
+  // (heads below, the two slots above), which takes its exponential; the lanes then pass the weights round.
+  constexpr int GP = G <= 1 ? 1 : G <= 2 ? 2 : G <= 4 ? 4 : 8, NS = 2 * GP;
+  static_assert(NS <= 2 * LPS, "a slot's lanes hold at most two sums each");
+  constexpr int PER = NS > LPS ? 2 : 1, ND = NS / PER;                  // sums a lane ends up with, lanes that differ
+  const int mine = sub & (ND - 1);
+  float o[G][8], m[PER], l[PER];                                        // of the lane's heads: maximum, the lane's share of the sum
+#pragma unroll
+  for (int g = 0; g < G; ++g)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) o[g][e] = 0.f;
+#pragma unroll
+  for (int r = 0; r < PER; ++r) { m[r] = -INFINITY; l[r] = 0.f; }
+  // sum i = u * GP + g; after the exchange lane `mine` holds sums mine + r * ND
+  auto work = [&](const Pair& x) {
+    float s[NS];
+    {
+      float f[2][8];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) unpack8(x.k[u], f[u]);
+#pragma unroll
+      for (int g = 0; g < GP; ++g) {
+        if (g < G) {
+          const float4 q0 = *reinterpret_cast<const float4*>(&sm_q[g][sub * 8]), q1 = *reinterpret_cast<const float4*>(&sm_q[g][sub * 8 + 4]);
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+            s[u * GP + g] = q0.x * f[u][0] + q0.y * f[u][1] + q0.z * f[u][2] + q0.w * f[u][3] + q1.x * f[u][4] + q1.y * f[u][5] + q1.z * f[u][6] + q1.w * f[u][7];
+        } else {
+          s[g] = s[GP + g] = 0.f;
+        }
+      }
+    }
+#pragma unroll
+    for (int off = LPS / 2; off >= ND; off >>= 1)
+#pragma unroll
+      for (int i = 0; i < NS; ++i) s[i] += __shfl_xor_sync(0xffffffffu, s[i], off);
+#pragma unroll
+    for (int off = ND / 2; off > 0; off >>= 1) {
+      const bool up = (sub & off) != 0;
+#pragma unroll
+      for (int r = 0; r < PER; ++r)
+#pragma unroll
+        for (int i = 0; i < off; ++i) {
+          const float keep = up ? s[r * ND + i + off] : s[r * ND + i], give = up ? s[r * ND + i] : s[r * ND + i + off];
+          s[r * ND + i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+        }
+    }
+    float c[PER], p[PER], mn[PER], sc[PER];
+#pragma unroll
+    for (int r = 0; r < PER; ++r) {
+      const int i = mine + r * ND, u = i / GP;
+      sc[r] = (u == 0 ? x.ok[0] : x.ok[1]) ? s[r * ND] : -INFINITY;
+      mn[r] = fmaxf(m[r], sc[r]);
+    }
+    if constexpr (PER == 2) {                                          // the lane holds both slots of its head
+      mn[0] = mn[1] = fmaxf(mn[0], mn[1]);
+    } else {
+      mn[0] = fmaxf(mn[0], __shfl_xor_sync(0xffffffffu, mn[0], GP));
+    }
+#pragma unroll
+    for (int r = 0; r < PER; ++r) {
+      const float mu = mn[r] == -INFINITY ? 0.f : mn[r];               // nothing seen so far in this group of lanes
+      c[r] = __expf(m[r] - mu);
+      p[r] = __expf(sc[r] - mu);
+      l[r] = l[r] * c[r] + p[r];
+      m[r] = mn[r];
+    }
+    float f[2][8];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) unpack8(x.v[u], f[u]);
+    const int lead = lane - sub;
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const float cg = __shfl_sync(0xffffffffu, c[0], lead + g);
+      const float p0 = __shfl_sync(0xffffffffu, p[0], lead + g), p1 = __shfl_sync(0xffffffffu, p[PER - 1], PER == 2 ? lead + g : lead + GP + g);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) o[g][e] = o[g][e] * cg + p0 * f[0][e] + p1 * f[1][e];
+    }
+  };
+#pragma unroll 1
+  for (int t = 0; t < trips; t += 2) {
+    work(A);
+    if (t + 2 < trips) fetch(A, t + 2, true, true);
+    if (t + 1 < trips) {
+      work(B2);
+      if (t + 3 < trips) fetch(B2, t + 3, true, true);
+    }
+  }
+  float lt = l[0];
+  if constexpr (PER == 2) lt += l[PER - 1];
+  else lt += __shfl_xor_sync(0xffffffffu, lt, GP);
+  // every group of lanes of every warp leaves its result, and the CTA adds them in their order
+  const int part = warp * SPW + grp;
+  if (sub < G) { sm_m[part][sub] = m[0]; sm_l[part][sub] = lt; }
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    float4* dst = reinterpret_cast<float4*>(&sm_o[part][g][sub * 8]);
+    dst[0] = make_float4(o[g][0], o[g][1], o[g][2], o[g][3]);
+    dst[1] = make_float4(o[g][4], o[g][5], o[g][6], o[g][7]);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < PARTS * G; i += 128) {
+    const int w0 = i / G, g = i - w0 * G;
+    float mm = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < PARTS; ++w) mm = fmaxf(mm, sm_m[w][g]);
+    sm_f[w0][g] = sm_m[w0][g] == -INFINITY ? 0.f : __expf(sm_m[w0][g] - mm);
+    if (w0 == 0) sm_m[PARTS][g] = mm;
+  }
+  __syncthreads();
+  if (threadIdx.x < G) {
+    float ll = 0.f;
+#pragma unroll
+    for (int w = 0; w < PARTS; ++w) ll += sm_l[w][threadIdx.x] * sm_f[w][threadIdx.x];
+    sm_l[PARTS][threadIdx.x] = ll;
+  }
+  for (int t = threadIdx.x; t < G * HD; t += 128) {
+    const int g = t / HD, c = t % HD;
+    float oo = 0.f;
+#pragma unroll
+    for (int w = 0; w < PARTS; ++w) oo += sm_o[w][g][c] * sm_f[w][g];
+    sm_o[PARTS][g][c] = oo;
+  }
+  cluster_sync_all();
+  auto remote = [](const float* p, int rank) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(mapa_shared(smem_u32(p), (uint32_t)rank)) : "memory");
+    return v;
+  };
+  for (int t = split * 128 + (int)threadIdx.x; t < G * HD; t += splits * 128) {      // the splits, in their order
+    const int g = t / HD, c = t % HD;
+    float ms[8], ls[8], os[8], mm = -INFINITY;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      ms[r] = -INFINITY;
+      ls[r] = os[r] = 0.f;
+      if (r < splits) { ms[r] = remote(&sm_m[PARTS][g], r); ls[r] = remote(&sm_l[PARTS][g], r); os[r] = remote(&sm_o[PARTS][g][c], r); }
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) mm = fmaxf(mm, ms[r]);
+    float ll = 0.f, oo = 0.f;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const float f = ms[r] == -INFINITY ? 0.f : __expf(ms[r] - mm);
+      ll += ls[r] * f;
+      oo += os[r] * f;
+    }
+    out[b * ld_o + (long long)(kvh * G + g) * HD + c] = Cvt<T>::from_f(ll > 0.f ? oo / ll : 0.f);
+  }
+  cluster_sync_all();                                  // the other CTAs have read this one's shared memory
+}
+
 // One block of HD threads per (sequence, head).  The split maxima and sums are read by one thread per split and the
 // per-split factors go through shared memory, so that the long loop over the splits carries no dependent load: the
 // earlier form (every thread walking all splits twice, each step waiting for its load) took 12 us per launch, a
@@ -895,6 +1116,30 @@ static int launch_decode_attn(const void* q, long long ld_q, const void* cK, con
                               int KV, int cap, int window, float scale, int* ticket, cudaStream_t st) {
   const int G = H / KV;
   if (!ticket && splits > 2 * HD) return -4;      // the merge kernel reads at most two splits per thread
+  // a cluster: no more than eight CTAs anywhere, and a slot's lanes hold its scores (heads of 32: up to four queries a key head)
+  if (!ticket && splits <= 8 && (splits & (splits - 1)) == 0 && G <= HD / 8) {
+    cudaLaunchAttribute at[2];
+    cudaLaunchConfig_t cfg = gb_pdl_config(dim3((unsigned)(B * KV * splits)), dim3(128), 0, st, &at[1]);
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)splits; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs += 1;
+#define ATT(GG)                                                                                                                              \
+  if constexpr (GG <= HD / 8)                                                                                                               \
+    (void)cudaLaunchKernelEx(&cfg, decode_attn_cluster_kernel<T, HD, GG>, (const T*)q, ld_q, (const T*)cK, (const T*)cV, slot_pos, state, splits, \
+                             H, KV, cap, window, scale, (T*)out, ld_o)
+    switch (G) {
+      case 1: ATT(1); break;
+      case 2: ATT(2); break;
+      case 3: ATT(3); break;
+      case 4: ATT(4); break;
+      case 6: ATT(6); break;
+      case 8: ATT(8); break;
+      default: return -3;
+    }
+#undef ATT
+    return gb_launch_rc();
+  }
   const dim3 grid(B * KV, splits);
 #define ATT(GG)                                                                                                   \
   GB_PDL_LAUNCH((decode_attn_kernel<T, HD, GG>), grid, dim3(128), st, (const T*)q, ld_q, (const T*)cK, (const T*)cV, slot_pos, \

@@ -273,6 +273,20 @@ __device__ __forceinline__ LlEight<T> ll_load_eight(const T* p, bool wide) {
   }
   return x;
 }
+// The same past the L1: of a cache whose lines may hold a row that is written while they are read.
+template <typename T>
+__device__ __forceinline__ LlEight<T> ll_load_eight_cg(const T* p, bool wide) {
+  LlEight<T> x;
+  if (wide) {
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(T) / 2; ++i) x.r[i] = __ldcg(reinterpret_cast<const uint4*>(p) + i);
+  } else {
+    T* y = reinterpret_cast<T*>(&x);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) y[i] = __ldcg(p + i);
+  }
+  return x;
+}
 template <typename T>
 __device__ __forceinline__ void ll_expand_eight(const LlEight<T>& x, float (&v)[8]) {
   if constexpr (sizeof(T) == 4) {
@@ -430,6 +444,194 @@ __global__ void __launch_bounds__(128, 4) ll_attn_decode_kernel(const __grid_con
   }
 }
 
+// The same for up to eight splits (1, 2, 4 or 8): the splits of a (sequence, key head, chunk of query heads) are a cluster, whose CTAs exchange their
+// results through distributed shared memory and apply sink and gate, so there is no merge kernel behind it.  The first keys and values are asked for
+// before the wait for the kernel ahead, which writes the queries and the cache row of the step's own position, and nothing else that is read
+// here; queries wait in shared memory.  Bound by the chain and by the instructions of the scores: 32 sequences, 16 heads, 4 key heads of 64, 128 to 190
+// keys, capped scores: 7.9 us of the step, before 9.5 and 3.1 for the merge.
+template <typename T, int LPS, int GQ>
+__global__ void __launch_bounds__(128, 4) ll_attn_decode_cluster_kernel(const __grid_constant__ gb_ll_attn_args a) {
+  constexpr int HD = LPS * 8, SPW = 32 / LPS, U = 2;
+  __shared__ __align__(16) float sm_q[GQ][HD];
+  constexpr int PARTS = 4 * SPW;                                       // groups of lanes that share a slot, in the CTA
+  __shared__ float sm_m[PARTS + 1][GQ], sm_l[PARTS + 1][GQ], sm_f[PARTS][GQ];           // theirs, and the CTA's
+  __shared__ __align__(16) float sm_o[PARTS + 1][GQ][HD];
+  const int R = a.H / a.G, chunks = (R + GQ - 1) / GQ;
+  const int split = (int)cluster_ctarank(), item = (int)cluster_id_x();
+  const int b = item / (a.G * chunks), rem = item - b * a.G * chunks;
+  const int g = rem / chunks, h0 = g * R + (rem - g * chunks) * GQ, nh = min(GQ, (g + 1) * R - h0);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane / LPS, sub = lane % LPS;
+  const int pos = a.st[b].abs_pos;
+  const LlKeyRange kr = ll_key_range(pos, pos, a.window, a.keep);
+  const int used = ll_splits_used(a.splits, kr.count);
+  const int per = (kr.count + used - 1) / used;
+  const int lo = split * per, hi = min(kr.count, lo + per);            // of a split beyond `used`: lo >= hi
+  const bool kl = sub * 8 < a.dkp, vl = sub * 8 < a.dvp;
+  const T* kb = reinterpret_cast<const T*>(a.cache_k) + g * a.dkp + sub * 8;
+  const T* vb = reinterpret_cast<const T*>(a.cache_v) + g * a.dvp + sub * 8;
+  const bool wide = ((reinterpret_cast<uintptr_t>(a.cache_k) | reinterpret_cast<uintptr_t>(a.cache_v) | (uintptr_t)(a.ld_k * sizeof(T)) |
+                      (uintptr_t)(a.ld_v * sizeof(T)) | (uintptr_t)(a.dkp * sizeof(T)) | (uintptr_t)(a.dvp * sizeof(T))) & 15) == 0;
+  LlEight<T> kx[U], vx[U];
+  int back[U];
+  bool ok[U];
+  auto fetch = [&](int e0, bool own, bool rest) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int e = e0 + u * 4 * SPW + grp;
+      const int p = e < kr.n_kept ? e : kr.win_lo + (e - kr.n_kept);
+      if (rest) {
+        ok[u] = e < hi;
+        back[u] = pos - p;
+        kx[u] = vx[u] = LlEight<T>{};
+      }
+      if (e < hi && (p == pos ? own : rest)) {
+        const long long crow = (long long)b * a.cap + ll_ring_row(p, a.keep, a.cap);
+        if (kl) kx[u] = ll_load_eight_cg<T>(kb + crow * a.ld_k, wide);
+        if (vl) vx[u] = ll_load_eight_cg<T>(vb + crow * a.ld_v, wide);
+      }
+    }
+  };
+  const int e_first = lo + warp * SPW;                                 // the warp's first key
+  fetch(e_first, false, true);
+  pdl_wait();
+  fetch(e_first, true, false);
+  for (int i = threadIdx.x; i < GQ * HD; i += 128) {
+    const int x = i / HD, c = i - x * HD;
+    sm_q[x][c] = x < nh && c < a.dkp ? Cvt<T>::to_f(reinterpret_cast<const T*>(a.q)[((long long)b * a.H + h0 + x) * a.dkp + c]) : 0.f;
+  }
+  __syncthreads();
+  // The U * GQ scores of a trip are one to a lane: the sums over the lanes of a slot are exchanged so that lane `sub` ends up with sum number
+  // sub & 7 (heads below, slots above), caps it and takes its exponential; the lanes then pass the weights round.  (Every lane working out all
+  // of them was most of the kernel's instructions.)  With one or two heads a chunk, lanes repeat them.
+  constexpr int NS = U * GQ;
+  const int mine = sub & (NS - 1), mu_ = mine / GQ, mx = mine - mu_ * GQ;               // this lane's slot and head
+  const float slope = a.slopes && mx < nh ? a.slopes[h0 + mx] : 0.f;
+  float o[GQ][8], m = -INFINITY, l = 0.f;                              // m: the head's maximum, l: this lane's share of its sum
+#pragma unroll
+  for (int x = 0; x < GQ; ++x)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) o[x][e] = 0.f;
+#pragma unroll 1
+  for (int e0 = e_first; e0 < hi; e0 += U * 4 * SPW) {
+    if (e0 != e_first) fetch(e0, true, true);
+    float s[NS];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float kf[8];
+      ll_expand_eight<T>(kx[u], kf);
+#pragma unroll
+      for (int x = 0; x < GQ; ++x) {
+        const float4 q0 = *reinterpret_cast<const float4*>(&sm_q[x][sub * 8]), q1 = *reinterpret_cast<const float4*>(&sm_q[x][sub * 8 + 4]);
+        s[u * GQ + x] = q0.x * kf[0] + q0.y * kf[1] + q0.z * kf[2] + q0.w * kf[3] + q1.x * kf[4] + q1.y * kf[5] + q1.z * kf[6] + q1.w * kf[7];
+      }
+    }
+#pragma unroll
+    for (int off = LPS / 2; off >= NS; off >>= 1)                      // more lanes than sums: whole sums first
+#pragma unroll
+      for (int i = 0; i < NS; ++i) s[i] += __shfl_xor_sync(0xffffffffu, s[i], off);
+#pragma unroll
+    for (int off = NS / 2; off > 0; off >>= 1) {                       // then half of them to each side
+      const bool up = (sub & off) != 0;
+#pragma unroll
+      for (int i = 0; i < off; ++i) {
+        const float keep = up ? s[i + off] : s[i], give = up ? s[i] : s[i + off];
+        s[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+      }
+    }
+    const bool live = mu_ == 0 ? ok[0] : ok[U - 1];
+    const float sc = live ? ll_score<T>(s[0], a.scale, a.softcap, slope, mu_ == 0 ? back[0] : back[U - 1]) : -INFINITY;
+    float mn = fmaxf(m, sc);
+#pragma unroll
+    for (int off = GQ; off < NS; off <<= 1) mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, off));       // the head's other slots
+    const float mu = mn == -INFINITY ? 0.f : mn;                       // no key so far in this group of lanes
+    const float c = expf(m - mu), p = expf(sc - mu);
+    l = l * c + p;
+    m = mn;
+    const int lead = lane - sub;                                       // the slot group's first lane
+    float vf[U][8];
+#pragma unroll
+    for (int u = 0; u < U; ++u) ll_expand_eight<T>(vx[u], vf[u]);
+#pragma unroll
+    for (int x = 0; x < GQ; ++x) {
+      const float cx = __shfl_sync(0xffffffffu, c, lead + x);
+      float px[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) px[u] = __shfl_sync(0xffffffffu, p, lead + u * GQ + x);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        float v = o[x][e] * cx;
+#pragma unroll
+        for (int u = 0; u < U; ++u) v += px[u] * vf[u][e];
+        o[x][e] = v;
+      }
+    }
+  }
+#pragma unroll
+  for (int off = GQ; off < NS; off <<= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
+  // every group of lanes of every warp leaves its result, and the CTA adds them in their order
+  const int part = warp * SPW + grp;
+  if (sub < GQ) { sm_m[part][sub] = m; sm_l[part][sub] = l; }
+#pragma unroll
+  for (int x = 0; x < GQ; ++x) {
+    float4* dst = reinterpret_cast<float4*>(&sm_o[part][x][sub * 8]);
+    dst[0] = make_float4(o[x][0], o[x][1], o[x][2], o[x][3]);
+    dst[1] = make_float4(o[x][4], o[x][5], o[x][6], o[x][7]);
+  }
+  __syncthreads();
+  if (threadIdx.x < PARTS * GQ) {                                      // at most 64
+    const int w0 = threadIdx.x / GQ, x = threadIdx.x - w0 * GQ;
+    float mm = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < PARTS; ++w) mm = fmaxf(mm, sm_m[w][x]);
+    sm_f[w0][x] = sm_m[w0][x] == -INFINITY ? 0.f : expf(sm_m[w0][x] - mm);
+    if (w0 == 0) sm_m[PARTS][x] = mm;
+  }
+  __syncthreads();
+  if (threadIdx.x < GQ) {
+    float ll = 0.f;
+#pragma unroll
+    for (int w = 0; w < PARTS; ++w) ll += sm_l[w][threadIdx.x] * sm_f[w][threadIdx.x];
+    sm_l[PARTS][threadIdx.x] = ll;
+  }
+  for (int i = threadIdx.x; i < nh * a.dvp; i += 128) {
+    const int x = i / a.dvp, c = i - x * a.dvp;
+    float oo = 0.f;
+#pragma unroll
+    for (int w = 0; w < PARTS; ++w) oo += sm_o[w][x][c] * sm_f[w][x];
+    sm_o[PARTS][x][c] = oo;
+  }
+  cluster_sync_all();
+  auto remote = [](const float* p, int rank) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(mapa_shared(smem_u32(p), (uint32_t)rank)) : "memory");
+    return v;
+  };
+  for (int i = split * 128 + (int)threadIdx.x; i < nh * a.dv; i += a.splits * 128) {    // the splits, in their order
+    const int x = i / a.dv, c = i - x * a.dv, h = h0 + x;
+    float ms[8], ls[8], os[8], mm = a.sink ? a.sink[h] : -INFINITY;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      ms[r] = -INFINITY;
+      ls[r] = os[r] = 0.f;
+      if (r < used) { ms[r] = remote(&sm_m[PARTS][x], r); ls[r] = remote(&sm_l[PARTS][x], r); os[r] = remote(&sm_o[PARTS][x][c], r); }
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) mm = fmaxf(mm, ms[r]);
+    float ll = 0.f, oo = 0.f;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const float f = ms[r] == -INFINITY ? 0.f : expf(ms[r] - mm);
+      ll += ls[r] * f;
+      oo += os[r] * f;
+    }
+    if (a.sink) ll += expf(a.sink[h] - mm);
+    float v = ll > 0.f ? oo * (1.f / ll) : 0.f;
+    if (a.gate) v *= ll_sigmoid(Cvt<T>::to_f(reinterpret_cast<const T*>(a.gate)[b * a.ld_gate + h * a.dv + c]));
+    reinterpret_cast<T*>(a.out)[b * a.ldo + h * a.dv + c] = Cvt<T>::from_f(v);
+  }
+  cluster_sync_all();                                                  // the other CTAs have read this one's shared memory
+}
+
 // One block per (sequence, head): the splits' results, the sink and the output gate.  Groups of threads take every g-th split.
 template <typename T>
 __global__ void __launch_bounds__(256) ll_attn_merge_kernel(const __grid_constant__ gb_ll_attn_args a) {
@@ -494,6 +696,19 @@ __global__ void __launch_bounds__(256) ll_attn_merge_kernel(const __grid_constan
 template <typename T, int LPS>
 static void ll_decode_go(const gb_ll_attn_args& a, cudaStream_t st) {
   const int R = a.H / a.G;
+  if (a.splits <= 8 && (a.splits & (a.splits - 1)) == 0) {             // a cluster: no more than eight CTAs anywhere
+    const int gq = R == 1 ? 1 : R == 2 ? 2 : 4;
+    cudaLaunchAttribute at[2];
+    cudaLaunchConfig_t cfg = gb_pdl_config(dim3((unsigned)(a.B * a.G * ((R + gq - 1) / gq) * a.splits)), dim3(128), 0, st, &at[1]);
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)a.splits; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs += 1;
+    if (gq == 1) (void)cudaLaunchKernelEx(&cfg, ll_attn_decode_cluster_kernel<T, LPS, 1>, a);
+    else if (gq == 2) (void)cudaLaunchKernelEx(&cfg, ll_attn_decode_cluster_kernel<T, LPS, 2>, a);
+    else (void)cudaLaunchKernelEx(&cfg, ll_attn_decode_cluster_kernel<T, LPS, 4>, a);
+    return;
+  }
 #define GO(GQ) GB_PDL_LAUNCH((ll_attn_decode_kernel<T, LPS, GQ>), dim3(a.B * a.G * ((R + GQ - 1) / GQ), a.splits), dim3(128), st, a)
   if (R == 1) GO(1);
   else if (R == 2) GO(2);

@@ -151,6 +151,9 @@ class InferenceEngine(TokenLoop):
         # split-KV: enough (sequence, kv head, split) blocks to cover the GPU; a warp walks its slots one by one,
         # so at batch 1 the cache is cut fine (a few slots per warp) and the partial results merged afterwards
         self.splits = int(min(64, max(8, 512 // (B * cfg.num_kv_heads))))
+        fit = 592 if cfg.num_heads <= 4 * cfg.num_kv_heads else 296              # four blocks to an SM at once, or two
+        while self.splits > 1 and self.splits * B * cfg.num_kv_heads > fit:
+            self.splits //= 2
         self.att_scratch = CA.zeros(B * cfg.num_heads * self.splits * (cfg.head_dim + 2), **f32)
         self.att_ticket = CA.zeros(B * cfg.num_kv_heads, **i32)
         self.cos_sin = K.rope_table(torch.from_numpy(cfg.rope_inv_freq()), max(cfg.max_seq_len, max_len) + 1, self.dev)

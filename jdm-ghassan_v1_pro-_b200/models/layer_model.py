@@ -252,6 +252,8 @@ class LayerModel:
             seen = cache.cap if not m.window else m.window + m.keep_first
             # four blocks fit an SM at once: a few more than that are a second round (32 sequences: 18.5 us with 5 splits, 13.3 with 4)
             a.splits = int(max(1, min(64, 592 // blocks, (seen + 15) // 16)))
+            if a.splits <= 8 or seen <= 512:                # a power of two up to eight: a cluster merges them, with no kernel behind it
+                a.splits = 1 << (min(a.splits, 8).bit_length() - 1)
             a.scratch = self.buf("att_scratch%d" % B, m.heads * a.splits * (a.dvp + 2), torch.float32, rows=B).data_ptr()
         a.st, a.pos0_max, a.status = st.data_ptr(), pos0_max, _lib.status_word(self.dev).data_ptr()
         return a
