@@ -150,6 +150,54 @@ __device__ __forceinline__ void load_row32(const T* src, float (&v)[32], int nco
   }
 }
 
+// A warp's 32 x 32 block of results goes through its 4 KB of shared memory, from a row a lane to eight lanes a row: what is read from and written to
+// global memory is then whole pieces of rows, four rows an access (a row a lane touched 32 rows 16 bytes at a time).  Pieces are swizzled, so that
+// every eight lanes hit all banks.  GEMM_EPILOGUE_FIGURES
+__device__ __forceinline__ void turn_in(float4* ws, const float (&v)[32]) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();                                         // the last block has been read
+#pragma unroll
+  for (int i = 0; i < 8; ++i) ws[lane * 8 + (i ^ (lane & 7))] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+  __syncwarp();
+}
+// Columns 4 * (lane % 8) .. of row 4 * it + lane / 8.
+__device__ __forceinline__ float4 turn_out(const float4* ws, int it) {
+  const int lane = threadIdx.x & 31, rr = it * 4 + (lane >> 3);
+  return ws[rr * 8 + ((lane & 7) ^ (rr & 7))];
+}
+template <typename OutT>
+__device__ __forceinline__ void store4(OutT* dst, const float4& q) {
+  if constexpr (sizeof(OutT) == 4) *reinterpret_cast<float4*>(dst) = q;
+  else *reinterpret_cast<uint2*>(dst) = make_uint2(Cvt<OutT>::pack2(q.x, q.y), Cvt<OutT>::pack2(q.z, q.w));
+}
+template <typename T>
+__device__ __forceinline__ float4 load4(const T* src) {
+  if constexpr (sizeof(T) == 4) {
+    return *reinterpret_cast<const float4*>(src);
+  } else {
+    const uint2 q = *reinterpret_cast<const uint2*>(src);
+    const float2 a = Cvt<T>::unpack2(q.x), b = Cvt<T>::unpack2(q.y);
+    return make_float4(a.x, a.y, b.x, b.y);
+  }
+}
+// Every row's pieces of four elements are aligned.
+template <typename T>
+__device__ __forceinline__ bool pieces_ok(const T* p, long long ld) {
+  return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t)(ld * (long long)sizeof(T))) & (4 * sizeof(T) - 1)) == 0;
+}
+// The block v (row `lane`) to out, whose row 0 is the block's; `rows` of them exist.
+template <typename OutT>
+__device__ __forceinline__ void store_block(float4* ws, const float (&v)[32], OutT* out, long long ld, int rows) {
+  const int lane = threadIdx.x & 31;
+  turn_in(ws, v);
+#pragma unroll
+  for (int it = 0; it < 8; ++it) {
+    const float4 q = turn_out(ws, it);
+    const int rr = it * 4 + (lane >> 3);
+    if (rr < rows) store4<OutT>(out + rr * ld + (lane & 7) * 4, q);
+  }
+}
+
 __device__ __forceinline__ float silu_f(float g) { return g / (1.f + __expf(-g)); }
 
 template <int BN, int STAGES, int EPI, typename OutT, typename InT>
@@ -169,8 +217,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   uint64_t* tempty_bar = tfull_bar + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  // 2 KB per epilogue warp: a 32 x 32 block of 16-bit results is turned from "one row per lane" into "four lanes per
-  // row" before it goes to a per-tile destination (another GPU's memory likes 64-byte pieces, not 16-byte ones)
+  // 4 KB per epilogue warp: see turn_in (a per-tile destination, maybe another GPU's memory, gets 64-byte pieces by way of the first 2 KB)
   uint8_t* stage = smem + STAGES * STAGE_BYTES + 256;
 
   const int warp = threadIdx.x >> 5;
@@ -191,6 +238,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
 
   int tiles_m = (p.mode == 1) ? *p.num_m_tiles : (p.M + BM - 1) / BM;
   const int tiles_n = (p.N + BN - 1) / BN;
@@ -291,11 +339,26 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         OutT* orow = p.tile_out ? reinterpret_cast<OutT*>(p.tile_out[t.tm]) + (long long)r_in_tile * p.ldo
                                 : reinterpret_cast<OutT*>(p.out) + t.out_off + (long long)row * p.ldo;
         const float* arow = p.addend ? p.addend + t.out_off + (long long)row * p.ld_add : nullptr;
+        // the warp's block: its first row, how many of its rows exist, whether rows fall into aligned pieces
+        float4* ws = reinterpret_cast<float4*>(stage + warp * 4096);
+        const int row0 = t.a_row0 + quarter * 32, rows = min(32, p.M - row0);
+        OutT* oblk = orow - (long long)lane * p.ldo;
+        const float* ablk = arow ? arow - (long long)lane * p.ld_add : nullptr;
+        const bool whole = EPI != EPI_STORE_TILED && pieces_ok(oblk, p.ldo) && (!ablk || (sizeof(OutT) == 4 && pieces_ok(ablk, p.ld_add)));
         constexpr int CH = BN / 64;            // 32-column chunks per half
+        constexpr int NB = CH >= 2 && sizeof(OutT) == 2 ? 2 : 1;   // chunks loaded per wait (one where an addend may want the registers)
 #pragma unroll 1
-        for (int c0 = half * CH; c0 < (half + 1) * CH; c0 += 2) {
-          constexpr int NB = CH >= 2 ? 2 : 1;   // chunks loaded per wait
+        for (int c0 = half * CH; c0 < (half + 1) * CH; c0 += NB) {
           uint32_t r[NB][32];
+          float4 add[8];
+          auto fetch = [&](int col) {
+#pragma unroll
+            for (int it = 0; it < 8; ++it) {
+              const int rr = it * 4 + (lane >> 3);
+              add[it] = rr < rows && p.N - col >= 32 ? load4<float>(ablk + rr * (long long)p.ld_add + col + (lane & 7) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+          };
+          if (sizeof(OutT) == 4 && whole && ablk) fetch(t.n0 + c0 * 32);      // under way while the accumulator is read
           if (!empty_k) {
 #pragma unroll
             for (int b = 0; b < NB; ++b) tmem_ld_32x32(taddr0 + (c0 + b) * 32, r[b]);
@@ -314,7 +377,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             const int nvalid = p.N - col;
             if constexpr (EPI == EPI_STORE_TILED && sizeof(OutT) == 2) {
               if (nvalid >= 32) {                               // warp-uniform: col and N are
-                uint4* ws = reinterpret_cast<uint4*>(stage + warp * 2048);
+                uint4* ws = reinterpret_cast<uint4*>(stage + warp * 4096);
                 __syncwarp();
 #pragma unroll
                 for (int pp = 0; pp < 4; ++pp) {
@@ -338,7 +401,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 continue;
               }
             }
-            if (row_ok && nvalid > 0) {
+            if (whole && nvalid >= 32) {                        // uniform over the warp
+              turn_in(ws, v);
+#pragma unroll
+              for (int it = 0; it < 8; ++it) {
+                float4 q = turn_out(ws, it);
+                const int rr = it * 4 + (lane >> 3);
+                if (sizeof(OutT) == 4 && ablk) { q.x += add[it].x; q.y += add[it].y; q.z += add[it].z; q.w += add[it].w; }
+                if (rr < rows) store4<OutT>(oblk + rr * (long long)p.ldo + col + (lane & 7) * 4, q);
+              }
+            } else if (row_ok && nvalid > 0) {
               if (arow) {
                 float a[32];
                 load_row32<float>(arow + col, a, nvalid);
@@ -371,7 +443,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             a[i] = silu_f(g[i]) * u[i];
           }
           const int nvalid = p.N - (t.n0 + gcol + 64);  // columns of the up half bound both halves
-          if (row_ok && nvalid > 0) {
+          OutT* gu_blk = gu_row ? gu_row - (long long)lane * p.ld_aux + t.n0 + gcol : nullptr;
+          OutT* act_blk = act_row - (long long)lane * p.ldo + (t.n0 >> 1) + (pp >> 1) * 64 + (pp & 1) * 32;
+          if (nvalid >= 32 && pieces_ok(act_blk, p.ldo) && (!gu_blk || pieces_ok(gu_blk, p.ld_aux))) {
+            float4* ws = reinterpret_cast<float4*>(stage + warp * 4096);
+            const int rows = min(32, p.M - (t.a_row0 + quarter * 32));
+            if (gu_blk) {
+              store_block<OutT>(ws, g, gu_blk, p.ld_aux, rows);
+              store_block<OutT>(ws, u, gu_blk + 64, p.ld_aux, rows);
+            }
+            store_block<OutT>(ws, a, act_blk, p.ldo, rows);
+          } else if (row_ok && nvalid > 0) {
             if (gu_row) {
               store_row32<OutT>(gu_row + t.n0 + gcol, g, nvalid);
               store_row32<OutT>(gu_row + t.n0 + gcol + 64, u, nvalid);
@@ -385,12 +467,53 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         OutT* dgu = reinterpret_cast<OutT*>(p.out) + (long long)row * p.ldo;
 #pragma unroll 1
         for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
+          const int j = t.n0 + c * 32;
+          const int nvalid = p.N - j;
+          const int at = (j >> 6) * 128 + (j & 63);
+          const InT* gblk = gu - (long long)lane * p.ld_aux + at;
+          OutT* dblk = dgu - (long long)lane * p.ldo + at;
+          const bool whole = nvalid >= 32 && pieces_ok(gblk, p.ld_aux) && pieces_ok(dblk, p.ldo);
+          const int rows = min(32, p.M - (t.a_row0 + quarter * 32));
+          uint2 gq[8], uq[8];
+          if (whole)                                            // under way while the accumulator is read
+#pragma unroll
+            for (int it = 0; it < 8; ++it) {
+              const int rr = it * 4 + (lane >> 3);
+              gq[it] = uq[it] = make_uint2(0u, 0u);
+              if (rr < rows) {
+                gq[it] = *reinterpret_cast<const uint2*>(gblk + rr * (long long)p.ld_aux + (lane & 7) * 4);
+                uq[it] = *reinterpret_cast<const uint2*>(gblk + rr * (long long)p.ld_aux + (lane & 7) * 4 + 64);
+              }
+            }
           uint32_t r[32];
           tmem_ld_32x32(taddr0 + c * 32, r);
           tmem_ld_wait();
-          const int j = t.n0 + c * 32;
-          const int nvalid = p.N - j;
-          if (row_ok && nvalid > 0) {
+          if (whole) {
+            float4* ws = reinterpret_cast<float4*>(stage + warp * 4096);
+            float da[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) da[i] = __uint_as_float(r[i]);
+            turn_in(ws, da);
+#pragma unroll
+            for (int it = 0; it < 8; ++it) {
+              const int rr = it * 4 + (lane >> 3);
+              const float4 d = turn_out(ws, it), g = load4<InT>(reinterpret_cast<const InT*>(&gq[it])), u = load4<InT>(reinterpret_cast<const InT*>(&uq[it]));
+              auto one = [](float da, float g, float u, float& dg, float& du) {
+                const float sg = 1.f / (1.f + __expf(-g));
+                du = da * (g * sg);
+                dg = da * u * (sg * (1.f + g * (1.f - sg)));
+              };
+              float4 dg, du;
+              one(d.x, g.x, u.x, dg.x, du.x);
+              one(d.y, g.y, u.y, dg.y, du.y);
+              one(d.z, g.z, u.z, dg.z, du.z);
+              one(d.w, g.w, u.w, dg.w, du.w);
+              if (rr < rows) {
+                store4<OutT>(dblk + rr * (long long)p.ldo + (lane & 7) * 4, dg);
+                store4<OutT>(dblk + rr * (long long)p.ldo + (lane & 7) * 4 + 64, du);
+              }
+            }
+          } else if (row_ok && nvalid > 0) {
             const int base = (j >> 6) * 128 + (j & 63);
             float g[32], u[32], dg[32], du[32];
             load_row32<InT>(gu + base, g, nvalid);
@@ -430,7 +553,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
 template <int BN, int STAGES>
 constexpr size_t gemm_smem_bytes() {
-  return size_t(STAGES) * (BM * BK * 2 + BN * BK * 2) + 256 /* barriers */ + 8 * 2048 /* epilogue staging */ + 1024;
+  return size_t(STAGES) * (BM * BK * 2 + BN * BK * 2) + 256 /* barriers */ + 8 * 4096 /* epilogue staging */ + 1024;
 }
 
 }  // namespace gb
@@ -489,7 +612,9 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const gb::GemmPara
   }
   int grid = max_tiles < num_sms() ? max_tiles : num_sms();
   if (grid < 1) grid = 1;
-  kern<<<grid, gb::GEMM_THREADS, smem, st>>>(ta, tb, p);
+  cudaLaunchAttribute at;
+  const cudaLaunchConfig_t cfg = gb_pdl_config(dim3((unsigned)grid), dim3(gb::GEMM_THREADS), smem, st, &at);
+  (void)cudaLaunchKernelEx(&cfg, kern, ta, tb, p);
   return gb_launch_rc();
 }
 
