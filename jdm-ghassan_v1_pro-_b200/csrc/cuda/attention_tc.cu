@@ -124,6 +124,7 @@ __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1) attn_tc_fwd_kern
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
   const uint32_t tmem_S = tmem_base, tmem_O = tmem_base + AT_N;
 
   // Visible key tiles of an item: [k_lo, k_lo + n_tiles * AT_N).  `lo` (start of the packed document) and the window
@@ -407,6 +408,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS) attn_tc_bwd_dq_kernel(const __
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
   const uint32_t tmem_S = tmem_base, tmem_dP = tmem_base + AT_N, tmem_dQ = tmem_base + 2 * AT_N;
 
   // visible key tiles of an item (`lo` and the window bound are non-decreasing along a sequence: the first row of the
@@ -628,6 +630,7 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dq64_kernel(co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
   const uint32_t tmem_S = tmem_base, tmem_dP = tmem_base + KN, tmem_dQ = tmem_base + 2 * KN;
 
   // visible key steps of an item: [k_lo, k_lo + n_steps * 64)
@@ -860,6 +863,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS) attn_tc_bwd_dkv_kernel(const _
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
   const uint32_t tmem_ST = tmem_base, tmem_dPT = tmem_base + AT_M, tmem_dV = tmem_base + 2 * AT_M,
                  tmem_dK = tmem_base + 2 * AT_M + HD;
 
@@ -1141,6 +1145,7 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
   const uint32_t tmem_ST = tmem_base, tmem_dPT = tmem_base + QN, tmem_dV = tmem_base + 2 * QN, tmem_dK = tmem_base + 2 * QN + HD;
 
   // the query steps of an item start at its key tile: n_qs steps of 64 queries for each head of the group
@@ -1413,6 +1418,7 @@ __global__ void __launch_bounds__(AT_DQ64_THREADS, 2) attn_tc_bwd_dkv64_kernel(c
 // first row of a tile has its smallest lo, the last one its largest).
 // One block of 1024 threads per sequence: running maximum of the run-start positions (chunked inclusive scan).
 __global__ void __launch_bounds__(1024) attn_seg_lo_kernel(const int* __restrict__ seg, int* __restrict__ lo, int B, int T) {
+  pdl_wait();
   __shared__ int s_warp[32], s_flag[32];
   __shared__ int s_carry, s_carry_f;
   const long long base = (long long)blockIdx.x * T;
@@ -1491,13 +1497,14 @@ int launch_tc_fwd(const gb_attn_args* a, int* lo, int* status, cudaStream_t st) 
   const long long n_items = (long long)((a->T + AT_M - 1) / AT_M) * a->B * a->H;
   if (n_items > 0x7fffffffll - resident) return -1;
   const unsigned grid = (unsigned)std::min<long long>(n_items, resident);
-  kern<<<grid, AT_THREADS, smem, st>>>(tq, tk, tv, p);
+  GB_PDL_LAUNCH_SMEM(kern, dim3(grid), dim3(AT_THREADS), smem, st, tq, tk, tv, p);
   return gb_launch_rc();
 }
 
 template <typename T>
 __global__ void attn_tc_delta_kernel(const T* __restrict__ d_o, long long ld_do, const T* __restrict__ o, long long ld_o,
                                      float* __restrict__ delta, long long n_tok, int H, int hd) {
+  pdl_wait();
   const long long gw = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (gw >= n_tok * H) return;
@@ -1516,6 +1523,7 @@ template <typename T, int HD>
 __global__ void __launch_bounds__(256) attn_tc_delta_vec_kernel(const T* __restrict__ d_o, long long ld_do,
                                                                 const T* __restrict__ o, long long ld_o,
                                                                 float* __restrict__ delta, long long n_tok, int H) {
+  pdl_wait();
   constexpr int LPI = HD / 8, IPW = 32 / LPI;
   const int lane = threadIdx.x & 31, sub = lane / LPI, j = lane % LPI;
   const long long item = (blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5)) * IPW + sub;
@@ -1546,10 +1554,10 @@ int launch_tc_bwd(const gb_attn_args* a, int* lo, int* status, cudaStream_t st) 
   if (gb_make_tmap_2d_16b(&tdo, a->d_o, rows, (uint64_t)a->H * HD, a->ld_do, AT_M, 64, a->is_bf16)) return -23;
   if (a->ld_do % 8 == 0 && a->ld_o % 8 == 0 && (((uintptr_t)a->d_o | (uintptr_t)a->o) & 15) == 0) {
     constexpr int per_block = 8 * (256 / HD);
-    attn_tc_delta_vec_kernel<T, HD><<<(unsigned)((rows * a->H + per_block - 1) / per_block), 256, 0, st>>>(
+    GB_PDL_LAUNCH_SMEM((attn_tc_delta_vec_kernel<T, HD>), dim3((unsigned)((rows * a->H + per_block - 1) / per_block)), dim3(256), 0, st, 
         reinterpret_cast<const T*>(a->d_o), a->ld_do, reinterpret_cast<const T*>(a->o), a->ld_o, a->delta, rows, a->H);
   } else {
-    attn_tc_delta_kernel<T><<<(unsigned)((rows * a->H + 7) / 8), 256, 0, st>>>(
+    GB_PDL_LAUNCH_SMEM((attn_tc_delta_kernel<T>), dim3((unsigned)((rows * a->H + 7) / 8)), dim3(256), 0, st, 
         reinterpret_cast<const T*>(a->d_o), a->ld_do, reinterpret_cast<const T*>(a->o), a->ld_o, a->delta, rows, a->H, HD);
   }
   AttnTcParams p{};
@@ -1593,9 +1601,9 @@ int launch_tc_bwd(const gb_attn_args* a, int* lo, int* status, cudaStream_t st) 
       (void)cudaFuncSetAttribute(kq64, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
       attr64 = true;
     }
-    kq64<<<(unsigned)std::min<long long>(items_q, 2ll * sms), AT_DQ64_THREADS, smem_q64, st>>>(tq, tk64, tv64, tdo, p);
+    GB_PDL_LAUNCH_SMEM(kq64, dim3((unsigned)std::min<long long>(items_q, 2ll * sms)), dim3(AT_DQ64_THREADS), smem_q64, st, tq, tk64, tv64, tdo, p);
   } else {
-    kq<<<(unsigned)std::min<long long>(items_q, sms), AT_BWD_THREADS, smem_q, st>>>(tq, tk, tv, tdo, p);
+    GB_PDL_LAUNCH_SMEM(kq, dim3((unsigned)std::min<long long>(items_q, sms)), dim3(AT_BWD_THREADS), smem_q, st, tq, tk, tv, tdo, p);
   }
   if constexpr (HD == 64) {
     // query steps of 64, two CTAs per SM
@@ -1614,16 +1622,12 @@ int launch_tc_bwd(const gb_attn_args* a, int* lo, int* status, cudaStream_t st) 
         (void)cudaFuncSetAttribute(ks, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         attr_s = true;
       }
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)(items_kv * group), 1, 1);
-      cfg.blockDim = dim3(AT_DQ64_THREADS, 1, 1);
-      cfg.dynamicSmemBytes = smem_kv64;
-      cfg.stream = st;
-      cudaLaunchAttribute at;
-      at.id = cudaLaunchAttributeClusterDimension;
-      at.val.clusterDim.x = (unsigned)group; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-      cfg.attrs = &at;
-      cfg.numAttrs = 1;
+      cudaLaunchAttribute at[2];
+      cudaLaunchConfig_t cfg = gb_pdl_config(dim3((unsigned)(items_kv * group)), dim3(AT_DQ64_THREADS), smem_kv64, st, &at[1]);
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = (unsigned)group; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs += 1;
       if (cudaLaunchKernelEx(&cfg, ks, tq64, tk, tv, tdo64, p) != cudaSuccess) return -10;
       return gb_launch_rc();
     }
@@ -1634,9 +1638,9 @@ int launch_tc_bwd(const gb_attn_args* a, int* lo, int* status, cudaStream_t st) 
       (void)cudaFuncSetAttribute(kkv64, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
       attr_kv64 = true;
     }
-    kkv64<<<(unsigned)std::min<long long>(items_kv, 2ll * sms), AT_DQ64_THREADS, smem_kv64, st>>>(tq64, tk, tv, tdo64, p);
+    GB_PDL_LAUNCH_SMEM(kkv64, dim3((unsigned)std::min<long long>(items_kv, 2ll * sms)), dim3(AT_DQ64_THREADS), smem_kv64, st, tq64, tk, tv, tdo64, p);
   } else {
-    kkv<<<(unsigned)std::min<long long>(items_kv, sms), AT_BWD_THREADS, smem_kv, st>>>(tq, tk, tv, tdo, p);
+    GB_PDL_LAUNCH_SMEM(kkv, dim3((unsigned)std::min<long long>(items_kv, sms)), dim3(AT_BWD_THREADS), smem_kv, st, tq, tk, tv, tdo, p);
   }
   return gb_launch_rc();
 }
@@ -1654,7 +1658,7 @@ extern "C" int gb_attn_tc_bwd(const gb_attn_args* a, int* lo_scratch, int lo_rea
   if (lo_ready) {
     lo = lo_scratch;                 // filled earlier by gb_attn_seg_lo for the same segment ids
   } else if (a->seg) {
-    attn_seg_lo_kernel<<<a->B, 1024, 0, st>>>(a->seg, lo_scratch, a->B, a->T);
+    GB_PDL_LAUNCH_SMEM(attn_seg_lo_kernel, dim3(a->B), dim3(1024), 0, st, a->seg, lo_scratch, a->B, a->T);
     lo = lo_scratch;
   }
   if (a->is_bf16) return a->hd == 64 ? launch_tc_bwd<__nv_bfloat16, 64>(a, lo, status, st) : launch_tc_bwd<__nv_bfloat16, 128>(a, lo, status, st);
@@ -1666,7 +1670,7 @@ extern "C" int gb_attn_tc_bwd(const gb_attn_args* a, int* lo_scratch, int lo_rea
 // lo[i] = start of the run of equal segment ids containing i; compute once per batch and pass lo_ready = 1 below.
 extern "C" int gb_attn_seg_lo(const int* seg, int* lo, int B, int T, cudaStream_t st) {
   if (!seg || !lo || B <= 0 || T <= 0) return -1;
-  attn_seg_lo_kernel<<<B, 1024, 0, st>>>(seg, lo, B, T);
+  GB_PDL_LAUNCH_SMEM(attn_seg_lo_kernel, dim3(B), dim3(1024), 0, st, seg, lo, B, T);
   return gb_launch_rc();
 }
 
@@ -1678,7 +1682,7 @@ extern "C" int gb_attn_tc_fwd(const gb_attn_args* a, int* lo_scratch, int lo_rea
   if (lo_ready) {
     lo = lo_scratch;                 // filled earlier by gb_attn_seg_lo for the same segment ids
   } else if (a->seg) {
-    attn_seg_lo_kernel<<<a->B, 1024, 0, st>>>(a->seg, lo_scratch, a->B, a->T);
+    GB_PDL_LAUNCH_SMEM(attn_seg_lo_kernel, dim3(a->B), dim3(1024), 0, st, a->seg, lo_scratch, a->B, a->T);
     lo = lo_scratch;
   }
   if (a->is_bf16) return a->hd == 64 ? launch_tc_fwd<__nv_bfloat16, 64>(a, lo, status, st) : launch_tc_fwd<__nv_bfloat16, 128>(a, lo, status, st);

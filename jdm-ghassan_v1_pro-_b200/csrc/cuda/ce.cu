@@ -14,6 +14,7 @@ __global__ void __launch_bounds__(256) ce_row_kernel(T* __restrict__ logits, lon
                                                      int V, float z, float grad_scale_val,
                                                      const float* __restrict__ grad_scale_dev, int write_grad,
                                                      float* __restrict__ row_loss) {
+  pdl_wait();
   __shared__ float red[8];
   __shared__ float bcast;
   const int row = blockIdx.x;
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(256) ce_row_kernel(T* __restrict__ logits, lon
 
 // acc[0] += sum of row losses, acc[1] += supervised rows; single block, fixed-order tree
 __global__ void ce_fold_kernel(const float* __restrict__ row_loss, int rows, double* __restrict__ acc) {
+  pdl_wait();
   __shared__ double s_l[256];
   __shared__ double s_n[256];
   double l = 0.0, n = 0.0;
@@ -123,11 +125,11 @@ extern "C" int gb_softmax_ce(void* logits, long long ld, const int* targets, int
                              cudaStream_t st) {
   if (rows <= 0 || V <= 0 || (ld * 2) % 16 || (reinterpret_cast<uintptr_t>(logits) & 15)) return -1;
   if (is_bf16)
-    ce_row_kernel<__nv_bfloat16><<<rows, 256, 0, st>>>((__nv_bfloat16*)logits, ld, targets, V, z_loss, grad_scale,
+    GB_PDL_LAUNCH_SMEM((ce_row_kernel<__nv_bfloat16>), dim3(rows), dim3(256), 0, st, (__nv_bfloat16*)logits, ld, targets, V, z_loss, grad_scale,
                                                        grad_scale_dev, write_grad, row_loss);
   else
-    ce_row_kernel<__half><<<rows, 256, 0, st>>>((__half*)logits, ld, targets, V, z_loss, grad_scale, grad_scale_dev,
+    GB_PDL_LAUNCH_SMEM((ce_row_kernel<__half>), dim3(rows), dim3(256), 0, st, (__half*)logits, ld, targets, V, z_loss, grad_scale, grad_scale_dev,
                                                 write_grad, row_loss);
-  ce_fold_kernel<<<1, 256, 0, st>>>(row_loss, rows, acc);
+  GB_PDL_LAUNCH_SMEM(ce_fold_kernel, dim3(1), dim3(256), 0, st, row_loss, rows, acc);
   return gb_launch_rc();
 }

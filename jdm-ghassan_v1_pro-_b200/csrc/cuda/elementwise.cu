@@ -49,6 +49,7 @@ constexpr int EMB_MAX_VOCAB = 1 << 19;     // ids covered by the first-occurrenc
 __device__ int g_emb_first[EMB_MAX_VOCAB];
 
 __global__ void embed_first_kernel(const int* __restrict__ ids, int n_tok, int vocab) {
+  pdl_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n_tok) return;
   const int id = ids[t];
@@ -57,6 +58,7 @@ __global__ void embed_first_kernel(const int* __restrict__ ids, int n_tok, int v
 
 __global__ void __launch_bounds__(EMB_THREADS) embed_bwd_kernel(const int* __restrict__ ids, const float* __restrict__ dx,
                                                                float* __restrict__ dtable, int n_tok, int d, int vocab) {
+  pdl_wait();
   __shared__ unsigned int mask[4][EMB_THREADS / 32];
   const int t = blockIdx.x;
   if (t >= n_tok) return;
@@ -110,6 +112,7 @@ __global__ void __launch_bounds__(EMB_THREADS) embed_bwd_sorted_kernel(const int
                                                                       const long long* __restrict__ order,
                                                                       const float* __restrict__ dx, float* __restrict__ dtable,
                                                                       int n_tok, int d, int vocab) {
+  pdl_wait();
   const int p = blockIdx.x;
   if (p >= n_tok) return;
   const int id = sid[p];
@@ -181,6 +184,7 @@ __global__ void rmsnorm_bwd_kernel(const T* __restrict__ g, const float* __restr
                                    const float* __restrict__ rrms, const float* __restrict__ dres,
                                    float* __restrict__ dx_out, T* __restrict__ dx16, float* __restrict__ part,
                                    int rows, int d, int rows_per_block) {
+  pdl_wait();
   extern __shared__ float sm_dw_all[];  // [nwarps][d]: every warp sums its own rows, lanes own distinct columns
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   for (int i = threadIdx.x; i < d * nwarps; i += blockDim.x) sm_dw_all[i] = 0.f;
@@ -245,6 +249,7 @@ __global__ void __launch_bounds__(256, 4) rmsnorm_bwd_vec_kernel(const T* __rest
                                                               const float* __restrict__ dres, float* __restrict__ dx_out,
                                                               T* __restrict__ dx16, float* __restrict__ part, int rows,
                                                               int rows_per_block) {
+  pdl_wait();
   constexpr int D = NV * 128;
   extern __shared__ float sm_dw_all[];  // [8][D] column sums of the warps, then [D] weights
   float* s_w = sm_dw_all + 8 * D;
@@ -406,6 +411,7 @@ __global__ void qk_norm_rope_bwd_kernel(const T* __restrict__ dout, int ld_dout,
                                         const int* __restrict__ pos, float* __restrict__ part_q,
                                         float* __restrict__ part_k, int n_tok, int H, int KV, float eps, int rope_type,
                                         int items_per_block) {
+  pdl_wait();
   constexpr int PAIRS = HD / 2;
   constexpr int PPL = (PAIRS + 31) / 32;
   __shared__ float s_dwq_all[8][HD], s_dwk_all[8][HD];  // launched with 8 warps; each warp sums its own items
@@ -577,6 +583,7 @@ __global__ void __launch_bounds__(256) qk_norm_rope_bwd_vec_kernel(
     const float* __restrict__ qw, const float* __restrict__ kw, const float* __restrict__ cs, const int* __restrict__ pos,
     float* __restrict__ part_q, float* __restrict__ part_k, int n_tok, int H, int KV, float eps, int rope_type,
     int items_per_block) {
+  pdl_wait();
   constexpr int PAIRS = HD / 2, LPI = HD / 8, IPW = 32 / LPI, U = 2;
   __shared__ __align__(16) float s_w[2][HD];        // q and k norm weights
   __shared__ float s_dw[2][8][HD];                  // [q|k][warp][column], summed over the warp's items
@@ -701,6 +708,7 @@ __global__ void __launch_bounds__(256, 3) qk_norm_rope_bwd_tok_kernel(
     const T* __restrict__ dout, int ld_dout, const T* __restrict__ qkv, int ld_in, T* __restrict__ dqkv, int ld_dqkv,
     const float* __restrict__ qw, const float* __restrict__ kw, const float* __restrict__ cs, const int* __restrict__ pos,
     float* __restrict__ part_q, float* __restrict__ part_k, int n_tok, int nq, int groups, float eps, int tok_per_block) {
+  pdl_wait();
   constexpr int PAIRS = HD / 2, LPI = HD / 8, IPW = 32 / LPI;
   __shared__ __align__(16) float s_w[2][HD];        // q and k norm weights
   __shared__ float s_dw[2][8][HD];                  // [q|k][warp][column], summed over the warp's items
@@ -810,6 +818,7 @@ __global__ void __launch_bounds__(256, 3) qk_norm_rope_bwd_tok_kernel(
 // ------------------------------------------------------------------------------------------ casts / fills
 template <typename T>
 __global__ void cast_f32_to_16_kernel(const float* __restrict__ src, T* __restrict__ dst, long long n) {
+  pdl_wait();
   long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * 8;
   const long long stride = (long long)gridDim.x * blockDim.x * 8;
   for (; i + 8 <= n; i += stride) {
@@ -837,8 +846,8 @@ extern "C" int gb_embed_bwd(const int* ids, const float* dx, float* dtable, int 
   void* first = nullptr;
   if (cudaGetSymbolAddress(&first, g_emb_first) != cudaSuccess) return -12;
   if (cudaMemsetAsync(first, 0x7f, (size_t)vocab * sizeof(int), st) != cudaSuccess) return -12;   // 0x7f7f7f7f > any token index
-  embed_first_kernel<<<(n_tok + 255) / 256, 256, 0, st>>>(ids, n_tok, vocab);
-  embed_bwd_kernel<<<n_tok, EMB_THREADS, 0, st>>>(ids, dx, dtable, n_tok, d, vocab);
+  GB_PDL_LAUNCH_SMEM(embed_first_kernel, dim3((n_tok + 255) / 256), dim3(256), 0, st, ids, n_tok, vocab);
+  GB_PDL_LAUNCH_SMEM(embed_bwd_kernel, dim3(n_tok), dim3(EMB_THREADS), 0, st, ids, dx, dtable, n_tok, d, vocab);
   return GB_LAUNCH_OK();
 }
 
@@ -849,7 +858,7 @@ extern "C" int gb_embed_bwd(const int* ids, const float* dx, float* dtable, int 
 extern "C" int gb_embed_bwd_sorted(const int* sorted_ids, const long long* order, const float* dx, float* dtable,
                                    int n_tok, int d, int vocab, cudaStream_t st) {
   if (d > EMB_THREADS * EMB_MAX_COLS || vocab <= 0 || n_tok <= 0) return -1;
-  embed_bwd_sorted_kernel<<<n_tok, EMB_THREADS, 0, st>>>(sorted_ids, order, dx, dtable, n_tok, d, vocab);
+  GB_PDL_LAUNCH_SMEM(embed_bwd_sorted_kernel, dim3(n_tok), dim3(EMB_THREADS), 0, st, sorted_ids, order, dx, dtable, n_tok, d, vocab);
   return GB_LAUNCH_OK();
 }
 
@@ -888,7 +897,7 @@ extern "C" int gb_rmsnorm_bwd(const void* g, const float* x, const float* w, con
   if (vec) {
     const size_t vsmem = (size_t)d * 9 * sizeof(float);
 #define GB_RMS_BWD_VEC(T, NV)                                                                                      \
-  rmsnorm_bwd_vec_kernel<T, NV><<<nb, 256, vsmem, st>>>((const T*)g, x, w, rrms, dres, dx_out, (T*)dx16, part, rows, rpb)
+  GB_PDL_LAUNCH_SMEM((rmsnorm_bwd_vec_kernel<T, NV>), dim3(nb), dim3(256), vsmem, st, (const T*)g, x, w, rrms, dres, dx_out, (T*)dx16, part, rows, rpb)
 #define GB_RMS_BWD_VEC_T(T)          \
   switch (d / 128) {                 \
     case 2: GB_RMS_BWD_VEC(T, 2); break; \
@@ -900,10 +909,10 @@ extern "C" int gb_rmsnorm_bwd(const void* g, const float* x, const float* w, con
 #undef GB_RMS_BWD_VEC_T
 #undef GB_RMS_BWD_VEC
   } else if (is_bf16)
-    rmsnorm_bwd_kernel<__nv_bfloat16><<<nb, threads, smem, st>>>((const __nv_bfloat16*)g, x, w, rrms, dres, dx_out,
+    GB_PDL_LAUNCH_SMEM((rmsnorm_bwd_kernel<__nv_bfloat16>), dim3(nb), dim3(threads), smem, st, (const __nv_bfloat16*)g, x, w, rrms, dres, dx_out,
                                                              (__nv_bfloat16*)dx16, part, rows, d, rpb);
   else
-    rmsnorm_bwd_kernel<__half><<<nb, threads, smem, st>>>((const __half*)g, x, w, rrms, dres, dx_out, (__half*)dx16, part,
+    GB_PDL_LAUNCH_SMEM((rmsnorm_bwd_kernel<__half>), dim3(nb), dim3(threads), smem, st, (const __half*)g, x, w, rrms, dres, dx_out, (__half*)dx16, part,
                                                       rows, d, rpb);
   if (dw) GB_PDL_LAUNCH(colsum_finalize_kernel, dim3((d + 31) / 32), dim3(1024), st, part, dw, (const float*)nullptr, (float*)nullptr, nb, d);
   return GB_LAUNCH_OK();
@@ -971,15 +980,15 @@ static int qk_bwd_t(const void* dout, int ld_dout, const void* qkv, int ld_in, v
   const bool aligned = ld_dout % 8 == 0 && ld_in % 8 == 0 && ld_dqkv % 8 == 0 && (qw == nullptr) == (kw == nullptr) &&
                        (((uintptr_t)dout | (uintptr_t)qkv | (uintptr_t)dqkv | (uintptr_t)cs) & 15) == 0;
 #define GB_QK_BWD_VEC(HD)                                                                                        \
-  qk_norm_rope_bwd_vec_kernel<T, HD><<<nb, 256, 0, st>>>((const T*)dout, ld_dout, (const T*)qkv, ld_in, (T*)dqkv, \
+  GB_PDL_LAUNCH_SMEM((qk_norm_rope_bwd_vec_kernel<T, HD>), dim3(nb), dim3(256), 0, st, (const T*)dout, ld_dout, (const T*)qkv, ld_in, (T*)dqkv, \
                                                          ld_dqkv, qw, kw, cs, pos, pq, pk, n_tok, H, KV, eps,   \
                                                          rope_type, ipb)
 #define GB_QK_BWD(HD)                                                                                                 \
-  qk_norm_rope_bwd_kernel<T, HD><<<nb, 256, 0, st>>>((const T*)dout, ld_dout, (const T*)qkv, ld_in, (T*)dqkv, ld_dqkv, \
+  GB_PDL_LAUNCH_SMEM((qk_norm_rope_bwd_kernel<T, HD>), dim3(nb), dim3(256), 0, st, (const T*)dout, ld_dout, (const T*)qkv, ld_in, (T*)dqkv, ld_dqkv, \
                                                      qw, kw, cs, pos, pq, pk, n_tok, H, KV, eps, rope_type, ipb)
   const int ipw = hd <= 256 ? 256 / hd : 1;
 #define GB_QK_BWD_TOK(HD, ROPE)                                                                                           \
-  qk_norm_rope_bwd_tok_kernel<T, HD, ROPE, 2><<<nb, 256, 0, st>>>((const T*)dout, ld_dout, (const T*)qkv, ld_in, (T*)dqkv, \
+  GB_PDL_LAUNCH_SMEM((qk_norm_rope_bwd_tok_kernel<T, HD, ROPE, 2>), dim3(nb), dim3(256), 0, st, (const T*)dout, ld_dout, (const T*)qkv, ld_in, (T*)dqkv, \
                                                                   ld_dqkv, qw, kw, cs, pos, pq, pk, n_tok, H / ipw, (H + KV) / ipw, eps, (n_tok + nb - 1) / nb)
   if (aligned && (hd == 64 || hd == 128) && H % ipw == 0 && KV % ipw == 0 && (rope_type == 0 || rope_type == 1)) {
     if (hd == 64) { if (rope_type == 0) GB_QK_BWD_TOK(64, 0); else GB_QK_BWD_TOK(64, 1); }
@@ -1022,6 +1031,7 @@ extern "C" int gb_qk_norm_rope_bwd(const void* dout, int ld_dout, const void* qk
 // out16[i] = sum_s part[s * n + i] (fixed order), the second stage of a split-K GEMM
 template <typename T>
 __global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits, long long n, T* __restrict__ out) {
+  pdl_wait();
   long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * 4;
   const long long stride = (long long)gridDim.x * blockDim.x * 4;
   for (; i < n; i += stride) {
@@ -1041,13 +1051,14 @@ extern "C" int gb_splitk_reduce(const float* part, int splits, long long n, void
   if (n <= 0 || n % 4 || splits < 1) return -1;
   long long blocks = (n / 4 + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  if (is_bf16) splitk_reduce_kernel<__nv_bfloat16><<<(int)blocks, 256, 0, st>>>(part, splits, n, (__nv_bfloat16*)out16);
-  else splitk_reduce_kernel<__half><<<(int)blocks, 256, 0, st>>>(part, splits, n, (__half*)out16);
+  if (is_bf16) GB_PDL_LAUNCH_SMEM((splitk_reduce_kernel<__nv_bfloat16>), dim3((int)blocks), dim3(256), 0, st, part, splits, n, (__nv_bfloat16*)out16);
+  else GB_PDL_LAUNCH_SMEM((splitk_reduce_kernel<__half>), dim3((int)blocks), dim3(256), 0, st, part, splits, n, (__half*)out16);
   return GB_LAUNCH_OK();
 }
 
 // out[i] += sum_s part[s * n + i] (fixed order): second stage of a split-K weight gradient
 __global__ void splitk_accumulate_kernel(const float* __restrict__ part, int splits, long long n, float* __restrict__ out) {
+  pdl_wait();
   long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * 4;
   const long long stride = (long long)gridDim.x * blockDim.x * 4;
   for (; i < n; i += stride) {
@@ -1065,7 +1076,7 @@ extern "C" int gb_splitk_accumulate(const float* part, int splits, long long n, 
   if ((reinterpret_cast<uintptr_t>(part) | reinterpret_cast<uintptr_t>(out)) & 15) return -2;
   long long blocks = (n / 4 + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  splitk_accumulate_kernel<<<(int)blocks, 256, 0, st>>>(part, splits, n, out);
+  GB_PDL_LAUNCH_SMEM(splitk_accumulate_kernel, dim3((int)blocks), dim3(256), 0, st, part, splits, n, out);
   return GB_LAUNCH_OK();
 }
 
@@ -1074,7 +1085,7 @@ extern "C" int gb_cast_f32_to_16(const float* src, void* dst, long long n, int i
   long long blocks = (n / 8 + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
   if (blocks < 1) blocks = 1;
-  if (is_bf16) cast_f32_to_16_kernel<__nv_bfloat16><<<(int)blocks, 256, 0, st>>>(src, (__nv_bfloat16*)dst, n);
-  else cast_f32_to_16_kernel<__half><<<(int)blocks, 256, 0, st>>>(src, (__half*)dst, n);
+  if (is_bf16) GB_PDL_LAUNCH_SMEM((cast_f32_to_16_kernel<__nv_bfloat16>), dim3((int)blocks), dim3(256), 0, st, src, (__nv_bfloat16*)dst, n);
+  else GB_PDL_LAUNCH_SMEM((cast_f32_to_16_kernel<__half>), dim3((int)blocks), dim3(256), 0, st, src, (__half*)dst, n);
   return GB_LAUNCH_OK();
 }

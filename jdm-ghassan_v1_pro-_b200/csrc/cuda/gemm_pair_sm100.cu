@@ -226,15 +226,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB); tma_prefetch_desc(&tmO);
     if (EPI != EPI_STORE && EPI != EPI_RELU2) tma_prefetch_desc(&tmX);
   }
-  if (EPI == EPI_STORE && sizeof(OutT) == 4 && p.part_slots && warp == 0)
-    plan_pieces(plan, p.seg_offsets, p.K, p.groups, ((p.M + TM - 1) / TM) * ((p.N + TN - 1) / TN), (long long)p.M * p.N,
-                (int)cluster_nctaid_x(), p.part_slots, p.part_cut);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();        // both CTAs' barriers exist before either signals the other's
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();                // behind the allocation of tensor memory: a kernel after this one must not come first to it and then wait for this one
   if (tmem_base != 0 && threadIdx.x == 0) { atomicCAS(p.status, 0, ST_BAD_ARGUMENT); *abort_flag = 1; }
+  if (EPI == EPI_STORE && sizeof(OutT) == 4 && p.part_slots) {
+    if (warp == 0)
+      plan_pieces(plan, p.seg_offsets, p.K, p.groups, ((p.M + TM - 1) / TM) * ((p.N + TN - 1) / TN), (long long)p.M * p.N,
+                  (int)cluster_nctaid_x(), p.part_slots, p.part_cut);
+    __syncthreads();
+  }
 
   const int tiles_m = (p.mode == 1) ? (*p.num_m_tiles + 1) / 2 : (p.M + TM - 1) / TM;
   const int tiles_n = (p.N + TN - 1) / TN;
@@ -590,7 +594,7 @@ constexpr size_t smem_bytes() {
 __global__ void __launch_bounds__(256) piece_add_kernel(const float* __restrict__ part, float* __restrict__ out, const int* seg, int K,
                                                         int groups, int per, long long mn, int n_pairs, int slots, int fixed) {
   __shared__ PiecePlan pl;
-  // the offsets come from kernels before the product, which is not itself launched ahead of them
+  // the offsets come from kernels before the product, which have ended: all blocks of the product are past their wait
   if (threadIdx.x < 32) plan_pieces(&pl, seg, K, groups, per, mn, n_pairs, slots, fixed);
   __syncthreads();
   pdl_wait();
@@ -684,7 +688,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   if (pairs < 1) pairs = 1;
   if (p.part_slots) pairs = max_pairs;
   if (used_pairs) *used_pairs = pairs;
-  kern<<<2 * pairs, gb::pr::THREADS, smem, st>>>(ta, tb, to, tx, p);
+  GB_PDL_LAUNCH_SMEM(kern, dim3(2 * pairs), dim3(gb::pr::THREADS), smem, st, ta, tb, to, tx, p);
   return gb_launch_rc();
 }
 

@@ -188,13 +188,4 @@ __device__ __forceinline__ void ll_row_norm(int d, int mode, const float* __rest
 // Cache row of a position: the first `keep` rows are never given up, the rest is a ring of cap - keep rows.
 __device__ __forceinline__ int ll_ring_row(int p, int keep, int cap) { return p < keep ? p : keep + (p - keep) % (cap - keep); }
 
-// kernel<<<grid, block, smem>>> with programmatic stream serialization, opting in to more than 48 KB of shared memory
-#define GB_PDL_LAUNCH_SMEM(kernel, grid, block, smem, st, ...)                                                       \
-  do {                                                                                                               \
-    cudaLaunchAttribute gb_attr_;                                                                                    \
-    cudaLaunchConfig_t gb_cfg_ = gb_pdl_config(grid, block, smem, st, &gb_attr_);                                    \
-    if ((smem) > 48 * 1024) (void)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem)); \
-    (void)cudaLaunchKernelEx(&gb_cfg_, kernel, __VA_ARGS__);                                                         \
-  } while (0)
-
 }  // namespace gb

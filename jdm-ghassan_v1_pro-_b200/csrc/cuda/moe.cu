@@ -50,6 +50,7 @@ __device__ __forceinline__ void warp_argmax(float& v, int& i) {
 // pieces the kernel was bound by load instructions, at a tenth of the bandwidth its 2 bytes per element need.
 template <typename T, int NV8>
 __global__ void __launch_bounds__(256) moe_route_kernel(const gb_moe_args a) {
+  pdl_wait();
   __shared__ int s_hist[MAX_NE + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ne = a.ne, K = a.top_k, d = a.d;
@@ -222,6 +223,7 @@ __global__ void __launch_bounds__(RT_THREADS) moe_route_tc_kernel(const __grid_c
   if (warp == 1) { tmem_alloc(tmem_slot, 32); tmem_relinquish(); }
   for (int i = threadIdx.x; i < nsub * (ne + 1); i += RT_THREADS) s_hist[i] = 0;
   __syncthreads();
+  pdl_wait();            // behind the allocation of tensor memory, as in the pair kernel of the GEMM
   // the first activation tiles are asked for before the weights are prepared, so that they arrive meanwhile
   const int pre = nkc < RT_ST ? nkc : RT_ST;
   if (threadIdx.x == 0)
@@ -384,6 +386,7 @@ __global__ void __launch_bounds__(RT_THREADS) moe_route_tc_kernel(const __grid_c
 // `staged` != 0: the histogram table fits the dynamic shared memory passed at launch and is scanned there
 // (the per-expert scans are chains of dependent loads; in global memory they dominate the kernel).
 __global__ void moe_scan_kernel(const gb_moe_args a, int n_blocks, int staged) {
+  pdl_wait();
   __shared__ int s_total[MAX_NE + 1];
   __shared__ int s_off[MAX_NE + 2];
   extern __shared__ int s_tab[];
@@ -509,6 +512,7 @@ __global__ void moe_scan_kernel(const gb_moe_args a, int n_blocks, int staged) {
 // fixed-order tree reduction
 __global__ void moe_colmean_kernel(const float* __restrict__ probs, float* __restrict__ out, int n_tok_all, int ne,
                                    int seg_tok) {
+  pdl_wait();
   __shared__ float s[256];
   const int e = blockIdx.x;
   const int t_lo = blockIdx.y * seg_tok;
@@ -529,6 +533,7 @@ __global__ void moe_colmean_kernel(const float* __restrict__ probs, float* __res
 // Row positions (stable: token order inside every expert) and the expert-sorted copy.
 template <typename T>
 __global__ void __launch_bounds__(256) moe_pack_kernel(const gb_moe_args a) {
+  pdl_wait();
   __shared__ int s_idx[BLK_TOK * MAX_K];
   __shared__ int s_pos[BLK_TOK * (MAX_K + 1)];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -574,6 +579,7 @@ constexpr int PAD_PARTS = 16;
 template <typename T>
 __global__ void moe_zero_pads_kernel(T* __restrict__ buf, const int* __restrict__ seg_offsets,
                                      const int* __restrict__ totals, int d) {
+  pdl_wait();
   const int e = blockIdx.x;
   const int r0 = seg_offsets[e] + totals[e], r1 = seg_offsets[e + 1];
   const int vec = d / 8;
@@ -583,6 +589,7 @@ __global__ void moe_zero_pads_kernel(T* __restrict__ buf, const int* __restrict_
 
 template <typename T>
 __global__ void __launch_bounds__(256) moe_combine_kernel(const gb_moe_args a) {
+  pdl_wait();
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= a.n_tok) return;
   const int K = a.top_k, S = K + (a.shared ? 1 : 0), d = a.d;
@@ -621,6 +628,7 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const gb_moe_args a) {
 // dy_perm[pos(t,k)] = w_k * dout[t]; dy_perm[pos(t,shared)] = dout[t]; gdot[t,k] = <dout[t], y_perm[pos(t,k)]>
 template <typename T>
 __global__ void __launch_bounds__(256) moe_combine_bwd_kernel(const gb_moe_args a) {
+  pdl_wait();
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= a.n_tok) return;
   const int K = a.top_k, S = K + (a.shared ? 1 : 0), d = a.d;
@@ -666,6 +674,7 @@ __global__ void __launch_bounds__(256) moe_combine_bwd_kernel(const gb_moe_args 
 // router-logit gradients (into `part`, [n_tok, ne]).
 template <typename T>
 __global__ void __launch_bounds__(256, 4) moe_router_bwd_kernel(const gb_moe_args a) {
+  pdl_wait();
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= a.n_tok) return;
   const int ne = a.ne, K = a.top_k, S = K + (a.shared ? 1 : 0), d = a.d;
@@ -748,6 +757,7 @@ __global__ void __launch_bounds__(256, 4) moe_router_bwd_kernel(const gb_moe_arg
 // broadcast loads of the logit gradients; the 24 KB of router rows are no longer re-read from L1 for every token
 // (sixteen 16-byte loads per 8 columns, three quarters of the one-kernel form's load instructions).
 __global__ void __launch_bounds__(256) moe_router_dlogit_kernel(const gb_moe_args a) {
+  pdl_wait();
   // one thread per token: with at most 8 experts everything of a token fits a thread's registers, and its dozen
   // loads are independent (a warp per token waited for them in sequence, round after round)
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -801,6 +811,7 @@ __global__ void __launch_bounds__(256) moe_router_dlogit_kernel(const gb_moe_arg
 constexpr int RD_LANES = 96, RD_GROUPS = 4;
 template <typename T, int NS>       // NS = slots per token (top_k + shared), so that the row buffers are exactly that long
 __global__ void __launch_bounds__(RD_LANES * RD_GROUPS) moe_router_dx_kernel(const gb_moe_args a) {
+  pdl_wait();
   const int g = threadIdx.x / RD_LANES, l = threadIdx.x - g * RD_LANES;
   const int c0 = (blockIdx.y * RD_LANES + l) * 8;
   const int ne = a.ne, d = a.d;
@@ -891,6 +902,7 @@ template <typename T>
 __global__ void __launch_bounds__(RW_LANES * RW_GROUPS) moe_router_wgrad_kernel(const float* __restrict__ dlogit,
                                                                               const T* __restrict__ x16, float* __restrict__ dw,
                                                                               int n_tok, int ne, int d) {
+  pdl_wait();
   __shared__ float red[RW_LANES][65];
   const int g = threadIdx.x / RW_LANES, l = threadIdx.x - g * RW_LANES;
   const int c0 = (blockIdx.x * RW_LANES + l) * 8;
@@ -988,6 +1000,7 @@ __global__ void __launch_bounds__(RW_LANES * RW_GROUPS) moe_router_wgrad_kernel(
 // chunks each (their loads independent), and the eight partial sums are added in order.
 __global__ void __launch_bounds__(256) moe_router_wgrad_fold_kernel(const float* __restrict__ part, float* __restrict__ dw,
                                                                     int chunks, int n) {
+  pdl_wait();
   __shared__ float red[8][32];
   const int o = threadIdx.x & 31, q = threadIdx.x >> 5;
   const int i = blockIdx.x * 32 + o;
@@ -1013,12 +1026,12 @@ using namespace gb;
 template <typename T>
 static void launch_router_dx(const gb_moe_args& a, int n_slots, dim3 grid, cudaStream_t st) {
   switch (n_slots) {
-    case 1: moe_router_dx_kernel<T, 1><<<grid, RD_LANES * RD_GROUPS, 0, st>>>(a); break;
-    case 2: moe_router_dx_kernel<T, 2><<<grid, RD_LANES * RD_GROUPS, 0, st>>>(a); break;
-    case 3: moe_router_dx_kernel<T, 3><<<grid, RD_LANES * RD_GROUPS, 0, st>>>(a); break;
-    case 4: moe_router_dx_kernel<T, 4><<<grid, RD_LANES * RD_GROUPS, 0, st>>>(a); break;
-    case 5: moe_router_dx_kernel<T, 5><<<grid, RD_LANES * RD_GROUPS, 0, st>>>(a); break;
-    default: moe_router_dx_kernel<T, 6><<<grid, RD_LANES * RD_GROUPS, 0, st>>>(a); break;
+    case 1: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 1>), dim3(grid), dim3(RD_LANES * RD_GROUPS), 0, st, a); break;
+    case 2: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 2>), dim3(grid), dim3(RD_LANES * RD_GROUPS), 0, st, a); break;
+    case 3: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 3>), dim3(grid), dim3(RD_LANES * RD_GROUPS), 0, st, a); break;
+    case 4: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 4>), dim3(grid), dim3(RD_LANES * RD_GROUPS), 0, st, a); break;
+    case 5: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 5>), dim3(grid), dim3(RD_LANES * RD_GROUPS), 0, st, a); break;
+    default: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 6>), dim3(grid), dim3(RD_LANES * RD_GROUPS), 0, st, a); break;
   }
 }
 
@@ -1062,7 +1075,7 @@ extern "C" int gb_moe_route(const gb_moe_args* a, cudaStream_t st) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -10;
         set_b = smem;
       }
-      kern<<<grid, RT_THREADS, smem, st>>>(tm, *a, a->status);
+      GB_PDL_LAUNCH_SMEM(kern, dim3(grid), dim3(RT_THREADS), smem, st, tm, *a, a->status);
     } else {
       auto kern = moe_route_tc_kernel<__half>;
       static size_t set_h = 0;
@@ -1070,17 +1083,17 @@ extern "C" int gb_moe_route(const gb_moe_args* a, cudaStream_t st) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -10;
         set_h = smem;
       }
-      kern<<<grid, RT_THREADS, smem, st>>>(tm, *a, a->status);
+      GB_PDL_LAUNCH_SMEM(kern, dim3(grid), dim3(RT_THREADS), smem, st, tm, *a, a->status);
     }
   }
   const bool vec = a->d % 256 == 0 && a->d <= 1024 && (((uintptr_t)a->x16 | (uintptr_t)a->router_w) & 15) == 0;
 #define GB_ROUTE(T)                                                           \
   switch (vec ? a->d / 256 : 0) {                                             \
-    case 1: moe_route_kernel<T, 1><<<nb, 256, 0, st>>>(*a); break;            \
-    case 2: moe_route_kernel<T, 2><<<nb, 256, 0, st>>>(*a); break;            \
-    case 3: moe_route_kernel<T, 3><<<nb, 256, 0, st>>>(*a); break;            \
-    case 4: moe_route_kernel<T, 4><<<nb, 256, 0, st>>>(*a); break;            \
-    default: moe_route_kernel<T, 0><<<nb, 256, 0, st>>>(*a); break;           \
+    case 1: GB_PDL_LAUNCH_SMEM((moe_route_kernel<T, 1>), dim3(nb), dim3(256), 0, st, *a); break;            \
+    case 2: GB_PDL_LAUNCH_SMEM((moe_route_kernel<T, 2>), dim3(nb), dim3(256), 0, st, *a); break;            \
+    case 3: GB_PDL_LAUNCH_SMEM((moe_route_kernel<T, 3>), dim3(nb), dim3(256), 0, st, *a); break;            \
+    case 4: GB_PDL_LAUNCH_SMEM((moe_route_kernel<T, 4>), dim3(nb), dim3(256), 0, st, *a); break;            \
+    default: GB_PDL_LAUNCH_SMEM((moe_route_kernel<T, 0>), dim3(nb), dim3(256), 0, st, *a); break;           \
   }
   if (!tc) {
     if (a->is_bf16) { GB_ROUTE(__nv_bfloat16) } else { GB_ROUTE(__half) }
@@ -1088,7 +1101,7 @@ extern "C" int gb_moe_route(const gb_moe_args* a, cudaStream_t st) {
 #undef GB_ROUTE
   if (a->aux_m) {
     const int seg_tok = a->seg_tokens > 0 ? a->seg_tokens : a->n_tok;
-    moe_colmean_kernel<<<dim3(a->ne, (a->n_tok + seg_tok - 1) / seg_tok), 256, 0, st>>>(a->probs, a->aux_m, a->n_tok, a->ne,
+    GB_PDL_LAUNCH_SMEM(moe_colmean_kernel, dim3(a->ne, (a->n_tok + seg_tok - 1) / seg_tok), dim3(256), 0, st, a->probs, a->aux_m, a->n_tok, a->ne,
                                                                                        seg_tok);
   }
   return GB_OK();
@@ -1102,14 +1115,14 @@ extern "C" int gb_moe_group(const gb_moe_args* a, cudaStream_t st) {
   const int ne1 = a->ne + (a->shared ? 1 : 0);
   const size_t tab_bytes = (size_t)nb * (a->ne + 1) * sizeof(int);
   const int staged = tab_bytes <= 40 * 1024;
-  moe_scan_kernel<<<1, 256, staged ? tab_bytes : 0, st>>>(*a, nb, staged);
+  GB_PDL_LAUNCH_SMEM(moe_scan_kernel, dim3(1), dim3(256), staged ? tab_bytes : 0, st, *a, nb, staged);
   const int* totals = a->block_base + (size_t)nb * (a->ne + 1);
   if (a->is_bf16) {
-    moe_pack_kernel<__nv_bfloat16><<<nb, 256, 0, st>>>(*a);
-    if (!a->forward_only) moe_zero_pads_kernel<__nv_bfloat16><<<dim3(ne1, PAD_PARTS), 256, 0, st>>>((__nv_bfloat16*)a->x_perm, a->seg_offsets, totals, a->d);
+    GB_PDL_LAUNCH_SMEM((moe_pack_kernel<__nv_bfloat16>), dim3(nb), dim3(256), 0, st, *a);
+    if (!a->forward_only) GB_PDL_LAUNCH_SMEM((moe_zero_pads_kernel<__nv_bfloat16>), dim3(ne1, PAD_PARTS), dim3(256), 0, st, (__nv_bfloat16*)a->x_perm, a->seg_offsets, totals, a->d);
   } else {
-    moe_pack_kernel<__half><<<nb, 256, 0, st>>>(*a);
-    if (!a->forward_only) moe_zero_pads_kernel<__half><<<dim3(ne1, PAD_PARTS), 256, 0, st>>>((__half*)a->x_perm, a->seg_offsets, totals, a->d);
+    GB_PDL_LAUNCH_SMEM((moe_pack_kernel<__half>), dim3(nb), dim3(256), 0, st, *a);
+    if (!a->forward_only) GB_PDL_LAUNCH_SMEM((moe_zero_pads_kernel<__half>), dim3(ne1, PAD_PARTS), dim3(256), 0, st, (__half*)a->x_perm, a->seg_offsets, totals, a->d);
   }
   return GB_OK();
 }
@@ -1118,8 +1131,8 @@ extern "C" int gb_moe_combine(const gb_moe_args* a, cudaStream_t st) {
   int rc = moe_check(a);
   if (rc) return rc;
   const int grid = (a->n_tok + 7) / 8;
-  if (a->is_bf16) moe_combine_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(*a);
-  else moe_combine_kernel<__half><<<grid, 256, 0, st>>>(*a);
+  if (a->is_bf16) GB_PDL_LAUNCH_SMEM((moe_combine_kernel<__nv_bfloat16>), dim3(grid), dim3(256), 0, st, *a);
+  else GB_PDL_LAUNCH_SMEM((moe_combine_kernel<__half>), dim3(grid), dim3(256), 0, st, *a);
   return GB_OK();
 }
 
@@ -1131,11 +1144,11 @@ extern "C" int gb_moe_combine_bwd(const gb_moe_args* a, cudaStream_t st) {
   const int ne1 = a->ne + (a->shared ? 1 : 0);
   const int* totals = a->block_base + (size_t)nb * (a->ne + 1);
   if (a->is_bf16) {
-    moe_combine_bwd_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(*a);
-    moe_zero_pads_kernel<__nv_bfloat16><<<dim3(ne1, PAD_PARTS), 256, 0, st>>>((__nv_bfloat16*)a->dy_perm, a->seg_offsets, totals, a->d);
+    GB_PDL_LAUNCH_SMEM((moe_combine_bwd_kernel<__nv_bfloat16>), dim3(grid), dim3(256), 0, st, *a);
+    GB_PDL_LAUNCH_SMEM((moe_zero_pads_kernel<__nv_bfloat16>), dim3(ne1, PAD_PARTS), dim3(256), 0, st, (__nv_bfloat16*)a->dy_perm, a->seg_offsets, totals, a->d);
   } else {
-    moe_combine_bwd_kernel<__half><<<grid, 256, 0, st>>>(*a);
-    moe_zero_pads_kernel<__half><<<dim3(ne1, PAD_PARTS), 256, 0, st>>>((__half*)a->dy_perm, a->seg_offsets, totals, a->d);
+    GB_PDL_LAUNCH_SMEM((moe_combine_bwd_kernel<__half>), dim3(grid), dim3(256), 0, st, *a);
+    GB_PDL_LAUNCH_SMEM((moe_zero_pads_kernel<__half>), dim3(ne1, PAD_PARTS), dim3(256), 0, st, (__half*)a->dy_perm, a->seg_offsets, totals, a->d);
   }
   return GB_OK();
 }
@@ -1158,27 +1171,27 @@ extern "C" int gb_moe_router_bwd(const gb_moe_args* a, cudaStream_t st) {
   dim3 gdx(std::max(1, std::min(sms, (a->n_tok + RD_GROUPS - 1) / RD_GROUPS)), (a->d / 8 + RD_LANES - 1) / RD_LANES);   // one resident block per SM
   if (a->is_bf16) {
     if (split) {
-      moe_router_dlogit_kernel<<<(a->n_tok + 255) / 256, 256, 0, st>>>(*a);
+      GB_PDL_LAUNCH_SMEM(moe_router_dlogit_kernel, dim3((a->n_tok + 255) / 256), dim3(256), 0, st, *a);
       launch_router_dx<__nv_bfloat16>(*a, n_slots, gdx, st);
     } else {
-      moe_router_bwd_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(*a);
+      GB_PDL_LAUNCH_SMEM((moe_router_bwd_kernel<__nv_bfloat16>), dim3(grid), dim3(256), 0, st, *a);
     }
     if (a->d_router_w)
-      moe_router_wgrad_kernel<__nv_bfloat16><<<g2, RW_LANES * RW_GROUPS, 0, st>>>(a->part, (const __nv_bfloat16*)a->x16, wout, a->n_tok,
+      GB_PDL_LAUNCH_SMEM((moe_router_wgrad_kernel<__nv_bfloat16>), dim3(g2), dim3(RW_LANES * RW_GROUPS), 0, st, a->part, (const __nv_bfloat16*)a->x16, wout, a->n_tok,
                                                                  a->ne, a->d);
   } else {
     if (split) {
-      moe_router_dlogit_kernel<<<(a->n_tok + 255) / 256, 256, 0, st>>>(*a);
+      GB_PDL_LAUNCH_SMEM(moe_router_dlogit_kernel, dim3((a->n_tok + 255) / 256), dim3(256), 0, st, *a);
       launch_router_dx<__half>(*a, n_slots, gdx, st);
     } else {
-      moe_router_bwd_kernel<__half><<<grid, 256, 0, st>>>(*a);
+      GB_PDL_LAUNCH_SMEM((moe_router_bwd_kernel<__half>), dim3(grid), dim3(256), 0, st, *a);
     }
     if (a->d_router_w)
-      moe_router_wgrad_kernel<__half><<<g2, RW_LANES * RW_GROUPS, 0, st>>>(a->part, (const __half*)a->x16, wout, a->n_tok, a->ne, a->d);
+      GB_PDL_LAUNCH_SMEM((moe_router_wgrad_kernel<__half>), dim3(g2), dim3(RW_LANES * RW_GROUPS), 0, st, a->part, (const __half*)a->x16, wout, a->n_tok, a->ne, a->d);
   }
   if (a->d_router_w && chunks > 1) {
     const int n = a->ne * a->d;
-    moe_router_wgrad_fold_kernel<<<(n + 31) / 32, 256, 0, st>>>(a->part2, a->d_router_w, chunks, n);
+    GB_PDL_LAUNCH_SMEM(moe_router_wgrad_fold_kernel, dim3((n + 31) / 32), dim3(256), 0, st, a->part2, a->d_router_w, chunks, n);
   }
   return GB_OK();
 }

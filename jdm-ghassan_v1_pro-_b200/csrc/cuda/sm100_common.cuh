@@ -57,13 +57,22 @@ static inline cudaLaunchConfig_t gb_pdl_config(dim3 grid, dim3 block, size_t sme
     cudaLaunchConfig_t gb_cfg_ = gb_pdl_config(grid, block, 0, st, &gb_attr_);        \
     (void)cudaLaunchKernelEx(&gb_cfg_, kernel, __VA_ARGS__);                          \
   } while (0)
+// The same with dynamic shared memory, opting in to more than 48 KB of it.
+#define GB_PDL_LAUNCH_SMEM(kernel, grid, block, smem, st, ...)                                                       \
+  do {                                                                                                               \
+    cudaLaunchAttribute gb_attr_;                                                                                    \
+    cudaLaunchConfig_t gb_cfg_ = gb_pdl_config(grid, block, smem, st, &gb_attr_);                                    \
+    if ((smem) > 48 * 1024) (void)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem)); \
+    (void)cudaLaunchKernelEx(&gb_cfg_, kernel, __VA_ARGS__);                                                         \
+  } while (0)
 
 namespace gb {
 
 // Wait until the kernels before this one have finished and their writes are visible, then let the kernel after it begin its own
 // set-up.  The first statement of every kernel that GB_PDL_LAUNCH starts, but for those that first ask for constants (weights in
-// gemm_skinny_sm100.cu, layers_gemv.cu and layers_latent.cu, prefetches in layers_mamba.cu, the offsets in piece_add_kernel): their launchers say
-// which arguments the launch ahead must not write.
+// gemm_skinny_sm100.cu, layers_gemv.cu and layers_latent.cu, prefetches in layers_mamba.cu, the offsets in piece_add_kernel, the state and
+// the cache rows of earlier steps in the token attention kernels): their launchers say which arguments the launch ahead must not write.  A kernel with tensor memory allocates
+// it first: were the next kernel let in before, its blocks could take the columns and then wait for this kernel, which waits for them.
 __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
