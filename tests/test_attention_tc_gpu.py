@@ -253,3 +253,35 @@ def test_tc_attention_scores_of_thousands(dt, T, H, KV, hd, use_seg):
             assert worst <= 1.0, (name, top, worst)
         err = float((heads(lse.repeat_interleave(hd, dim=1), H)[..., 0] - torch.logsumexp(S, dim=-1)).abs().max())
         assert err <= 8 * 2.0 ** -23 * terms, ("lse", top, err)
+
+
+# Two CTAs an item: from four query tiles on, and while all pairs are resident (148 items); 385 is the shortest, 8 x 18 items and more fall back.
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("B,T,H,KV,window,use_seg", [(1, 385, 3, 1, 0, False), (1, 1501, 12, 4, 0, False), (2, 700, 8, 2, 0, True), (1, 1000, 8, 2, 129, True),
+                                                     (3, 512, 12, 4, 1, False), (1, 2304, 8, 2, 0, False), (1, 2305, 8, 2, 0, False), (1, 384, 4, 2, 0, False)])
+def test_tc_forward_with_shared_items(dt, B, T, H, KV, window, use_seg):
+    """Rows whose keys all lie in one CTA's tiles, documents that begin in the second half, windows shorter than a tile; log-sum-exp included."""
+    from ghassan_b200.ops import kernels as K
+    hd = 64
+    n = B * T
+    g = torch.Generator(device="cuda").manual_seed(T + H)
+    q, k, v = (torch.randn(n, h * hd, device="cuda", generator=g).to(dt) * s for h, s in ((H, 2.0), (KV, 2.0), (KV, 1.0)))
+    seg = torch.arange(T, device="cuda", dtype=torch.int32).div(317, rounding_mode="floor").to(torch.int32).repeat(B) if use_seg else None
+    o, lse = torch.full((n, H * hd), 7.0, device="cuda", dtype=dt), torch.full((n, H), 7.0, device="cuda")
+    lo = torch.zeros(n, dtype=torch.int32, device="cuda")
+    K.attn_tc_fwd(q, k, v, o, lse, seg, lo, B, T, H, KV, hd, window, hd ** -0.5)
+    i, j = torch.arange(T, device="cuda")[:, None], torch.arange(T, device="cuda")[None, :]
+    see = j <= i
+    if window:
+        see = see & (j > i - window)
+    if use_seg:
+        see = see & (seg[:T, None] == seg[None, :T])
+    for b in range(B):
+        rows = slice(b * T, (b + 1) * T)
+        for h in range(H):
+            s = (q[rows, h * hd:(h + 1) * hd].float() @ k[rows, (h * KV // H) * hd:(h * KV // H + 1) * hd].float().t() * hd ** -0.5).masked_fill(~see, float("-inf"))
+            want = torch.softmax(s, -1) @ v[rows, (h * KV // H) * hd:(h * KV // H + 1) * hd].float()
+            ok, worst = near(o[rows, h * hd:(h + 1) * hd], want)[:2]
+            assert ok, (b, h, worst)
+            assert float((lse[rows, h] - torch.logsumexp(s, -1)).abs().max()) <= 2e-3          # fp32, fast exponentials, values up to about 30
+
