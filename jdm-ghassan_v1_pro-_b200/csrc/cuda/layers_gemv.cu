@@ -58,13 +58,12 @@ struct LlGemv {
 // went from 26.6 to 25.6 ms: 12 layers, width 1024).
 __host__ __device__ constexpr int ll_norm_vectors(int pro) { return pro == 1 || pro == 5 ? 2 : pro == 3 || pro == 4 ? 1 : 0; }
 
-// Input vector of sequence b into xs[0, K).  w1, w2: the norm weights in shared memory (w2: the last norm's, or the norm's bias).
-template <int PRO, typename XT>
+// Input vector of sequence b into xs[0, K).  KEEP: values per thread of a row that stay in registers (the rest is made again).  w1, w2: the norm weights in shared memory (w2: the last norm's, or the norm's bias).
+template <int PRO, typename XT, int KEEP>
 __device__ __forceinline__ void ll_prologue(const LlGemv& a, int b, XT* __restrict__ xs, float* red, float* part_inv, const float* w1, const float* w2) {
   const int tid = threadIdx.x, d = a.d;
   if constexpr (PRO == 1) {
     const float* xr = a.x + (long long)b * d;
-    constexpr int KEEP = 16;                       // values per thread kept in registers (d up to 4096)
     float v[KEEP];
     const bool writes = blockIdx.x == 0 && a.x_out != nullptr;
     if (a.y) {
@@ -135,7 +134,6 @@ __device__ __forceinline__ void ll_prologue(const LlGemv& a, int b, XT* __restri
     const float* yr = a.y ? a.y + b * a.ldy : nullptr;
     const float* x0 = a.x0 ? a.x0 + (long long)b * d : nullptr;
     float* xo = blockIdx.x == 0 && a.x_out ? a.x_out + (long long)b * d : nullptr;
-    constexpr int KEEP = 16;                       // values per thread kept in registers (d up to 4096); the rest is made again
     auto value = [&](int i) {
       float v = xr[i];
       if (yr) v += a.alpha * yr[i];
@@ -173,6 +171,10 @@ __device__ __forceinline__ void ll_prologue(const LlGemv& a, int b, XT* __restri
     const float* vr = a.v32 + (long long)b * d;
     const float* sq = a.sq + (long long)b * a.n_sq;
     const int per = d / a.parts, nq = a.n_sq / a.parts, warp = tid >> 5, lane = tid & 31;
+    constexpr int NV = 8;                          // values asked for with the sums, not behind them (one round trip instead of two)
+    float v[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = tid + k * LV_THREADS < d ? vr[tid + k * LV_THREADS] : 0.f;
     for (int p = warp; p < a.parts; p += LV_WARPS) {
       float ss = 0.f;
       for (int i = lane; i < nq; i += 32) ss += sq[p * nq + i];
@@ -180,8 +182,12 @@ __device__ __forceinline__ void ll_prologue(const LlGemv& a, int b, XT* __restri
       if (lane == 0) part_inv[p] = ll_inv_rms(ss, per, a.eps);
     }
     __syncthreads();
+    auto put = [&](int i, float x) { xs[i] = Cvt<XT>::from_f(x * part_inv[a.parts == 1 ? 0 : i / per] * w1[i]); };
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+      if (tid + k * LV_THREADS < d) put(tid + k * LV_THREADS, v[k]);
 #pragma unroll 4
-    for (int i = tid; i < d; i += LV_THREADS) xs[i] = Cvt<XT>::from_f(vr[i] * part_inv[i / per] * w1[i]);
+    for (int i = tid + NV * LV_THREADS; i < d; i += LV_THREADS) put(i, vr[i]);
     __syncthreads();                               // part_inv is the next sequence's, too
   } else {                                         // PRO == 2: gated norm in equal parts, one warp per part
     const XT* yr = reinterpret_cast<const XT*>(a.y16) + b * a.ldy16;
@@ -202,26 +208,26 @@ __device__ __forceinline__ void ll_prologue(const LlGemv& a, int b, XT* __restri
       }
     } else {
       for (int p = 0; p < a.parts; ++p) {          // few parts: the whole block works on each
-        constexpr int KEEP = 8;
-        float v[KEEP];
+        constexpr int KEEP2 = 8;
+        float v[KEEP2];
         float ss = 0.f;
 #pragma unroll
-        for (int k = 0; k < KEEP; ++k) {
+        for (int k = 0; k < KEEP2; ++k) {
           const int i = tid + k * LV_THREADS;
           v[k] = i < per ? Cvt<XT>::to_f(yr[p * per + i]) * ll_silu_t<XT>(Cvt<XT>::to_f(zr[p * per + i])) : 0.f;
           ss += v[k] * v[k];
         }
-        for (int i = tid + KEEP * LV_THREADS; i < per; i += LV_THREADS) {
+        for (int i = tid + KEEP2 * LV_THREADS; i < per; i += LV_THREADS) {
           const float t = Cvt<XT>::to_f(yr[p * per + i]) * ll_silu_t<XT>(Cvt<XT>::to_f(zr[p * per + i]));
           ss += t * t;
         }
         const float inv = ll_inv_rms(ll_block_sum(ss, red), per, a.eps);
 #pragma unroll
-        for (int k = 0; k < KEEP; ++k) {
+        for (int k = 0; k < KEEP2; ++k) {
           const int i = tid + k * LV_THREADS;
           if (i < per) xs[p * per + i] = Cvt<XT>::from_f(v[k] * inv * a.w1[p * per + i]);
         }
-        for (int i = tid + KEEP * LV_THREADS; i < per; i += LV_THREADS) {
+        for (int i = tid + KEEP2 * LV_THREADS; i < per; i += LV_THREADS) {
           const float t = Cvt<XT>::to_f(yr[p * per + i]) * ll_silu_t<XT>(Cvt<XT>::to_f(zr[p * per + i]));
           xs[p * per + i] = Cvt<XT>::from_f(t * inv * a.w1[p * per + i]);
         }
@@ -262,29 +268,41 @@ __device__ __forceinline__ void ll_accum(const LlRaw<FMT>& raw, int u, const XT*
     if (j < nb) acc[j] += ll_dot8(w, x + j * ldx + 8 * u);
 }
 
-// KS warps share a stored row (short rows spread over more of the machine); NB sequences per pass over the row.
-template <int FMT, typename XT, int PRO, int SWI, int NB, int KS>
+// KS warps share a stored row (short rows spread over more of the machine).
+// One sequence (R > 0): a warp takes R rows at a time, as many as eight units a lane, 32 registers, hold.  All of them are asked for
+// before the wait for the kernel ahead, and their sums are reduced side by side with one barrier.  The product was a chain of trips of
+// one row, 0.75 us each, with a DRAM round trip from the second on.  Width 1024, each kernel's time behind the one ahead: 4384 rows
+// 5.6 -> 3.5 us, 5632 with SwiGLU 5.7 -> 3.5, 1024 of 2816 numbers 3.6 -> 2.9, of 2048 with the gated norm 5.6 -> 4.0, the vocabulary
+// 18.5 -> 14.0; a request of 64 tokens 25.8 -> 21.0 ms.
+// Several sequences (R == 0), and rows of more units: NB sequences a pass over a row, PF units ahead, the rest in a loop.
+template <int FMT, typename XT, int PRO, int SWI, int NB, int KS, int R, int UPL, int KEEP>
 __global__ void __launch_bounds__(LV_THREADS) ll_gemv_kernel(const __grid_constant__ LlGemv a) {
-  constexpr int PF = (SWI ? 4 : 8) / (FMT == GB_W_F32 ? 2 : 1);      // units per lane and row that are loaded ahead
+  constexpr int ROWS = R ? R : 1, PF = R ? UPL : (SWI ? 4 : 8) / (FMT == GB_W_F32 ? 2 : 1);      // rows, and units per lane of each, that are loaded ahead
+  static_assert(R == 0 || NB == 1, "rows side by side are for one sequence");
   extern __shared__ __align__(16) uint8_t lv_dyn[];
   __shared__ float red[LV_WARPS];
   __shared__ float part_inv[PRO == 3 ? 256 : 1];
-  __shared__ float part[2][LV_WARPS][NB];
+  __shared__ float part[2][LV_WARPS][NB * ROWS];
   XT* xs = reinterpret_cast<XT*>(lv_dyn);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ric = warp / KS, ks = warp % KS;
   const int n_out = SWI ? a.N / 2 : a.N, units = a.K >> 3, u0 = lane + 32 * ks;
   constexpr int RPB = LV_WARPS / KS, US = 32 * KS;
   auto row_of = [&](int j) { return a.W + (SWI ? (long long)(j >> 6) * 128 + (j & 63) : (long long)j) * a.row_bytes; };
-  LlRaw<FMT> g[PF], up[SWI ? PF : 1];
-  auto fetch = [&](int j) {
-    if (j >= n_out) return;
-    const uint8_t* w = row_of(j);
+  LlRaw<FMT> g[ROWS][PF], up[ROWS][SWI ? PF : 1];
+  const int step = gridDim.x * RPB;
+  auto fetch = [&](int j0) {
 #pragma unroll
-    for (int k = 0; k < PF; ++k)
-      if (u0 + k * US < units) {
-        g[k].load(w, u0 + k * US);
-        if constexpr (SWI != 0) up[k].load(w + 64 * a.row_bytes, u0 + k * US);
-      }
+    for (int r = 0; r < ROWS; ++r) {
+      const int j = j0 + r * step;
+      if (j >= n_out) return;
+      const uint8_t* w = row_of(j);
+#pragma unroll
+      for (int k = 0; k < PF; ++k)
+        if (u0 + k * US < units) {
+          g[r][k].load(w, u0 + k * US);
+          if constexpr (SWI != 0) up[r][k].load(w + 64 * a.row_bytes, u0 + k * US);
+        }
+    }
   };
   fetch(blockIdx.x * RPB + ric);
   constexpr int NV = ll_norm_vectors(PRO);
@@ -301,72 +319,118 @@ __global__ void __launch_bounds__(LV_THREADS) ll_gemv_kernel(const __grid_consta
   const XT* xin = reinterpret_cast<const XT*>(a.x16);
   long long ldx = a.ldx;
   if constexpr (PRO != 0) {
-    for (int b = 0; b < a.B; ++b) ll_prologue<PRO, XT>(a, b, xs + (long long)b * a.K, red, part_inv, a.staged ? norm_w : a.w1, a.staged ? norm_w + a.d : second);
+    for (int b = 0; b < a.B; ++b)
+      ll_prologue<PRO, XT, KEEP>(a, b, xs + (long long)b * a.K, red, part_inv, a.staged ? norm_w : a.w1, a.staged ? norm_w + a.d : second);
     __syncthreads();
     xin = xs;
     ldx = a.K;
   }
+  auto store = [&](int b, int j, float v, float u) {
+    if constexpr (SWI != 0) v = ll_silu(v) * u;
+    if (a.softcap > 0.f) v = a.softcap * tanhf(v / a.softcap);
+    if (a.n1 > 0 && j >= a.n1) {
+      v = fmaxf(v, 0.f);
+      reinterpret_cast<XT*>(a.out2)[(long long)b * a.ldo2 + j - a.n1] = Cvt<XT>::from_f(v * v);
+    } else if (a.out_f32) reinterpret_cast<float*>(a.out)[(long long)b * a.ldo + j] = v;
+    else reinterpret_cast<XT*>(a.out)[(long long)b * a.ldo + j] = Cvt<XT>::from_f(v);
+  };
   // every warp of the block makes the same number of trips: rows past the end still take part in the barriers
-  for (int j0 = blockIdx.x * RPB; j0 < n_out; j0 += gridDim.x * RPB) {
+#pragma unroll 1
+  for (int j0 = blockIdx.x * RPB; j0 < n_out; j0 += ROWS * step) {
     const int j = j0 + ric;
-    const bool live = j < n_out;
-    for (int b0 = 0; b0 < a.B; b0 += NB) {
-      const int nb = min(NB, a.B - b0);
-      float acc[NB], acu[NB];
+    if constexpr (R > 0) {
+      float acc[R], acu[R];
 #pragma unroll
-      for (int k = 0; k < NB; ++k) { acc[k] = 0.f; acu[k] = 0.f; }
-      if (live) {
-        if (b0 > 0) fetch(j);
-        const XT* xb = xin + b0 * ldx;
+      for (int r = 0; r < R; ++r) { acc[r] = 0.f; acu[r] = 0.f; }
 #pragma unroll
-        for (int k = 0; k < PF; ++k)
-          if (u0 + k * US < units) {
-            ll_accum<FMT, NB, XT>(g[k], u0 + k * US, xb, ldx, nb, acc);
-            if constexpr (SWI != 0) ll_accum<FMT, NB, XT>(up[k], u0 + k * US, xb, ldx, nb, acu);
-          }
-        const uint8_t* w = row_of(j);
-#pragma unroll 4
-        for (int u = u0 + PF * US; u < units; u += US) {
-          LlRaw<FMT> r0, r1;
-          r0.load(w, u);
-          if constexpr (SWI != 0) r1.load(w + 64 * a.row_bytes, u);
-          ll_accum<FMT, NB, XT>(r0, u, xb, ldx, nb, acc);
-          if constexpr (SWI != 0) ll_accum<FMT, NB, XT>(r1, u, xb, ldx, nb, acu);
+      for (int k = 0; k < PF; ++k)
+        if (u0 + k * US < units) {
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+            if (j + r * step < n_out) {
+              ll_accum<FMT, 1, XT>(g[r][k], u0 + k * US, xin, ldx, 1, reinterpret_cast<float (&)[1]>(acc[r]));
+              if constexpr (SWI != 0) ll_accum<FMT, 1, XT>(up[r][k], u0 + k * US, xin, ldx, 1, reinterpret_cast<float (&)[1]>(acu[r]));
+            }
         }
-      }
-      if (b0 + NB >= a.B) fetch(j + gridDim.x * RPB);
+      if (j0 + ROWS * step < n_out) fetch(j + ROWS * step);
 #pragma unroll
-      for (int k = 0; k < NB; ++k) {
-        acc[k] = warp_sum(acc[k]);
-        if constexpr (SWI != 0) acu[k] = warp_sum(acu[k]);
+      for (int r = 0; r < R; ++r) {
+        acc[r] = warp_sum(acc[r]);
+        if constexpr (SWI != 0) acu[r] = warp_sum(acu[r]);
       }
       if constexpr (KS > 1) {
         if (lane == 0) {
 #pragma unroll
-          for (int k = 0; k < NB; ++k) { part[0][warp][k] = acc[k]; part[1][warp][k] = acu[k]; }
-        }
-        __syncthreads();
-        if (ks == 0) {
-#pragma unroll
-          for (int k = 0; k < NB; ++k) {
-            acc[k] = 0.f; acu[k] = 0.f;
-#pragma unroll
-            for (int s = 0; s < KS; ++s) { acc[k] += part[0][ric * KS + s][k]; acu[k] += part[1][ric * KS + s][k]; }
-          }
+          for (int r = 0; r < R; ++r) { part[0][warp][r] = acc[r]; part[1][warp][r] = acu[r]; }
         }
         __syncthreads();
       }
-      if (live && ks == 0 && lane == 0) {
+      // one lane a row
+      if (ks == 0 && lane < R && j + lane * step < n_out) {
+        float v = 0.f, u = 0.f;
+        if constexpr (KS > 1) {
+#pragma unroll
+          for (int s = 0; s < KS; ++s) { v += part[0][ric * KS + s][lane]; u += part[1][ric * KS + s][lane]; }
+        } else {
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+            if (lane == r) { v = acc[r]; u = acu[r]; }
+        }
+        store(0, j + lane * step, v, u);
+      }
+      if (KS > 1 && j0 + ROWS * step < n_out) __syncthreads();
+    } else {
+      const bool live = j < n_out;
+      for (int b0 = 0; b0 < a.B; b0 += NB) {
+        const int nb = min(NB, a.B - b0);
+        float acc[NB], acu[NB];
+#pragma unroll
+        for (int k = 0; k < NB; ++k) { acc[k] = 0.f; acu[k] = 0.f; }
+        if (live) {
+          if (b0 > 0) fetch(j);
+          const XT* xb = xin + b0 * ldx;
+#pragma unroll
+          for (int k = 0; k < PF; ++k)
+            if (u0 + k * US < units) {
+              ll_accum<FMT, NB, XT>(g[0][k], u0 + k * US, xb, ldx, nb, acc);
+              if constexpr (SWI != 0) ll_accum<FMT, NB, XT>(up[0][k], u0 + k * US, xb, ldx, nb, acu);
+            }
+          const uint8_t* w = row_of(j);
+#pragma unroll 4
+          for (int u = u0 + PF * US; u < units; u += US) {
+            LlRaw<FMT> r0, r1;
+            r0.load(w, u);
+            if constexpr (SWI != 0) r1.load(w + 64 * a.row_bytes, u);
+            ll_accum<FMT, NB, XT>(r0, u, xb, ldx, nb, acc);
+            if constexpr (SWI != 0) ll_accum<FMT, NB, XT>(r1, u, xb, ldx, nb, acu);
+          }
+        }
+        if (b0 + NB >= a.B) fetch(j + step);
 #pragma unroll
         for (int k = 0; k < NB; ++k) {
-          if (k >= nb) continue;
-          float v = SWI ? ll_silu(acc[k]) * acu[k] : acc[k];
-          if (a.softcap > 0.f) v = a.softcap * tanhf(v / a.softcap);
-          if (a.n1 > 0 && j >= a.n1) {
-            v = fmaxf(v, 0.f);
-            reinterpret_cast<XT*>(a.out2)[(long long)(b0 + k) * a.ldo2 + j - a.n1] = Cvt<XT>::from_f(v * v);
-          } else if (a.out_f32) reinterpret_cast<float*>(a.out)[(long long)(b0 + k) * a.ldo + j] = v;
-          else reinterpret_cast<XT*>(a.out)[(long long)(b0 + k) * a.ldo + j] = Cvt<XT>::from_f(v);
+          acc[k] = warp_sum(acc[k]);
+          if constexpr (SWI != 0) acu[k] = warp_sum(acu[k]);
+        }
+        if constexpr (KS > 1) {
+          if (lane == 0) {
+#pragma unroll
+            for (int k = 0; k < NB; ++k) { part[0][warp][k] = acc[k]; part[1][warp][k] = acu[k]; }
+          }
+          __syncthreads();
+          if (ks == 0) {
+#pragma unroll
+            for (int k = 0; k < NB; ++k) {
+              acc[k] = 0.f; acu[k] = 0.f;
+#pragma unroll
+              for (int s = 0; s < KS; ++s) { acc[k] += part[0][ric * KS + s][k]; acu[k] += part[1][ric * KS + s][k]; }
+            }
+          }
+          __syncthreads();
+        }
+        if (live && ks == 0 && lane == 0) {
+#pragma unroll
+          for (int k = 0; k < NB; ++k)
+            if (k < nb) store(b0 + k, j, acc[k], acu[k]);
         }
       }
     }
@@ -383,19 +447,35 @@ static int ll_gemv_go(LlGemv a, cudaStream_t st) {
   // warps per row: enough of them to keep loads in flight on every SM, more for long rows
   const int units = a.K >> 3;
   const int ks = (n_out < 148 * 16 || units > 512) ? 4 : (n_out < 148 * 64 || units > 256) ? 2 : 1;
-  // blocks: what is resident at once, and then so many that all of them make the same number of trips
-#define GO(NB, KS)                                                                                                                 \
+  // blocks: what is resident at once, and then so many that all of them make the same number of trips (of rpt rows)
+#define GO(NB, KS, R, UPL, KEEP)                                                                                                   \
   do {                                                                                                                             \
-    auto kern = ll_gemv_kernel<FMT, XT, PRO, SWI, NB, KS>;                                                                         \
+    auto kern = ll_gemv_kernel<FMT, XT, PRO, SWI, NB, KS, R, UPL, KEEP>;                                                           \
     static int occ = 0;                                                                                                            \
     if (!occ && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, LV_THREADS, 16 * 1024) != cudaSuccess || occ < 1)) occ = 2; \
-    const int groups = (n_out + LV_WARPS / KS - 1) / (LV_WARPS / KS), trips = (groups + 148 * occ - 1) / (148 * occ);              \
+    const int rpt = R ? R : 1, groups = (n_out + LV_WARPS / KS - 1) / (LV_WARPS / KS);                                             \
+    const int trips = (groups + 148 * occ * rpt - 1) / (148 * occ * rpt) * rpt;                                                    \
     GB_PDL_LAUNCH_SMEM(kern, dim3((groups + trips - 1) / trips), dim3(LV_THREADS), smem, st, a);                                   \
   } while (0)
-#define GOK(NB) do { if (ks == 4) GO(NB, 4); else if (ks == 2) GO(NB, 2); else GO(NB, 1); } while (0)
-  if (a.B == 1) GOK(1);
-  else GOK(4);
-#undef GOK
+  if constexpr (FMT == GB_W_BF16) if (a.B == 1) {
+    // rows of up to 2 or 4 units a lane: rows x units x matrices are 8 units, 32 registers.  Longer rows are few blocks' work and
+    // mostly loads: side by side they would leave one block an SM.  The prologues that keep the row take four numbers a thread up to 1024.
+    const int upl = (units + 32 * ks - 1) / (32 * ks);
+    const bool small = a.d <= 4 * LV_THREADS || (PRO != 1 && PRO != 5);
+#define ROWS_OF(KS)                                                                                                                \
+    do {                                                                                                                           \
+      if (upl <= 2 && small) { GO(1, KS, (SWI ? 2 : 4), 2, 4); return gb_launch_rc(); }                                             \
+      if (upl <= 4 && small) { GO(1, KS, (SWI ? 1 : 2), 4, 4); return gb_launch_rc(); }                                             \
+      if constexpr (PRO == 1 || PRO == 5)                                                                                          \
+        if (upl <= 4) { GO(1, KS, (SWI ? 1 : 2), 4, 16); return gb_launch_rc(); }                                                  \
+    } while (0)
+    if (ks == 4) ROWS_OF(4); else if (ks == 2) ROWS_OF(2); else ROWS_OF(1);
+#undef ROWS_OF
+  }
+#define GOB(NB) do { if (ks == 4) GO(NB, 4, 0, 1, 16); else if (ks == 2) GO(NB, 2, 0, 1, 16); else GO(NB, 1, 0, 1, 16); } while (0)
+  if (a.B == 1) GOB(1);
+  else GOB(4);
+#undef GOB
 #undef GO
   return gb_launch_rc();
 }

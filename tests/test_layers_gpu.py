@@ -431,6 +431,43 @@ def test_gemv_prologues(dtype, B, d, N):
         near(run(N, out, prologue=2, y16=x16, ldy16=Kp, z16=z, ldz=d, w1=w1, parts=parts), v @ W[:N].t())
 
 
+@pytest.mark.parametrize("d, N", [(40, 9), (512, 4387), (520, 40011), (1024, 9501), (1032, 2501), (2048, 19001), (4096, 9473), (4104, 2399)])
+def test_gemv_rows_side_by_side(d, N):
+    """One sequence: rows that a warp takes together, at the ends of a row's units and of the rows of a block's trips."""
+    from ghassan_b200.ops import layers as K
+    g = torch.Generator(device="cuda").manual_seed(d + N)
+    E = (N + 63) // 64 * 64
+    w = (torch.randn(2 * E, d, generator=g, device="cuda") * d ** -0.5).to(BF)
+    x = torch.randn(1, d, generator=g, device="cuda").to(BF)
+    x32 = x.float()
+    W, xd = w.double(), x.double()
+    for pro in (0, 1, 5):
+        ones = torch.ones(d, device="cuda")
+        for swi in (0, 1) if pro < 5 else (0,):
+            a = K.GemvArgs()
+            a.W, a.fmt, a.N, a.K, a.B, a.dtype, a.d, a.eps, a.prologue, a.swiglu = w.data_ptr(), K.W_FMT[BF], 2 * E if swi else N, d, 1, K.DTYPE[BF], d, 1e-4, pro, swi
+            out = torch.full((1, E + 8), 7.0, dtype=BF if swi else F32, device="cuda")
+            a.out, a.ldo, a.out_f32 = out.data_ptr(), E + 8, int(not swi)
+            v = xd
+            if pro == 0:
+                a.x16, a.ldx = x.data_ptr(), d
+            else:
+                a.x = x32.data_ptr()
+                if pro == 5:
+                    a.norm_mode, a.w1, a.alpha = K.NORM["rms"], ones.data_ptr(), 1.0
+                    v = xd / torch.sqrt((xd * xd).mean() + 1e-4)
+            K.gemv(a)
+            n = E if swi else N
+            j = torch.arange(n, device="cuda")
+            y = v @ (W[(j // 64) * 128 + j % 64] if swi else W[:N]).t()
+            if swi:
+                y = y * torch.sigmoid(y) * (v @ W[(j // 64) * 128 + j % 64 + 64].t())
+            # prologue 5 rounds the vector to 16 bits, SwiGLU the result; sums are of 32 bits
+            tol = 2.0 ** -6 if pro == 5 or swi else 1e-5
+            assert float((out[:, :n].double() - y).abs().max()) < tol * float(y.abs().max())
+            assert bool((out[:, n:] == 7.0).all())
+
+
 # ------------------------------------------------------------------------------------------------ long decoding, slots, batches
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_long_decoding_through_wrapping_rings(dtype):
