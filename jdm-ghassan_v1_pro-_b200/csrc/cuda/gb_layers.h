@@ -180,7 +180,8 @@ int gb_ll_ssd_ok(const gb_ll_mamba_args* a);                        // 0 when th
 long long gb_ll_ssd_ws_floats(int B, int H, int P, int Ns, int n, int segments);
 int gb_ll_ssd(const gb_ll_mamba_args* a, int segments, cudaStream_t st);
 int gb_ll_gated_norm(const gb_ll_mamba_args* a, cudaStream_t st);
-int gb_ll_mamba_step(const gb_ll_mamba_args* a, cudaStream_t st);   // n == 1: convolution + recurrence in one kernel
+int gb_ll_mamba_step(const gb_ll_mamba_args* a, cudaStream_t st);   // n == 1: convolution + recurrence in one kernel; of what it reads
+                                                                    // the launch directly ahead may write proj alone
 
 #ifdef __cplusplus
 }

@@ -172,6 +172,10 @@ struct LlState {
       s[4 * r] = v.x; s[4 * r + 1] = v.y; s[4 * r + 2] = v.z; s[4 * r + 3] = v.w;
     }
   }
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int r = 0; r < NR; ++r) s[r] = 0.f;
+  }
   __device__ __forceinline__ void store(float* row, int Ns, int slice) const {
 #pragma unroll
     for (int r = 0; r < NR / 4; ++r) {
@@ -253,9 +257,15 @@ __global__ void __launch_bounds__(256) ll_scan_kernel(const __grid_constant__ gb
 
 // One token: convolution of this head's channels and of its group's B and C, then the recurrence.  The carried inputs
 // are a ring of `taps` rows, so the new row never overwrites one that another block still reads.
-template <typename T, int NR>
+//
+// Between two tokens the weights of the whole model pass through L2, so the state, the last inputs of the convolution and its weights come
+// from DRAM.  Only the input product's rows are the launch ahead's, so all the rest is loaded before the wait for it: the position, the
+// state, and with up to four taps (TAPS4) the inputs and weights of the convolution; past the wait a block reads a few of the product's
+// values a thread, side by side.  In the chain of a token (32 heads of 64 x 128) 6.2 -> 2.5 us; all of it read behind the wait, with only
+// prefetches ahead of it, a request of 64 tokens and nine such layers took 21.0 ms, now 18.4.
+template <typename T, int NR, bool TAPS4>
 __global__ void __launch_bounds__(256) ll_mamba_step_kernel(const __grid_constant__ gb_ll_mamba_args a) {
-  constexpr int NW = NR * 8;
+  constexpr int NW = NR * 8, NCH = 32 + 2 * NW, PER = (NCH + 255) / 256;
   __shared__ __align__(16) float sB[NW], sC[NW];
   __shared__ float sX[32];
   const int h = blockIdx.y, b = blockIdx.z, pt = blockIdx.x * 32, rep = a.H / a.G, g = h / rep;
@@ -266,47 +276,74 @@ __global__ void __launch_bounds__(256) ll_mamba_step_kernel(const __grid_constan
   const bool live = p < a.P;
   float* srow = a.ssm + (((long long)b * a.H + h) * a.P + (live ? p : 0)) * a.Ns;
   auto channel = [&](int i) {                 // of the convolution: this block's 32 of x, then the group's B and C
+    if (i >= NCH) return -1;
     if (i < 32) return pt + i < a.P ? h * a.P + pt + i : -1;
     const int e = (i - 32) % NW, which = (i - 32) / NW;
     return e < a.N ? n + which * gn + g * a.N + e : -1;
   };
-  // Between two tokens the weights of the whole model pass through L2, so the state, the last inputs of the convolution and its
-  // weights come from DRAM.  They are asked of L2 before the wait for the input product (a hint: what the kernels ahead still
-  // write is read after the wait): 13.4 -> 12.1 us in the chain of a token (32 heads of 64 x 128).
-  if (live && slice * 32 < a.Ns) asm volatile("prefetch.global.L2 [%0];" ::"l"(srow + slice * 32));
-  for (int i = tid; i < 32 + 2 * NW; i += 256) {
-    const int c = channel(i);
-    if (c < 0) continue;
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(a.conv_w + (long long)c * a.taps));
-    if ((c & 31) == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.conv_b + c));
-    if ((c & 63) == 0)
-      for (int t = 0; t < a.taps; ++t) asm volatile("prefetch.global.L2 [%0];" ::"l"(ring + (long long)t * C + c));
-  }
-  pdl_wait();
-  const int pos = a.st[b].abs_pos;
+  const int pos = *reinterpret_cast<const volatile int*>(&a.st[b].abs_pos);
   LlState<NR> S;
-  S.load(srow, a.Ns, slice, pos == 0 || !live);
+  S.load(srow, a.Ns, slice, !live);
+  int ch[PER];
+  float bias[PER], cw[PER][4];
+  T last[PER][3];
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    ch[q] = channel(tid + 256 * q);
+    if (TAPS4 && ch[q] >= 0) {
+      bias[q] = a.conv_b[ch[q]];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) cw[q][k] = k < a.taps ? a.conv_w[(long long)ch[q] * a.taps + a.taps - 1 - k] : 0.f;
+    }
+  }
+  const int at = pos % a.taps;                // row of this position; k positions ago: at - k, round the ring
+  if constexpr (TAPS4) {
+#pragma unroll
+    for (int q = 0; q < PER; ++q)
+#pragma unroll
+      for (int k = 1; k < 4; ++k)
+        if (ch[q] >= 0 && k < a.taps && pos - k >= 0)
+          last[q][k - 1] = __ldcg(ring + (long long)(at - k < 0 ? at - k + a.taps : at - k) * C + ch[q]);
+  }
+  const float dt_bias = a.dt_bias[h], A = -expf(a.A_log[h]), D = a.D[h];
+  pdl_wait();
+  T cur[PER], z{};
+#pragma unroll
+  for (int q = 0; q < PER; ++q)
+    if (ch[q] >= 0) cur[q] = row[n + ch[q]];
+  const T dt_in = row[2 * n + 2 * gn + h];
+  if (a.gated && live && slice == 0) z = row[h * a.P + p];
   const bool owner = (h % rep) == 0 && blockIdx.x == 0;      // writes the group's B and C inputs
-  for (int i = tid; i < 32 + 2 * NW; i += 256) {
-    const int c = channel(i);
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const int i = tid + 256 * q, c = ch[q];
+    if (i >= NCH) break;
     float v = 0.f;
     if (c >= 0) {
-      const T cur = row[n + c];
-      float s = a.conv_b[c] + a.conv_w[(long long)c * a.taps + a.taps - 1] * Cvt<T>::to_f(cur);
-      for (int k = 1; k < a.taps; ++k)
-        if (pos - k >= 0) s += a.conv_w[(long long)c * a.taps + a.taps - 1 - k] * Cvt<T>::to_f(ring[(long long)((pos - k) % a.taps) * C + c]);
+      float s;
+      if constexpr (TAPS4) {
+        s = bias[q] + cw[q][0] * Cvt<T>::to_f(cur[q]);
+#pragma unroll
+        for (int k = 1; k < 4; ++k)
+          if (k < a.taps && pos - k >= 0) s += cw[q][k] * Cvt<T>::to_f(last[q][k - 1]);
+      } else {
+        s = a.conv_b[c] + a.conv_w[(long long)c * a.taps + a.taps - 1] * Cvt<T>::to_f(cur[q]);
+        for (int k = 1; k < a.taps; ++k)
+          if (pos - k >= 0) s += a.conv_w[(long long)c * a.taps + a.taps - 1 - k] * Cvt<T>::to_f(ring[(long long)((pos - k) % a.taps) * C + c]);
+      }
       v = Cvt<T>::to_f(Cvt<T>::from_f(ll_silu_t<T>(s)));
-      if (i < 32 || owner) ring[(long long)(pos % a.taps) * C + c] = cur;
+      if (i < 32 || owner) ring[(long long)at * C + c] = cur[q];
     }
     if (i < 32) sX[i] = v;
     else if (i < 32 + NW) sB[i - 32] = v;
     else sC[i - 32 - NW] = v;
   }
-  const float dt = ll_softplus(Cvt<T>::to_f(row[2 * n + 2 * gn + h]) + a.dt_bias[h]);
-  const float decay = expf(-expf(a.A_log[h]) * dt);
+  const float dt = ll_softplus(Cvt<T>::to_f(dt_in) + dt_bias);
+  const float decay = expf(A * dt);
+  if (pos == 0) S.clear();                    // whatever the slot held before
   __syncthreads();
   const float x = sX[pr];
-  const float y = ll_sum8(S.step(decay, dt * x, sB, sC, slice)) + a.D[h] * x;
+  const float y = ll_sum8(S.step(decay, dt * x, sB, sC, slice)) + D * x;
   if (live) S.store(srow, a.Ns, slice);
   if (a.gated == nullptr) {
     if (live && slice == 0) reinterpret_cast<T*>(a.y)[b * a.ld_y + h * a.P + p] = Cvt<T>::from_f(y);
@@ -316,7 +353,7 @@ __global__ void __launch_bounds__(256) ll_mamba_step_kernel(const __grid_constan
   __shared__ float s_sq[8];
   float v = 0.f;
   if (live && slice == 0) {
-    v = Cvt<T>::to_f(Cvt<T>::from_f(y)) * ll_silu_t<T>(Cvt<T>::to_f(row[h * a.P + p]));
+    v = Cvt<T>::to_f(Cvt<T>::from_f(y)) * ll_silu_t<T>(Cvt<T>::to_f(z));
     a.gated[(long long)b * n + h * a.P + p] = v;
   }
   v = warp_sum(v * v);
@@ -421,7 +458,8 @@ static bool ll_vec_ok(const gb_ll_mamba_args& a) {
 template <typename T>
 static int ll_scan_go(const gb_ll_mamba_args& a, bool step, cudaStream_t st) {
   const dim3 grid((a.P + 31) / 32, a.H, a.B);
-#define GO(NR) do { if (step) GB_PDL_LAUNCH((ll_mamba_step_kernel<T, NR>), grid, dim3(256), st, a); \
+#define GO(NR) do { if (step && a.taps <= 4) GB_PDL_LAUNCH((ll_mamba_step_kernel<T, NR, true>), grid, dim3(256), st, a); \
+                    else if (step) GB_PDL_LAUNCH((ll_mamba_step_kernel<T, NR, false>), grid, dim3(256), st, a); \
                     else GB_PDL_LAUNCH((ll_scan_kernel<T, NR>), grid, dim3(256), st, a); } while (0)
   if (a.N <= 64) GO(8);
   else if (a.N <= 128) GO(16);

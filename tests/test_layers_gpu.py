@@ -321,6 +321,33 @@ def test_one_token_step_equals_the_portion_kernels(dtype):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("taps, P, N", [(1, 32, 64), (2, 33, 60), (3, 64, 128), (4, 20, 132), (5, 40, 128), (9, 64, 256)])
+def test_one_token_step_loads_its_history_early(dtype, taps, P, N):
+    """Convolutions inside and beyond the registers, every size of the state, a slot that is used again with old contents."""
+    from ghassan_b200.ops import layers as K
+    out = {}
+    for step in (False, True):
+        raw, m, mem, state = _one_layer(C.mamba(4, P, N, 2, taps, 1), dtype=dtype)
+        mem.layers[0].ssm.fill_(float("nan"))
+        mem.layers[0].conv.fill_(float("nan"))
+        src = m.buf("proj", (m.weights[0].w_in.shape[0] + 7) // 8 * 8)
+        _mamba_inputs(m, 24, taps)
+        whole, ys = src[:24].clone(), []
+        for t in range(24):
+            src[:1] = whole[t:t + 1]
+            a = m.mamba_args(0, mem.layers[0], state, 0, 1, 1)
+            if step:
+                K.mamba_step(a)
+            else:
+                K.conv(a)
+                K.scan(a)
+            ys.append(m.buf("ssm_y", 4 * P)[:1].float().clone())
+            state[:, 0] += 1
+        out[step] = torch.cat(ys)
+    assert float((out[True] - out[False]).abs().max()) <= 1e-6 * float(out[False].abs().max())
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("parts, P", [(1, 20), (2, 50), (6, 30), (12, 36), (1, 1500)])
 def test_gated_group_norm(dtype, parts, P):
     from ghassan_b200.ops import layers as K
