@@ -751,11 +751,7 @@ __global__ void __launch_bounds__(256, 4) moe_router_bwd_kernel(const gb_moe_arg
 }
 
 // The same for at most 8 experts, in two kernels.  moe_router_dlogit_kernel is the router-logit part above (one thread
-// per token, a few hundred bytes); moe_router_dx_kernel then streams the input gradient with the router rows held in
-// registers: a lane owns 8 columns of all (<= 8) experts for the life of the block, 4 token groups x 96 lanes per
-// block, blocks walk the tokens with a grid stride.  Per token a lane issues its slot rows' 16-byte loads and two
-// broadcast loads of the logit gradients; the 24 KB of router rows are no longer re-read from L1 for every token
-// (sixteen 16-byte loads per 8 columns, three quarters of the one-kernel form's load instructions).
+// per token, a few hundred bytes); moe_router_dx_kernel then streams the input gradient.
 __global__ void __launch_bounds__(256) moe_router_dlogit_kernel(const gb_moe_args a) {
   pdl_wait();
   // one thread per token: with at most 8 experts everything of a token fits a thread's registers, and its dozen
@@ -808,86 +804,68 @@ __global__ void __launch_bounds__(256) moe_router_dlogit_kernel(const gb_moe_arg
     }
 }
 
-constexpr int RD_LANES = 96, RD_GROUPS = 4;
+// A warp takes RD_TOKENS tokens and 256 columns, eight a lane.  The tokens' slot positions and logit gradients are one load each, spread
+// by shuffles, all of their slot rows are in flight together, and the block's columns of the router rows are in shared memory, read once for
+// the warp's tokens.  Only the logit gradients are the launch ahead's, so the rest is asked for before the wait for it.  Bound by bytes
+// (NS + 1 rows of 16 bits a token): 32768 tokens of 768, 3 slots, bytes 31 us: 66.7 -> 40.4 us; the form with the router rows in registers held
+// one block of 12 warps an SM, each with one token ahead.
+constexpr int RD_TOKENS = 4, RD_WARPS = 8;
 template <typename T, int NS>       // NS = slots per token (top_k + shared), so that the row buffers are exactly that long
-__global__ void __launch_bounds__(RD_LANES * RD_GROUPS) moe_router_dx_kernel(const gb_moe_args a) {
+__global__ void __launch_bounds__(RD_WARPS * 32) moe_router_dx_kernel(const gb_moe_args a) {
+  __shared__ __align__(16) float s_w[8][256];
+  const int lane = threadIdx.x & 31, ne = a.ne, d = a.d, c0 = blockIdx.y * 256 + lane * 8;
+  const int t0 = (blockIdx.x * RD_WARPS + (threadIdx.x >> 5)) * RD_TOKENS, nt = min(RD_TOKENS, a.n_tok - t0);
+  const bool live = c0 < d;                       // d % 8 == 0: a live lane has all 8 columns
+  const int my_pos = lane < nt * NS ? a.slot_pos[(size_t)t0 * NS + lane] : 0;
+  for (int i = threadIdx.x; i < ne * 64; i += RD_WARPS * 32) {
+    const int e = i >> 6, c = (i & 63) * 4;
+    if (blockIdx.y * 256 + c < d) *reinterpret_cast<float4*>(&s_w[e][c]) = *reinterpret_cast<const float4*>(a.router_w + (size_t)e * d + blockIdx.y * 256 + c);
+  }
+  const T* dxp = reinterpret_cast<const T*>(a.dx_perm) + c0;
+  uint4 q[RD_TOKENS][NS];
+#pragma unroll
+  for (int u = 0; u < RD_TOKENS; ++u)
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      const int pos = __shfl_sync(0xffffffffu, my_pos, u * NS + s);
+      if (live && u < nt) q[u][s] = *reinterpret_cast<const uint4*>(dxp + (size_t)pos * d);
+    }
   pdl_wait();
-  const int g = threadIdx.x / RD_LANES, l = threadIdx.x - g * RD_LANES;
-  const int c0 = (blockIdx.y * RD_LANES + l) * 8;
-  const int ne = a.ne, d = a.d;
-  constexpr int S = NS;
-  if (c0 >= d) return;                            // no block-wide barrier below
-  float w[8][8];                                  // router rows of this lane's 8 columns (zero beyond ne)
+  const int te = lane >> 3, e = lane & 7;         // this lane's token and expert of the logit gradients
+  const float my_dl = te < nt && e < ne ? a.part[(size_t)(t0 + te) * ne + e] : 0.f;
+  __syncthreads();
+  float acc[RD_TOKENS][8];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    float4 w0 = make_float4(0.f, 0.f, 0.f, 0.f), w1 = w0;
-    if (e < ne) {
-      w0 = *reinterpret_cast<const float4*>(a.router_w + (size_t)e * d + c0);
-      w1 = *reinterpret_cast<const float4*>(a.router_w + (size_t)e * d + c0 + 4);
+  for (int u = 0; u < RD_TOKENS; ++u) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[u][j] = 0.f;
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      const float2 v0 = Cvt<T>::unpack2(q[u][s].x), v1 = Cvt<T>::unpack2(q[u][s].y), v2 = Cvt<T>::unpack2(q[u][s].z), v3 = Cvt<T>::unpack2(q[u][s].w);
+      acc[u][0] += v0.x; acc[u][1] += v0.y; acc[u][2] += v1.x; acc[u][3] += v1.y;
+      acc[u][4] += v2.x; acc[u][5] += v2.y; acc[u][6] += v3.x; acc[u][7] += v3.y;
     }
-    w[e][0] = w0.x; w[e][1] = w0.y; w[e][2] = w0.z; w[e][3] = w0.w;
-    w[e][4] = w1.x; w[e][5] = w1.y; w[e][6] = w1.z; w[e][7] = w1.w;
   }
-  const T* dxp = reinterpret_cast<const T*>(a.dx_perm);
-  T* dx = reinterpret_cast<T*>(a.dx16);
-  const bool vec = ne == 8;
-  // Two tokens in flight: a token's slot rows depend on its slot positions, a chain of two global loads.  The positions
-  // are fetched two tokens ahead and the rows one token ahead, so that every trip waits for one load, not two.
-  const int stride = gridDim.x * RD_GROUPS;
-  auto load_pos = [&](int t, int (&pos)[NS]) {
 #pragma unroll
-    for (int s = 0; s < NS; ++s)
-      pos[s] = t < a.n_tok ? a.slot_pos[(size_t)t * S + s] : 0;
-  };
-  auto load_rows = [&](int t, const int (&pos)[NS], uint4 (&q)[NS], float (&dl)[8]) {
-    if (t >= a.n_tok) return;
+  for (int x = 0; x < 8; ++x) {
+    if (x >= ne) break;
+    const float4 w0 = *reinterpret_cast<const float4*>(&s_w[x][lane * 8]), w1 = *reinterpret_cast<const float4*>(&s_w[x][lane * 8 + 4]);
+    const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
-    for (int s = 0; s < NS; ++s)
-      q[s] = *reinterpret_cast<const uint4*>(dxp + (size_t)pos[s] * d + c0);
-    if (vec) {
-      const float4 a4 = *reinterpret_cast<const float4*>(a.part + (size_t)t * 8);
-      const float4 b4 = *reinterpret_cast<const float4*>(a.part + (size_t)t * 8 + 4);
-      dl[0] = a4.x; dl[1] = a4.y; dl[2] = a4.z; dl[3] = a4.w; dl[4] = b4.x; dl[5] = b4.y; dl[6] = b4.z; dl[7] = b4.w;
-    } else {
+    for (int u = 0; u < RD_TOKENS; ++u) {
+      const float dl = __shfl_sync(0xffffffffu, my_dl, u * 8 + x);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) dl[e] = e < ne ? a.part[(size_t)t * ne + e] : 0.f;
+      for (int j = 0; j < 8; ++j) acc[u][j] += dl * w[j];
     }
-  };
-  int t0 = blockIdx.x * RD_GROUPS + g;
-  int pos0[NS], pos1[NS];
-  uint4 q0[NS], q1[NS];
-  float dl0[8], dl1[8];
-  load_pos(t0, pos0);
-  load_pos(t0 + stride, pos1);
-  load_rows(t0, pos0, q0, dl0);
-  for (; t0 < a.n_tok; t0 += stride) {
-    load_rows(t0 + stride, pos1, q1, dl1);          // the next token's rows
-    load_pos(t0 + 2 * stride, pos0);                // positions of the one after (pos0 is free: its rows are loaded)
-    float acc[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-#pragma unroll
-    for (int s = 0; s < NS; ++s)
-      {
-        const float2 v0 = Cvt<T>::unpack2(q0[s].x), v1 = Cvt<T>::unpack2(q0[s].y), v2 = Cvt<T>::unpack2(q0[s].z),
-                     v3 = Cvt<T>::unpack2(q0[s].w);
-        acc[0] += v0.x; acc[1] += v0.y; acc[2] += v1.x; acc[3] += v1.y; acc[4] += v2.x; acc[5] += v2.y; acc[6] += v3.x; acc[7] += v3.y;
-      }
-#pragma unroll
-    for (int e = 0; e < 8; ++e)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] += dl0[e] * w[e][j];
-    uint4 o;
-    o.x = Cvt<T>::pack2(acc[0], acc[1]); o.y = Cvt<T>::pack2(acc[2], acc[3]);
-    o.z = Cvt<T>::pack2(acc[4], acc[5]); o.w = Cvt<T>::pack2(acc[6], acc[7]);
-    *reinterpret_cast<uint4*>(dx + (size_t)t0 * d + c0) = o;
-    // hand over: next token's rows become current, the freshly loaded positions become next
-#pragma unroll
-    for (int s = 0; s < NS; ++s)
-      { q0[s] = q1[s]; const int tmp = pos0[s]; pos0[s] = pos1[s]; pos1[s] = tmp; }
-#pragma unroll
-    for (int e = 0; e < 8; ++e) dl0[e] = dl1[e];
   }
+#pragma unroll
+  for (int u = 0; u < RD_TOKENS; ++u)
+    if (live && u < nt) {
+      uint4 o;
+      o.x = Cvt<T>::pack2(acc[u][0], acc[u][1]); o.y = Cvt<T>::pack2(acc[u][2], acc[u][3]);
+      o.z = Cvt<T>::pack2(acc[u][4], acc[u][5]); o.w = Cvt<T>::pack2(acc[u][6], acc[u][7]);
+      *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.dx16) + (size_t)(t0 + u) * d + c0) = o;
+    }
 }
 
 // d_router_w[e, c] += sum_t dlogit[t, e] * x16[t, c], in a fixed order (deterministic).
@@ -1026,12 +1004,12 @@ using namespace gb;
 template <typename T>
 static void launch_router_dx(const gb_moe_args& a, int n_slots, dim3 grid, cudaStream_t st) {
   switch (n_slots) {
-    case 1: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 1>), dim3(grid), dim3(RD_LANES * RD_GROUPS), 0, st, a); break;
-    case 2: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 2>), dim3(grid), dim3(RD_LANES * RD_GROUPS), 0, st, a); break;
-    case 3: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 3>), dim3(grid), dim3(RD_LANES * RD_GROUPS), 0, st, a); break;
-    case 4: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 4>), dim3(grid), dim3(RD_LANES * RD_GROUPS), 0, st, a); break;
-    case 5: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 5>), dim3(grid), dim3(RD_LANES * RD_GROUPS), 0, st, a); break;
-    default: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 6>), dim3(grid), dim3(RD_LANES * RD_GROUPS), 0, st, a); break;
+    case 1: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 1>), dim3(grid), dim3(RD_WARPS * 32), 0, st, a); break;
+    case 2: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 2>), dim3(grid), dim3(RD_WARPS * 32), 0, st, a); break;
+    case 3: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 3>), dim3(grid), dim3(RD_WARPS * 32), 0, st, a); break;
+    case 4: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 4>), dim3(grid), dim3(RD_WARPS * 32), 0, st, a); break;
+    case 5: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 5>), dim3(grid), dim3(RD_WARPS * 32), 0, st, a); break;
+    default: GB_PDL_LAUNCH_SMEM((moe_router_dx_kernel<T, 6>), dim3(grid), dim3(RD_WARPS * 32), 0, st, a); break;
   }
 }
 
@@ -1162,13 +1140,10 @@ extern "C" int gb_moe_router_bwd(const gb_moe_args* a, cudaStream_t st) {
   if (chunks > GB_ROUTER_WGRAD_CHUNKS) chunks = GB_ROUTER_WGRAD_CHUNKS;
   dim3 g2((a->d / 8 + RW_LANES - 1) / RW_LANES, chunks, (a->ne + 7) / 8);
   float* wout = chunks > 1 ? a->part2 : a->d_router_w;
-  // up to 8 experts: logit gradients first, then the input gradient with the router rows in registers
+  // up to 8 experts: logit gradients first, then the input gradient
   const int n_slots = a->top_k + (a->shared ? 1 : 0);
   const bool split = a->ne <= 8 && n_slots <= 6;
-  int sms = 0, dev = 0;
-  if (split && (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess))
-    return -10;
-  dim3 gdx(std::max(1, std::min(sms, (a->n_tok + RD_GROUPS - 1) / RD_GROUPS)), (a->d / 8 + RD_LANES - 1) / RD_LANES);   // one resident block per SM
+  const dim3 gdx((a->n_tok + RD_WARPS * RD_TOKENS - 1) / (RD_WARPS * RD_TOKENS), (a->d + 255) / 256);
   if (a->is_bf16) {
     if (split) {
       GB_PDL_LAUNCH_SMEM(moe_router_dlogit_kernel, dim3((a->n_tok + 255) / 256), dim3(256), 0, st, *a);

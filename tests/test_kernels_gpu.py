@@ -296,6 +296,28 @@ def test_moe_layer_forward_backward(aux, jit):
 
 
 @pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("n, d, ne, Kk, shared", [(1, 8, 2, 1, False), (3, 256, 8, 2, True), (37, 264, 5, 2, False), (130, 1000, 8, 3, True),
+                                                  (33, 768, 8, 4, True), (258, 512, 7, 5, True), (70, 128, 8, 1, True)])
+def test_router_input_gradient_of_token_groups(dt, n, d, ne, Kk, shared):
+    """Remainders of a warp's tokens and of its columns, fewer experts than eight, one to six slots."""
+    k = K()
+    x16, rw = rnd(n, d, seed=131).to(dt), rnd(ne, d, seed=132, scale=0.05)
+    ws = k.MoeWorkspace(n, d, ne, Kk, shared, dt, "cuda")
+    xp = torch.empty(ws.cap, d, dtype=dt, device="cuda")
+    k.moe_route_group(ws, x16, rw, None, xp, None)
+    gdot, dxp = rnd(n, Kk, seed=133), rnd(ws.cap, d, seed=134).to(dt)
+    dx16 = torch.full((n + 1, d), 7.0, dtype=dt, device="cuda")
+    part = torch.empty(n, ne, device="cuda")
+    k.moe_router_bwd(ws, x16, rw, gdot, dxp, dx16, torch.zeros(ne, d, device="cuda"), part)
+    S = Kk + int(shared)
+    want = dxp.double()[ws.slot_pos[:n * S].view(-1).long()].view(n, S, d).sum(1) + part.double() @ rw.double()
+    # sums of at most 14 terms in 32 bits, rounded to 16 bits once
+    tol = 2.0 ** (-8 if dt == torch.bfloat16 else -11) + 1e-5
+    assert bool(((dx16[:n].double() - want).abs() <= tol * want.abs() + 1e-5).all())
+    assert bool((dx16[n] == 7.0).all())
+
+
+@pytest.mark.parametrize("dt", DT)
 @pytest.mark.parametrize("V,z", [(32000, 1e-4), (600, 0.0), (1003, 1e-3)])
 def test_softmax_ce(dt, V, z):
     k = K()
