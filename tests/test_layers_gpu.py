@@ -348,6 +348,23 @@ def test_one_token_step_loads_its_history_early(dtype, taps, P, N):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("d", [1024, 1028, 2048, 3068, 3072, 3076, 5000])
+def test_postnorm_of_long_rows(dtype, d):
+    """Rows of a block: what its registers hold, and beyond; the result may take the residual's place."""
+    from ghassan_b200.ops import layers as K
+    rows, ld = 5, d + 12
+    g = torch.Generator(device="cuda").manual_seed(d)
+    y, x = (torch.randn(rows, n, generator=g, device="cuda") for n in (ld, d))
+    w = 1 + 0.1 * torch.randn(d, generator=g, device="cuda")
+    v = y[:, :d].double()
+    want = x.double() + v / torch.sqrt((v * v).mean(1, keepdim=True) + 1e-4) * w.double()
+    x16 = torch.full((rows, ld), 7.0, dtype=dtype, device="cuda")
+    K.postnorm(y, x, w, 1e-4, x, x16, rows, d)
+    assert float((x.double() - want).abs().max()) < 3e-6 * float(want.abs().max())
+    assert torch.equal(x16[:, :d], x.to(dtype)) and float(x16[:, d:].float().abs().sum()) == 0.0
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("parts, P", [(1, 20), (2, 50), (6, 30), (12, 36), (1, 1500)])
 def test_gated_group_norm(dtype, parts, P):
     from ghassan_b200.ops import layers as K
