@@ -220,6 +220,26 @@ def test_pair_dense(dtype, out_dtype, M, N, K):
     assert torch.equal(out, out2)
 
 
+@pytest.mark.parametrize("M,N,K", [(2305, 1000, 1024), (9473, 136, 1032), (300, 4616, 2048), (1500, 1544, 1090), (1280, 2048, 1024)])
+def test_one_round_of_pairs_in_every_form(M, N, K):
+    """38 to 59 tiles go to the two-CTA kernel: orders, types, pitches and addends that the one-CTA kernel takes there."""
+    G, L = _ops()
+    assert 38 <= G.pair_tiles(M, N) < 60
+    Mp, Kp = (M + 7) // 8 * 8, (K + 7) // 8 * 8
+    for a_mn in (False, True):
+        for b_mn in (False, True):
+            A, B = _rand(Kp if a_mn else M, Mp if a_mn else Kp, seed=5), _rand(Kp if b_mn else N, N if b_mn else Kp, seed=6)
+            a, b = (A[:K, :M] if a_mn else A[:, :K]), (B[:K, :N] if b_mn else B[:, :K])
+            ref = (a.t() if a_mn else a).float() @ (b if b_mn else b.t()).float()
+            for dt, pitch, add in ((torch.float16, N, 0), (torch.float16, N + 3, 0), (torch.float32, N, 0), (torch.float32, N, N), (torch.float32, N + 1, N + 1)):
+                out = torch.zeros(M, pitch, dtype=dt, device="cuda")[:, :N]
+                res = _rand(M, add, dtype=torch.float32, seed=7)[:, :N] if add else None
+                G.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=out, addend=res)
+                rel, ok = _close(out, ref if res is None else ref + res)
+                assert ok, (a_mn, b_mn, dt, pitch, add, rel)
+    L.check_status(what="one round of pairs")
+
+
 @pytest.mark.parametrize("a_mn,b_mn", [(False, True), (True, False), (True, True)])
 def test_pair_operand_majors(a_mn, b_mn):
     G, L = _ops()
