@@ -70,7 +70,7 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   return t;
 }
 
-// ------------------------------------------------------------------------------------------------ grid barrier
+// ------------------------------------------------------------------------------------------------ grid barrier, once a step
 // Arrivals are counted in sync[0], which only ever grows; barrier k of a launch opens at base + k * grid, where base
 // (sync[1]) is the count the previous launch left behind.
 struct GridBar {
@@ -412,7 +412,7 @@ __device__ __forceinline__ void run_phase(const Phase& ph, const Plan& pl, const
 // The layer phases do not pull their rows through registers: lane 0 of a warp issues one bulk asynchronous copy per
 // contiguous run of super-units of ALL the warp's work in the phase into the warp's own slice of shared memory (no
 // other warp touches it), signalled on the warp's own mbarriers, and it does so right after the warp has finished the
-// phase before: the weights of a phase are in flight while the previous phase's results cross the grid barrier.
+// phase before: the weights of a phase are in flight while the previous phase's results are exchanged.
 constexpr int MAXI = 4;               // outputs a warp stages at once (checked on the host)
 constexpr int MAX_DYN = 220 * 1024;   // dynamic shared memory the kernel may ask for (227 KB per CTA, less than 7 KB static)
 
@@ -978,7 +978,7 @@ __device__ __forceinline__ void route_phase(const gb_mega_args& a, const gb_mega
 
 // Vocabulary projection.  A warp has far more rows here than its staging slice holds, so the slice is a ring of
 // `items` row slots (as many whole rows as fit, at most MAXI): row k lands in slot k % items, and the slot is refilled
-// with row k + items as soon as the warp has read it.  head_issue before the last grid barrier starts the first rows.
+// with row k + items as soon as the warp has read it.  head_issue before the last exchange starts the first rows.
 // (Pulling the rows through registers one group ahead ran this phase at a fifth of the memory bandwidth.)
 template <int FMT>
 __device__ __forceinline__ int head_items(const gb_mega_args& a) {

@@ -220,6 +220,35 @@ def test_moe_route_group_matches_reference(n, ne, Kk, shared, jit, d):
         assert float(xp[so[e] + tot[e]:so[e + 1]].abs().max() if so[e + 1] > so[e] + tot[e] else 0) == 0.0
 
 
+@pytest.mark.parametrize("n, ne, Kk, shared", [(1, 8, 2, True), (9, 8, 1, False), (6144, 8, 2, True), (6145, 8, 2, True), (8191, 2, 1, True),
+                                              (8192, 8, 4, True), (33000, 8, 2, False), (2000, 64, 6, True), (840, 64, 2, False)])
+def test_moe_grouping_beside_its_scan(n, ne, Kk, shared):
+    """Positions, totals, tile map and pads where every copying block adds up the histograms ahead of it, and where a scan did before."""
+    k = K()
+    d, dt = 64, torch.float16
+    x16, rw = rnd(n, d, seed=141).to(dt), rnd(ne, d, seed=142, scale=0.05)
+    ws = k.MoeWorkspace(n, d, ne, Kk, shared, dt, "cuda")
+    xp = torch.full((ws.cap, d), 7.0, dtype=dt, device="cuda")
+    counts = torch.zeros(ne, device="cuda")
+    k.moe_route_group(ws, x16, rw, None, xp, counts, want_aux=True)
+    ne1, S = ne + int(shared), Kk + int(shared)
+    idx = ws.idx.view(n, Kk).long()
+    hit = torch.zeros(n, ne1, dtype=torch.long, device="cuda").scatter_(1, idx, 1)
+    hit[:, ne:] = 1
+    tot = hit.sum(0)
+    pad = (tot + 255) // 256 * 256
+    off = torch.cat([torch.zeros(1, dtype=torch.long, device="cuda"), pad.cumsum(0)])
+    assert torch.equal(ws.seg_offsets[:ne1 + 1].long(), off) and int(ws.num_tiles[0]) == int(off[-1]) // 128
+    assert torch.equal(counts.long(), tot[:ne])
+    assert torch.equal(ws.tile_expert[:int(off[-1]) // 128].long(), torch.repeat_interleave(torch.arange(ne1, device="cuda"), pad // 128))
+    order = hit.cumsum(0) - 1 + off[:ne1]                                  # stable: token order inside every expert
+    want = torch.cat([order.gather(1, idx)] + ([order[:, ne:]] if shared else []), 1)
+    assert torch.equal(ws.slot_pos.reshape(-1)[:n * S].view(n, S).long(), want)
+    full = torch.zeros(int(off[-1]), d, dtype=dt, device="cuda")
+    full[want.reshape(-1)] = x16.repeat_interleave(S, 0)
+    assert torch.equal(xp[:int(off[-1])], full)
+
+
 @pytest.mark.parametrize("aux,jit", [(0.0, 0.0), (0.01, 0.01)])
 def test_moe_layer_forward_backward(aux, jit):
     """route -> grouped SwiGLU GEMM -> grouped down GEMM -> combine, and the whole backward, vs autograd."""
