@@ -26,7 +26,6 @@ import torch
 from ..models.config import ModelConfig
 from ..models.cuda_model import CudaModel
 from ..ops import decode as D
-from ..ops import gemm as G
 from ..ops import kernels as K
 from ..utils import canary as CA
 from .token_loop import SamplingParams, TokenLoop  # noqa: F401  (SamplingParams is re-exported)
@@ -344,29 +343,10 @@ class InferenceEngine(TokenLoop):
             self._prompt_graph = g
         self._prompt_graph.replay()
 
-    def _pass_has_step_weights(self) -> bool:
-        """True where the prompt pass multiplies by the very weights of the token step: 16-bit formats of the compute type, and the step that
-        runs on the pass's copies.  (A pass over a quantised file's 16-bit values would give its last token other logits than the step.)"""
-        own = {torch.float16: D.W_F16, torch.bfloat16: D.W_BF16}[self.dt]
-        return self.batched or all(w.fmt == own for L in self.layers for w in (L.wqkv, L.wo, L.wg, L.wu, L.wd))
-
-    def _logits_of_rows(self, m: CudaModel, x: torch.Tensor):
-        """Final norm and vocabulary projection of ``x`` [B, width] (fp32, any row pitch), as the token step does them.  The step of the last
-        token read all active weights again: 0.54 ms of a prompt of 1501 tokens (26 layers)."""
-        cfg = self.cfg
-        if self.batched or not D.gemv_norm_fits(self.B, cfg.hidden_size):
-            K.rmsnorm_fwd(x.contiguous(), self.final_norm, self.xb, self.rr, cfg.rms_eps)
-            if self.batched:
-                G.gemm(self.xb, m._head_weight16(), out=self.logits, block_n=256 if cfg.vocab_size >= 4096 else 0)
-            else:
-                D.gemv(self.head, self.xb, self.logits)
-        else:
-            D.gemv_norm(self.head, x, self.final_norm, cfg.rms_eps, self.logits, self.dt == torch.bfloat16)
-
     def prefill(self, prompts: torch.Tensor):
         """``prompts``: int32 [B, n] (same length for every sequence).  The first ``prefill_chunk`` tokens go through
-        the batched forward pass, whose K/V land in the cache, and the rest through the decode step.  The logits come from the last
-        row of the pass where it holds the whole prompt and its weights are those of the decode step, else from the step of the last token."""
+        the batched forward pass, whose K/V land in the cache; the rest (and the last prompt token, which produces
+        the first logits) go through the decode step."""
         B, n = prompts.shape
         if B != self.B or n < 1:
             raise ValueError("prefill needs [%d, n >= 1] token ids, got %s" % (self.B, tuple(prompts.shape)))
@@ -377,8 +357,6 @@ class InferenceEngine(TokenLoop):
         # A prompt longer than the cache goes token by token: the ring keeps the first tokens and the most recent ones
         # (inference/kv_cache.h:11-106 in the reference), which the batched pass cannot express.
         head = min(n - 1, self.prefill_chunk) if (n - 1 >= 64 and n <= self.cap) else 0
-        if head and n <= self.prefill_chunk and self._pass_has_step_weights():
-            head = n
         if head > 0:
             m = self._prefill_net()
             T = self.prefill_chunk
@@ -390,9 +368,6 @@ class InferenceEngine(TokenLoop):
             self.state[:, 0] = head
             self.state[:, 1] = head
             self.pos.fill_(head)
-            if head == n:
-                self.cur_tok.copy_(prompts[:, n - 1])
-                self._logits_of_rows(m, m.x[self.cfg.num_layers % 2].view(B, T, -1)[:, n - 1])
         for j in range(head, n):
             self.cur_tok.copy_(prompts[:, j])
             self._forward_token()

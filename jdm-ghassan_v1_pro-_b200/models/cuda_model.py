@@ -434,8 +434,8 @@ class CudaModel:
             G.gemm(b.act, self.w16(p + "w_down"), out=x_out, addend=b.x_mid)
 
     def prompt_forward(self, eng):
-        """The rows in ``ids`` through all layers, for the keys and values that they leave in the cache of ``eng`` (which takes a
-        prompt's logits from its last row here, or from the token step of its last token)."""
+        """The rows in ``ids`` through all layers, for the keys and values that they leave in the cache of ``eng`` (the logits of a
+        prompt come from the token step of its last token)."""
         self.kv_sink = eng
         try:
             K.embed_fwd(self.ids, self.w("tok_embeddings"), self.x[0])

@@ -295,6 +295,25 @@ def test_prefill_pass_equals_token_by_token():
     assert torch.allclose(a.layers[1].cK[:, :100].float(), b.layers[1].cK[:, :100].float(), atol=3e-2)
 
 
+@pytest.mark.parametrize("fmt,B,gemm_min_batch,n", [("f16", 1, 0, 100), ("f16", 2, 0, 128), ("f16", 2, 2, 100), ("q8_0", 2, 2, 66), ("q4_0", 1, 0, 90)])
+def test_prompt_logits_are_the_token_steps(fmt, B, gemm_min_batch, n):
+    """A prompt's logits have the precision of every other token's: they are the step's over the cache that the pass has left, bit for bit.
+    (The pass rounds probabilities and experts' outputs to 16 bits, the step does not.)"""
+    from ghassan_b200.inference.engine import InferenceEngine
+    from ghassan_b200.models.config import init_parameters
+    cfg = _tiny_cfg(num_heads=4, num_kv_heads=2, hidden_size=256)
+    e = InferenceEngine(cfg, init_parameters(cfg, 5), fmt=fmt, batch=B, max_len=160, prefill_chunk=128, gemm_min_batch=gemm_min_batch)
+    prompt = torch.randint(16, 512, (B, n), generator=torch.Generator().manual_seed(n), dtype=torch.int32)
+    e.reset(1)
+    e.prefill(prompt)
+    got, state = e.logits.clone(), e.state.clone()
+    e.state[:, :2] = n - 1                                  # the last token once more, through the step
+    e.pos.fill_(n - 1)
+    e.cur_tok.copy_(prompt[:, -1])
+    e._forward_token()
+    assert torch.equal(e.state, state) and torch.equal(e.logits, got)
+
+
 def test_generator_host_and_device_routes(tmp_path):
     from ghassan_b200.data.tokenizer import Tokenizer
     from ghassan_b200.inference.engine import InferenceEngine, SamplingParams
