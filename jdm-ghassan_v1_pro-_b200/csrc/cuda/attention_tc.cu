@@ -59,7 +59,7 @@ __device__ __forceinline__ float at_order_back(int i) { return __int_as_float(i 
 // ============================================================================================ forward
 // SPLIT (head size 64): two CTAs, a cluster, share an item's key tiles, where there are so few items that the longest one is the whole kernel; each has a
 // soft-max of its own, and they meet at the end: every CTA takes over half of the output columns, whose other part it reads from the other's shared
-// memory.  1501 tokens, 12 heads (144 items, up to twelve tiles of about 2 us): 24.3 -> 19.1 us; 1000 tokens, 8 heads 16.8 -> 14.7.
+// memory.  1501 tokens, 12 heads (144 items, up to twelve tiles of about 2 us): 24.0 -> 20.7 us.  The launcher says where it is taken.
 template <typename T, int HD, bool SPLIT>
 __global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1) attn_tc_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
                                                                  const __grid_constant__ CUtensorMap tmK,
@@ -1543,9 +1543,9 @@ int launch_tc_fwd(const gb_attn_args* a, int* lo, int* status, cudaStream_t st) 
     attr = true;
   }
   // persistent: as many CTAs as fit the device at once (two per SM at head_dim 64), each walking its share of the items
-  static int resident = 0;
+  static int resident = 0, sms = 0;
   if (!resident) {
-    int dev = 0, sms = 0, per_sm = 0;
+    int dev = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       return -10;
     // two 112 KB CTAs share an SM at head_dim 64 (the carve-out preference above); the occupancy query does not see
@@ -1555,10 +1555,14 @@ int launch_tc_fwd(const gb_attn_args* a, int* lo, int* status, cudaStream_t st) 
   }
   const long long n_items = (long long)((a->T + AT_M - 1) / AT_M) * a->B * a->H;
   if (n_items > 0x7fffffffll - resident) return -1;
-  // Two CTAs an item where all of them are resident at once and the longest item has four key tiles or more (with three, two and one tile
-  // a CTA, the exchange costs as much as the tile that it saves).
+  // Two CTAs an item where they are few and items are long.  What an item saves is half of its tiles, what it pays is the exchange, and where two CTAs share
+  // an SM also the other's time: with an SM for every CTA four tiles are enough, else ten.  us, one CTA an item -> two: 8 heads, 1000 tokens 16.8 -> 12.5,
+  // 385 tokens 9.6 -> 9.2; 12 heads, 1501 tokens 24.0 -> 20.7, 1200 20.4 -> 18.0, but 1024 (eight tiles) 15.3 -> 15.6, and 4 x 512 tokens, 8 heads 9.7 -> 13.3.  A
+  // window bounds an item's tiles (12 heads, 1501 tokens, window 256: 9.0 -> 13.6).  Packed documents have lengths that the host does not know, and most are
+  // short: 12 heads, 1501 tokens, documents of 200 9.5 -> 13.8, of 400 11.0 -> 13.9; they stay with one CTA.
   if constexpr (HD == 64) {
-    if (2 * n_items <= resident && a->T > 3 * AT_M) {
+    const long long tiles_q = (a->T + AT_M - 1) / AT_M, most = a->window > 0 ? std::min<long long>(tiles_q, (a->window + 2ll * (AT_N - 1)) / AT_N) : tiles_q;
+    if (!lo && ((2 * n_items <= sms && most >= 4) || (2 * n_items <= resident && most >= 10))) {
       auto ks = attn_tc_fwd_kernel<T, HD, true>;
       static bool attr_s = false;
       if (!attr_s) {

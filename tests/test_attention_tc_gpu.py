@@ -255,10 +255,13 @@ def test_tc_attention_scores_of_thousands(dt, T, H, KV, hd, use_seg):
         assert err <= 8 * 2.0 ** -23 * terms, ("lse", top, err)
 
 
-# Two CTAs an item: from four query tiles on, and while all pairs are resident (148 items); 385 is the shortest, 8 x 18 items and more fall back.
+# Two CTAs an item: from four key tiles on while every CTA has an SM (74 items; 385 is the shortest), from ten on up to 148 items; windows bound the tiles.
+# Documents, short windows and many short items have one CTA each and are here for the other side of the line.
 @pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("B,T,H,KV,window,use_seg", [(1, 385, 3, 1, 0, False), (1, 1501, 12, 4, 0, False), (2, 700, 8, 2, 0, True), (1, 1000, 8, 2, 129, True),
-                                                     (3, 512, 12, 4, 1, False), (1, 2304, 8, 2, 0, False), (1, 2305, 8, 2, 0, False), (1, 384, 4, 2, 0, False)])
+                                                     (3, 512, 12, 4, 1, False), (1, 2304, 8, 2, 0, False), (1, 2305, 8, 2, 0, False), (1, 384, 4, 2, 0, False),
+                                                     (1, 1000, 8, 2, 385, False), (1, 700, 3, 1, 386, False), (1, 2304, 8, 2, 1153, False), (1, 2304, 8, 2, 1154, False),
+                                                     (1, 1153, 12, 4, 0, False), (1, 1152, 12, 4, 0, False)])
 def test_tc_forward_with_shared_items(dt, B, T, H, KV, window, use_seg):
     """Rows whose keys all lie in one CTA's tiles, documents that begin in the second half, windows shorter than a tile; log-sum-exp included."""
     from ghassan_b200.ops import kernels as K
@@ -285,3 +288,19 @@ def test_tc_forward_with_shared_items(dt, B, T, H, KV, window, use_seg):
             assert ok, (b, h, worst)
             assert float((lse[rows, h] - torch.logsumexp(s, -1)).abs().max()) <= 2e-3          # fp32, fast exponentials, values up to about 30
 
+
+@pytest.mark.parametrize("B,T,H,KV,window,doc", [(1, 1501, 12, 4, 256, 0), (1, 1000, 8, 2, 0, 100), (4, 512, 8, 2, 0, 0), (1, 1024, 12, 4, 0, 0)])
+def test_tc_forward_of_short_items_does_not_depend_on_the_batch(B, T, H, KV, window, doc):
+    """Items that two CTAs would not make faster are worked on as they are in a large batch: the same bits."""
+    from ghassan_b200.ops import kernels as K
+    hd, many = 64, 8
+    g = torch.Generator(device="cuda").manual_seed(T)
+    qkv = torch.randn(B * T, (H + 2 * KV) * hd, device="cuda", generator=g).half()
+    outs = []
+    for n in (B, B * many):
+        x = qkv.repeat(n // B, 1)
+        seg = torch.arange(T, device="cuda", dtype=torch.int32).div(doc, rounding_mode="floor").to(torch.int32).repeat(n) if doc else None
+        o, lse, lo = torch.empty(n * T, H * hd, device="cuda", dtype=torch.float16), torch.empty(n * T, H, device="cuda"), torch.zeros(n * T, dtype=torch.int32, device="cuda")
+        K.attn_tc_fwd(x[:, :H * hd], x[:, H * hd:(H + KV) * hd], x[:, (H + KV) * hd:], o, lse, seg, lo, n, T, H, KV, hd, window, hd ** -0.5)
+        outs.append((o[:B * T], lse[:B * T]))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
