@@ -1116,8 +1116,10 @@ static int launch_decode_attn(const void* q, long long ld_q, const void* cK, con
                               int KV, int cap, int window, float scale, int* ticket, cudaStream_t st) {
   const int G = H / KV;
   if (!ticket && splits > 2 * HD) return -4;      // the merge kernel reads at most two splits per thread
-  // a cluster: no more than eight CTAs anywhere, and a slot's lanes hold its scores (heads of 32: up to four queries a key head)
-  if (!ticket && splits <= 8 && (splits & (splits - 1)) == 0 && G <= HD / 8) {
+  // a cluster: no more than eight CTAs anywhere, and a slot's lanes hold its scores (heads of 32: up to four queries a key head).  Eight splits only
+  // while all CTAs fit at once (four to an SM, two with more than four queries a key head): beyond that the plain kernel and its merge are faster (48 sequences,
+  // 8 heads of 64 without groups, 4000 slots 65 us, the cluster 82; 96 sequences, 12/4 heads, 2000 slots 61 and 69)
+  if (!ticket && splits <= 8 && (splits & (splits - 1)) == 0 && G <= HD / 8 && (splits < 8 || (long long)B * KV * splits <= (G <= 4 ? 592 : 296))) {
     cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg = gb_pdl_config(dim3((unsigned)(B * KV * splits)), dim3(128), 0, st, &at[1]);
     at[0].id = cudaLaunchAttributeClusterDimension;

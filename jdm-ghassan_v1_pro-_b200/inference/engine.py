@@ -42,6 +42,29 @@ class _Layer:
     pass
 
 
+def attention_splits(batch: int, heads: int, kv_heads: int, head_dim: int, max_len: int) -> int:
+    """Pieces that the token step cuts a sequence's cache into: enough (sequence, key head, piece) blocks to cover the GPU; a warp walks its
+    slots one by one, so at batch 1 the cache is cut fine and the partial results merged afterwards.
+
+    Where that is more blocks than fit at once (four to an SM, two with more than four query heads a key head) fewer pieces, whose results a cluster
+    merges without a kernel behind it, are faster while caches are short: 32 sequences of 500 slots, 12/4 heads of 64, 8 pieces 10.2 us, 4 pieces 7.9.  With long
+    caches they are not, since the last round of blocks leaves the GPU half empty: 96 sequences of 4000 slots 106 and 126, 48 sequences of 4000 slots, 8/8
+    heads 65 and 97.  The bounds, in keys of 64 values, lie where both are equal, for one, two and more query heads a key head: with a full
+    last round (0.8 of it) and with an emptier one (half where it is not the only one).  Eight pieces and more, which eight query heads a key head leave, are
+    always enough (16 sequences, 32 pieces -> 16: 12.9 -> 7.8 us with 500 slots, 20.7 -> 17.0 with 4000)."""
+    splits = int(min(64, max(8, 512 // (batch * kv_heads))))
+    group, fit = heads // kv_heads, 592 if heads <= 4 * kv_heads else 296
+    fewer = splits
+    while fewer > 1 and fewer * batch * kv_heads > fit:
+        fewer //= 2
+    rounds = -(-fewer * batch * kv_heads // fit)
+    full, empty = {1: (640, 576), 2: (2176, 1152)}.get(group, (4352, 1152))
+    if rounds > 1 and group <= 2:
+        empty //= 2
+    keys = full if fewer * batch * kv_heads >= 0.8 * fit * rounds else empty
+    return fewer if fewer >= 8 or max_len * head_dim <= keys * 64 else splits
+
+
 class InferenceEngine(TokenLoop):
     """Weights in decode formats + KV cache + one captured decode step for ``batch`` sequences."""
 
@@ -148,12 +171,7 @@ class InferenceEngine(TokenLoop):
         self.r_w = CA.zeros(B, max(1, cfg.moe_top_k), **f32)
         self.dense_idx = CA.zeros(B, 1, **i32)          # dense FFN = one "expert" with weight 1
         self.dense_w = torch.ones(B, 1, **f32)
-        # split-KV: enough (sequence, kv head, split) blocks to cover the GPU; a warp walks its slots one by one,
-        # so at batch 1 the cache is cut fine (a few slots per warp) and the partial results merged afterwards
-        self.splits = int(min(64, max(8, 512 // (B * cfg.num_kv_heads))))
-        fit = 592 if cfg.num_heads <= 4 * cfg.num_kv_heads else 296              # four blocks to an SM at once, or two
-        while self.splits > 1 and self.splits * B * cfg.num_kv_heads > fit:
-            self.splits //= 2
+        self.splits = attention_splits(B, cfg.num_heads, cfg.num_kv_heads, cfg.head_dim, max_len)
         self.att_scratch = CA.zeros(B * cfg.num_heads * self.splits * (cfg.head_dim + 2), **f32)
         self.att_ticket = CA.zeros(B * cfg.num_kv_heads, **i32)
         self.cos_sin = K.rope_table(torch.from_numpy(cfg.rope_inv_freq()), max(cfg.max_seq_len, max_len) + 1, self.dev)

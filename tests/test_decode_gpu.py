@@ -668,6 +668,26 @@ def test_decode_attention_at_slot_edges(hd, H, KV, n, splits, window, off):
         assert (out.float()[:, h * hd:(h + 1) * hd] - ref).abs().max() < 2e-3, (h, lo)
 
 
+@pytest.mark.parametrize("hd,H,KV,B", [(64, 3, 1, 75), (64, 3, 1, 74), (64, 8, 1, 38), (128, 4, 2, 38), (32, 2, 2, 38)])
+def test_decode_attention_of_large_batches(hd, H, KV, B):
+    """Eight splits while their clusters fit at once, and beyond that, where the plain kernel and its merge take over; one to four splits either way."""
+    D = _D()
+    n, cap = 150, 160
+    cK, cV = (_rand(B, cap, KV * hd, seed=s).cuda().half() for s in (1, 2))
+    slot_pos = torch.arange(cap, dtype=torch.int32, device="cuda").repeat(B, 1)
+    state = torch.zeros(B, D.STATE_INTS, dtype=torch.int32, device="cuda")
+    state[:, :2] = n - 1 - torch.arange(B, device="cuda")[:, None] % 7                   # lengths differ
+    q, g = _rand(B, H * hd, seed=3).cuda().half(), H // KV
+    k, v = (c.float().view(B, cap, KV, hd).repeat_interleave(g, 2) for c in (cK, cV))
+    s = torch.einsum("bhd,blhd->bhl", q.float().view(B, H, hd), k) * hd ** -0.5
+    s = s.masked_fill(torch.arange(cap, device="cuda")[None, None, :] > state[:, 1, None, None], float("-inf"))
+    want = torch.einsum("bhl,blhd->bhd", torch.softmax(s, -1), v)
+    for splits in (1, 4, 8):
+        out = torch.zeros(B, H * hd, device="cuda", dtype=torch.float16)
+        D.decode_attn(q, cK, cV, slot_pos, state, out, torch.zeros(B * H * splits * (hd + 2), device="cuda"), splits, H, KV, hd, cap, 0, hd ** -0.5)
+        assert float((out.float().view(B, H, hd) - want).abs().max()) < 2e-3, splits         # fp32 throughout, rounded once, values below 4
+
+
 def test_prompt_pass_replays_for_other_prompts():
     """An engine's first prompt runs as it comes (it may be the only one), the second is captured and replayed, as are all others: other
     lengths and tokens, two sequences; cache rows behind the prompt stay as they were."""
