@@ -59,6 +59,19 @@ class LayerWeights:
     w_kv: Optional[torch.Tensor] = None      # [H * dkp + H * dvp, latent row] keys and values from cache rows
 
 
+def attention_splits(blocks: int, seen: int, dkp: int) -> int:
+    """Pieces of a token's attention over ``seen`` keys in rows of ``dkp`` values, where ``blocks`` have one piece each.  Four blocks fit an SM at once: a few
+    more than that are a second round (32 sequences: 18.5 us with 5 pieces, 13.3 with 4).
+
+    One, two, four or eight pieces are merged by a cluster, with no kernel behind it; other numbers are rounded down to that while few keys are
+    walked.  Rows of 64, four heads a key head, us as many pieces as fit -> rounded down: 1 sequence of 512 keys (32 -> 8) 6.3 -> 5.5, of 1032 (64 -> 8) 7.6 -> 8.3; 20
+    sequences of 512 (7 -> 4) 13.8 -> 11.4, of 2048 33 -> 36.5.  Rows of 128: 1 sequence of 256 keys 7.3 -> 6.0, of 700 8.6 -> 10.0; 32 sequences of 256 (3 -> 2) 22.7 -> 22.0, of 512
+    36.7 -> 38.5.  Rows of 256 gain nothing (1 sequence of 512 keys 9.7 -> 13.8)."""
+    splits = int(max(1, min(64, 592 // blocks, (seen + 15) // 16)))
+    few = 1 << (min(splits, 8).bit_length() - 1)
+    return few if dkp <= 128 and seen * dkp <= 512 * 64 else splits
+
+
 class LayerModel:
     def __init__(self, cfg: LayerListConfig, named: Dict[str, torch.Tensor], slots: int, chunk_rows: int, dtype=torch.bfloat16,
                  device=None, use_tensor_cores: bool = True):
@@ -250,10 +263,7 @@ class LayerModel:
             per_key_head = m.heads // m.kv_heads
             blocks = B * m.kv_heads * ((per_key_head + 3) // 4)
             seen = cache.cap if not m.window else m.window + m.keep_first
-            # four blocks fit an SM at once: a few more than that are a second round (32 sequences: 18.5 us with 5 splits, 13.3 with 4)
-            a.splits = int(max(1, min(64, 592 // blocks, (seen + 15) // 16)))
-            if a.splits <= 8 or seen <= 512:                # a power of two up to eight: a cluster merges them, with no kernel behind it
-                a.splits = 1 << (min(a.splits, 8).bit_length() - 1)
+            a.splits = attention_splits(blocks, seen, a.dkp)
             a.scratch = self.buf("att_scratch%d" % B, m.heads * a.splits * (a.dvp + 2), torch.float32, rows=B).data_ptr()
         a.st, a.pos0_max, a.status = st.data_ptr(), pos0_max, _lib.status_word(self.dev).data_ptr()
         return a

@@ -13,3 +13,11 @@ import pytest
 def test_pieces_of_a_sequence_in_token_attention(batch, heads, kv, hd, max_len, want):
     from ghassan_b200.inference.engine import attention_splits
     assert attention_splits(batch, heads, kv, hd, max_len) == want
+
+
+@pytest.mark.parametrize("blocks,seen,dkp,want", [
+    (4, 16, 64, 1), (4, 64, 64, 4), (4, 512, 64, 8), (4, 513, 64, 33), (4, 1032, 64, 64), (80, 512, 64, 4), (80, 513, 64, 7), (128, 4096, 64, 4), (600, 4096, 64, 1),
+    (5, 256, 128, 8), (5, 257, 128, 17), (160, 256, 128, 2), (160, 1024, 128, 3), (4, 128, 256, 8), (4, 144, 256, 9), (192, 64, 256, 3)])
+def test_pieces_of_a_layer_list_token(blocks, seen, dkp, want):
+    from ghassan_b200.models.layer_model import attention_splits
+    assert attention_splits(blocks, seen, dkp) == want
