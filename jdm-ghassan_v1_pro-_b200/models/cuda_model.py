@@ -182,6 +182,20 @@ class _LayerBuf:
     pass
 
 
+def few_through_all(N: int, top_k: int, ne: int, ne1: int, E: int, d: int) -> bool:
+    """True where all of ``N`` rows go through all ``ne1`` experts (``ne`` routed ones), with no sorting and no rows padded to 256.
+
+    Few tokens visit nearly all experts, 1 - (1 - top_k / ne)^N of them: two thirds from N * top_k == ne on.  What it costs is rows: the down product's operand is
+    ne1 * E wide, and each of its d / 64 tiles reads all of it, so the more experts' columns there are to a column of the result, the fewer rows pay.  Width
+    768, 2 of 8 experts and a shared one of 768, us a layer's feed-forward sorted -> all: 32 rows 42.5 -> 17.5, 128 rows 42.4 -> 28.4.  ne1 * E of 15 d, 128
+    rows: 51.2 -> 39.4.  20 d: 64 rows 71 -> 65, 128 rows 71 -> 76.  32 d: 32 rows 88 -> 80, 33 rows (another size of tile) 87 -> 94; 4 rows for 16 experts, 4 picks 77 ->
+    79.  64 d: 64 rows 156 -> 201."""
+    if N > 128 or N * top_k < ne or ne > 64 or top_k > 8 or E % 64 or d > 20480:
+        return False
+    columns = ne1 * E
+    return columns <= 16 * d or (columns <= 22 * d and N <= 64) or (columns <= 32 * d and N <= 32 and N * top_k >= 2 * ne)
+
+
 class CudaModel:
     """Parameters, activations and the forward/backward schedule for a fixed micro-batch shape (B, T)."""
 
@@ -250,10 +264,7 @@ class CudaModel:
         f32 = dict(dtype=torch.float32, device=dev)
         c16 = dict(dtype=dt, device=dev)
         nl = cfg.num_layers if train else 1     # evaluation reuses one layer's buffers
-        # Few tokens visit nearly all experts: 1 - (1 - top_k / ne)^N of them, two thirds from here on.  All rows then go through all experts, with no
-        # sorting and no rows padded to 256 (32 tokens, 2 of 8 experts and a shared one of 768, width 768: 47 us a layer's feed-forward -> 20).
-        self.experts_few = (not train and cfg.use_moe and N <= 128 and N * cfg.moe_top_k >= cfg.num_experts and cfg.num_experts <= 64
-                            and cfg.moe_top_k <= 8 and E % 64 == 0 and d <= 20480)
+        self.experts_few = not train and cfg.use_moe and few_through_all(N, cfg.moe_top_k, cfg.num_experts, self.layout.ne1, E, d)
         self.x = [CA.empty(N, d, **f32) for _ in range((cfg.num_layers + 1) if train else 2)]
         self.layers: List[_LayerBuf] = []
         for _ in range(nl):

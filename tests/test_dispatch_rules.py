@@ -21,3 +21,14 @@ def test_pieces_of_a_sequence_in_token_attention(batch, heads, kv, hd, max_len, 
 def test_pieces_of_a_layer_list_token(blocks, seen, dkp, want):
     from ghassan_b200.models.layer_model import attention_splits
     assert attention_splits(blocks, seen, dkp) == want
+
+
+@pytest.mark.parametrize("N,top,ne,ne1,E,d,want", [
+    (3, 2, 8, 9, 768, 768, False), (4, 2, 8, 9, 768, 768, True), (128, 2, 8, 9, 768, 768, True), (129, 2, 8, 9, 768, 768, False),      # most experts are visited
+    (128, 4, 8, 9, 1280, 768, True), (128, 2, 16, 16, 1024, 1024, True), (64, 2, 16, 16, 1088, 1024, True), (65, 2, 16, 16, 1088, 1024, False),
+    (64, 2, 4, 5, 4096, 1024, True), (96, 2, 4, 5, 4096, 1024, False), (4, 4, 16, 16, 2048, 1024, False), (8, 4, 16, 16, 2048, 1024, True),
+    (32, 4, 16, 16, 2048, 1024, True), (33, 4, 16, 16, 2048, 1024, False), (64, 1, 64, 64, 1024, 1024, False), (32, 8, 64, 64, 576, 1024, False),
+    (32, 2, 65, 65, 64, 768, False), (32, 9, 16, 16, 64, 768, False), (32, 2, 8, 8, 96, 768, False), (32, 2, 8, 8, 64, 20488, False)])
+def test_when_all_rows_go_through_all_experts(N, top, ne, ne1, E, d, want):
+    from ghassan_b200.models.cuda_model import few_through_all
+    assert few_through_all(N, top, ne, ne1, E, d) is want
