@@ -21,24 +21,33 @@ EPI_STORE, EPI_SWIGLU_FWD, EPI_SWIGLU_BWD, EPI_RELU2 = 0, 1, 2, 4
 # (74 CTA pairs on a B200); GB200_GEMM_PAIR=0 keeps every product on the one-CTA kernel.
 PAIR_ENABLED = os.environ.get("GB200_GEMM_PAIR", "1") != "0"
 PAIR_MIN_TILES = int(os.environ.get("GB200_GEMM_PAIR_MIN_TILES", "60"))
-# One product that is neither grouped nor short (K of 1024 and more) goes to the pairs from 38 tiles on: its 128 x 128 tiles are more
-# than 148 there, two rounds of the one-CTA kernel, and a pair has the same products to do in one round and reads half of B for them.
-# 40 to 56 tiles, bf16, one CTA -> pair: K 1024 15.3 -> 13.9 us (SwiGLU 14 -> 14, its gradient 22 -> 17.5), 2048 22.5 -> 17.7 (21 -> 18.3,
-# 29.8 -> 24), 6912 58 -> 41.5 (57 -> 45, 74 -> 60), 32000 243 -> 165, with B in [K, N] order 290 -> 170.  Up to 768 they differ by
-# less than their calls.  Grouped rows keep the line above: their count is a bound, and what the experts got is known on the device.
-PAIR_MIN_TILES_ONE = int(os.environ.get("GB200_GEMM_PAIR_MIN_TILES", "38"))
+# One product that is neither grouped nor short (K of 1024 and more) goes to the pairs from 38 tiles on where the one-CTA kernel would take a second round for
+# its own tiles: a pair has the same products to do in one round and reads half of B for them.  40 to 56 tiles, bf16, one CTA -> pair: K 1024 15.3 -> 13.9 us (SwiGLU
+# 14 -> 14, its gradient 22 -> 17.5), 2048 22.5 -> 17.7 (21 -> 18.3, 29.8 -> 24), 6912 58 -> 41.5 (57 -> 45, 74 -> 60), 32000 243 -> 165, with B in [K, N] order
+# 290 -> 170.  Up to 768 they differ by less than their calls.  In one round the one-CTA kernel is the faster one, since a pair's tiles then are rows that do not
+# exist: 300 x 4616 x 2048 (111 tiles of 128 x 128) 12.8 and 14.9, 64 x 6912 with SwiGLU, K 2560, 17.3 and 23.7; 128 x 9728 x 2048 (152 tiles of 128 x 64) 19.4 and
+# 16.2.  Grouped rows keep the line above: their count is a bound, and what the experts got is known on the device.
+PAIR_MIN_TILES_ONE = int(os.environ.get("GB200_GEMM_PAIR_MIN_TILES_ONE", os.environ.get("GB200_GEMM_PAIR_MIN_TILES", "38")))
 PAIR_MIN_K_ONE = 1024
+SMS = 148
 
 
 def pair_tiles(M, N, groups=1):
     return ((M + 255) // 256) * ((N + 255) // 256) * groups
 
 
-def pair_ok(M, N, out, groups=1, extra=(), K=0):
-    """True when the two-CTA kernel can and should run this product: enough 256 x 256 tiles, and every matrix that
-    its epilogue moves with TMA (the output, saved gate/up) 16-byte aligned with a 16-byte row pitch.
-    ``K``: of a product that is not grouped."""
-    if not PAIR_ENABLED or pair_tiles(M, N, groups) < (PAIR_MIN_TILES_ONE if K >= PAIR_MIN_K_ONE else PAIR_MIN_TILES):
+def pair_fits(M, N, groups=1, K=0, block_n=128):
+    """True when a product has enough 256 x 256 tiles for the two-CTA kernel.  ``K``, ``block_n``: of a product that is not grouped, and the
+    tile width that the one-CTA kernel would take for it."""
+    if K >= PAIR_MIN_K_ONE and ((M + 127) // 128) * ((N + block_n - 1) // block_n) > SMS:
+        return pair_tiles(M, N, groups) >= PAIR_MIN_TILES_ONE
+    return pair_tiles(M, N, groups) >= PAIR_MIN_TILES
+
+
+def pair_ok(M, N, out, groups=1, extra=(), K=0, block_n=128):
+    """True when the two-CTA kernel can and should run this product: enough 256 x 256 tiles (:func:`pair_fits`), and every matrix that
+    its epilogue moves with TMA (the output, saved gate/up) 16-byte aligned with a 16-byte row pitch."""
+    if not PAIR_ENABLED or not pair_fits(M, N, groups, K, block_n):
         return False
     for t in (out,) + tuple(extra):
         if t is not None and (t.data_ptr() % 16 or (t.stride(-2) * t.element_size()) % 16):
@@ -114,11 +123,12 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_dtype=None, addend=None,
     if out is None:
         out = torch.empty(M, N, dtype=out_dtype or a.dtype, device=a.device)
     skinny = pair is None and not (block_n or a_mn or b_mn) and skinny_ok(M, N, out, addend)
-    if pair is None:
-        pair = (not skinny and block_n in (0, 256) and (addend is None or out.dtype == torch.float32) and
-                pair_ok(M, N, out, K=K))
+    wide = block_n in (0, 256)
     if not block_n:
         block_n = pick_block_n(M, N, mn_major=a_mn and b_mn)
+    if pair is None:
+        pair = (not skinny and wide and (addend is None or out.dtype == torch.float32) and
+                pair_ok(M, N, out, K=K, block_n=block_n))
     g = _base_args(a, b, M, N, K, a_mn, b_mn, out, block_n)
     if relu2 and (addend is not None or out.dtype != torch.bfloat16):
         raise ValueError("relu2 needs a bf16 output and no addend")
@@ -194,7 +204,8 @@ def gemm_swiglu(a, w_gu, *, act_out=None, gu_out=None, tile_expert=None, num_m_t
         g.N, g.skinny, g.b_static = N // 2, 1, int(b_static)
         _launch(g)
         return act_out
-    g.pair = int(pair_ok(M, N, act_out, extra=(gu_out,), K=K if tile_expert is None and act_out.element_size() == 2 else 0) if pair is None else bool(pair))
+    one_k = K if tile_expert is None and act_out.element_size() == 2 else 0
+    g.pair = int(pair_ok(M, N, act_out, extra=(gu_out,), K=one_k, block_n=g.block_n) if pair is None else bool(pair))
     if gu_out is not None:
         g.aux_out, g.ld_aux = gu_out.data_ptr(), gu_out.stride(0)
     if tile_expert is not None:
@@ -218,7 +229,8 @@ def gemm_swiglu_bwd(dy, w_down, gu, *, dgu_out=None, b_mn=True, tile_expert=None
     g = _base_args(dy, w_down, M, N, K, False, b_mn, dgu_out,
                    256 if (N % 256 == 0 and M >= 4096) else (128 if N % 128 == 0 else 64))
     g.epilogue = EPI_SWIGLU_BWD
-    g.pair = int((N % 64 == 0 and pair_ok(M, N, dgu_out, extra=(gu,), K=K if tile_expert is None and dgu_out.element_size() == 2 else 0)) if pair is None else bool(pair))
+    one_k = K if tile_expert is None and dgu_out.element_size() == 2 else 0
+    g.pair = int((N % 64 == 0 and pair_ok(M, N, dgu_out, extra=(gu,), K=one_k, block_n=g.block_n)) if pair is None else bool(pair))
     g.aux_in, g.ld_aux = gu.data_ptr(), gu.stride(0)
     if tile_expert is not None:
         g.mode = 1

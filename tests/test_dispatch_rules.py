@@ -32,3 +32,24 @@ def test_pieces_of_a_layer_list_token(blocks, seen, dkp, want):
 def test_when_all_rows_go_through_all_experts(N, top, ne, ne1, E, d, want):
     from ghassan_b200.models.cuda_model import few_through_all
     assert few_through_all(N, top, ne, ne1, E, d) is want
+
+
+@pytest.mark.parametrize("M,N,K,want", [
+    (1280, 2048, 1024, True), (1280, 2048, 1023, False), (1536, 2560, 768, True),            # one round of pairs for two of the one-CTA kernel; 60 tiles for any K
+    (300, 4616, 2048, False), (300, 6144, 2048, False), (128, 15104, 2048, False), (500, 4864, 2048, True),      # 111, 144 and 118 tiles of 128 x 128, 152
+    (128, 9728, 2048, True), (128, 9408, 2048, False), (128, 15360, 2048, True)])            # 152 tiles of 128 x 64, 147; 60 of 256 x 256
+def test_products_that_the_pairs_take(M, N, K, want):
+    from ghassan_b200.ops import gemm as G
+    assert G.pair_fits(M, N, K=K, block_n=G.pick_block_n(M, N)) is want
+
+
+def test_pair_lines_from_the_environment():
+    """One variable moves both lines, as it did when there was one; the second has a variable of its own."""
+    import os
+    import subprocess
+    import sys
+    code = "from ghassan_b200.ops import gemm as G; print(G.PAIR_MIN_TILES, G.PAIR_MIN_TILES_ONE)"
+    for env, want in (({}, "60 38"), ({"GB200_GEMM_PAIR_MIN_TILES": "70"}, "70 70"), ({"GB200_GEMM_PAIR_MIN_TILES_ONE": "50"}, "60 50")):
+        clean = {k: v for k, v in os.environ.items() if not k.startswith("GB200_GEMM_PAIR")}
+        out = subprocess.run([sys.executable, "-c", code], env=dict(clean, **env), capture_output=True, text=True, check=True).stdout
+        assert out.split("\n")[-2] == want

@@ -220,11 +220,12 @@ def test_pair_dense(dtype, out_dtype, M, N, K):
     assert torch.equal(out, out2)
 
 
-@pytest.mark.parametrize("M,N,K", [(2305, 1000, 1024), (9473, 136, 1032), (300, 4616, 2048), (1500, 1544, 1090), (1280, 2048, 1024)])
+@pytest.mark.parametrize("M,N,K", [(2305, 1000, 1024), (9473, 136, 1032), (300, 4616, 2048), (500, 4864, 1032), (1500, 1544, 1090), (1280, 2048, 1024)])
 def test_one_round_of_pairs_in_every_form(M, N, K):
-    """38 to 59 tiles go to the two-CTA kernel: orders, types, pitches and addends that the one-CTA kernel takes there."""
+    """38 to 59 tiles go to the two-CTA kernel where the one-CTA kernel would need a second round (300 x 4616 does not): orders, types, pitches and
+    addends that the one-CTA kernel takes there."""
     G, L = _ops()
-    assert 38 <= G.pair_tiles(M, N) < 60
+    assert 38 <= G.pair_tiles(M, N) < 60 and G.pair_fits(M, N, K=K) == (M != 300)
     Mp, Kp = (M + 7) // 8 * 8, (K + 7) // 8 * 8
     for a_mn in (False, True):
         for b_mn in (False, True):
