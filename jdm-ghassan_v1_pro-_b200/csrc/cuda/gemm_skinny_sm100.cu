@@ -5,9 +5,9 @@
 // into the shared memory of each of the others with a bulk copy; every CTA then adds and stores its share of the tile, the parts in the order of K.
 // Row by row, in pieces of four columns, the same writes took 1 us; fetched from the others when all were there, another round trip and a second wait
 // for the cluster so that nobody leaves early, 1 to 1.8 us more than now (from the last product to the last store 1.3 us).
-// us, the persistent kernel -> this one with early weights (floor by bytes at 6.5 TB/s), before the exchange by bulk copies: 32 x 3840 x 1024
-// 16.7 -> 7.7 (1.2), 32 x 1024 x 2816 7.5 -> 6.0 (0.9), 32 x 768 x 1280 6.6 -> 4.5 (0.3), 8 x 6912 x 2560 26.9 -> 11.2 (5.5), 128 x 6912 x 2560
-// 28.9 -> 14.3, 100 x 2816 x 1024 14.2 -> 7.0.  What is left is launch, the round trips of the first loads and the exchange.
+// A CTA's own part of its share stays where it is.  us, the persistent kernel -> this one with early weights (floor by bytes at 6.5 TB/s): 32 x 3840 x 1024 16.7 -> 5.0
+// (1.2), 32 x 1024 x 2816 7.5 -> 5.3 (0.9), 8 x 6912 x 2560 26.9 -> 10.3 (5.5), 128 x 6912 x 2560 28.9 -> 13.4.  With its own part copied, too, and
+// four columns a thread whatever the rows: 128 x 2816 x 1024 7.4 instead of 6.2, 128 x 2560 x 6912 18.0 instead of 16.7.  What is left is launch, the round trips of the first loads and the exchange.
 //
 // The kernel is launched with programmatic dependency: barriers, tensor memory and, where the caller says that W is not what
 // the kernel before writes (weights), the first eight k-blocks of W are under way before griddepcontrol.wait.
@@ -46,7 +46,9 @@ struct Params {
   int n1; void* out2; int ldo2;                    // relu2: columns below n1 as they are into out, the others into out2
 };
 
-template <typename OutT, bool SWIGLU>
+// Q: fours of columns that a thread takes at a time.  One while rows are few, so that all threads have some; two beyond 32 rows, in half as many turns with
+// stores of 16 bytes.
+template <typename OutT, bool SWIGLU, int Q>
 __global__ void __launch_bounds__(THREADS) gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW,
                                                               const Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -72,7 +74,7 @@ __global__ void __launch_bounds__(THREADS) gemm_skinny_kernel(const __grid_const
     mbar_init(&parts_bar, 1);
     abort_word = 0;
     fence_barrier_init();
-    if (p.split > 1) mbar_arrive_expect_tx(&parts_bar, (uint32_t)(p.split * share) * 4);
+    if (p.split > 1) mbar_arrive_expect_tx(&parts_bar, (uint32_t)((p.split - 1) * share) * 4);
   }
   if (warp == W_MMA) { tmem_alloc(&tmem_slot, BN); tmem_relinquish(); }
   tc_fence_before();
@@ -80,25 +82,25 @@ __global__ void __launch_bounds__(THREADS) gemm_skinny_kernel(const __grid_const
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");       // waited for before the first write to another CTA
-  // units of four columns; what a thread's first two are added to or scaled by is asked for before the sums are there
-  constexpr int LG_ROW = SWIGLU ? 3 : 4;
+  // units of Q fours of columns; what a thread's first two are added to or scaled by is asked for before the sums are there
+  constexpr int LG_ROW = (SWIGLU ? 3 : 4) - (Q - 1);
   const int per_row = 1 << (LG_ROW - p.lg), units = p.M * per_row;
-  auto column = [&](int u) { return n0 + rank * (COLS >> p.lg) + (u & (per_row - 1)) * 4; };
-  auto addend_of = [&](int u) {
+  auto column = [&](int u) { return n0 + rank * (COLS >> p.lg) + (u & (per_row - 1)) * (4 * Q); };
+  struct Add { float4 v[Q]; float scale; };
+  auto add_of = [&](int u) {
+    Add a;
     const int row = u >> (LG_ROW - p.lg), col = column(u);
-    return p.addend && u < units && col < p.N ? *reinterpret_cast<const float4*>(p.addend + (long long)row * p.ld_add + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool in = u < units && col < p.N;
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      a.v[q] = p.addend && in ? reinterpret_cast<const float4*>(p.addend + (long long)row * p.ld_add + col)[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+    a.scale = SWIGLU && p.scale && in ? p.scale[(long long)row * p.ld_scale + col / p.scale_cols] : 1.f;
+    return a;
   };
-  float4 add0 = make_float4(0.f, 0.f, 0.f, 0.f), add1 = add0;
-  float scale0 = 1.f, scale1 = 1.f;
-  auto scale_of = [&](int u) {
-    const int col = column(u);
-    return SWIGLU && p.scale && u < units && col < p.N ? p.scale[(long long)(u >> (LG_ROW - p.lg)) * p.ld_scale + col / p.scale_cols] : 1.f;
-  };
+  Add add0, add1;
   auto ahead = [&]() {
-    add0 = addend_of(threadIdx.x);
-    add1 = addend_of(threadIdx.x + THREADS);
-    scale0 = scale_of(threadIdx.x);
-    scale1 = scale_of(threadIdx.x + THREADS);
+    add0 = add_of(threadIdx.x);
+    add1 = add_of(threadIdx.x + THREADS);
   };
 
   if (warp == W_TMA) {
@@ -178,9 +180,10 @@ __global__ void __launch_bounds__(THREADS) gemm_skinny_kernel(const __grid_const
     __syncthreads();
   }
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");          // the others have begun, their barriers are set up
+  const float* mine = reinterpret_cast<const float*>(smem) + rank * share;      // this CTA's part of its own share stays where it is
   if (p.split > 1) {
     if (threadIdx.x == 0)
-      for (int r = 0; r < p.split; ++r) {
+      for (int r = 1; r < p.split; ++r) {
         const uint32_t own = (uint32_t)((rank + r) & (p.split - 1));
         asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                          mapa_shared(smem_u32(parts) + (uint32_t)(rank * share) * 4, own)),
@@ -188,43 +191,51 @@ __global__ void __launch_bounds__(THREADS) gemm_skinny_kernel(const __grid_const
                      : "memory");
       }
     wait_or_report(&parts_bar, 0, p.status, ST_TIMEOUT_AUX, abort_flag);
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // all copies into this CTA have landed
-  } else {
-    parts = reinterpret_cast<float*>(smem);
   }
   for (int u = (int)threadIdx.x; u < units; u += THREADS) {
     const int row = u >> (LG_ROW - p.lg), col = column(u);
     if (col >= p.N) continue;                          // N is a multiple of 8
-    const int turn = u / THREADS;
-    const float4 add = turn == 0 ? add0 : turn == 1 ? add1 : addend_of(u);
-    const float scale = turn == 0 ? scale0 : turn == 1 ? scale1 : scale_of(u);
-    const float* src = parts + row * pitch + (u & (per_row - 1)) * 4;
-    auto total = [&](const float* from) {
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int turn = u / THREADS, at = row * pitch + (u & (per_row - 1)) * (4 * Q);
+    const Add add = turn == 0 ? add0 : turn == 1 ? add1 : add_of(u);
+    auto total = [&](int from, float (&v)[4 * Q]) {
+#pragma unroll
+      for (int k = 0; k < 4 * Q; ++k) v[k] = 0.f;
 #pragma unroll 4
       for (int g = 0; g < p.split; ++g) {
-        const float4 x = *reinterpret_cast<const float4*>(from + g * share);
-        v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
-      }
-      return v;
-    };
-    const float4 t = total(src);
-    float v[4] = {t.x, t.y, t.z, t.w};
-    if constexpr (SWIGLU) {
-      const float4 t2 = total(src + (width >> 1));
-      const float up[4] = {t2.x, t2.y, t2.z, t2.w};
+        const float4* src = reinterpret_cast<const float4*>((g == rank ? mine : parts + g * share) + from);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) v[k] = scale == 0.f ? 0.f : v[k] / (1.f + __expf(-v[k])) * up[k] * scale;   // not chosen: zero, whatever the product is
+        for (int q = 0; q < Q; ++q) {
+          const float4 x = src[q];
+          v[4 * q] += x.x; v[4 * q + 1] += x.y; v[4 * q + 2] += x.z; v[4 * q + 3] += x.w;
+        }
+      }
+    };
+    float v[4 * Q];
+    total(at, v);
+    if constexpr (SWIGLU) {
+      float up[4 * Q];
+      total(at + (width >> 1), up);
+#pragma unroll
+      for (int k = 0; k < 4 * Q; ++k) v[k] = add.scale == 0.f ? 0.f : v[k] / (1.f + __expf(-v[k])) * up[k] * add.scale;   // not chosen: zero, whatever the product is
     }
-    v[0] += add.x; v[1] += add.y; v[2] += add.z; v[3] += add.w;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) { v[4 * q] += add.v[q].x; v[4 * q + 1] += add.v[q].y; v[4 * q + 2] += add.v[q].z; v[4 * q + 3] += add.v[q].w; }
     OutT* dst = reinterpret_cast<OutT*>(p.out) + (long long)row * p.ldo + col;
     if (p.relu2 && col >= p.n1) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) { v[k] = fmaxf(v[k], 0.f); v[k] *= v[k]; }
+      for (int k = 0; k < 4 * Q; ++k) { v[k] = fmaxf(v[k], 0.f); v[k] *= v[k]; }
       if (p.out2) dst = reinterpret_cast<OutT*>(p.out2) + (long long)row * p.ldo2 + col - p.n1;
     }
-    if constexpr (sizeof(OutT) == 4) *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
-    else *reinterpret_cast<uint2*>(dst) = make_uint2(Cvt<OutT>::pack2(v[0], v[1]), Cvt<OutT>::pack2(v[2], v[3]));
+    if constexpr (sizeof(OutT) == 4) {
+#pragma unroll
+      for (int q = 0; q < Q; ++q) reinterpret_cast<float4*>(dst)[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    } else if constexpr (Q == 2) {
+      *reinterpret_cast<uint4*>(dst) = make_uint4(Cvt<OutT>::pack2(v[0], v[1]), Cvt<OutT>::pack2(v[2], v[3]), Cvt<OutT>::pack2(v[4], v[5]), Cvt<OutT>::pack2(v[6], v[7]));
+    } else {
+      *reinterpret_cast<uint2*>(dst) = make_uint2(Cvt<OutT>::pack2(v[0], v[1]), Cvt<OutT>::pack2(v[2], v[3]));
+    }
   }
   if (warp == W_MMA) { tc_fence_after(); tmem_dealloc(tmem, BN); }
   __syncwarp();
@@ -238,12 +249,13 @@ __global__ void __launch_bounds__(THREADS) gemm_skinny_kernel(const __grid_const
 
 namespace {
 
-constexpr size_t MOST_SMEM = 226 * 1024;
+constexpr size_t MOST_SMEM = 226 * 1024, TWO_SMEM = 111 * 1024;       // of one CTA an SM, and of two (3 KB of each are static or the system's)
 
-// Shared memory of a launch: stages, and behind them the larger of the parts and of the rows that the MMAs read past the last stage.
+// Shared memory of a launch: stages, and behind them the larger of the parts (in the stages where a CTA has the whole reduction) and of the rows that the
+// MMAs read past the last stage.
 size_t skinny_smem(const gb::sk::Params& p) {
   namespace sk = gb::sk;
-  const size_t parts = (size_t)p.M * (sk::BN + 4 * p.split) * 4, tail = (size_t)(128 - p.a_rows) * 128;
+  const size_t parts = p.split > 1 ? (size_t)p.M * (sk::BN + 4 * p.split) * 4 : 0, tail = (size_t)(128 - p.a_rows) * 128;
   return (size_t)p.stages * (p.a_rows * 128 + sk::W_BYTES) + (parts > tail ? parts : tail) + 1024;
 }
 
@@ -259,36 +271,38 @@ cudaLaunchConfig_t skinny_config(const gb::sk::Params& p, cudaStream_t st, cudaL
   return cfg;
 }
 
-template <typename OutT, bool SWIGLU = false>
-int launch_skinny(const CUtensorMap& ta, const CUtensorMap& tw, gb::sk::Params p, cudaStream_t st) {
+template <typename OutT, bool SWIGLU, int Q>
+int launch_skinny_q(const CUtensorMap& ta, const CUtensorMap& tw, gb::sk::Params p, cudaStream_t st) {
   namespace sk = gb::sk;
-  auto kern = sk::gemm_skinny_kernel<OutT, SWIGLU>;
+  auto kern = sk::gemm_skinny_kernel<OutT, SWIGLU, Q>;
   static bool attr = false;
   if (!attr) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST_SMEM) != cudaSuccess) { (void)cudaGetLastError(); return -10; }
+    (void)cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     attr = true;
   }
-  // CTAs of a tile: as many as leave all tiles resident at once, which the driver is asked for (296 CTAs of half an SM each do not all fit where they come
-  // in fours: 32 x 4352 x 1024 with four CTAs a tile had a few late clusters, 10.2 us, with two it has none, 6.0).  Fewer than two k-blocks per
-  // CTA do not pay for the exchange.
+  // CTAs of a tile: as many as leave all tiles resident at once (32 x 4352 x 1024, four CTAs a tile, had a few late clusters, 10.2 us; with two it has none, 6.0).
+  // The driver is asked how many clusters fit with an SM for every CTA; up to 32 rows two CTAs share one, which its query does not see: counted as one they had
+  // half as many CTAs, 8 x 2560 x 6912 15.0 us and 11.4, 8 x 6912 x 2560 12.0 and 10.3.  Fewer than two k-blocks per CTA do not pay for the exchange.
   constexpr int COLS = SWIGLU ? sk::BN / 2 : sk::BN, MOST = SWIGLU ? 4 : 8;
   const int tiles = (p.N + COLS - 1) / COLS, blocks = (p.K + sk::BK - 1) / sk::BK;
-  static std::atomic<int> fits[4][17];                // clusters of 2, 4, 8 CTAs that fit, plus one, by rows of A in eights
+  static std::atomic<int> fits[4];                    // clusters of 2, 4, 8 CTAs that fit an SM each, plus one
   cudaLaunchAttribute at[2];
   p.split = 1;
   for (int lg = 1; (1 << lg) <= MOST && blocks >= (1 << lg) * 2; ++lg) {
     sk::Params q = p;
     q.split = 1 << lg;
     q.lg = lg;
-    q.M = q.a_rows;
     for (q.stages = sk::STAGES; skinny_smem(q) > MOST_SMEM;) --q.stages;
-    int n = fits[lg][p.a_rows / 8].load(std::memory_order_relaxed);
+    int n = fits[lg].load(std::memory_order_relaxed);
     if (!n) {
-      const cudaLaunchConfig_t cfg = skinny_config<OutT, SWIGLU>(q, st, at);
+      cudaLaunchConfig_t cfg = skinny_config<OutT, SWIGLU>(q, st, at);
+      cfg.dynamicSmemBytes = MOST_SMEM;
       if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = 0; }
-      fits[lg][p.a_rows / 8].store(++n, std::memory_order_relaxed);
+      fits[lg].store(++n, std::memory_order_relaxed);
     }
-    if (tiles > n - 1) break;
+    const int an_sm = skinny_smem(q) <= TWO_SMEM ? 2 : 1;
+    if (tiles > (n - 1) * an_sm) break;
     p.split = q.split;
     p.lg = lg;
   }
@@ -296,6 +310,11 @@ int launch_skinny(const CUtensorMap& ta, const CUtensorMap& tw, gb::sk::Params p
   const cudaLaunchConfig_t cfg = skinny_config<OutT, SWIGLU>(p, st, at);
   if (cudaLaunchKernelEx(&cfg, kern, ta, tw, p) != cudaSuccess) return -10;
   return gb_launch_rc();
+}
+
+template <typename OutT, bool SWIGLU = false>
+int launch_skinny(const CUtensorMap& ta, const CUtensorMap& tw, const gb::sk::Params& p, cudaStream_t st) {
+  return p.M > 32 ? launch_skinny_q<OutT, SWIGLU, 2>(ta, tw, p, st) : launch_skinny_q<OutT, SWIGLU, 1>(ta, tw, p, st);
 }
 
 }  // namespace

@@ -91,6 +91,24 @@ def test_two_outputs_of_few_rows(M, n1, n2, K):
     assert float((both[:, 8:].float() - up).abs().max()) <= eps * float(up.abs().max()) and bool((both[:, :8] == 3).all())
 
 
+# a share of eight columns at 33 rows and more (one unit a row), shares of 16 to 64 on both sides of 32 rows, columns past the end, one CTA a tile
+@pytest.mark.parametrize("M,N,K", [(32, 8, 1024), (33, 8, 1024), (33, 72, 4096), (128, 200, 2048), (64, 2560, 1000), (32, 4352, 1024), (40, 6912, 512), (127, 9472, 64), (1, 2568, 6912)])
+@pytest.mark.parametrize("f32", [False, True])
+def test_products_of_few_rows_share_by_share(M, N, K, f32):
+    from ghassan_b200.ops import _lib, gemm as G
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a, w = torch.randn(M, K, device="cuda", generator=g).half(), (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).half()
+    out = torch.full((M + 1, N), 3.0, device="cuda", dtype=torch.float32 if f32 else torch.float16)
+    add = torch.randn(M, N, device="cuda", generator=g) if f32 else None
+    assert G.skinny_ok(M, N, out, add)
+    G.gemm(a, w, out=out[:M], addend=add, b_static=True)
+    _lib.check_status(what="few rows")
+    want = a.double() @ w.double().t() + (add if f32 else 0)
+    # fp32 sums of products that are exact in fp32; half a unit in the last place where they are rounded
+    tol = 1e-6 * K ** 0.5 if f32 else torch.finfo(torch.float16).eps * float(want.abs().max())
+    assert float((out[:M].double() - want).abs().max()) <= tol and bool((out[M] == 3).all())
+
+
 @pytest.mark.parametrize("splits", [1, 4, 8])
 def test_decode_attention_of_a_full_ring(splits):
     """A cluster's splits over a cache whose next slot lies inside the ring."""
