@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(RT_THREADS) moe_route_tc_kernel(const __grid_c
       const int i = i0 + u * RT_THREADS, e = i / (d / 8), c = (i - e * (d / 8)) * 8;
       if (i >= cells) break;
       const float f[8] = {w[u][0].x, w[u][0].y, w[u][0].z, w[u][0].w, w[u][1].x, w[u][1].y, w[u][1].z, w[u][1].w};
-      T hi[8], lo[8];
+      alignas(16) T hi[8], lo[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         hi[k] = Cvt<T>::from_f(f[k]);
@@ -537,7 +537,7 @@ __global__ void moe_colmean_kernel(const float* __restrict__ probs, float* __res
 // Row positions (stable: token order inside every expert) and the expert-sorted copy.
 // SCAN: the scan is block 0 of this launch, beside the blocks that copy, which add up the histograms of the blocks before them for
 // themselves (L2 holds them).  As a launch of its own, of one block, it stood between the router and the copy: with it 9.7 -> 5.9 us
-// (1501 tokens), 49 -> 37 us (32768).
+// (1501 tokens).
 template <typename T, bool SCAN>
 __global__ void __launch_bounds__(256) moe_pack_kernel(const gb_moe_args a, int n_blocks) {
   pdl_wait();
@@ -1103,13 +1103,18 @@ extern "C" int gb_moe_route(const gb_moe_args* a, cudaStream_t st) {
     }
   }
   const bool vec = a->d % 256 == 0 && a->d <= 1024 && (((uintptr_t)a->x16 | (uintptr_t)a->router_w) & 15) == 0;
-#define GB_ROUTE(T)                                                           \
-  switch (vec ? a->d / 256 : 0) {                                             \
-    case 1: GB_PDL_LAUNCH_SMEM((moe_route_kernel<T, 1>), dim3(nb), dim3(256), 0, st, *a); break;            \
-    case 2: GB_PDL_LAUNCH_SMEM((moe_route_kernel<T, 2>), dim3(nb), dim3(256), 0, st, *a); break;            \
-    case 3: GB_PDL_LAUNCH_SMEM((moe_route_kernel<T, 3>), dim3(nb), dim3(256), 0, st, *a); break;            \
-    case 4: GB_PDL_LAUNCH_SMEM((moe_route_kernel<T, 4>), dim3(nb), dim3(256), 0, st, *a); break;            \
-    default: GB_PDL_LAUNCH_SMEM((moe_route_kernel<T, 0>), dim3(nb), dim3(256), 0, st, *a); break;           \
+  // Blocks of 64 tokens are about one to an SM and run long: set up while the kernel ahead drains, they share the SMs that it leaves idle, and the last of these
+  // is what the launch lasts (8192 tokens, 64 experts 163 us as an ordinary launch, 211 as a programmatic one; 5 experts, width 264 38 and 42).
+  cudaLaunchAttribute attr;
+  cudaLaunchConfig_t cfg = gb_pdl_config(dim3(nb), dim3(256), 0, st, &attr);
+  if (blk_tok(a->n_tok) > 8) cfg.numAttrs = 0;
+#define GB_ROUTE(T)                                                                     \
+  switch (vec ? a->d / 256 : 0) {                                                       \
+    case 1: (void)cudaLaunchKernelEx(&cfg, moe_route_kernel<T, 1>, *a); break;          \
+    case 2: (void)cudaLaunchKernelEx(&cfg, moe_route_kernel<T, 2>, *a); break;          \
+    case 3: (void)cudaLaunchKernelEx(&cfg, moe_route_kernel<T, 3>, *a); break;          \
+    case 4: (void)cudaLaunchKernelEx(&cfg, moe_route_kernel<T, 4>, *a); break;          \
+    default: (void)cudaLaunchKernelEx(&cfg, moe_route_kernel<T, 0>, *a); break;         \
   }
   if (!tc) {
     if (a->is_bf16) { GB_ROUTE(__nv_bfloat16) } else { GB_ROUTE(__half) }
@@ -1132,12 +1137,17 @@ extern "C" int gb_moe_group(const gb_moe_args* a, cudaStream_t st) {
   const size_t tab_bytes = (size_t)nb * (a->ne + 1) * sizeof(int);
   const int staged = tab_bytes <= 40 * 1024;
   const bool one = tab_bytes <= 27 * 1024;         // with the copy's own tables (20 KB) within 48
-  if (!one) GB_PDL_LAUNCH_SMEM(moe_scan_kernel, dim3(1), dim3(256), staged ? tab_bytes : 0, st, *a, nb, staged);
+  if (!one) moe_scan_kernel<<<1, 256, staged ? tab_bytes : 0, st>>>(*a, nb, staged);
   const int* totals = a->block_base + (size_t)nb * (a->ne + 1);
+  cudaLaunchAttribute attr;
+  cudaLaunchConfig_t cfg = gb_pdl_config(dim3(one ? nb + 1 : nb), dim3(256), one ? tab_bytes : 0, st, &attr);
+  // an ordinary launch behind the scan, which is one long block, and for blocks of many tokens (see gb_moe_route): 16384 tokens of 768, 8 experts, router and
+  // grouping 34 us, as a programmatic launch 55
+  if (!one || blk_tok(a->n_tok) > 8) cfg.numAttrs = 0;
 #define GB_PACK(T)                                                                                                            \
   do {                                                                                                                        \
-    if (one) GB_PDL_LAUNCH_SMEM((moe_pack_kernel<T, true>), dim3(nb + 1), dim3(256), tab_bytes, st, *a, nb);                   \
-    else GB_PDL_LAUNCH_SMEM((moe_pack_kernel<T, false>), dim3(nb), dim3(256), 0, st, *a, nb);                                  \
+    if (one) (void)cudaLaunchKernelEx(&cfg, moe_pack_kernel<T, true>, *a, nb);                                                 \
+    else (void)cudaLaunchKernelEx(&cfg, moe_pack_kernel<T, false>, *a, nb);                                                    \
     if (!a->forward_only) GB_PDL_LAUNCH_SMEM((moe_zero_pads_kernel<T>), dim3(ne1, PAD_PARTS), dim3(256), 0, st, (T*)a->x_perm, a->seg_offsets, totals, a->d); \
   } while (0)
   if (a->is_bf16) GB_PACK(__nv_bfloat16);
