@@ -23,14 +23,16 @@ __global__ void ll_embed_kernel(const int* __restrict__ ids, const T* __restrict
   }
 }
 
-// A block per row, d a multiple of 4: rows of more than 1024 numbers.  The norm's weights are asked for before the wait for the kernel ahead,
-// which must not write them.  A warp per row (below) keeps 1024 numbers, reads the rest twice and leaves an SM 14 warps of 2048 rows:
-// 17.2 -> 11.7 us behind the product ahead (2048 rows of 2560 numbers, 73 MB).
+// A block per row, d a multiple of 4, up to 49152: rows of more than 1024 numbers.  The norm's weights are asked for before the wait for the kernel ahead, which must
+// not write them.  A warp per row (below) keeps 1024 numbers, reads the rest twice and leaves an SM 14 warps of 2048 rows: 17.2 -> 11.7 us
+// behind the product ahead (2048 rows of 2560 numbers, 73 MB).  The squares go through shared memory and are added in the order of the warp per
+// row, so a row's result does not depend on which of the two has it.
+constexpr int PN_MOST = 49152;                          // a square sum of every four numbers in 48 KB
 template <typename T>
 __global__ void __launch_bounds__(256) ll_postnorm_row_kernel(const float* __restrict__ y, long long ldy, const float* x, const float* __restrict__ w,
                                                               float eps, float* x_out, T* __restrict__ x16, long long ld16, int rows, int d) {
   constexpr int KEEP = 3;
-  __shared__ float red[8];
+  extern __shared__ float sq[];
   const int r = blockIdx.x, tid = threadIdx.x, n4 = d >> 2;
   const float4* wr = reinterpret_cast<const float4*>(w);
   const float4* yr = reinterpret_cast<const float4*>(y + r * ldy);
@@ -40,7 +42,7 @@ __global__ void __launch_bounds__(256) ll_postnorm_row_kernel(const float* __res
   for (int k = 0; k < KEEP; ++k)
     if (tid + 256 * k < n4) g[k] = wr[tid + 256 * k];
   pdl_wait();
-  float ss = 0.f;
+  auto squares = [](const float4& u) { return u.x * u.x + u.y * u.y + u.z * u.z + u.w * u.w; };
 #pragma unroll
   for (int k = 0; k < KEEP; ++k) {
     const int i = tid + 256 * k;
@@ -48,16 +50,14 @@ __global__ void __launch_bounds__(256) ll_postnorm_row_kernel(const float* __res
     if (i < n4) xk[k] = xr[i];
   }
 #pragma unroll
-  for (int k = 0; k < KEEP; ++k) ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
-  for (int i = tid + 256 * KEEP; i < n4; i += 256) {
-    const float4 u = yr[i];
-    ss += u.x * u.x + u.y * u.y + u.z * u.z + u.w * u.w;
-  }
-  ss = warp_sum(ss);
-  if ((tid & 31) == 0) red[tid >> 5] = ss;
+  for (int k = 0; k < KEEP; ++k)
+    if (tid + 256 * k < n4) sq[tid + 256 * k] = squares(v[k]);
+  for (int i = tid + 256 * KEEP; i < n4; i += 256) sq[i] = squares(yr[i]);
   __syncthreads();
-  ss = ((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]));      // in pairs: the error of one after the other is larger
-  const float inv = ll_inv_rms(ss, d, eps);
+  float ss = 0.f;                                      // every warp adds all of them: lane l every 32nd from l on
+#pragma unroll 8
+  for (int i = tid & 31; i < n4; i += 32) ss += sq[i];
+  const float inv = ll_inv_rms(warp_sum(ss), d, eps);
   auto put = [&](int i, const float4& u, const float4& xv, const float4& gv) {
     float4 o;
     o.x = xv.x + u.x * inv * gv.x; o.y = xv.y + u.y * inv * gv.y; o.z = xv.z + u.z * inv * gv.z; o.w = xv.w + u.w * inv * gv.w;
@@ -301,9 +301,11 @@ extern "C" int gb_ll_postnorm(const float* y, long long ldy, const float* x, con
   if (!y || !x || !w || !x_out || rows <= 0 || d <= 0) return -1;
   const bool vec = d % 4 == 0 && ldy % 4 == 0 && ld16 % 4 == 0;
   const dim3 grid((rows + 7) / 8);
-  if (vec && d > 1024) {
-    if (dtype == 1) GB_PDL_LAUNCH(ll_postnorm_row_kernel<__nv_bfloat16>, dim3(rows), dim3(256), st, y, ldy, x, w, eps, x_out, (__nv_bfloat16*)x16, ld16, rows, d);
-    else if (dtype == 2) GB_PDL_LAUNCH(ll_postnorm_row_kernel<float>, dim3(rows), dim3(256), st, y, ldy, x, w, eps, x_out, (float*)x16, ld16, rows, d);
+  if (vec && d > 1024 && d <= PN_MOST && (d >= 1536 || rows <= 2048)) {        // 8192 rows of 1028: a block 20 us, a warp 17
+    if (dtype == 1)
+      GB_PDL_LAUNCH_SMEM(ll_postnorm_row_kernel<__nv_bfloat16>, dim3(rows), dim3(256), d, st, y, ldy, x, w, eps, x_out, (__nv_bfloat16*)x16, ld16, rows, d);
+    else if (dtype == 2)
+      GB_PDL_LAUNCH_SMEM(ll_postnorm_row_kernel<float>, dim3(rows), dim3(256), d, st, y, ldy, x, w, eps, x_out, (float*)x16, ld16, rows, d);
     else return -2;
     return gb_launch_rc();
   }

@@ -347,8 +347,24 @@ def test_one_token_step_loads_its_history_early(dtype, taps, P, N):
     assert float((out[True] - out[False]).abs().max()) <= 1e-6 * float(out[False].abs().max())
 
 
+@pytest.mark.parametrize("d", [1028, 1500])
+def test_postnorm_does_not_depend_on_the_number_of_rows(d):
+    """A warp per row where rows are many, a block where they are few: the same sums in the same order."""
+    from ghassan_b200.ops import layers as K
+    rows = 2049
+    g = torch.Generator(device="cuda").manual_seed(d)
+    y, x = (torch.randn(rows, d, generator=g, device="cuda") * s for s in (3.0, 1.0))
+    w = 1 + 0.1 * torch.randn(d, generator=g, device="cuda")
+    outs = []
+    for n in (rows, rows - 1, 1):
+        out, x16 = torch.empty(rows, d, device="cuda"), torch.empty(rows, d, device="cuda", dtype=BF)
+        K.postnorm(y, x, w, 1e-4, out, x16, n, d)
+        outs.append((out[:1], x16[:1], out[:rows - 1], x16[:rows - 1]))
+    assert all(torch.equal(a, b) for a, b in zip(outs[0], outs[1])) and all(torch.equal(a, b) for a, b in zip(outs[0][:2], outs[2][:2]))
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("d", [1024, 1028, 2048, 3068, 3072, 3076, 5000])
+@pytest.mark.parametrize("d", [1024, 1028, 2048, 3068, 3072, 3076, 5000, 49152, 49156])
 def test_postnorm_of_long_rows(dtype, d):
     """Rows of a block: what its registers hold, and beyond; the result may take the residual's place."""
     from ghassan_b200.ops import layers as K
