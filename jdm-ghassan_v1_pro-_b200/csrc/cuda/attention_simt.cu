@@ -299,7 +299,7 @@ int launch_fwd(const AttnArgs& a, cudaStream_t st) {
   constexpr int ROWS = 128 / TPR;
   const size_t smem = (size_t)2 * KT * HD * 4 + KT * 4;
   auto kern = attn_fwd_kernel<T, HD, TPR, KT>;
-  if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  (void)gb_allow_smem(reinterpret_cast<const void*>(kern), smem);
   dim3 grid((a.T + ROWS - 1) / ROWS, a.H, a.B);
   kern<<<grid, 128, smem, st>>>(a);
   return gb_launch_rc();
@@ -317,10 +317,8 @@ int launch_bwd(const AttnArgs& a, cudaStream_t st) {
   const size_t smem_kv = (size_t)2 * KT * HD * 4 + KT * 12;
   auto kq = attn_bwd_dq_kernel<T, HD, TPR, KT>;
   auto kkv = attn_bwd_dkv_kernel<T, HD, TPR, KT>;
-  if (smem_kv > 48 * 1024) {
-    cudaFuncSetAttribute(kq, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_q);
-    cudaFuncSetAttribute(kkv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv);
-  }
+  (void)gb_allow_smem(reinterpret_cast<const void*>(kq), smem_q);
+  (void)gb_allow_smem(reinterpret_cast<const void*>(kkv), smem_kv);
   dim3 gq((a.T + ROWS - 1) / ROWS, a.H, a.B), gkv((a.T + ROWS - 1) / ROWS, a.KV, a.B);
   kq<<<gq, 128, smem_q, st>>>(a);
   kkv<<<gkv, 128, smem_kv, st>>>(a);

@@ -1084,23 +1084,8 @@ extern "C" int gb_moe_route(const gb_moe_args* a, cudaStream_t st) {
     if (gb_make_tmap_2d_16b(&tm, a->x16, (uint64_t)a->n_tok, (uint64_t)a->d, (uint64_t)a->d, RT_TOK, RT_KC, a->is_bf16)) return -20;
     const size_t smem = rt_smem_bytes(a->d, a->ne);
     const unsigned grid = (unsigned)((a->n_tok + RT_TOK - 1) / RT_TOK);
-    if (a->is_bf16) {
-      auto kern = moe_route_tc_kernel<__nv_bfloat16>;
-      static size_t set_b = 0;                   // the attribute only ever grows
-      if (smem > set_b) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -10;
-        set_b = smem;
-      }
-      GB_PDL_LAUNCH_SMEM(kern, dim3(grid), dim3(RT_THREADS), smem, st, tm, *a, a->status);
-    } else {
-      auto kern = moe_route_tc_kernel<__half>;
-      static size_t set_h = 0;
-      if (smem > set_h) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -10;
-        set_h = smem;
-      }
-      GB_PDL_LAUNCH_SMEM(kern, dim3(grid), dim3(RT_THREADS), smem, st, tm, *a, a->status);
-    }
+    if (a->is_bf16) GB_PDL_LAUNCH_SMEM(moe_route_tc_kernel<__nv_bfloat16>, dim3(grid), dim3(RT_THREADS), smem, st, tm, *a, a->status);
+    else GB_PDL_LAUNCH_SMEM(moe_route_tc_kernel<__half>, dim3(grid), dim3(RT_THREADS), smem, st, tm, *a, a->status);
   }
   const bool vec = a->d % 256 == 0 && a->d <= 1024 && (((uintptr_t)a->x16 | (uintptr_t)a->router_w) & 15) == 0;
   // Blocks of 64 tokens are about one to an SM and run long: set up while the kernel ahead drains, they share the SMs that it leaves idle, and the last of these

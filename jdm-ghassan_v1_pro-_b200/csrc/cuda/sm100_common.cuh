@@ -38,6 +38,7 @@ static inline int gb_launch_rc() {
 // visible.  What only earlier launches write may be read before: a launch starts once every block of the one ahead is past its own
 // wait.  GB200_NO_PDL=1 turns the attribute off.
 #include <cstdlib>
+#include "smem_limit.h"
 static inline cudaLaunchConfig_t gb_pdl_config(dim3 grid, dim3 block, size_t smem, cudaStream_t st, cudaLaunchAttribute* attr) {
   static const int enabled = []() { const char* e = std::getenv("GB200_NO_PDL"); return (e && e[0] == '1') ? 0 : 1; }();
   cudaLaunchConfig_t cfg = {};
@@ -57,12 +58,12 @@ static inline cudaLaunchConfig_t gb_pdl_config(dim3 grid, dim3 block, size_t sme
     cudaLaunchConfig_t gb_cfg_ = gb_pdl_config(grid, block, 0, st, &gb_attr_);        \
     (void)cudaLaunchKernelEx(&gb_cfg_, kernel, __VA_ARGS__);                          \
   } while (0)
-// The same with dynamic shared memory, opting in to more than 48 KB of it.
+// The same with dynamic shared memory, opting in to more than 48 KB of it.  (Where that is refused, so is the launch, which says why.)
 #define GB_PDL_LAUNCH_SMEM(kernel, grid, block, smem, st, ...)                                                       \
   do {                                                                                                               \
     cudaLaunchAttribute gb_attr_;                                                                                    \
     cudaLaunchConfig_t gb_cfg_ = gb_pdl_config(grid, block, smem, st, &gb_attr_);                                    \
-    if ((smem) > 48 * 1024) (void)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem)); \
+    (void)gb_allow_smem(reinterpret_cast<const void*>(kernel), smem);                                                \
     (void)cudaLaunchKernelEx(&gb_cfg_, kernel, __VA_ARGS__);                                                         \
   } while (0)
 

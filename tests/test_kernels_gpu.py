@@ -502,3 +502,30 @@ def test_router_rows_at_any_address():
         outs.append((ws.probs.clone(), ws.w.clone()))
     assert rows[1:].data_ptr() % 16 == 4
     assert float((outs[0][0] - outs[1][0]).abs().max()) <= 1e-5
+
+
+def test_a_narrow_model_beside_a_wide_one():
+    """Two threads whose launches of one kernel need different amounts of shared memory: neither takes the other's limit back."""
+    import threading
+    from ghassan_b200.ops import kernels as K
+    failed, go = [], threading.Barrier(2)
+
+    def work(d):
+        try:
+            torch.cuda.set_device(0)
+            with torch.cuda.stream(torch.cuda.Stream()):
+                x, w = torch.zeros(256, d, device="cuda", dtype=torch.float16), torch.zeros(8, d, device="cuda")
+                ws = K.MoeWorkspace(256, d, 8, 2, False, torch.float16, "cuda")
+                go.wait()
+                for i in range(8000):
+                    K.moe_route_only(ws, x, w, None)
+                    if i % 500 == 0:
+                        torch.cuda.current_stream().synchronize()
+        except Exception as e:                              # a launch that was refused
+            failed.append((d, repr(e)))
+    threads = [threading.Thread(target=work, args=(d,)) for d in (4096, 256)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
