@@ -431,15 +431,16 @@ __global__ void __launch_bounds__(128) decode_attn_kernel(const T* __restrict__ 
 
 // The same for up to eight splits (1, 2, 4 or 8): the splits of a (sequence, kv head) are a cluster, whose CTAs exchange their results through
 // distributed shared memory and write the output, so there is no merge kernel behind it.  Keys and values are loaded two slots a lane ahead of
-// the ones being worked on, the first ones before the wait for the kernel ahead, which writes the step's own row and the queries and nothing
-// else that is read here (a full ring's next slot is not known here, so it loads behind the wait).
+// the ones being worked on, with `early` the first ones before the wait for the kernel ahead, which then writes the step's own row and the queries and
+// nothing else that is read here (a full ring's next slot is not known here, so it loads behind the wait).
 // Bound by the latency of the chain and the instructions of the scores at short caches, by memory at long ones: 32 sequences, 500 slots, 3 query
 // heads a key head, 4 splits (16 MB, 2.5 us at the copy rate): 8.3 us of the step, before 9.9 with 8 splits and 2.4 for the merge.
 template <typename T, int HD, int G>
 __global__ void __launch_bounds__(128, G <= 4 ? 4 : 2) decode_attn_cluster_kernel(const T* __restrict__ q, long long ld_q, const T* __restrict__ cK,
                                                                      const T* __restrict__ cV, const int* __restrict__ slot_pos,
                                                                      const gb_seq_state* __restrict__ st, int splits, int H, int KV, int cap, int window,
-                                                                     float scale, T* __restrict__ out, long long ld_o) {
+                                                                     float scale, int early, T* __restrict__ out, long long ld_o) {
+  if (!early) pdl_wait();                                               // the launch ahead may have written the state or the cache
   constexpr int LPS = HD / 8, SPW = 32 / LPS, TRIP = 2 * 4 * SPW;       // lanes per slot, slots side by side, slots of a trip of the CTA
   __shared__ __align__(16) float sm_q[G][HD];
   constexpr int PARTS = 4 * SPW;                                        // groups of lanes that share a slot, in the CTA
@@ -1113,7 +1114,7 @@ extern "C" int gb_decode_advance(gb_seq_state* state, int* pos_out, int B, int c
 template <typename T, int HD>
 static int launch_decode_attn(const void* q, long long ld_q, const void* cK, const void* cV, const int* slot_pos,
                               const gb_seq_state* state, void* out, long long ld_o, float* scratch, int splits, int B, int H,
-                              int KV, int cap, int window, float scale, int* ticket, cudaStream_t st) {
+                              int KV, int cap, int window, float scale, int early, int* ticket, cudaStream_t st) {
   const int G = H / KV;
   if (!ticket && splits > 2 * HD) return -4;      // the merge kernel reads at most two splits per thread
   // a cluster: no more than eight CTAs anywhere, and a slot's lanes hold its scores (heads of 32: up to four queries a key head).  Eight splits only
@@ -1129,7 +1130,7 @@ static int launch_decode_attn(const void* q, long long ld_q, const void* cK, con
 #define ATT(GG)                                                                                                                              \
   if constexpr (GG <= HD / 8)                                                                                                               \
     (void)cudaLaunchKernelEx(&cfg, decode_attn_cluster_kernel<T, HD, GG>, (const T*)q, ld_q, (const T*)cK, (const T*)cV, slot_pos, state, splits, \
-                             H, KV, cap, window, scale, (T*)out, ld_o)
+                             H, KV, cap, window, scale, early, (T*)out, ld_o)
     switch (G) {
       case 1: ATT(1); break;
       case 2: ATT(2); break;
@@ -1162,10 +1163,10 @@ static int launch_decode_attn(const void* q, long long ld_q, const void* cK, con
 
 static int decode_attn_any(const void* q16, long long ld_q, const void* cacheK, const void* cacheV, const int* slot_pos,
                            const gb_seq_state* state, void* out16, long long ld_o, float* scratch, int splits, int B, int H,
-                           int KV, int hd, int cap, int window, float scale, int is_bf16, int* ticket, cudaStream_t st) {
+                           int KV, int hd, int cap, int window, float scale, int is_bf16, int early, int* ticket, cudaStream_t st) {
   if (!q16 || !cacheK || !cacheV || !slot_pos || !state || !out16 || !scratch || splits < 1 || B <= 0 || KV <= 0 || H % KV)
     return -1;
-#define GO(T, HD) return launch_decode_attn<T, HD>(q16, ld_q, cacheK, cacheV, slot_pos, state, out16, ld_o, scratch, splits, B, H, KV, cap, window, scale, ticket, st)
+#define GO(T, HD) return launch_decode_attn<T, HD>(q16, ld_q, cacheK, cacheV, slot_pos, state, out16, ld_o, scratch, splits, B, H, KV, cap, window, scale, early, ticket, st)
   if (hd == 64) { if (is_bf16) GO(__nv_bfloat16, 64); else GO(__half, 64); }
   if (hd == 128) { if (is_bf16) GO(__nv_bfloat16, 128); else GO(__half, 128); }
   if (hd == 32) { if (is_bf16) GO(__nv_bfloat16, 32); else GO(__half, 32); }
@@ -1175,9 +1176,9 @@ static int decode_attn_any(const void* q16, long long ld_q, const void* cacheK, 
 
 extern "C" int gb_decode_attn(const void* q16, long long ld_q, const void* cacheK, const void* cacheV, const int* slot_pos,
                               const gb_seq_state* state, void* out16, long long ld_o, float* scratch, int splits, int B, int H,
-                              int KV, int hd, int cap, int window, float scale, int is_bf16, cudaStream_t st) {
+                              int KV, int hd, int cap, int window, float scale, int is_bf16, int early, cudaStream_t st) {
   return decode_attn_any(q16, ld_q, cacheK, cacheV, slot_pos, state, out16, ld_o, scratch, splits, B, H, KV, hd, cap, window,
-                         scale, is_bf16, nullptr, st);
+                         scale, is_bf16, early, nullptr, st);
 }
 
 // The same with the merge of the splits done by the last block to finish; `ticket` is B*KV ints, zero before the first call.
@@ -1187,7 +1188,7 @@ extern "C" int gb_decode_attn_fused(const void* q16, long long ld_q, const void*
                                     cudaStream_t st) {
   if (!ticket) return -1;
   return decode_attn_any(q16, ld_q, cacheK, cacheV, slot_pos, state, out16, ld_o, scratch, splits, B, H, KV, hd, cap, window,
-                         scale, is_bf16, ticket, st);
+                         scale, is_bf16, 0, ticket, st);
 }
 
 // RMSNorm of x32 [B, K] (fp32) fused into out = W @ norm(x32).  Shared memory holds the normalised rows: B*K*2 bytes.

@@ -56,9 +56,11 @@ int gb_kv_append(const void* k16, long long ld_k, const void* v16, long long ld_
                  int* slot_pos, const gb_seq_state* state, int B, int cap, int pinned, int kv_dim, cudaStream_t st);
 // out[b, h*hd:(h+1)*hd] = softmax(q_h . K^T * scale) V over the cached slots (the new token's slot included, so
 // call after gb_kv_append).  window > 0 masks slots older than `window` positions.  scratch: B*H*splits*(hd+2) floats.
+// early != 0: the launch directly ahead has written nothing of state, slot_pos and the caches but the step's own row (gb_kv_append, gb_qk_rope_append), so
+// they may be read before it has ended.  After gb_decode_advance or gb_kv_rows, for instance, early is 0.
 int gb_decode_attn(const void* q16, long long ld_q, const void* cacheK, const void* cacheV, const int* slot_pos,
                    const gb_seq_state* state, void* out16, long long ld_o, float* scratch, int splits, int B, int H,
-                   int KV, int hd, int cap, int window, float scale, int is_bf16, cudaStream_t st);
+                   int KV, int hd, int cap, int window, float scale, int is_bf16, int early, cudaStream_t st);
 // The first *n (device) of T prompt rows per sequence into slots 0 .. *n - 1 of the caches [B, cap, kv_dim], 16-bit values, and their
 // positions; pointers 16-byte aligned, kv_dim and row pitches multiples of 8, cap >= T.
 int gb_kv_rows(const void* k, long long ld_k, const void* v, long long ld_v, void* cK, void* cV, int* slot_pos, const int* n, int B, int T,
@@ -91,7 +93,7 @@ int gb_gemv_norm(const void* W, int fmt, int N, int K, const float* x32, int ldx
 int gb_route_norm(const float* x32, const float* norm_w, float eps, const float* router_w, const float* bias, int B, int d,
                   int ne, int top_k, int* idx_out, float* w_out, int is_bf16, cudaStream_t st);
 // The same for a batch whose tokens go through all experts: the normed rows x16 [B, d] and weights [B, ne (+ 1 shared)], zero where an expert
-// is not chosen.
+// is not chosen; ne == 0: the rows alone.  norm_w, router_w and bias are read before the wait for the launch ahead, which must not write them.
 int gb_norm_route_few(const float* x32, const float* norm_w, float eps, const float* router_w, const float* bias, int B, int d,
                       int ne, int top_k, int shared, void* x16, float* weights, int is_bf16, cudaStream_t st);
 // act = SwiGLU(gate, up) of the experts named by idx [B, top_k] (+ the shared one) applied to rmsnorm(x32).

@@ -19,7 +19,8 @@ extern "C" {
 // x[r, :] = table[ids[r], :] in fp32 (pitch d) and in the compute type (pitch ld16; the columns past d are zeroed).
 int gb_ll_embed(const int* ids, const void* table, long long ld_table, int vocab, float* x, void* x16, long long ld16, int rows,
                 int d, int dtype, cudaStream_t st);
-// x_out = x + (y / rms(y)) * w, x16 = compute-type copy of x_out.  x16 may be NULL; x_out may be x.
+// x_out = x + (y / rms(y)) * w, x16 = compute-type copy of x_out.  x16 may be NULL; x_out may be x.  w is a constant: it is read before the wait for
+// the launch ahead, which must not write it.
 int gb_ll_postnorm(const float* y, long long ldy, const float* x, const float* w, float eps, float* x_out, void* x16,
                    long long ld16, int rows, int d, int dtype, cudaStream_t st);
 // out[r, :] = compute-type copy of (x / rms(x)) * w for x row `row_idx[r]` (NULL: row r).
@@ -106,6 +107,8 @@ typedef struct gb_ll_attn_args {
   const gb_seq_state* st;
   int pos0_max;                          // host's upper bound of abs_pos over the B sequences (tile counts); -1 unknown
   int* status;
+  int early;                             // gb_ll_attn_decode: the launch directly ahead has written nothing of st and the caches but the rows of
+                                         // the step's own positions (gb_ll_qkv_store), so they may be read before it has ended
 } gb_ll_attn_args;
 // gb_ll_qkv_store writes caches with ld_k = G*dkp and ld_v = G*dvp.
 int gb_ll_rotations(const double* freq, int pairs, const gb_seq_state* st, int B, int n, float* cs, cudaStream_t stream);
@@ -171,6 +174,8 @@ typedef struct gb_ll_mamba_args {
   const gb_seq_state* st;
   float* chunk_ws;                       // chunked scan: gb_ll_ssd_ws_floats floats, or NULL (no cutting into segments)
   int* status;
+  int early;                             // gb_ll_mamba_step: of what it reads the launch directly ahead has written proj alone, so all the rest may be
+                                         // read before that has ended
 } gb_ll_mamba_args;
 int gb_ll_conv(const gb_ll_mamba_args* a, cudaStream_t st);
 int gb_ll_scan(const gb_ll_mamba_args* a, cudaStream_t st);         // recurrence token by token, any dtype
@@ -180,8 +185,7 @@ int gb_ll_ssd_ok(const gb_ll_mamba_args* a);                        // 0 when th
 long long gb_ll_ssd_ws_floats(int B, int H, int P, int Ns, int n, int segments);
 int gb_ll_ssd(const gb_ll_mamba_args* a, int segments, cudaStream_t st);
 int gb_ll_gated_norm(const gb_ll_mamba_args* a, cudaStream_t st);
-int gb_ll_mamba_step(const gb_ll_mamba_args* a, cudaStream_t st);   // n == 1: convolution + recurrence in one kernel; of what it reads
-                                                                    // the launch directly ahead may write proj alone
+int gb_ll_mamba_step(const gb_ll_mamba_args* a, cudaStream_t st);   // n == 1: convolution + recurrence in one kernel
 
 #ifdef __cplusplus
 }

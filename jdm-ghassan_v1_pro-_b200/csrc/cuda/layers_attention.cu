@@ -445,12 +445,13 @@ __global__ void __launch_bounds__(128, 4) ll_attn_decode_kernel(const __grid_con
 }
 
 // The same for up to eight splits (1, 2, 4 or 8): the splits of a (sequence, key head, chunk of query heads) are a cluster, whose CTAs exchange their
-// results through distributed shared memory and apply sink and gate, so there is no merge kernel behind it.  The first keys and values are asked for
-// before the wait for the kernel ahead, which writes the queries and the cache row of the step's own position, and nothing else that is read
-// here; queries wait in shared memory.  Bound by the chain and by the instructions of the scores: 32 sequences, 16 heads, 4 key heads of 64, 128 to 190
+// results through distributed shared memory and apply sink and gate, so there is no merge kernel behind it.  With `early` the first keys and values are asked
+// for before the wait for the kernel ahead, which then writes the queries and the cache row of the step's own position, and nothing else that is
+// read here; queries wait in shared memory.  Bound by the chain and by the instructions of the scores: 32 sequences, 16 heads, 4 key heads of 64, 128 to 190
 // keys, capped scores: 7.9 us of the step, before 9.5 and 3.1 for the merge.
 template <typename T, int LPS, int GQ>
 __global__ void __launch_bounds__(128, 4) ll_attn_decode_cluster_kernel(const __grid_constant__ gb_ll_attn_args a) {
+  if (!a.early) pdl_wait();                                            // the launch ahead may have written positions or the cache
   constexpr int HD = LPS * 8, SPW = 32 / LPS, U = 2;
   __shared__ __align__(16) float sm_q[GQ][HD];
   constexpr int PARTS = 4 * SPW;                                       // groups of lanes that share a slot, in the CTA

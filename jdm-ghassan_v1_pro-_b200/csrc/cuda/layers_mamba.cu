@@ -259,12 +259,13 @@ __global__ void __launch_bounds__(256) ll_scan_kernel(const __grid_constant__ gb
 // are a ring of `taps` rows, so the new row never overwrites one that another block still reads.
 //
 // Between two tokens the weights of the whole model pass through L2, so the state, the last inputs of the convolution and its weights come
-// from DRAM.  Only the input product's rows are the launch ahead's, so all the rest is loaded before the wait for it: the position, the
+// from DRAM.  Where only the input product's rows are the launch ahead's (`early`), all the rest is loaded before the wait for it: the position, the
 // state, and with up to four taps (TAPS4) the inputs and weights of the convolution; past the wait a block reads a few of the product's
 // values a thread, side by side.  In the chain of a token (32 heads of 64 x 128) 6.2 -> 2.5 us; all of it read behind the wait, with only
 // prefetches ahead of it, a request of 64 tokens and nine such layers took 21.0 ms, now 18.4.
 template <typename T, int NR, bool TAPS4>
 __global__ void __launch_bounds__(256) ll_mamba_step_kernel(const __grid_constant__ gb_ll_mamba_args a) {
+  if (!a.early) pdl_wait();                    // the launch ahead may have written the position, the state or the ring
   constexpr int NW = NR * 8, NCH = 32 + 2 * NW, PER = (NCH + 255) / 256;
   __shared__ __align__(16) float sB[NW], sC[NW];
   __shared__ float sX[32];

@@ -69,11 +69,12 @@ static inline cudaLaunchConfig_t gb_pdl_config(dim3 grid, dim3 block, size_t sme
 
 namespace gb {
 
-// Wait until the kernels before this one have finished and their writes are visible, then let the kernel after it begin its own
-// set-up.  The first statement of every kernel that GB_PDL_LAUNCH starts, but for those that first ask for constants (weights in
-// gemm_skinny_sm100.cu, layers_gemv.cu and layers_latent.cu, the state and weights in layers_mamba.cu, the offsets in piece_add_kernel, the state and
-// the cache rows of earlier steps in the token attention kernels): their launchers say which arguments the launch ahead must not write.  A kernel with tensor memory allocates
-// it first: were the next kernel let in before, its blocks could take the columns and then wait for this kernel, which waits for them.
+// Wait until the kernels before this one have finished and their writes are visible, then let the kernel after it begin its own set-up.  The first
+// statement of every kernel that GB_PDL_LAUNCH starts, but for those that first ask for constants (weights in gemm_skinny_sm100.cu, layers_gemv.cu,
+// layers_latent.cu, the norms of decode.cu and layers_common.cu, the offsets in piece_add_kernel) or, where the caller says that the launch ahead leaves them
+// alone (`early`, `b_static`), for state and cache rows of earlier steps (token attention, the Mamba step): the headers say which arguments the
+// launch ahead must not write.  A kernel with tensor memory allocates it first: were the next kernel let in before, its blocks could take the columns
+// and then wait for this kernel, which waits for them.
 __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

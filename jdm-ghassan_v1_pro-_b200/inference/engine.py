@@ -265,7 +265,7 @@ class InferenceEngine(TokenLoop):
             D.qk_rope_append(self.qkv, self.qk, L.qn, L.kn, self.cos_sin, self.pos, L.cK, L.cV, self.slot_pos, self.state,
                              Hh, KV, hd, self.cap, PINNED_TOKENS, cfg.rms_eps, cfg.rope_type)
             D.decode_attn(self.qk[:, :qd], L.cK, L.cV, self.slot_pos, self.state, self.att, self.att_scratch, self.splits,
-                          Hh, KV, hd, self.cap, cfg.sliding_window, cfg.attn_scale())
+                          Hh, KV, hd, self.cap, cfg.sliding_window, cfg.attn_scale(), early=True)
             D.gemv(L.wo, self.att, self.x_mid, addend=x_in)
             if cfg.use_moe:
                 D.route_norm(self.x_mid, L.ffn_norm, cfg.rms_eps, L.router, L.bias, cfg.moe_top_k, self.r_idx, self.r_w, bf)
@@ -282,7 +282,7 @@ class InferenceEngine(TokenLoop):
         K.qk_norm_rope_fwd(self.qkv, self.qk, L.qn, L.kn, self.cos_sin, self.pos, Hh, KV, hd, cfg.rms_eps, cfg.rope_type)
         D.kv_append(self.qk[:, qd:], self.qkv[:, qd + kvd:], L.cK, L.cV, self.slot_pos, self.state, self.cap, PINNED_TOKENS)
         D.decode_attn(self.qk[:, :qd], L.cK, L.cV, self.slot_pos, self.state, self.att, self.att_scratch, self.splits,
-                      Hh, KV, hd, self.cap, cfg.sliding_window, cfg.attn_scale())
+                      Hh, KV, hd, self.cap, cfg.sliding_window, cfg.attn_scale(), early=True)
         D.gemv(L.wo, self.att, self.x_mid, addend=x_in)
         K.rmsnorm_fwd(self.x_mid, L.ffn_norm, self.xb, self.rr, cfg.rms_eps)
         if cfg.use_moe:

@@ -394,7 +394,7 @@ class CudaModel:
             D.qk_rope_append(b.qkv, b.qk, qw, kw, dec.cos_sin, dec.pos, Lc.cK, Lc.cV, dec.slot_pos, dec.state, H, KV, hd,
                              dec.cap, dec.pinned, cfg.rms_eps, cfg.rope_type)
             D.decode_attn(b.qk[:, :qd], Lc.cK, Lc.cV, dec.slot_pos, dec.state, b.att, dec.att_scratch, dec.splits, H, KV, hd,
-                          dec.cap, cfg.sliding_window, cfg.attn_scale())
+                          dec.cap, cfg.sliding_window, cfg.attn_scale(), early=True)
         else:
             self._attention_forward(l, b, qw, kw)
         G.gemm(b.att, self.w16(p + "wo"), out=b.x_mid, addend=x_in, b_static=dec is not None)

@@ -264,6 +264,7 @@ class LayerModel:
             blocks = B * m.kv_heads * ((per_key_head + 3) // 4)
             seen = cache.cap if not m.window else m.window + m.keep_first
             a.splits = attention_splits(blocks, seen, a.dkp)
+            a.early = 1                                     # behind qkv_store, which writes this token's rows
             a.scratch = self.buf("att_scratch%d" % B, m.heads * a.splits * (a.dvp + 2), torch.float32, rows=B).data_ptr()
         a.st, a.pos0_max, a.status = st.data_ptr(), pos0_max, _lib.status_word(self.dev).data_ptr()
         return a
@@ -354,6 +355,7 @@ class LayerModel:
         out = self.mixed(i)
         a.y, a.ld_y, a.out, a.ld_out = y.data_ptr(), y.stride(0), out.data_ptr(), out.stride(0)
         a.st, a.status = st.data_ptr(), _lib.status_word(self.dev).data_ptr()
+        a.early = int(n == 1)                      # behind the input product
         return a
 
     # ------------------------------------------------------------------ many rows

@@ -139,13 +139,15 @@ def kv_append(k16, v16, cacheK, cacheV, slot_pos, state, cap, pinned):
     _lib.check_rc(rc, "gb_kv_append")
 
 
-def decode_attn(q16, cacheK, cacheV, slot_pos, state, out16, scratch, splits, H, KV, hd, cap, window, scale):
+def decode_attn(q16, cacheK, cacheV, slot_pos, state, out16, scratch, splits, H, KV, hd, cap, window, scale, early=False):
+    """``early``: the launch directly ahead has written nothing of ``state``, ``slot_pos`` and the caches but the step's own row, so reading
+    them may begin before that ends."""
     B = q16.shape[0]
     rc = _lib.lib().gb_decode_attn(c_vp(q16.data_ptr()), c_ll(q16.stride(0)), c_vp(cacheK.data_ptr()),
                                    c_vp(cacheV.data_ptr()), c_vp(slot_pos.data_ptr()), c_vp(state.data_ptr()),
                                    c_vp(out16.data_ptr()), c_ll(out16.stride(0)), c_vp(scratch.data_ptr()), c_int(splits),
                                    c_int(B), c_int(H), c_int(KV), c_int(hd), c_int(cap), c_int(window), c_float(scale),
-                                   c_int(_bf(q16)), _lib.stream_ptr())
+                                   c_int(_bf(q16)), c_int(int(early)), _lib.stream_ptr())
     _lib.check_rc(rc, "gb_decode_attn")
 
 

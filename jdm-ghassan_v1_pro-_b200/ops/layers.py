@@ -45,7 +45,7 @@ class AttnArgs(ctypes.Structure):
         ("proj", c_vp), ("ld_proj", c_ll), ("gate", c_vp), ("ld_gate", c_ll), ("sink", c_vp),
         ("softcap", c_float), ("slopes", c_vp), ("temp_coef", c_float), ("temp_every", c_int),
         ("q", c_vp), ("cache_k", c_vp), ("cache_v", c_vp), ("ld_k", c_ll), ("ld_v", c_ll), ("out", c_vp), ("ldo", c_ll),
-        ("scratch", c_vp), ("splits", c_int), ("st", c_vp), ("pos0_max", c_int), ("status", c_vp),
+        ("scratch", c_vp), ("splits", c_int), ("st", c_vp), ("pos0_max", c_int), ("status", c_vp), ("early", c_int),
     ]
 
 
@@ -73,7 +73,7 @@ class MambaArgs(ctypes.Structure):
         ("norm_w", c_vp), ("norm_groups", c_int), ("eps", c_float),
         ("conv_state", c_vp), ("ssm", c_vp), ("xh", c_vp), ("bc", c_vp), ("cc", c_vp),
         ("y", c_vp), ("ld_y", c_ll), ("out", c_vp), ("ld_out", c_ll), ("gated", c_vp), ("gated_sq", c_vp),
-        ("st", c_vp), ("chunk_ws", c_vp), ("status", c_vp),
+        ("st", c_vp), ("chunk_ws", c_vp), ("status", c_vp), ("early", c_int),
     ]
 
 

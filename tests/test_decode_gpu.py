@@ -688,6 +688,37 @@ def test_decode_attention_of_large_batches(hd, H, KV, B):
         assert float((out.float().view(B, H, hd) - want).abs().max()) < 2e-3, splits         # fp32 throughout, rounded once, values below 4
 
 
+def test_decode_attention_directly_behind_what_writes_its_inputs():
+    """The state advanced, or the cache filled, by the launch directly ahead: what the kernel reads is read behind it."""
+    D = _D()
+    B, H, KV, hd, cap, splits = 2, 12, 4, 64, 4096, 8
+    cK, cV = (_rand(B, cap, KV * hd, seed=s).cuda().half() for s in (1, 2))
+    slot_pos = torch.arange(cap, dtype=torch.int32, device="cuda").repeat(B, 1)
+    state, pos = torch.zeros(B, D.STATE_INTS, dtype=torch.int32, device="cuda"), torch.zeros(B, dtype=torch.int32, device="cuda")
+    q, scratch = _rand(B, H * hd, seed=3).cuda().half(), torch.zeros(B * H * splits * (hd + 2), device="cuda")
+    outs = [torch.zeros(B, H * hd, device="cuda", dtype=torch.float16) for _ in range(40)]
+    args = (scratch, splits, H, KV, hd, cap, 0, hd ** -0.5)
+    state[:, :2] = 100
+    for o in outs:                                          # each over one slot more than the one before
+        D.decode_advance(state, pos, cap, 8)
+        D.decode_attn(q, cK, cV, slot_pos, state, o, *args)
+    torch.cuda.synchronize()
+    for i, o in enumerate(outs):
+        state[:, :2] = 101 + i
+        alone = torch.zeros_like(o)
+        D.decode_attn(q, cK, cV, slot_pos, state, alone, *args)
+        assert torch.equal(o, alone), i
+    k, n = cK[:, :1024].reshape(-1, KV * hd).contiguous(), torch.tensor([1024], dtype=torch.int32, device="cuda")
+    state[:, :2] = 1023
+    want = torch.zeros_like(outs[0])
+    D.decode_attn(q, cK, cK, slot_pos, state, want, *args)
+    for o in outs:
+        other = torch.zeros_like(cK)
+        D.kv_rows(k, k, other, other, slot_pos, n, 1024)
+        D.decode_attn(q, other, other, slot_pos, state, o, *args)
+        assert torch.equal(o, want)
+
+
 def test_prompt_pass_replays_for_other_prompts():
     """An engine's first prompt runs as it comes (it may be the only one), the second is captured and replayed, as are all others: other
     lengths and tokens, two sequences; cache rows behind the prompt stay as they were."""

@@ -347,6 +347,49 @@ def test_one_token_step_loads_its_history_early(dtype, taps, P, N):
     assert float((out[True] - out[False]).abs().max()) <= 1e-6 * float(out[False].abs().max())
 
 
+def test_token_kernels_directly_behind_what_writes_their_positions():
+    """Positions advanced by the launch directly ahead, without the promise that they are not: read behind it."""
+    from ghassan_b200.ops import layers as K
+    raw, m, mem, state = _one_layer(C.mamba(8, 64, 128, 2, 4, 1), dtype=BF)
+    pos, src, c = torch.zeros(1, dtype=torch.int32, device="cuda"), m.buf("proj", (m.weights[0].w_in.shape[0] + 7) // 8 * 8), mem.layers[0]
+    _mamba_inputs(m, 24, 3)
+    whole, got = src[:24].clone(), {}
+    for together in (False, True):
+        state.zero_()
+        c.ssm.fill_(float("nan"))
+        ys = []
+        for t in range(24):
+            src[:1] = whole[t:t + 1]
+            a = m.mamba_args(0, c, state, 0, 1, 1)
+            a.early = 0
+            if t:
+                K.advance(state, pos, 1)
+                if not together:
+                    torch.cuda.synchronize()
+            K.mamba_step(a)
+            ys.append(m.buf("ssm_y", 8 * 64)[:1].clone())
+        got[together] = torch.cat(ys)
+    assert bool(torch.isfinite(got[True].float()).all()) and torch.equal(got[False], got[True])
+    H, G, dk, cap, splits = 8, 2, 64, 300, 8
+    q, k, v = (torch.randn(1, n, device="cuda").to(BF) for n in (H * dk, cap * G * dk, cap * G * dk))
+    out, scratch = torch.zeros(1, H * dk, device="cuda", dtype=BF), torch.zeros(1, H * splits * (dk + 2), device="cuda")
+    a = K.AttnArgs()
+    a.dtype, a.B, a.n, a.H, a.G, a.dk, a.dv, a.dkp, a.dvp = K.DTYPE[BF], 1, 1, H, G, dk, dk, dk, dk
+    a.eps, a.scale, a.cap, a.q, a.cache_k, a.cache_v, a.ld_k, a.ld_v = 1e-5, dk ** -0.5, cap, q.data_ptr(), k.data_ptr(), v.data_ptr(), G * dk, G * dk
+    a.out, a.ldo, a.scratch, a.splits, a.st = out.data_ptr(), H * dk, scratch.data_ptr(), splits, state.data_ptr()
+    for together in (False, True):
+        state.zero_()
+        outs = []
+        for t in range(200):
+            K.advance(state, pos, 1)
+            if not together:
+                torch.cuda.synchronize()
+            K.attn_decode(a)
+            outs.append(out.clone())
+        got[together] = torch.cat(outs)
+    assert torch.equal(got[False], got[True])
+
+
 @pytest.mark.parametrize("d", [1028, 1500])
 def test_postnorm_does_not_depend_on_the_number_of_rows(d):
     """A warp per row where rows are many, a block where they are few: the same sums in the same order."""
