@@ -230,8 +230,11 @@ class CudaModel:
         self.Gr = CA.zeros(L.total, **f32) if train else None        # fp32 gradients
         self.moe_bias = None
         self.bias_counts = None
+        # All rows through all experts multiplies an unchosen expert's down rows by zero, which only leaves no trace where they are finite: a 16-bit
+        # copy that is not (an overflow of a wider file's numbers) keeps the rows sorted, so that it reaches the tokens that chose it and no others.
+        self.down_finite = True
         if share_weights is not None:
-            self.moe_bias = share_weights.moe_bias
+            self.moe_bias, self.down_finite = share_weights.moe_bias, share_weights.down_finite
         elif cfg.use_moe and cfg.moe_aux_free:
             self.moe_bias = CA.zeros(cfg.num_layers, cfg.num_experts, **f32)
         if cfg.use_moe and train:
@@ -349,6 +352,8 @@ class CudaModel:
     def load_named(self, named, missing_ok=False):
         absent = self.layout.to_internal(named, self.P, missing_ok)
         self.refresh_shadows()
+        if self.Gr is None and self.cfg.use_moe:
+            self.down_finite = bool(torch.stack([torch.isfinite(self.w16(f"L{i}.w_down")).all() for i in range(self.cfg.num_layers)]).all())
         return absent
 
     def export_named(self, flat=None) -> Dict[str, np.ndarray]:
@@ -398,7 +403,7 @@ class CudaModel:
         else:
             self._attention_forward(l, b, qw, kw)
         G.gemm(b.att, self.w16(p + "wo"), out=b.x_mid, addend=x_in, b_static=dec is not None)
-        if self.experts_few and not train and self.ep is None:
+        if self.experts_few and self.down_finite and not train and self.ep is None:
             from ..ops import decode as D
             D.norm_route_few(b.x_mid, self.w(p + "ffn_norm"), cfg.rms_eps, self.w(p + "router"), self.moe_bias[l] if self.moe_bias is not None else None,
                              cfg.moe_top_k, cfg.moe_shared, b.xb2, b.few_w)

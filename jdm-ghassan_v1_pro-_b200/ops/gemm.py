@@ -160,7 +160,8 @@ def gemm_two(a, w, n1, out1, out2):
 def experts_few(a, w_gu, w_down, weights, act, out, addend):
     """All rows of ``a`` through all experts, for batches so small that their tokens visit nearly every expert: ``out = addend +
     sum_e weights[:, e] * expert_e(a)``.  ``w_gu`` ``[ne * 2E, d]`` interleaved, ``w_down`` ``[ne * d, E]``, ``weights`` fp32 ``[M, ne]``,
-    ``act`` 16-bit ``[M, ne * E]`` scratch, ``out`` and ``addend`` fp32 ``[M, d]``.  Weights may be read ahead of the launch before."""
+    ``act`` 16-bit ``[M, ne * E]`` scratch, ``out`` and ``addend`` fp32 ``[M, d]``.  Weights may be read ahead of the launch before.  Where a weight
+    is zero the expert's gate and up rows may hold anything; ``w_down`` is finite everywhere."""
     (M, d), ne, E = a.shape, weights.shape[1], w_down.shape[1]
     if M > 128 or act.shape != (M, ne * E) or w_gu.shape != (ne * 2 * E, d) or w_down.shape != (ne * d, E) or E % 64:
         raise ValueError("experts_few: shapes")

@@ -606,6 +606,32 @@ def test_tensor_core_token_step_matches_gemv_chain(moe, fmt, B):
     assert out.shape == (B, 13) and int(gemm.state[0, 0]) == 9 + 12
 
 
+def test_an_expert_with_infinities_reaches_only_its_tokens():
+    """Down rows that overflow in 16 bits, of an expert that the selection bias keeps out: the batch's logits are those of finite rows, in the
+    token step and in a short prompt."""
+    from ghassan_b200.inference.engine import InferenceEngine
+    from ghassan_b200.models.config import init_parameters
+    cfg = _tiny_cfg(num_heads=4, num_kv_heads=2, hidden_size=256, use_moe=True, moe_aux_free=True, moe_aux_scale=0.0)
+    bias = [np.where(np.arange(cfg.num_experts) == 1, -100.0, 0.0).astype(np.float32) for _ in range(cfg.num_layers)]
+    got, prompt = [], torch.randint(16, 512, (8, 70), generator=torch.Generator().manual_seed(9), dtype=torch.int32)
+    for fill in (0.0, 1e30):
+        named = init_parameters(cfg, 31)
+        for i in range(cfg.num_layers):
+            key = "layers.%d.moe_down" % i
+            down = np.array(named[key], dtype=np.float32)
+            down.reshape(cfg.num_experts, -1)[1] = fill
+            named[key] = down
+        e = InferenceEngine(cfg, named, fmt="f16", batch=8, max_len=80, prefill_chunk=72, moe_bias=bias, gemm_min_batch=2)
+        e.reset(1)
+        e.prefill(prompt)
+        e.cur_tok.copy_(prompt[:, 0])
+        e._forward_token()
+        assert e._step_net().down_finite == (fill == 0.0)
+        got.append(e.logits.clone())
+    assert bool(torch.isfinite(got[1]).all())
+    assert float((got[0] - got[1]).abs().max()) <= 1e-2 * max(1.0, float(got[0].abs().max()))       # sorted rows round the experts' outputs
+
+
 @pytest.mark.parametrize("V,top_k", [(300, 300), (1000, 40), (5000, 512), (5000, 513), (32001, 40), (32001, 1024)])
 def test_device_sampler_candidate_edges(V, top_k):
     """Fewer logits than threads, both ways to the k-th largest value, ties across it (values on a grid of 1/16)."""

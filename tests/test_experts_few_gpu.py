@@ -49,7 +49,7 @@ def test_experts_few(case, dtype):
 
 
 def test_unchosen_expert_does_not_matter():
-    """An expert that no token has chosen may hold infinities."""
+    """The gate and up rows of an expert that no token has chosen may hold infinities."""
     from ghassan_b200.ops import gemm as G
     B, d, ne, E = 16, 256, 4, 64
     g = torch.Generator(device="cuda").manual_seed(5)
