@@ -492,22 +492,23 @@ def test_single_kernel_step_matches_kernel_chain(case):
 
 # Query heads per key head (one to four are passes of their own, eight go four at a time), head sizes, and how many slots the cache holds: up to 64 a
 # CTA is one trip, more is several; 1537 and up make a CTA walk more than 64; a full ring wraps.
-@pytest.mark.parametrize("n", [1, 64, 65, 700, 1537, 2500])
+@pytest.mark.parametrize("n,window", [(1, 0), (64, 0), (65, 0), (700, 0), (1537, 0), (2500, 0), (65, 16), (700, 100), (1537, 1000), (2500, 100), (2500, 2000), (6000, 2300)])
 @pytest.mark.parametrize("hidden,H,KV", [(256, 4, 4), (512, 8, 4), (768, 12, 4), (512, 8, 2), (512, 8, 1), (256, 2, 1), (256, 8, 4)])
-def test_single_kernel_step_over_long_caches(hidden, H, KV, n):
-    """One step of the cooperative kernel against the kernel chain, from the same cache of ``n`` - 1 drawn keys and values."""
-    from ghassan_b200.inference.engine import InferenceEngine
+def test_single_kernel_step_over_long_caches(hidden, H, KV, n, window):
+    """One step of the cooperative kernel against the kernel chain, from the same cache of ``n`` - 1 drawn keys and values: where it is full, the first tokens
+    and a ring that has gone round; windows that hide slots in the middle of a CTA's and whole CTAs."""
+    from ghassan_b200.inference.engine import PINNED_TOKENS, InferenceEngine
     from ghassan_b200.models.config import init_parameters
     from ghassan_b200.ops import _lib
     cap = 2400
-    cfg = _tiny_cfg(hidden_size=hidden, num_heads=H, num_kv_heads=KV, moe_expert_dim=256, max_seq_len=4096)
+    cfg = _tiny_cfg(hidden_size=hidden, num_heads=H, num_kv_heads=KV, moe_expert_dim=256, max_seq_len=8192, sliding_window=window)
     named = init_parameters(cfg, 7)
     one = InferenceEngine(cfg, named, fmt="f16", batch=1, max_len=cap, prefill_chunk=32, single_kernel=True)
     chain = InferenceEngine(cfg, named, fmt="f16", batch=1, max_len=cap, prefill_chunk=32, single_kernel=False)
     assert one.mega is not None and chain.mega is None
     g = torch.Generator(device="cuda").manual_seed(n)
-    seen, held = n - 1, min(n - 1, cap)
-    ring = max(0, seen - cap) % (cap - 8)
+    seen, held, turn = n - 1, min(n - 1, cap), cap - PINNED_TOKENS
+    ring = max(0, seen - cap) % turn
     for e in (one, chain):
         e.reset(1)
     for La, Lb in zip(one.layers, chain.layers):
@@ -515,9 +516,12 @@ def test_single_kernel_step_over_long_caches(hidden, H, KV, n):
         La.cV.copy_(torch.randn(La.cV.shape, device="cuda", generator=g))
         Lb.cK.copy_(La.cK)
         Lb.cV.copy_(La.cV)
-    one.slot_pos.copy_(torch.randint(0, max(1, seen), one.slot_pos.shape, device="cuda", generator=g, dtype=torch.int32))
+    at = torch.arange(cap)                                  # the last position that went into a slot
+    last = torch.where(at < PINNED_TOKENS, at, at + torch.div(seen - 1 - at, turn, rounding_mode="floor").clamp(min=0) * turn)
+    assert held < cap or sorted(last.tolist()) == list(range(PINNED_TOKENS)) + list(range(seen - turn, seen))
+    one.slot_pos.copy_(last.int()[None])
     chain.slot_pos.copy_(one.slot_pos)
-    one.state.copy_(torch.tensor([[held, seen, ring, 0][:one.state.shape[1]]], dtype=torch.int32))
+    one.state.copy_(torch.tensor([[seen, held, ring, 0]], dtype=torch.int32))
     chain.state.copy_(one.state)
     for e in (one, chain):
         e.pos.fill_(seen)
@@ -663,7 +667,7 @@ def test_device_sampler_candidate_edges(V, top_k):
             assert 0 <= out.tolist()[3] < V
 
 
-@pytest.mark.parametrize("hd,H,KV", [(64, 3, 1), (64, 8, 1), (32, 6, 1), (128, 2, 2), (128, 4, 2)])
+@pytest.mark.parametrize("hd,H,KV", [(64, 3, 1), (64, 8, 1), (64, 6, 1), (32, 6, 1), (128, 2, 2), (128, 4, 2), (128, 4, 1), (128, 12, 2), (128, 8, 1)])
 @pytest.mark.parametrize("n,splits,window", [(1, 1, 0), (15, 1, 0), (16, 1, 0), (17, 1, 7), (64, 2, 0), (129, 1, 0), (200, 8, 33)])
 @pytest.mark.parametrize("off", [0, 1])
 def test_decode_attention_at_slot_edges(hd, H, KV, n, splits, window, off):

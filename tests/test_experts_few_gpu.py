@@ -109,18 +109,24 @@ def test_products_of_few_rows_share_by_share(M, N, K, f32):
     assert float((out[:M].double() - want).abs().max()) <= tol and bool((out[M] == 3).all())
 
 
+@pytest.mark.parametrize("window", [0, 40, 260])
 @pytest.mark.parametrize("splits", [1, 4, 8])
-def test_decode_attention_of_a_full_ring(splits):
-    """A cluster's splits over a cache whose next slot lies inside the ring."""
+def test_decode_attention_of_a_full_ring(splits, window):
+    """A cluster's splits over a cache whose next slot lies inside the ring; windows that begin before it and behind it."""
     from ghassan_b200.ops import decode as D
-    B, H, KV, hd, cap = 2, 6, 2, 64, 300
+    B, H, KV, hd, cap, pinned, seen = 2, 6, 2, 64, 300, 8, 1001                            # position 1000 has been appended and is not counted yet
     g = torch.Generator(device="cuda").manual_seed(splits)
     cK, cV = (torch.randn(B, cap, KV * hd, device="cuda", generator=g).half() for _ in range(2))
     q, out = torch.randn(B, H * hd, device="cuda", generator=g).half(), torch.zeros(B, H * hd, device="cuda", dtype=torch.float16)
+    at, turn = torch.arange(cap, device="cuda"), cap - pinned
+    slot_pos = torch.where(at < pinned, at, at + torch.div(seen - 1 - at, turn, rounding_mode="floor") * turn).int()
     state = torch.zeros(B, D.STATE_INTS, dtype=torch.int32, device="cuda")
-    state[:, 0], state[:, 1], state[:, 2] = 1000, cap, 17
-    D.decode_attn(q, cK, cV, torch.zeros(B, cap, dtype=torch.int32, device="cuda"), state, out, torch.zeros(B * H * splits * (hd + 2), device="cuda"), splits,
-                  H, KV, hd, cap, 0, hd ** -0.5)
+    state[:, 0], state[:, 1], state[:, 2] = seen - 1, cap, (seen - 1 - cap) % turn
+    assert int(slot_pos[pinned + int(state[0, 2])]) == seen - 1
+    D.decode_attn(q, cK, cV, slot_pos.repeat(B, 1), state, out, torch.zeros(B * H * splits * (hd + 2), device="cuda"), splits, H, KV, hd, cap, window, hd ** -0.5)
     k, v = (c.float().view(B, cap, KV, hd).repeat_interleave(H // KV, 2) for c in (cK, cV))
-    want = torch.einsum("bhl,blhd->bhd", torch.softmax(torch.einsum("bhd,blhd->bhl", q.float().view(B, H, hd), k) * hd ** -0.5, -1), v)
+    s = torch.einsum("bhd,blhd->bhl", q.float().view(B, H, hd), k) * hd ** -0.5
+    if window:
+        s = s.masked_fill(seen - 1 - slot_pos >= window, float("-inf"))
+    want = torch.einsum("bhl,blhd->bhd", torch.softmax(s, -1), v)
     assert float((out.float().view(B, H, hd) - want).abs().max()) < 2e-3          # fp32 throughout, rounded once, values below 4
