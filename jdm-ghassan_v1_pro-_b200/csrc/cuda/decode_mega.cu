@@ -27,7 +27,7 @@
 // What bounds it: the chain of dependent steps, six exchanges a layer of 1.2 to 1.5 us with what they wait for, and the instructions between them.  A step,
 // us (five grid-wide barriers a layer, 360 bytes of spilled registers -> this form): 36 layers of 768, 12/4 heads, 5 of 9 experts of 1280, fp16,
 // 1024 slots 1694 -> 930 (weights at the copy rate: 196); 26 layers, 3 of 9 experts of 768, 4 bits, 3001 slots 1061 -> 619 (36).  On the way: words and
-// counts in place of barriers 1694 -> 1490, nothing spilled -> 1077, fewer instructions -> 966 (eager times, 36 layers).
+// counts in place of barriers 1694 -> 1490, hardly anything spilled -> 1077, fewer instructions -> 966 (eager times, 36 layers).
 //
 // Every wait is bounded: a word that does not arrive within about two seconds writes status 401, a copy that
 // never signals its mbarrier 402; the CTA then skips the rest of the step (the others follow when their own waits run
@@ -46,7 +46,7 @@ namespace mg {
 
 constexpr int WARPS = 16;
 constexpr int THREADS = WARPS * 32;
-constexpr int GROUP = 4;              // super-units a warp keeps in flight
+constexpr int ROUTER_AREA = 32 * 1024;   // shared memory for a layer's router rows
 constexpr int SU = 256;               // values per super-unit
 constexpr int MAX_SLOTS = 9;          // top_k <= 8 routed experts plus the shared one
 constexpr int MAX_HEADS = 128;
@@ -56,14 +56,8 @@ constexpr int ST_TIMEOUT_COPY = 402;      // a bulk copy of weight rows never si
 template <int FMT> struct Fmt {
   static constexpr bool k16 = FMT == GB_W_F16 || FMT == GB_W_BF16;
   static constexpr int bytes = k16 ? 512 : FMT == GB_W_GGML_Q8_0 ? 272 : FMT == GB_W_Q4_0 ? 144 : FMT == GB_W_Q8_64 ? 272 : 160;
-  static constexpr int words = bytes / 16;    // 16-byte words per super-unit (<= 32: one per lane)
 };
 
-__device__ __forceinline__ uint4 ld_stream(const uint8_t* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-  return v;
-}
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
@@ -108,8 +102,7 @@ __device__ __forceinline__ bool grid_sync(GridBar& gb) {
 }
 
 // ------------------------------------------------------------------------------------------------ exchange words
-// Relaxed loads at GPU scope on purpose: an acquire empties this SM's L1, and with it the registers the kernel has spilled to
-// local memory.  A word carries its own epoch, so nothing has to be ordered behind it.
+// Relaxed loads at GPU scope: a word carries its own epoch, so nothing has to be ordered behind it, and an acquire would empty this SM's L1 every time.
 __device__ __forceinline__ void put_f32(unsigned long long* p, float v, uint32_t epoch) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"((unsigned long long)epoch << 32 | __float_as_uint(v)) : "memory");
 }
@@ -227,17 +220,14 @@ __host__ __device__ inline Words words_of(const gb_mega_args& a) {
 }
 
 // ------------------------------------------------------------------------------------------------ row engine
-// One projection phase: every output is a sum over P super-units.  Super-unit p of an output lives at
-//   W + row_off(output) + off[p / nsu] + (p % nsu) * bytes,
-// is multiplied with the 256 activations at xs + (x_mod ? p % nsu : p) * 256, weighted by wt[p / nsu], and added to
-// accumulator (acc_split ? p / nsu : 0).  That covers a plain row (off, wt absent), a gate/up pair (two rows, two
-// accumulators) and the down projection of several experts into one output (one stored row per slot, weighted).
+// One projection phase: every output is a sum over super-units.  They lie in stretches of nsu, super-unit su of stretch s of an output at
+//   W + row_off(output) + off[s] + su * bytes
+// (off absent: 0).  A plain row is one stretch, a gate/up pair two (two rows), the down projection of several experts one per slot.
 struct Phase {
   const uint8_t* W;
   const long long* off;
-  const float* wt;
-  int nsu, P;
-  bool x_mod, acc_split;
+  const float* wt;            // weights of the stretches, where stream_run is WEIGHTED
+  int nsu;
 };
 
 // Which outputs of the CTA a warp computes: local output i = first + k * stride for k < n, super-units [pb, pe).
@@ -267,19 +257,6 @@ __device__ __forceinline__ Plan make_plan(int N, int P, int nsu) {
     pl.n = warp < pl.rows ? (pl.rows - warp + WARPS - 1) / WARPS : 0;
   }
   return pl;
-}
-
-template <int FMT>
-__device__ __forceinline__ void load_group(const Phase& ph, const uint8_t* row, int p0, int pe, uint4 (&r)[GROUP]) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int i = 0; i < GROUP; ++i) {
-    const int p = p0 + i;
-    if (p < pe && lane < Fmt<FMT>::words) {
-      const int s = p / ph.nsu, su = p - s * ph.nsu;
-      r[i] = ld_stream(row + (ph.off ? ph.off[s] : 0ll) + (long long)su * Fmt<FMT>::bytes + 16 * lane);
-    }
-  }
 }
 
 // A byte of four small unsigned numbers as a float, plus 2^23: one permutation where a conversion takes two instructions, one of them slow.
@@ -334,78 +311,6 @@ __device__ __forceinline__ void x_of(const XT* x, float (&f)[8]) {
 template <int FMT> __device__ __forceinline__ uint4 su_word(const uint8_t* slot) {
   if constexpr (Fmt<FMT>::k16) return *reinterpret_cast<const uint4*>(slot + 16 * (threadIdx.x & 31));
   else return make_uint4(0u, 0u, 0u, 0u);
-}
-
-template <int FMT, typename XT>
-__device__ __forceinline__ void dot_group(const Phase& ph, const XT* xs, int p0, int pe, const uint4 (&r)[GROUP], uint8_t* stage,
-                                          float (&acc)[2]) {
-  const int lane = threadIdx.x & 31;
-  if constexpr (!Fmt<FMT>::k16) {
-#pragma unroll
-    for (int i = 0; i < GROUP; ++i)
-      if (p0 + i < pe && lane < Fmt<FMT>::words) *reinterpret_cast<uint4*>(stage + i * Fmt<FMT>::bytes + 16 * lane) = r[i];
-    __syncwarp();
-  }
-#pragma unroll
-  for (int i = 0; i < GROUP; ++i) {
-    const int p = p0 + i;
-    if (p < pe) {
-      const int s = p / ph.nsu, su = p - s * ph.nsu;
-      float x[8];
-      x_of<XT>(xs + (ph.x_mod ? su : p) * SU, x);
-      const float v = su_dot<FMT>(r[i], stage + i * Fmt<FMT>::bytes, x);
-      if (ph.acc_split && s == 1) acc[1] += v;
-      else acc[0] += (ph.wt ? ph.wt[s] : 1.f) * v;
-    }
-  }
-  if constexpr (!Fmt<FMT>::k16) __syncwarp();
-}
-
-// The first group of the warp's first output, issued before the barrier that precedes the phase.
-template <int FMT, class RowOff>
-__device__ __forceinline__ void preload(const Phase& ph, const Plan& pl, RowOff row_off, uint4 (&cur)[GROUP]) {
-  if (pl.n > 0) load_group<FMT>(ph, ph.W + row_off(blockIdx.x + pl.first * (int)gridDim.x), pl.pb, pl.pe, cur);
-}
-
-// Runs the warp's outputs.  row_off(o): byte offset of output o's stored row; epi(o, a0, a1): called by one thread
-// per finished output.  `cur` holds the preloaded first group.
-template <int FMT, typename XT, class RowOff, class Epi>
-__device__ __forceinline__ void run_phase(const Phase& ph, const Plan& pl, const XT* xs, uint8_t* stage, float (*red)[WARPS],
-                                          uint4 (&cur)[GROUP], RowOff row_off, Epi epi) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int grid = gridDim.x, cta = blockIdx.x;
-  const int gpi = (pl.pe - pl.pb + GROUP - 1) / GROUP;
-  const int total = pl.n * gpi;
-  float acc[2] = {0.f, 0.f};
-  int k = 0, g = 0;
-  for (int t = 0; t < total; ++t) {
-    uint4 nxt[GROUP];
-    int k2 = k, g2 = g + 1;
-    if (g2 == gpi) { g2 = 0; ++k2; }
-    if (t + 1 < total)
-      load_group<FMT>(ph, ph.W + row_off(cta + (pl.first + k2 * pl.stride) * grid), pl.pb + GROUP * g2, pl.pe, nxt);
-    dot_group<FMT, XT>(ph, xs, pl.pb + GROUP * g, pl.pe, cur, stage, acc);
-    if (g == gpi - 1) {
-      const float a0 = warp_sum(acc[0]);
-      const float a1 = ph.acc_split ? warp_sum(acc[1]) : 0.f;
-      if (lane == 0) {
-        if (pl.KS == 1) epi(cta + (pl.first + k * pl.stride) * grid, a0, a1);
-        else { red[0][warp] = a0; red[1][warp] = a1; }
-      }
-      acc[0] = acc[1] = 0.f;
-    }
-#pragma unroll
-    for (int i = 0; i < GROUP; ++i) cur[i] = nxt[i];
-    k = k2; g = g2;
-  }
-  if (pl.KS > 1) {                        // uniform over the CTA: rows and P are
-    __syncthreads();
-    if ((int)threadIdx.x < pl.rows) {
-      float a0 = 0.f, a1 = 0.f;
-      for (int j = 0; j < pl.KS; ++j) { a0 += red[0][threadIdx.x * pl.KS + j]; a1 += red[1][threadIdx.x * pl.KS + j]; }
-      epi(cta + (int)threadIdx.x * grid, a0, a1);
-    }
-  }
 }
 
 // ------------------------------------------------------------------------------------------------ row streaming
@@ -979,7 +884,8 @@ __device__ __forceinline__ void route_phase(const gb_mega_args& a, const gb_mega
 // Vocabulary projection.  A warp has far more rows here than its staging slice holds, so the slice is a ring of
 // `items` row slots (as many whole rows as fit, at most MAXI): row k lands in slot k % items, and the slot is refilled
 // with row k + items as soon as the warp has read it.  head_issue before the last exchange starts the first rows.
-// (Pulling the rows through registers one group ahead ran this phase at a fifth of the memory bandwidth.)
+// (Pulling the rows through registers one group ahead ran this phase at a fifth of the memory bandwidth.)  One row fits wherever the layers' rows do:
+// 16 slices of a row of 4096 16-bit values beside the largest activations that MAXI rows a warp allow; gb_decode_mega_ok checks it.
 template <int FMT>
 __device__ __forceinline__ int head_items(const gb_mega_args& a) {
   const long long rb = (long long)(a.d / SU) * Fmt<FMT>::bytes;
@@ -1006,20 +912,12 @@ __device__ __forceinline__ void head_issue(const gb_mega_args& a, const Plan& pl
 }
 
 template <int FMT, typename XT>
-__device__ __forceinline__ void head_phase(const gb_mega_args& a, const XT* xs, uint8_t* stage, Smem& sm, Stage& st) {
+__device__ __forceinline__ void head_phase(const gb_mega_args& a, const XT* xs, Stage& st) {
   constexpr int SB = Fmt<FMT>::bytes;
   const int nsu = a.d / SU;
   const long long rb = (long long)nsu * SB;
-  Phase ph{reinterpret_cast<const uint8_t*>(a.head), nullptr, nullptr, nsu, nsu, false, false};
-  const Plan pl = make_plan(a.V, ph.P, ph.P);
+  const Plan pl = make_plan(a.V, nsu, nsu);
   const int items = head_items<FMT>(a);
-  if (items < 1) {                               // a row does not fit the slice: through registers
-    auto row = [&](int o) { return (long long)o * rb; };
-    uint4 cur[GROUP];
-    preload<FMT>(ph, pl, row, cur);
-    run_phase<FMT, XT>(ph, pl, xs, stage, sm.red, cur, row, [&](int o, float v, float) { a.logits[o] = v; });
-    return;
-  }
   const int lane = threadIdx.x & 31;
   constexpr int NX = 4;                          // activations of that many super-units stay in registers: a warp has a dozen rows
   float x[NX][8];
@@ -1062,12 +960,11 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
   extern __shared__ __align__(16) uint8_t dyn[];
   __shared__ Smem sm;
   __shared__ __align__(8) uint64_t bars[WARPS * MAXI];         // of the warps' staging slices
-  // the router rows of a layer (ne x d fp32, the same for every token) are staged a phase and a half ahead too, into the
-  // area that only the vocabulary projection of block formats uses
+  // the router rows of a layer (ne x d fp32, the same for every token) are staged a phase and a half ahead too, into an area of their own
   __shared__ __align__(8) uint64_t rbar;
   const int warp_id = threadIdx.x >> 5;
   XT* xs = reinterpret_cast<XT*>(dyn);
-  uint8_t* stage_all = dyn + a.at_stage;
+  uint8_t* router_area = dyn + a.at_stage;
   float* amerge = reinterpret_cast<float*>(dyn + a.at_merge);
   Stage st{dyn + a.at_rows + (size_t)warp_id * a.stage_bytes, bars + warp_id * MAXI, 0u, 0u, &sm.dead, a.status};
   const Gate gate{a.words, sm.base, sm.warps, &sm.dead, a.status};
@@ -1121,7 +1018,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
       reinterpret_cast<unsigned long long*>(&sm.layer[0])[threadIdx.x] = reinterpret_cast<const unsigned long long*>(a.layers)[threadIdx.x];
     __syncthreads();
     // rows of the first projection of the first layer: nothing to wait for
-    Phase ph{reinterpret_cast<const uint8_t*>(sm.layer[0].wqkv), nullptr, nullptr, d / SU, d / SU, false, false};
+    Phase ph{reinterpret_cast<const uint8_t*>(sm.layer[0].wqkv), nullptr, nullptr, d / SU};
     stream_issue<FMT, 1>(ph, sm.plan[0][warp_id], 1, st, [&](int, int o) { return o * row_bytes(a.d); });
     int tok = a.cur_tok[0];
     if (tok < 0 || tok >= a.V) tok = 0;
@@ -1145,9 +1042,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
         asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(reinterpret_cast<unsigned long long*>(&sm.layer[(li + 1) & 1]) + threadIdx.x)),
                      "l"(reinterpret_cast<const unsigned long long*>(a.layers + li + 1) + threadIdx.x)
                      : "memory");
-      Phase ph{reinterpret_cast<const uint8_t*>(L.wqkv), nullptr, nullptr, a.d / SU, a.d / SU, false, false};
+      Phase ph{reinterpret_cast<const uint8_t*>(L.wqkv), nullptr, nullptr, a.d / SU};
       stream_run<FMT, XT, false, false>(ph, sm.plan[0][warp_id], xs, st, sm.red, gate, V_QKV, [&](int, int o, float v, float) { put_16<XT>(sm.wqkv + o, Cvt<XT>::from_f(v), epoch); });
-      Phase phC{reinterpret_cast<const uint8_t*>(L.wo), nullptr, nullptr, a.H * a.hd / SU, a.H * a.hd / SU, false, false};
+      Phase phC{reinterpret_cast<const uint8_t*>(L.wo), nullptr, nullptr, a.H * a.hd / SU};
       stream_issue<FMT, 1>(phC, sm.plan[1][warp_id], 1, st, [&](int, int o) { return o * row_bytes(a.H * a.hd); });
       const int S = sm.splits;
       if ((int)blockIdx.x < a.KV * S) {
@@ -1164,11 +1061,11 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
           }
       }
       const uint32_t router_bytes = a.ne > 0 ? (uint32_t)a.ne * (uint32_t)a.d * 4u : 0u;
-      if (router_bytes > 0 && router_bytes <= (uint32_t)(WARPS * GROUP * 512)) {
+      if (router_bytes > 0 && router_bytes <= (uint32_t)ROUTER_AREA) {
         if (threadIdx.x == THREADS - 32) {       // every thread's reads of the previous layer's rows lie barriers back
           fence_proxy_async();
           mbar_arrive_expect_tx(&rbar, router_bytes);
-          bulk_g2s(smem_u32(stage_all), L.router, router_bytes, smem_u32(&rbar));
+          bulk_g2s(smem_u32(router_area), L.router, router_bytes, smem_u32(&rbar));
         }
         rpending = true;
       }
@@ -1192,7 +1089,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
     if (sm.dead) { ok = false; break; }
     mark();
     {
-      Phase phC{reinterpret_cast<const uint8_t*>(L.wo), nullptr, nullptr, a.H * a.hd / SU, a.H * a.hd / SU, false, false};
+      Phase phC{reinterpret_cast<const uint8_t*>(L.wo), nullptr, nullptr, a.H * a.hd / SU};
       stream_run<FMT, XT, false, false>(phC, sm.plan[1][warp_id], xs, st, sm.red, gate, V_MID, [&](int i, int o, float v, float) {
         v += sm.res[0][i];
         sm.res[1][i] = v;
@@ -1211,11 +1108,11 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
         }
         rparity ^= 1u;
       }
-      if (rpending) route_phase<XT, true>(a, L, xs, sm, row_bytes(a.E), reinterpret_cast<const float*>(stage_all));
+      if (rpending) route_phase<XT, true>(a, L, xs, sm, row_bytes(a.E), reinterpret_cast<const float*>(router_area));
       else route_phase<XT, false>(a, L, xs, sm, row_bytes(a.E), L.router);
       rpending = false;
       mark();
-      Phase ph{reinterpret_cast<const uint8_t*>(L.wg), sm.off_gu, nullptr, a.d / SU, 2 * (a.d / SU), true, true};
+      Phase ph{reinterpret_cast<const uint8_t*>(L.wg), sm.off_gu, nullptr, a.d / SU};
       stream_issue<FMT, 2>(ph, sm.plan[2][warp_id], 2, st, [&](int k, int) {
         const int i = sm.plan[2][warp_id].first + k * sm.plan[2][warp_id].stride;
         return ((long long)sm.esel[sm.d_slot[i]] * a.E + sm.d_row[i]) * row_bytes(a.d);
@@ -1225,7 +1122,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
     }
     {
       const int slots = n_slots_of(), nsu_E = a.E / SU;
-      Phase phE{reinterpret_cast<const uint8_t*>(L.wd), sm.off_e, sm.wsel, nsu_E, slots * nsu_E, false, false};
+      Phase phE{reinterpret_cast<const uint8_t*>(L.wd), sm.off_e, sm.wsel, nsu_E};
       stream_issue<FMT, 0>(phE, sm.plan[3][warp_id], slots, st, [&](int, int o) { return o * row_bytes(a.E); });
       mark();
       asm volatile("cp.async.wait_all;" ::: "memory");         // the next layer's pointers, before the barriers of gather16
@@ -1240,7 +1137,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
       });
     }
     if (!last) {
-      Phase ph{reinterpret_cast<const uint8_t*>(sm.layer[(li + 1) & 1].wqkv), nullptr, nullptr, a.d / SU, a.d / SU, false, false};
+      Phase ph{reinterpret_cast<const uint8_t*>(sm.layer[(li + 1) & 1].wqkv), nullptr, nullptr, a.d / SU};
       stream_issue<FMT, 1>(ph, sm.plan[0][warp_id], 1, st, [&](int, int o) { return o * row_bytes(a.d); });
     }
     mark();
@@ -1255,10 +1152,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
     }
     block_norm<XT>(gate, V_X, a.n_layers * gridDim.x, sm.wx, nullptr, epoch, a.final_norm, xs, a.d, a.eps, sm.nred);
     if (!sm.dead) {
-      uint8_t* stage = stage_all + (size_t)warp_id * GROUP * 512;
-      if (a.head_fmt == FMT) head_phase<FMT, XT>(a, xs, stage, sm, st);
-      else if (a.head_fmt == GB_W_F16) head_phase<GB_W_F16, XT>(a, xs, stage, sm, st);
-      else head_phase<GB_W_BF16, XT>(a, xs, stage, sm, st);
+      if (a.head_fmt == FMT) head_phase<FMT, XT>(a, xs, st);
+      else if (a.head_fmt == GB_W_F16) head_phase<GB_W_F16, XT>(a, xs, st);
+      else head_phase<GB_W_BF16, XT>(a, xs, st);
     }
   }
   // a step that was given up: the copies this warp still has in flight must land (or run out of time) before the
@@ -1290,12 +1186,12 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
   }
 }
 
-// Dynamic shared memory: activations, staging of the vocabulary projection (and router rows), merge of the warps' attention, staged rows.
+// Dynamic shared memory: activations, router rows, merge of the warps' attention, staged rows.
 static size_t dyn_bytes(gb_mega_args& a, long long stage_per_warp) {
   const int slots = a.ne > 0 ? a.top_k + (a.shared ? 1 : 0) : 1;
   const int xs_vals = std::max(std::max(a.d, a.H * a.hd), slots * a.E);
   a.at_stage = (int)(((size_t)xs_vals * 2 + 15) & ~(size_t)15);
-  a.at_merge = a.at_stage + WARPS * GROUP * 512;
+  a.at_merge = a.at_stage + ROUTER_AREA;
   a.at_rows = a.at_merge + (WARPS * 8 + WARPS * 4 * a.hd) * 4;
   return (size_t)a.at_rows + (size_t)WARPS * (size_t)stage_per_warp;
 }
@@ -1350,7 +1246,7 @@ extern "C" int gb_decode_mega_ok(const gb_mega_args* a) {
   if (grid <= 0 || grid < a->KV || a->d < grid) return -9;           // a.d < grid: a CTA without rows would not be waited for
   gb_mega_args b = *a;
   const long long per_warp = mg::stage_bytes_per_warp(b, grid, mg::su_bytes_of(a->fmt));
-  if (per_warp < 0 || mg::dyn_bytes(b, per_warp) > mg::MAX_DYN) return -7;
+  if (per_warp < 0 || per_warp < (long long)(a->d / mg::SU) * mg::su_bytes_of(a->head_fmt) || mg::dyn_bytes(b, per_warp) > mg::MAX_DYN) return -7;
   return 0;
 }
 
