@@ -283,7 +283,8 @@ int launch_skinny_q(const CUtensorMap& ta, const CUtensorMap& tw, gb::sk::Params
   }
   // CTAs of a tile: as many as leave all tiles resident at once (32 x 4352 x 1024, four CTAs a tile, had a few late clusters, 10.2 us; with two it has none, 6.0).
   // The driver is asked how many clusters fit with an SM for every CTA; up to 32 rows two CTAs share one, which its query does not see: counted as one they had
-  // half as many CTAs, 8 x 2560 x 6912 15.0 us and 11.4, 8 x 6912 x 2560 12.0 and 10.3.  Fewer than two k-blocks per CTA do not pay for the exchange.
+  // half as many CTAs, 8 x 2560 x 6912 15.0 us and 11.4, 8 x 6912 x 2560 12.0 and 10.3.  More CTAs than SMs pay for themselves from ten k-blocks a CTA
+  // on (8 x 9472 x 768, six: 5.1 us with 148 CTAs, 6.2 with 296).  Fewer than two k-blocks per CTA do not pay for the exchange.
   constexpr int COLS = SWIGLU ? sk::BN / 2 : sk::BN, MOST = SWIGLU ? 4 : 8;
   const int tiles = (p.N + COLS - 1) / COLS, blocks = (p.K + sk::BK - 1) / sk::BK;
   static std::atomic<int> fits[4];                    // clusters of 2, 4, 8 CTAs that fit an SM each, plus one
@@ -301,7 +302,7 @@ int launch_skinny_q(const CUtensorMap& ta, const CUtensorMap& tw, gb::sk::Params
       if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = 0; }
       fits[lg].store(++n, std::memory_order_relaxed);
     }
-    const int an_sm = skinny_smem(q) <= TWO_SMEM ? 2 : 1;
+    const int an_sm = skinny_smem(q) <= TWO_SMEM && ((tiles << lg) <= 148 || blocks >> lg >= 10) ? 2 : 1;
     if (tiles > (n - 1) * an_sm) break;
     p.split = q.split;
     p.lg = lg;
