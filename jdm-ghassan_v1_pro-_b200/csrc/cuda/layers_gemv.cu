@@ -274,9 +274,12 @@ __device__ __forceinline__ void ll_accum(const LlRaw<FMT>& raw, int u, const XT*
 // one row, 0.75 us each, with a DRAM round trip from the second on.  Width 1024, each kernel's time behind the one ahead: 4384 rows
 // 5.6 -> 3.5 us, 5632 with SwiGLU 5.7 -> 3.5, 1024 of 2816 numbers 3.6 -> 2.9, of 2048 with the gated norm 5.6 -> 4.0, the vocabulary
 // 18.5 -> 14.0; a request of 64 tokens 25.8 -> 21.0 ms.
+// Rows of five to eight units a lane behind SwiGLU or the gated norm (R == 1): all of them are asked for ahead, two blocks an SM.  With four of them
+// ahead and the rest in the loop below, 13824 rows of 2560 with SwiGLU took 17.8 us before the rows were side by side, 21.2 since, and take 14.2;
+// 8192 of 4096 20.5, 22.6 and 13.5; 2560 of 5120 with the gated norm 11.3, 11.9 and 10.5.
 // Several sequences (R == 0), and rows of more units: NB sequences a pass over a row, PF units ahead, the rest in a loop.
 template <int FMT, typename XT, int PRO, int SWI, int NB, int KS, int R, int UPL, int KEEP>
-__global__ void __launch_bounds__(LV_THREADS) ll_gemv_kernel(const __grid_constant__ LlGemv a) {
+__global__ void __launch_bounds__(LV_THREADS, UPL > 4 ? 2 : 0) ll_gemv_kernel(const __grid_constant__ LlGemv a) {
   constexpr int ROWS = R ? R : 1, PF = R ? UPL : (SWI ? 4 : 8) / (FMT == GB_W_F32 ? 2 : 1);      // rows, and units per lane of each, that are loaded ahead
   static_assert(R == 0 || NB == 1, "rows side by side are for one sequence");
   extern __shared__ __align__(16) uint8_t lv_dyn[];
@@ -459,7 +462,8 @@ static int ll_gemv_go(LlGemv a, cudaStream_t st) {
   } while (0)
   if constexpr (FMT == GB_W_BF16) if (a.B == 1) {
     // rows of up to 2 or 4 units a lane: rows x units x matrices are 8 units, 32 registers.  Longer rows are few blocks' work and
-    // mostly loads: side by side they would leave one block an SM.  The prologues that keep the row take four numbers a thread up to 1024.
+    // mostly loads: side by side they would leave one block an SM; one at a time up to 8 units a lane pay with two matrices or the gated norm
+    // (with one matrix eight units are ahead in the loop's form, too).  The prologues that keep the row take four numbers a thread up to 1024.
     const int upl = (units + 32 * ks - 1) / (32 * ks);
     const bool small = a.d <= 4 * LV_THREADS || (PRO != 1 && PRO != 5);
 #define ROWS_OF(KS)                                                                                                                \
@@ -468,6 +472,10 @@ static int ll_gemv_go(LlGemv a, cudaStream_t st) {
       if (upl <= 4 && small) { GO(1, KS, (SWI ? 1 : 2), 4, 4); return gb_launch_rc(); }                                             \
       if constexpr (PRO == 1 || PRO == 5)                                                                                          \
         if (upl <= 4) { GO(1, KS, (SWI ? 1 : 2), 4, 16); return gb_launch_rc(); }                                                  \
+      if constexpr (SWI || PRO == 3) {                                                                                             \
+        if (upl <= 6) { GO(1, KS, 1, 6, 16); return gb_launch_rc(); }                                                              \
+        if (upl <= 8) { GO(1, KS, 1, 8, 16); return gb_launch_rc(); }                                                              \
+      }                                                                                                                            \
     } while (0)
     if (ks == 4) ROWS_OF(4); else if (ks == 2) ROWS_OF(2); else ROWS_OF(1);
 #undef ROWS_OF

@@ -534,6 +534,46 @@ def test_gemv_prologues(dtype, B, d, N):
         near(run(N, out, prologue=2, y16=x16, ldy16=Kp, z16=z, ldz=d, w1=w1, parts=parts), v @ W[:N].t())
 
 
+@pytest.mark.parametrize("d, N", [(2048, 9601), (2056, 2499), (3072, 2499), (3080, 4739), (4096, 2371), (4104, 130), (6144, 77), (6152, 2499), (8192, 130), (8200, 130)])
+def test_gemv_long_rows_asked_for_ahead(d, N):
+    """One sequence, four to nine units a lane: SwiGLU without a norm and with the residual, and the gated norm; the same sums as for several."""
+    from ghassan_b200.ops import layers as K
+    g = torch.Generator(device="cuda").manual_seed(d + N)
+    E = (N + 63) // 64 * 64
+    w = (torch.randn(2 * E, d, generator=g, device="cuda") * d ** -0.5).to(BF)
+    x, y = (torch.randn(2, d, generator=g, device="cuda").to(BF) for _ in range(2))
+    x32, w1, sq = x.float(), 1 + 0.1 * torch.randn(d, generator=g, device="cuda"), torch.rand(2, 16, generator=g, device="cuda") * d / 8
+    W, xd = w.double(), x.double()
+    for pro, swi in ((0, 1), (1, 1), (3, 0)):
+        n = E if swi else N
+        outs = []
+        for B in (1, 2):
+            a = K.GemvArgs()
+            a.W, a.fmt, a.N, a.K, a.B, a.dtype, a.d, a.eps, a.prologue, a.swiglu = w.data_ptr(), K.W_FMT[BF], 2 * E if swi else N, d, B, K.DTYPE[BF], d, 1e-4, pro, swi
+            out = torch.full((2, E + 8), 7.0, dtype=F32, device="cuda")
+            a.out, a.ldo, a.out_f32 = out.data_ptr(), E + 8, 1
+            if pro == 0:
+                a.x16, a.ldx = x.data_ptr(), d
+            elif pro == 1:
+                a.x = x32.data_ptr()
+            else:
+                a.v32, a.sq, a.n_sq, a.parts, a.w1 = x32.data_ptr(), sq.data_ptr(), 16, 1, w1.data_ptr()
+            K.gemv(a)
+            outs.append(out)
+        v = xd
+        if pro == 3:
+            v = (xd / torch.sqrt(sq.double().sum(1, keepdim=True) / d + 1e-4) * w1.double())
+        j = torch.arange(n, device="cuda")
+        ref = v @ (W[(j // 64) * 128 + j % 64] if swi else W[:N]).t()
+        if swi:
+            ref = ref * torch.sigmoid(ref) * (v @ W[(j // 64) * 128 + j % 64 + 64].t())
+        # the gated norm rounds the vector to 16 bits; sums are of 32 bits
+        tol = 2.0 ** -6 if pro == 3 else 1e-5
+        assert float((outs[1][:, :n].double() - ref).abs().max()) < tol * float(ref.abs().max())
+        assert torch.equal(outs[0][0, :n], outs[1][0, :n])
+        assert float((outs[0][:1, n:] - 7).abs().max()) == 0 and float((outs[0][1] - 7).abs().max()) == 0
+
+
 @pytest.mark.parametrize("d, N", [(40, 9), (512, 4387), (520, 40011), (1024, 9501), (1032, 2501), (2048, 19001), (4096, 9473), (4104, 2399)])
 def test_gemv_rows_side_by_side(d, N):
     """One sequence: rows that a warp takes together, at the ends of a row's units and of the rows of a block's trips."""
