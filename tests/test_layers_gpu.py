@@ -574,6 +574,26 @@ def test_gemv_long_rows_asked_for_ahead(d, N):
         assert float((outs[0][:1, n:] - 7).abs().max()) == 0 and float((outs[0][1] - 7).abs().max()) == 0
 
 
+@pytest.mark.parametrize("B, d", [(2, 4096), (1, 4088), (1, 4912), (3, 3504), (2, 3072)])
+def test_gemv_at_the_line_of_shared_memory(B, d):
+    """Vectors and norms of just below and above 48 KB together, next to what the kernel has of its own."""
+    from ghassan_b200.ops import layers as K
+    g = torch.Generator(device="cuda").manual_seed(B + d)
+    N = 24
+    w = (torch.randn(N, d, generator=g, device="cuda") * d ** -0.5).to(BF)
+    x, y = (torch.randn(B, d, generator=g, device="cuda") for _ in range(2))
+    w1, w2 = (1 + 0.1 * torch.randn(d, generator=g, device="cuda") for _ in range(2))
+    a = K.GemvArgs()
+    a.W, a.fmt, a.N, a.K, a.B, a.dtype, a.d, a.eps, a.prologue = w.data_ptr(), K.W_FMT[BF], N, d, B, K.DTYPE[BF], d, 1e-4, 1
+    a.x, a.y, a.ldy, a.w1 = x.data_ptr(), y.data_ptr(), d, w1.data_ptr()
+    out = torch.empty(B, N, device="cuda")
+    a.out, a.ldo, a.out_f32 = out.data_ptr(), N, 1
+    K.gemv(a)
+    rms = lambda v: v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-4)
+    ref = (x.double() + rms(y.double()) * w1.double()) @ w.double().t()
+    assert float((out.double() - ref).abs().max()) < 2.0 ** -6 * float(ref.abs().max())      # the vector is rounded to 16 bits
+
+
 @pytest.mark.parametrize("d, N", [(40, 9), (512, 4387), (520, 40011), (1024, 9501), (1032, 2501), (2048, 19001), (4096, 9473), (4104, 2399)])
 def test_gemv_rows_side_by_side(d, N):
     """One sequence: rows that a warp takes together, at the ends of a row's units and of the rows of a block's trips."""

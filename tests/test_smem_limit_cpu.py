@@ -26,9 +26,10 @@ extern "C" cudaError_t CUDARTAPI cudaFuncSetAttribute(const void* f, cudaFuncAtt
 }
 int main() {
   const char k = 0, other = 0;
-  assert(gb_allow_smem(&k, 48 * 1024) == 0 && sets == 0);                       // nothing to ask for
+  assert(gb_allow_smem(&k, 16 * 1024) == 0 && sets == 0);                       // nothing to ask for
+  assert((gb_allow_smem(&k, 48 * 1024) == 0 && now[{&k, 0}] == 48 * 1024));     // with static memory this is above the limit of a fresh kernel
   assert(gb_allow_smem(&k, 100000) == 0 && gb_allow_smem(&k, 200000) == 0 && gb_allow_smem(&k, 60000) == 0);
-  assert((now[{&k, 0}] == 200000 && sets == 2));                                // raised twice, never lowered
+  assert((now[{&k, 0}] == 200000 && sets == 3));                                // raised twice more, never lowered
   assert((gb_allow_smem(&other, 60000) == 0 && now[{&other, 0}] == 60000));
   device = 1;                                                                   // a limit of its own
   assert((gb_allow_smem(&k, 60000) == 0 && now[{&k, 1}] == 60000 && now[{&k, 0}] == 200000));
