@@ -301,7 +301,7 @@ extern "C" int gb_ll_postnorm(const float* y, long long ldy, const float* x, con
   if (!y || !x || !w || !x_out || rows <= 0 || d <= 0) return -1;
   const bool vec = d % 4 == 0 && ldy % 4 == 0 && ld16 % 4 == 0;
   const dim3 grid((rows + 7) / 8);
-  if (vec && d > 1024 && d <= PN_MOST && (d >= 1536 || rows <= 2048)) {        // 8192 rows of 1028: a block 20 us, a warp 17
+  if (vec && d > 1024 && d <= PN_MOST && (d >= 1536 || rows <= 1024)) {        // 8192 rows of 1028: a block 20 us, a warp 17; 2048: 7.3 and 5.9
     if (dtype == 1)
       GB_PDL_LAUNCH_SMEM(ll_postnorm_row_kernel<__nv_bfloat16>, dim3(rows), dim3(256), d, st, y, ldy, x, w, eps, x_out, (__nv_bfloat16*)x16, ld16, rows, d);
     else if (dtype == 2)

@@ -394,7 +394,7 @@ def test_token_kernels_directly_behind_what_writes_their_positions():
 def test_postnorm_does_not_depend_on_the_number_of_rows(d):
     """A warp per row where rows are many, a block where they are few: the same sums in the same order."""
     from ghassan_b200.ops import layers as K
-    rows = 2049
+    rows = 1025
     g = torch.Generator(device="cuda").manual_seed(d)
     y, x = (torch.randn(rows, d, generator=g, device="cuda") * s for s in (3.0, 1.0))
     w = 1 + 0.1 * torch.randn(d, generator=g, device="cuda")
