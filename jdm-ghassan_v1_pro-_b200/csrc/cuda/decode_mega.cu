@@ -219,7 +219,7 @@ __host__ __device__ inline Words words_of(const gb_mega_args& a) {
   return w;
 }
 
-// ------------------------------------------------------------------------------------------------ row engine
+// ------------------------------------------------------------------------------------------------ rows of a phase
 // One projection phase: every output is a sum over super-units.  They lie in stretches of nsu, super-unit su of stretch s of an output at
 //   W + row_off(output) + off[s] + su * bytes
 // (off absent: 0).  A plain row is one stretch, a gate/up pair two (two rows), the down projection of several experts one per slot.
